@@ -11,18 +11,22 @@
 //
 //   gla_decay   c = 1 - sigmoid(z)^(1 / tau) = -expm1(-softplus(-z) / tau) in place over rows of logits z (softplus in its
 //               stable form max(x, 0) + log1p(exp(-|x|)); no fast-math)
-//   gla_scan    a warp owns GL_CW = 4 columns of one head's state for one request and walks the request's new tokens in
-//               order.  Its lanes are 8 groups of rows x 4 columns: lane (lr, lc) keeps, of column lc, the rows
-//               32 j + 4 lr + {0, 1, 2, 3} (j = 0, 1, ...; d <= 256) in registers, so a token's read-out crosses 8
-//               lanes in three exchanges; four rows of q, k and a are one 16-byte load each where the operands allow
-//               it.  The next token's operands are fetched while this one is worked on.  The order of every sum is
-//               fixed by d alone, so a cut of a prompt changes nothing at all, and the same kernel serves prompt
-//               portions and single tokens.  (A chunked form -- per chunk of 16 tokens the products with e^(L_i - L_j),
-//               L the running sum of log a, every exponent <= 0, the chunks' own term for all chunks at once and a walk
-//               over the chunks with 16 columns of the state per block -- was built and gave the same numbers, but took
-//               1,931 us where this walk takes 745 us on 2,048 tokens of 16 heads of 128 x 128, and 6,105 against 4,569 us
-//               on eight such requests: the walk over 128 chunks with one block of four warps per SM is the longer chain.)
+//   gla_walk    for portions.  A block of eight warps owns 16 columns of one head's state for one request and walks the
+//               request's new tokens in order, the state in registers (walk.cuh says which lane holds what).  What bounds
+//               a walk is not the recurrence -- two dependent multiply-adds a token -- but its operands: with each warp
+//               fetching a token ahead by itself a token took 700 ns behind a product that had left the operands in
+//               DRAM and the far L2 (2,048 tokens of 16 heads of 128 x 128: 1,433 us inside the mixer).  So 16 tokens
+//               of q, k and the decays are copied into shared memory together, asynchronously, two tiles ahead, by all
+//               warps for all, and the read-outs of eight tokens cross the lanes together: 259 us alone (745 before, the operands
+//               in L2) and about as long inside the mixer, whose pass went from 1,613 to 428 us.
+//   gla_tokens  for steps of few tokens a request (decoding): 16 columns of a head and 8 groups of rows to a block, so that
+//               a row of the state is read and written in whole sectors (64 requests: 46 -> 24 us).
+//
+// The order of every sum is fixed by d and by the kernel.  (A chunked form -- per chunk of 16 tokens the products with
+// e^(L_i - L_j), L the running sum of log a, every exponent <= 0 -- needs an exponential per pair of tokens and channel and
+// was slower than a walk.)
 #include "common.cuh"
+#include "walk.cuh"
 
 struct GlaArgs {
     const float* q;
@@ -40,91 +44,227 @@ struct GlaArgs {
     float q_scale;
 };
 
-#define GL_CW 4   // columns of a warp
+#define GL_STAGES 3
+#define GL_TT 16   // tokens of a tile
 
-// R: rows of a column that a lane keeps (d <= 8 R).  VEC: the rows of q, k and a of a head start on 16-byte boundaries
-// and d is a multiple of 4, so four rows are one load.
-template <int R, bool VEC>
-__global__ void __launch_bounds__(128) gla_scan_kernel(const GlaArgs a, int col_groups) {
+// RPL: rows of a column that a lane keeps, of two columns (d <= 32 RPL).  VEC: the rows of q, k and a of a head start on
+// 16-byte boundaries and d is a multiple of 4, so four rows are one copy.
+template <int RPL, bool VEC>
+__global__ void __launch_bounds__(32 * WALK_WARPS, 2) gla_walk_kernel(const GlaArgs a, int col_blocks) {
+    constexpr int DP = 32 * RPL, CB = WALK_CW * WALK_WARPS, TT = GL_TT, TILE = TT * (3 * DP + 2 * CB), NT = 32 * WALK_WARPS;
+    constexpr int RV = RPL < 4 ? RPL : 4;                // rows of a load
+    extern __shared__ __align__(16) float walk_smem[];   // [GL_STAGES][q, k, a: [TT][DP]; v: [TT][CB], every value twice]
+    __shared__ float read[2][TT][CB];                    // a tile's read-outs, by the tile's parity
     pdl_entry();
     pdl_trigger();
-    constexpr int CW = GL_CW, NG = 32 / CW;
-    const int lane = threadIdx.x & 31, lr = lane / CW, lc = lane % CW;
-    const int unit = blockIdx.x * 4 + (threadIdx.x >> 5);  // (head, column group)
-    const int seg = blockIdx.y;
-    if (unit >= a.H * col_groups) return;
-    const int qn = a.seg_qn[seg];
-    const int h = unit / col_groups, col = (unit % col_groups) * CW + lc;
-    const int d = a.d, dv = a.dv, q0 = a.seg_q0[seg];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int seg = blockIdx.y, h = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * CB;
+    const int qn = a.seg_qn[seg], q0 = a.seg_q0[seg];
+    if (qn <= 0) return;
+    const int d = a.d, dv = a.dv, wc = wid * WALK_CW;
+    float* S = a.state + static_cast<size_t>(a.state_slots[seg]) * a.slot_stride + static_cast<size_t>(h) * d * dv;
+
+    // rows d .. DP of the tiles are never copied: they stay zero, and so do the state's rows there
+    if (d < DP)
+        for (int i = tid; i < GL_STAGES * TT * 3 * (DP - d); i += NT) {
+            const int row = i / (DP - d), r = d + i % (DP - d);
+            walk_smem[(row / (3 * TT)) * TILE + (row % (3 * TT)) * DP + r] = 0.f;
+        }
+    const float* src[3] = {a.q + a.off_q + h * d, a.k + a.off_k + h * d, a.a + a.off_a + h * d};
+    const int ld[3] = {a.ldq, a.ldk, a.lda};
+    const float* vsrc = a.v + a.off_v + h * dv + col0;
+    auto fetch = [&](int tile) {   // a tile's operands into its buffer; tokens behind the last one are zeros
+        float* buf = walk_smem + (tile % GL_STAGES) * TILE;
+#pragma unroll
+        for (int w = 0; w < 3; ++w)
+#pragma unroll
+            for (int i = 0; i < TT / WALK_WARPS; ++i) {
+                const int t = wid + i * WALK_WARPS, tok = tile * TT + t;
+                const bool live = tok < qn;
+                const float* row = src[w] + static_cast<size_t>(q0 + (live ? tok : 0)) * ld[w];
+                float* dst = buf + (w * TT + t) * DP;
+                if (VEC) {
+                    for (int r = 4 * lane; r < d; r += 128) walk_copy<16>(dst + r, row + r, live);
+                } else {
+                    for (int r = lane; r < d; r += 32) walk_copy<4>(dst + r, row + r, live);
+                }
+            }
+        for (int i = tid; i < 2 * TT * CB; i += NT) {
+            const int t = i / (2 * CB), c = (i % (2 * CB)) >> 1, tok = tile * TT + t;
+            const bool live = tok < qn && col0 + c < dv;
+            walk_copy<4>(buf + 3 * TT * DP + i, vsrc + (live ? static_cast<size_t>(q0 + tok) * a.ldv + c : 0), live);
+        }
+    };
+    auto read_out = [&](int tile) {   // the read-outs of a tile that all warps have left
+        for (int i = tid; i < TT * CB; i += NT) {
+            const int t = i / CB, c = i % CB, tok = tile * TT + t;
+            if (tok < qn && col0 + c < dv)
+                a.out[static_cast<size_t>(q0 + tok) * a.ldo + h * dv + col0 + c] = read[tile & 1][t][c] * a.q_scale;
+        }
+    };
+    const int n_tiles = (qn + TT - 1) / TT;
+#pragma unroll
+    for (int i = 0; i < GL_STAGES - 1; ++i) {
+        if (i < n_tiles) fetch(i);
+        walk_commit();
+    }
+    auto row_of = [&](int i) { return 128 * (i / RV) + RV * lane + (i % RV); };
+    f2 s[WALK_CW][RPL / 2];
+#pragma unroll
+    for (int c = 0; c < WALK_CW; ++c)
+#pragma unroll
+        for (int i = 0; i < RPL / 2; ++i) {
+            const int r = row_of(2 * i), col = col0 + wc + c;
+            s[c][i] = f2_pack((r < d && col < dv) ? S[static_cast<size_t>(r) * dv + col] : 0.f,
+                              (r + 1 < d && col < dv) ? S[static_cast<size_t>(r + 1) * dv + col] : 0.f);
+        }
+    const int mine = walk_sum_index<16>(lane);   // the value (token, column) of eight tokens that this lane ends up with
+    for (int tile = 0; tile < n_tiles; ++tile) {
+        walk_wait<GL_STAGES - 2>();
+        __syncthreads();   // the tile is there for all warps, and nobody reads the buffer that is filled next
+        if (tile + GL_STAGES - 1 < n_tiles) fetch(tile + GL_STAGES - 1);
+        walk_commit();
+        if (tile > 0) read_out(tile - 1);
+        const float* buf = walk_smem + (tile % GL_STAGES) * TILE;
+        struct Ops {
+            f2 q[RPL / 2], k[RPL / 2], a[RPL / 2], v[WALK_CW];
+        };
+        auto load = [&](Ops& x, int t) {
+            const float* qp = buf + t * DP + RV * lane;
+#pragma unroll
+            for (int b = 0; b < RPL / RV; ++b) {
+                if constexpr (RV == 4) {
+                    const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qp + 128 * b);
+                    const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(qp + TT * DP + 128 * b);
+                    const ulonglong2 a4 = *reinterpret_cast<const ulonglong2*>(qp + 2 * TT * DP + 128 * b);
+                    x.q[2 * b] = q4.x; x.q[2 * b + 1] = q4.y; x.k[2 * b] = k4.x; x.k[2 * b + 1] = k4.y; x.a[2 * b] = a4.x; x.a[2 * b + 1] = a4.y;
+                } else {
+                    x.q[b] = *reinterpret_cast<const f2*>(qp);
+                    x.k[b] = *reinterpret_cast<const f2*>(qp + TT * DP);
+                    x.a[b] = *reinterpret_cast<const f2*>(qp + 2 * TT * DP);
+                }
+            }
+            const ulonglong2 v4 = *reinterpret_cast<const ulonglong2*>(buf + 3 * TT * DP + 2 * (t * CB + wc));
+            x.v[0] = v4.x; x.v[1] = v4.y;
+        };
+        auto token = [&](const Ops& x, float* o) {
+            f2 na[RPL / 2];   // minus the rates
+#pragma unroll
+            for (int i = 0; i < RPL / 2; ++i) na[i] = x.a[i] ^ 0x8000000080000000ull;
+#pragma unroll
+            for (int c = 0; c < WALK_CW; ++c) {
+                f2 acc = 0;   // (+0, +0)
+#pragma unroll
+                for (int i = 0; i < RPL / 2; ++i) {
+                    s[c][i] = f2_fma(x.k[i], x.v[c], f2_fma(na[i], s[c][i], s[c][i]));
+                    acc = f2_fma(s[c][i], x.q[i], acc);
+                }
+                float e, f;
+                f2_unpack(acc, e, f);
+                o[c] = e + f;
+            }
+        };
+        auto leave = [&](const float* o, int t0) {
+            const float sum = walk_sum<16>(o, lane);
+            if (lane < 16) read[tile & 1][t0 + (mine >> 1)][wc + (mine & 1)] = sum;
+        };
+        if (qn - tile * TT >= TT) {
+            float o[2 * TT];
+            Ops x[2];
+            load(x[0], 0);
+#pragma unroll
+            for (int t = 0; t < TT; ++t) {
+                if (t + 1 < TT) load(x[(t + 1) & 1], t + 1);   // the next token's operands are on their way
+                token(x[t & 1], o + 2 * t);
+            }
+            leave(o, 0);
+            leave(o + TT, 8);
+        } else {   // (a token that is not there leaves the state alone, whatever it holds)
+#pragma unroll 1
+            for (int t0 = 0; t0 < TT; t0 += 8) {
+                float o[16];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    o[2 * u] = o[2 * u + 1] = 0.f;
+                    if (tile * TT + t0 + u < qn) {
+                        Ops x;
+                        load(x, t0 + u);
+                        token(x, o + 2 * u);
+                    }
+                }
+                leave(o, t0);
+            }
+        }
+    }
+    __syncthreads();
+    read_out(n_tiles - 1);
+#pragma unroll
+    for (int c = 0; c < WALK_CW; ++c)
+#pragma unroll
+        for (int i = 0; i < RPL / 2; ++i) {
+            const int r = row_of(2 * i), col = col0 + wc + c;
+            float e, f;
+            f2_unpack(s[c][i], e, f);
+            if (r < d && col < dv) S[static_cast<size_t>(r) * dv + col] = e;
+            if (r + 1 < d && col < dv) S[static_cast<size_t>(r + 1) * dv + col] = f;
+        }
+}
+
+// Few tokens a request.  128 threads: 16 columns x 8 groups of R consecutive rows (d <= 8 R).
+template <int R>
+__global__ void __launch_bounds__(128) gla_tokens_kernel(const GlaArgs a, int col_blocks) {
+    constexpr int DP = 8 * R;
+    __shared__ __align__(16) float ops[3][DP];
+    __shared__ float part[4][16];
+    pdl_entry();
+    pdl_trigger();
+    const int tid = threadIdx.x, rg = tid >> 4, c = tid & 15, wid = tid >> 5;
+    const int seg = blockIdx.y, h = blockIdx.x / col_blocks, col = (blockIdx.x % col_blocks) * 16 + c;
+    const int qn = a.seg_qn[seg], q0 = a.seg_q0[seg];
+    if (qn <= 0) return;
+    const int d = a.d, dv = a.dv;
     const bool col_ok = col < dv;
     float* S = a.state + static_cast<size_t>(a.state_slots[seg]) * a.slot_stride + static_cast<size_t>(h) * d * dv;
-    auto row_of = [&](int i) { return 4 * NG * (i >> 2) + 4 * lr + (i & 3); };
     float s[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-        const int r = row_of(i);
+        const int r = rg * R + i;
         s[i] = (r < d && col_ok) ? S[static_cast<size_t>(r) * dv + col] : 0.f;
     }
-    const int off_q = a.off_q + h * d, off_k = a.off_k + h * d, off_a = a.off_a + h * d, off_v = a.off_v + h * dv;
-    float qn_[R], kn_[R], an_[R], vn_ = 0.f;
-    auto fetch = [&](int t) {  // token t's operands into the look-ahead registers
-        if (t >= qn) return;
-        const size_t row = static_cast<size_t>(q0 + t);
-        const float* qp = a.q + row * a.ldq + off_q;
-        const float* kp = a.k + row * a.ldk + off_k;
-        const float* ap = a.a + row * a.lda + off_a;
-        if (VEC) {
-#pragma unroll
-            for (int b = 0; b < R / 4; ++b) {
-                const int r = 4 * NG * b + 4 * lr;
-                float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv, av = qv;
-                if (r < d) {
-                    qv = *reinterpret_cast<const float4*>(qp + r);
-                    kv = *reinterpret_cast<const float4*>(kp + r);
-                    av = *reinterpret_cast<const float4*>(ap + r);
-                }
-                qn_[4 * b] = qv.x; qn_[4 * b + 1] = qv.y; qn_[4 * b + 2] = qv.z; qn_[4 * b + 3] = qv.w;
-                kn_[4 * b] = kv.x; kn_[4 * b + 1] = kv.y; kn_[4 * b + 2] = kv.z; kn_[4 * b + 3] = kv.w;
-                an_[4 * b] = av.x; an_[4 * b + 1] = av.y; an_[4 * b + 2] = av.z; an_[4 * b + 3] = av.w;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const int r = row_of(i);
-                qn_[i] = r < d ? qp[r] : 0.f;
-                kn_[i] = r < d ? kp[r] : 0.f;
-                an_[i] = r < d ? ap[r] : 0.f;
-            }
-        }
-        vn_ = col_ok ? a.v[row * a.ldv + off_v + col] : 0.f;
-    };
-    fetch(0);
     for (int t = 0; t < qn; ++t) {
-        float qq[R], kk[R], aa[R];
-        const float vv = vn_;
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-            qq[i] = qn_[i];
-            kk[i] = kn_[i];
-            aa[i] = an_[i];
+        const size_t row = static_cast<size_t>(q0 + t);
+        const float vv = col_ok ? a.v[row * a.ldv + a.off_v + h * dv + col] : 0.f;
+        for (int r = tid; r < DP; r += 128) {
+            ops[0][r] = r < d ? a.q[row * a.ldq + a.off_q + h * d + r] : 0.f;
+            ops[1][r] = r < d ? a.k[row * a.ldk + a.off_k + h * d + r] : 0.f;
+            ops[2][r] = r < d ? a.a[row * a.lda + a.off_a + h * d + r] : 0.f;
         }
-        fetch(t + 1);  // the next token's operands are on their way while this one is worked on
+        __syncthreads();
         float o0 = 0.f, o1 = 0.f;
 #pragma unroll
-        for (int i = 0; i < R; i += 2) {
-            s[i] = fmaf(kk[i], vv, fmaf(-aa[i], s[i], s[i]));
-            s[i + 1] = fmaf(kk[i + 1], vv, fmaf(-aa[i + 1], s[i + 1], s[i + 1]));
-            o0 = fmaf(s[i], qq[i], o0);
-            o1 = fmaf(s[i + 1], qq[i + 1], o1);
+        for (int i = 0; i < R; i += 4) {
+            const float4 qv = *reinterpret_cast<const float4*>(&ops[0][rg * R + i]);
+            const float4 kv = *reinterpret_cast<const float4*>(&ops[1][rg * R + i]);
+            const float4 av = *reinterpret_cast<const float4*>(&ops[2][rg * R + i]);
+            s[i] = fmaf(kv.x, vv, fmaf(-av.x, s[i], s[i]));
+            s[i + 1] = fmaf(kv.y, vv, fmaf(-av.y, s[i + 1], s[i + 1]));
+            s[i + 2] = fmaf(kv.z, vv, fmaf(-av.z, s[i + 2], s[i + 2]));
+            s[i + 3] = fmaf(kv.w, vv, fmaf(-av.w, s[i + 3], s[i + 3]));
+            o0 = fmaf(s[i], qv.x, o0);
+            o1 = fmaf(s[i + 1], qv.y, o1);
+            o0 = fmaf(s[i + 2], qv.z, o0);
+            o1 = fmaf(s[i + 3], qv.w, o1);
         }
         float o = o0 + o1;
-#pragma unroll
-        for (int m = CW; m < 32; m <<= 1) o += __shfl_xor_sync(0xffffffffu, o, m);  // across the row groups of this column
-        if (lr == 0 && col_ok) a.out[static_cast<size_t>(q0 + t) * a.ldo + h * dv + col] = o * a.q_scale;
+        o += __shfl_xor_sync(0xffffffffu, o, 16);
+        if ((tid & 31) < 16) part[wid][c] = o;
+        __syncthreads();   // (also: nobody reads the operands any more)
+        if (tid < 16 && col_ok)
+            a.out[row * a.ldo + h * dv + col] = ((part[0][c] + part[1][c]) + (part[2][c] + part[3][c])) * a.q_scale;
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-        const int r = row_of(i);
+        const int r = rg * R + i;
         if (r < d && col_ok) S[static_cast<size_t>(r) * dv + col] = s[i];
     }
 }
@@ -152,31 +292,43 @@ extern "C" int locus_gla_decay(float* z, int ld, int off, int n, int T, float ta
     return locus_launch_status();
 }
 
+template <int RPL>
+static int gla_walk(const GlaArgs& a, bool vec, int n_seg, cudaStream_t stream) {
+    constexpr int CB = WALK_CW * WALK_WARPS;
+    constexpr size_t smem = sizeof(float) * GL_STAGES * GL_TT * (3 * 32 * RPL + 2 * CB);
+    const int col_blocks = (a.dv + CB - 1) / CB;
+    auto* kernel = vec ? gla_walk_kernel<RPL, true> : gla_walk_kernel<RPL, false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    locus_launch(kernel, dim3(a.H * col_blocks, n_seg), dim3(32 * WALK_WARPS), smem, stream, a, col_blocks);
+    return locus_launch_status();
+}
+
+// n_rows: the rows of `out`, which bound the tokens of all segments together.  Where they are at most GL_FEW a segment the
+// walk's copies would mostly be of tokens that are not there.
+#define GL_FEW 2
 extern "C" int locus_gla_scan(const float* q, int ldq, int off_q, const float* k, int ldk, int off_k, const float* v, int ldv,
                               int off_v, const float* dec, int lda, int off_a, float* state, long long slot_stride,
-                              const int* state_slots, const int* seg_q0, const int* seg_qn, int n_seg, float* out, int ldo,
-                              int H, int d, int dv, float q_scale, cudaStream_t stream) {
+                              const int* state_slots, const int* seg_q0, const int* seg_qn, int n_seg, int n_rows, float* out,
+                              int ldo, int H, int d, int dv, float q_scale, cudaStream_t stream) {
     if (n_seg <= 0) return 0;
     if (H <= 0 || d <= 0 || d > 256 || dv <= 0 || n_seg > 65535 || H > 65535) return LOCUS_ERR_UNSUPPORTED;
     GlaArgs a;
     a.q = q; a.k = k; a.v = v; a.a = dec; a.state = state; a.state_slots = state_slots; a.seg_q0 = seg_q0; a.seg_qn = seg_qn;
     a.out = out; a.slot_stride = slot_stride; a.ldq = ldq; a.off_q = off_q; a.ldk = ldk; a.off_k = off_k; a.ldv = ldv;
     a.off_v = off_v; a.lda = lda; a.off_a = off_a; a.ldo = ldo; a.H = H; a.d = d; a.dv = dv; a.q_scale = q_scale;
-    {   // (the scope of the launch macro)
-        const bool vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(dec)) & 15) == 0 &&
-                         ((ldq | off_q | ldk | off_k | lda | off_a | d) & 3) == 0;
-        const int col_groups = (dv + GL_CW - 1) / GL_CW;
-        const dim3 grid((H * col_groups + 3) / 4, n_seg);
-#define GL_SCAN(R)                                                                              \
-    do {                                                                                        \
-        if (vec) locus_launch(gla_scan_kernel<R, true>, grid, dim3(128), 0, stream, a, col_groups);  \
-        else locus_launch(gla_scan_kernel<R, false>, grid, dim3(128), 0, stream, a, col_groups);     \
-    } while (0)
-        if (d <= 32) GL_SCAN(4);
-        else if (d <= 64) GL_SCAN(8);
-        else if (d <= 128) GL_SCAN(16);
-        else GL_SCAN(32);
-#undef GL_SCAN
+    if (n_rows <= static_cast<long long>(GL_FEW) * n_seg) {
+        const int col_blocks = (dv + 15) / 16;
+        const dim3 grid(H * col_blocks, n_seg);
+        if (d <= 32) locus_launch(gla_tokens_kernel<4>, grid, dim3(128), 0, stream, a, col_blocks);
+        else if (d <= 64) locus_launch(gla_tokens_kernel<8>, grid, dim3(128), 0, stream, a, col_blocks);
+        else if (d <= 128) locus_launch(gla_tokens_kernel<16>, grid, dim3(128), 0, stream, a, col_blocks);
+        else locus_launch(gla_tokens_kernel<32>, grid, dim3(128), 0, stream, a, col_blocks);
+        return locus_launch_status();
     }
-    return locus_launch_status();
+    const bool vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(dec)) & 15) == 0 &&
+                     ((ldq | off_q | ldk | off_k | lda | off_a | d) & 3) == 0;
+    if (d <= 64) return gla_walk<2>(a, vec, n_seg, stream);
+    if (d <= 128) return gla_walk<4>(a, vec, n_seg, stream);
+    return gla_walk<8>(a, vec, n_seg, stream);
 }

@@ -2019,7 +2019,8 @@ def delta_rule(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torc
     code = _lib("delta_rule").locus_delta_scan(
         _p(q), I(q.stride(0)), I(off_q), _p(k), I(k.stride(0)), I(off_k), _p(v), I(v.stride(0)), I(off_v), _p(beta),
         _p(decay), ctypes.c_void_p(state.data_ptr() + 4 * state_offset), LL(state.stride(0)), _p(state_slots), _p(seg_q0),
-        _p(seg_qn), I(n_seg), _p(out), I(out.stride(0)), I(n_heads), I(heads_per_group), I(dim), I(v_dim), _stream())
+        _p(seg_qn), I(n_seg), I(out.shape[0]), _p(out), I(out.stride(0)), I(n_heads), I(heads_per_group), I(dim), I(v_dim),
+        _stream())
     _check(code, "delta_scan", f"(heads {n_heads}, dim {dim}, v_dim {v_dim})")
 
 
@@ -2135,8 +2136,8 @@ def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.
     code = _lib("gla").locus_gla_scan(
         _p(q), I(q.stride(0)), I(off_q), _p(k), I(k.stride(0)), I(off_k), _p(v), I(v.stride(0)), I(off_v), _p(decay),
         I(decay.stride(0)), I(off_a), ctypes.c_void_p(state.data_ptr() + 4 * state_offset), LL(state.stride(0)),
-        _p(state_slots), _p(seg_q0), _p(seg_qn), I(n_seg), _p(out), I(out.stride(0)), I(n_heads), I(dim), I(v_dim),
-        F(q_scale), _stream())
+        _p(state_slots), _p(seg_q0), _p(seg_qn), I(n_seg), I(out.shape[0]), _p(out), I(out.stride(0)), I(n_heads), I(dim),
+        I(v_dim), F(q_scale), _stream())
     _check(code, "gla_scan", f"(heads {n_heads}, dim {dim}, v_dim {v_dim})")
 
 

@@ -161,6 +161,31 @@ def precise(monkeypatch):
     monkeypatch.setattr(EK, "PRECISE", True)
 
 
+@pytest.mark.parametrize("H,d,dv", [(2, 24, 16), (1, 7, 5), (3, 72, 40), (2, 128, 128), (1, 256, 17)])
+def test_gla_scan_of_few_tokens_and_of_tiles_edges(H, d, dv, precise):
+    """Steps whose rows are few a segment go to a kernel of their own (none, one and two tokens), longer ones end on, in
+    front of and behind a tile of 16 tokens and a group of 8."""
+    import locus_b200.kernels as K
+
+    g = torch.Generator().manual_seed(d)
+    for qn in ([1, 0, 2, 1], [16, 8, 33, 7, 1]):
+        T, W = sum(qn), 2 * H * d + H * dv
+        proj, z = torch.randn(T, W, generator=g), torch.rand(T, H * d, generator=g) * 0.3
+        state = torch.randn(len(qn), H * d * dv, generator=g)
+        slots = torch.arange(len(qn), dtype=torch.int32).flip(0).contiguous()
+        n = torch.tensor(qn, dtype=torch.int32)
+        q0 = (n.cumsum(0) - n).to(torch.int32)
+        kw = dict(n_heads=H, dim=d, v_dim=dv, q_scale=d ** -0.5)
+        ref_state, ref = state.double(), torch.zeros(T, H * dv, dtype=torch.float64)
+        args = (0, H * d, 2 * H * d)
+        EK.gla_scan(proj.double(), args[0], proj.double(), args[1], proj.double(), args[2], z.double(), 0, ref_state, 0, slots,
+                    q0, n, len(qn), ref, **kw)
+        p, st, out = proj.to(DEV), state.to(DEV), torch.zeros(T, H * dv, device=DEV)
+        K.gla_scan(p, args[0], p, args[1], p, args[2], z.to(DEV), 0, st, 0, slots.to(DEV), q0.to(DEV), n.to(DEV), len(qn), out, **kw)
+        _cmp(out, ref, 2e-5)
+        _cmp(st, ref_state, 2e-5)
+
+
 @pytest.mark.parametrize("H,d,dv", [(2, 24, 16), (1, 7, 5), (3, 72, 40), (2, 128, 64), (1, 200, 12)])
 def test_gla_scan_and_decay_against_twin(H, d, dv, precise):
     import locus_b200.kernels as K

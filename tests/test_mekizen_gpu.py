@@ -221,6 +221,38 @@ def test_delta_rule_against_its_twin(heads, per_group, dim, v_dim, aligned):
     assert _close(out2, out_w, 3e-5) and _close(state2, st_w, 3e-5)
 
 
+@pytest.mark.parametrize("heads,per_group,dim,v_dim", [(2, 1, 24, 16), (1, 1, 7, 5), (4, 2, 72, 40), (2, 1, 128, 128), (1, 1, 256, 17)])
+def test_delta_rule_of_few_tokens_and_of_tiles_edges(heads, per_group, dim, v_dim):
+    """Steps whose rows are few a segment go to a kernel of their own (none, one and two tokens), longer ones end on, in
+    front of and behind a tile of 16 tokens and a group of 8."""
+    import locus_b200.kernels as K
+
+    G = heads // per_group
+    for qn in ([1, 0, 2, 1], [16, 8, 33, 7, 1]):
+        T = sum(qn)
+        rows = _rand((T, 2 * G * dim + heads * v_dim), 5, 0.6)
+        k = rows[:, G * dim:2 * G * dim].view(T, G, dim)
+        k /= k.norm(dim=-1, keepdim=True)
+        beta = torch.rand(T, heads, generator=torch.Generator().manual_seed(2)).cuda()
+        decay = torch.rand(T, heads, generator=torch.Generator().manual_seed(1)).cuda()
+        state = _rand((len(qn), heads * dim * v_dim), 6, 0.3)
+        q0 = _dev([sum(qn[:i]) for i in range(len(qn))])
+        st_w, out_w = state.cpu().double(), torch.zeros(T, heads * v_dim, dtype=torch.float64)
+        out = torch.zeros(T, heads * v_dim, device="cuda")
+
+        def run(fn, r, b, g, s, to, o):
+            fn(r, 0, r, G * dim, r, 2 * G * dim, b, g, s, 0, to(_dev(list(range(len(qn))))), to(q0), to(_dev(qn)), len(qn), o,
+               n_heads=heads, heads_per_group=per_group, dim=dim, v_dim=v_dim)
+
+        EK.PRECISE = True
+        try:
+            run(EK.delta_rule, rows.cpu(), beta.cpu(), decay.cpu(), st_w, lambda x: x.cpu(), out_w)
+        finally:
+            EK.PRECISE = False
+        run(K.delta_rule, rows, beta, decay, state, lambda x: x, out)
+        assert _close(out, out_w, 3e-5) and _close(state, st_w, 3e-5)
+
+
 @pytest.mark.parametrize("odt", DTYPES, ids=IDS)
 @pytest.mark.parametrize("heads,v_dim,shared", [(2, 8, True), (3, 10, False), (1, 40, True), (4, 128, True)])
 def test_delta_output_stage_and_gate_rows_against_their_twins(heads, v_dim, shared, odt):
