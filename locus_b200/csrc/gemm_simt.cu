@@ -13,7 +13,19 @@
 //                each 64-row tile, its expert, first row and row count; W of expert e
 //                starts at W + e * w_expert_stride
 //   * epilogue   store as float32 or bfloat16, or add into a float32 tensor (residual)
+//
+// Two kernels.  gemm_f32: float32 rows and weights that 16-byte copies can fetch.  Bound by the multiply-adds (148 SMs x 128
+// lanes x 2 x 1.965 GHz = 74.4 TFLOP/s), so everything else is kept off their issue slots: 32 columns of k of 64 rows
+// and 128 weight rows are copied into shared memory asynchronously, two stages ahead, k contiguous as they lie in memory (rows
+// 36 floats apart meet in no bank), a thread owns 8 x 8 outputs, and a multiply-add works on two k at once, so each
+// output has a sum over the even k and one over the odd k, added at the end -- in the same order whatever the tile.  A
+// tile's rows are worked on in eights, so that an expert's 34 rows cost 40 and not 64.  gemm_simt: every other type,
+// width and alignment.  Measured: 2,048 x
+// 6,144 x 2,048 1.18 ms = 43.8 TFLOP/s (20 before, with the 64 x 64 x 16 tiles of gemm_simt), 512 x 6,144 x 2,048 343 us, the
+// routed experts of 512 tokens (60 x (2,048 -> 1,408 -> 2,048), 4 picks) 1.02 ms; one multiply-add at a time instead of
+// two, with up to twice the warps, 1.26 to 1.5 ms on the first.
 #include "common.cuh"
+#include "walk.cuh"
 
 #define BM 64
 #define BN 64
@@ -47,6 +59,34 @@ struct GemmArgs {
     const int* n_tiles;
     long long w_expert_stride;
 };
+
+// One output: activation, bias, row scale (rs), softcap, store.  v2: the second weight's sum.
+template <bool SWIGLU>
+__device__ __forceinline__ void epilogue(const GemmArgs& a, int r, int n, float rs, float v, float v2) {
+    if (SWIGLU && a.act == 2) {
+        const float g = fminf(v * rs, a.act_param);
+        const float u = fminf(fmaxf(v2 * rs, -a.act_param), a.act_param);
+        v = g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
+    } else if (SWIGLU && a.act == 4) {
+        v = fmaxf(v + pair_bias(a.bias, a.bias_dt, n), 0.f) * (v2 + pair_bias(a.bias, a.bias_dt, a.N + n));
+    } else if (SWIGLU) {
+        const float g = v;
+        v = g / (1.0f + expf(-g)) * v2;
+    }
+    if (a.bias && a.act != 4) v += ld_dyn(a.bias, a.bias_dt, n);
+    if (a.act == 1) {
+        v = fmaxf(v, 0.f);
+        v *= v;
+    }
+    if (a.row_scale && a.act != 2) v *= rs;
+    if (a.act == 3) v = a.act_param * tanhf(v * a.act_scale / a.act_param);
+    const size_t o = static_cast<size_t>(r) * a.ldo + n;
+    if (a.accumulate) {
+        static_cast<float*>(a.out)[o] += v;
+    } else {
+        st_dyn(a.out, a.out_dt, o, v);
+    }
+}
 
 template <typename TX, typename TW, bool SWIGLU>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs a) {
@@ -139,33 +179,139 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = col0 + tx * 4 + j;
-            if (n >= a.N) continue;
-            float v = acc[i][j];
-            if (SWIGLU && a.act == 2) {
-                const float g = fminf(v * rs, a.act_param);
-                const float u = fminf(fmaxf(acc2[i][j] * rs, -a.act_param), a.act_param);
-                v = g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
-            } else if (SWIGLU && a.act == 4) {
-                v = fmaxf(v + pair_bias(a.bias, a.bias_dt, n), 0.f) * (acc2[i][j] + pair_bias(a.bias, a.bias_dt, a.N + n));
-            } else if (SWIGLU) {
-                const float g = v;
-                v = g / (1.0f + expf(-g)) * acc2[i][j];
-            }
-            if (a.bias && a.act != 4) v += ld_dyn(a.bias, a.bias_dt, n);
-            if (a.act == 1) {
-                v = fmaxf(v, 0.f);
-                v *= v;
-            }
-            if (a.row_scale && a.act != 2) v *= rs;
-            if (a.act == 3) v = a.act_param * tanhf(v * a.act_scale / a.act_param);
-            const size_t o = static_cast<size_t>(r) * a.ldo + n;
-            if (a.accumulate) {
-                static_cast<float*>(a.out)[o] += v;
-            } else {
-                st_dyn(a.out, a.out_dt, o, v);
-            }
+            if (n < a.N) epilogue<SWIGLU>(a, r, n, rs, acc[i][j], SWIGLU ? acc2[i][j] : 0.f);
         }
     }
+}
+
+#define FM 64          // rows of a tile
+#define FK 32          // columns of k of a stage
+#define FLD (FK + 4)   // floats from row to row of a stage
+#define F_STAGES 3
+
+// A stage's share of eight-row groups 0 .. NI - 1: thread (ty, tx) owns the rows ty + 8 i and the weight rows tx + TX j.
+template <int NI, int TX>
+__device__ __forceinline__ void f32_stage(const float* xs, const float* ws, f2 (&acc)[8][8]) {
+#pragma unroll
+    for (int k = 0; k < FK; k += 4) {
+        ulonglong2 x[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(xs + 8 * i * FLD + k);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(ws + TX * j * FLD + k);
+#pragma unroll
+            for (int i = 0; i < NI; ++i) acc[i][j] = f2_fma(x[i].x, w.x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < NI; ++i) acc[i][j] = f2_fma(x[i].y, w.y, acc[i][j]);
+        }
+    }
+}
+
+// TX: threads across the weight rows of a tile (8 TX of them; with SWIGLU 4 TX of each weight).
+template <int TX, bool SWIGLU>
+__global__ void __launch_bounds__(8 * TX) gemm_f32_kernel(GemmArgs a) {
+    constexpr int BNW = 8 * TX, COLS = SWIGLU ? BNW / 2 : BNW, NT = 8 * TX, STAGE = (FM + BNW) * FLD;
+    extern __shared__ __align__(16) float f32_smem[];
+    int row0, rows;
+    const float* W = static_cast<const float*>(a.w);
+    const float* W2 = static_cast<const float*>(a.w2);
+    if (a.tile_expert != nullptr) {
+        const int tile = blockIdx.y;
+        if (tile >= *a.n_tiles) return;
+        const long long e = a.tile_expert[tile];
+        row0 = a.tile_row0[tile];
+        rows = a.tile_rows[tile];
+        W += e * a.w_expert_stride;
+        if (SWIGLU) W2 += e * a.w_expert_stride;
+    } else {
+        row0 = blockIdx.y * FM;
+        rows = min(FM, a.M - row0);
+    }
+    const int col0 = blockIdx.x * COLS, tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    // the copies of this thread: 16 bytes of k (chunk tid & 7) of every NT / 8-th row
+    constexpr int PER = NT / 8;
+    const int chunk = (tid & 7) * 4, lrow = tid >> 3;
+    int xrow[FM / PER];
+#pragma unroll
+    for (int i = 0; i < FM / PER; ++i) {
+        const int r = row0 + lrow + i * PER;
+        xrow[i] = lrow + i * PER >= rows ? -1 : a.x_rows ? a.x_rows[r] / a.x_row_div : r;
+    }
+    const int n_k = (a.K + FK - 1) / FK, live_rows = (rows + 7) & ~7;
+    auto fetch = [&](int kb) {   // columns behind K and rows that are not there are zeros
+        float* st = f32_smem + (kb % F_STAGES) * STAGE + lrow * FLD + chunk;
+        const int k = kb * FK + chunk;
+        const bool in = k < a.K;
+#pragma unroll
+        for (int i = 0; i < FM / PER; ++i)
+            if (lrow + i * PER < live_rows) {
+                const bool live = in && xrow[i] >= 0;
+                walk_copy<16>(st + i * PER * FLD, live ? static_cast<const float*>(a.x) + xrow[i] * a.ldx + k : W, live);
+            }
+#pragma unroll
+        for (int i = 0; i < BNW / PER; ++i) {
+            const int c = lrow + i * PER, n = col0 + (SWIGLU ? c % COLS : c);
+            const bool live = in && n < a.N;
+            const float* w = SWIGLU && i * PER >= COLS ? W2 : W;   // (COLS is a multiple of PER)
+            walk_copy<16>(st + (FM + i * PER) * FLD, live ? w + static_cast<long long>(n) * a.K + k : W, live);
+        }
+    };
+    f2 acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+#pragma unroll
+    for (int i = 0; i < F_STAGES - 1; ++i) {
+        if (i < n_k) fetch(i);
+        walk_commit();
+    }
+    const int groups = (rows + 7) >> 3;
+    auto walk_k = [&](auto stage) {
+        for (int kb = 0; kb < n_k; ++kb) {
+            walk_wait<F_STAGES - 2>();
+            __syncthreads();   // the stage is there for all warps, and nobody reads the one that is filled next
+            if (kb + F_STAGES - 1 < n_k) fetch(kb + F_STAGES - 1);
+            walk_commit();
+            const float* st = f32_smem + (kb % F_STAGES) * STAGE;
+            stage(st + ty * FLD, st + (FM + tx) * FLD);
+        }
+    };
+    if (groups <= 2) walk_k([&](const float* x, const float* w) { f32_stage<2, TX>(x, w, acc); });
+    else if (groups <= 4) walk_k([&](const float* x, const float* w) { f32_stage<4, TX>(x, w, acc); });
+    else if (groups == 5) walk_k([&](const float* x, const float* w) { f32_stage<5, TX>(x, w, acc); });
+    else if (groups == 6) walk_k([&](const float* x, const float* w) { f32_stage<6, TX>(x, w, acc); });
+    else walk_k([&](const float* x, const float* w) { f32_stage<8, TX>(x, w, acc); });
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = ty + 8 * i;
+        if (m >= rows) continue;
+        const int r = row0 + m;
+        const float rs = a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
+#pragma unroll
+        for (int j = 0; j < (SWIGLU ? 4 : 8); ++j) {
+            const int n = col0 + tx + TX * j;
+            if (n >= a.N) continue;
+            float even, odd, even2 = 0.f, odd2 = 0.f;
+            f2_unpack(acc[i][j], even, odd);
+            if (SWIGLU) f2_unpack(acc[i][j + 4], even2, odd2);
+            epilogue<SWIGLU>(a, r, n, rs, even + odd, even2 + odd2);
+        }
+    }
+}
+
+template <int TX>
+static int launch_f32(const GemmArgs& a, int tiles, bool swiglu, cudaStream_t stream) {
+    constexpr size_t smem = sizeof(float) * F_STAGES * (FM + 8 * TX) * FLD;
+    const dim3 grid(ceil_div(a.N, swiglu ? 4 * TX : 8 * TX), tiles);
+    if (grid.y == 0 || grid.x == 0) return 0;
+    if (grid.y > 65535) return LOCUS_ERR_UNSUPPORTED;
+    auto* kernel = swiglu ? gemm_f32_kernel<TX, true> : gemm_f32_kernel<TX, false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    kernel<<<grid, 8 * TX, smem, stream>>>(a);
+    return locus_launch_status();
 }
 
 template <typename TX, typename TW>
@@ -207,6 +353,13 @@ extern "C" int locus_gemm_simt(const void* x, int x_dt, const void* w, const voi
     a.n_tiles = n_tiles; a.w_expert_stride = w_expert_stride;
     const int tiles = tile_expert ? max_tiles : ceil_div(M, BM);
     const bool swiglu = w2 != nullptr;
+    static_assert(FM == BM, "the grouped tile lists serve both kernels");
+    if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32 && ((K | ldx) & 3) == 0 &&
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w2)) & 15) == 0) {
+        // tiles of 64 weight rows where tiles of 128 would leave SMs without one
+        const long long wide = static_cast<long long>(ceil_div(N, swiglu ? 64 : 128)) * tiles;
+        return wide < 148 ? launch_f32<8>(a, tiles, swiglu, stream) : launch_f32<16>(a, tiles, swiglu, stream);
+    }
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32) return launch<float, float>(a, tiles, swiglu, stream);
     if (x_dt == LOCUS_DT_BF16 && w_dt == LOCUS_DT_BF16) return launch<bf16, bf16>(a, tiles, swiglu, stream);
     if (x_dt == LOCUS_DT_BF16 && w_dt == LOCUS_DT_F32) return launch<bf16, float>(a, tiles, swiglu, stream);

@@ -518,6 +518,53 @@ def test_attn_chunk_tensor_cores(nh, nkv, hd, P, window):
     assert 1 < K.attn_chunk_mma_splits(1, 16, 30000) <= K.MMA_ATTN_MAX_SPLITS
 
 
+@pytest.mark.parametrize("nh,nkv,hd,P,more", [
+    (4, 4, 16, 16, {}), (6, 2, 32, 48, {}), (5, 1, 48, 64, dict(window=24)), (2, 2, 64, 16, dict(window=1, sink=True)),
+    (3, 1, 80, 64, dict(chunk=50)), (4, 2, 112, 16, dict(window=100, keep_first=5, sink="learned")),
+    (4, 2, 128, 64, dict(slopes=True)), (2, 1, 128, 128, dict(window=70, keep_first=70))])
+def test_attn_chunk_float32_tiles(nh, nkv, hd, P, more):
+    """Portions of 2 to 200 tokens at contexts that straddle the 64-key tiles and the pages, whole and with the keys cut into
+    ranges; whatever lies in a request's pages behind its last token is NaN and must not reach the result."""
+    segs = [(0, 5), (33, 17), (100, 2), (15, 140), (64, 64), (190, 200), (63, 65)]
+    pool, q, meta, T = _paged_case(torch.float32, nh, nkv, hd, P, segs, seed=hd + 9, n_pages=120)
+    for s, (c, n) in enumerate(segs):
+        if (c + n) % P:
+            pool[int(meta["block_table"][s, (c + n) // P]), :, :, (c + n) % P :, :] = float("nan")
+    items_t = torch.tensor([(s, o) for s, (c, n) in enumerate(segs) for o in range(0, n, 64)], dtype=torch.int32)
+    kw = dict(n_heads=nh, n_kv_heads=nkv, head_dim=hd, page_tokens=P, window=0, scale=1 / math.sqrt(hd), **{})
+    kw.update(more)
+    if kw.get("sink") == "learned":
+        kw["sink"] = rnd(nh, seed=3)
+    if kw.get("slopes"):
+        kw["slopes"] = torch.tensor([2.0 ** -(h + 1) for h in range(nh)], dtype=torch.float32)
+    dev_kw = {k: v.to(DEV) if torch.is_tensor(v) else v for k, v in kw.items()}
+    ref = torch.zeros(T, nh * hd, dtype=torch.float64)
+    EK.attn_chunk(q, torch.nan_to_num(pool, nan=1e4), ref, items=items_t, n_items=len(items_t), **meta, **kw)
+    dq, dpool = q.to(DEV), pool.to(DEV)
+    assert K.attn_chunk_f32_takes(dq, hd) and not K.attn_chunk_f32_takes(dq, 144) and not K.attn_chunk_f32_takes(dq.bfloat16(), hd)
+    for n_splits in (1, 2, 7):
+        units = len(items_t) * nh * n_splits * 64
+        part_o, part_ml = torch.full((units * hd,), float("nan"), device=DEV), torch.full((units * 2,), float("nan"), device=DEV)
+        out = torch.full((T, nh * hd), float("nan"), device=DEV)
+        K.attn_chunk_f32(dq, dpool, out, items=items_t.to(DEV), n_items=len(items_t), n_splits=n_splits, part_o=part_o,
+                         part_ml=part_ml, **_dev(meta), **dev_kw)
+        close(out, ref, torch.float32, f"attn_chunk_f32 in {n_splits} key ranges")
+
+
+@pytest.mark.parametrize("dual", [False, True])
+@pytest.mark.parametrize("M,N,K_", [(9, 64, 36), (64, 129, 60), (65, 200, 4), (17, 1000, 2052), (40, 33, 100), (130, 300, 128)])
+def test_linear_float32_tiles(M, N, K_, dual):
+    """The float32 product's tiles of 64 rows worked on in eights, 64 and 128 weight rows and 32 columns of k, at their edges."""
+    x, w, w2 = rnd(M, K_ + 4, seed=1)[:, :K_], rnd(N, K_, seed=2), rnd(N, K_, seed=3)
+    dx = torch.zeros(M, K_ + 4, device=DEV)[:, :K_]   # (rows wider than the product's)
+    dx.copy_(x)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    K.linear(dx, w.to(DEV), out, w2=w2.to(DEV) if dual else None)
+    g = x.double() @ w.double().T
+    ref = torch.nn.functional.silu(g) * (x.double() @ w2.double().T) if dual else g
+    close(out, ref, torch.float32, f"linear {M} x {N} x {K_} dual={dual}")
+
+
 @pytest.mark.parametrize("nh,nkv,P,window", [(2, 2, 64, 0), (4, 1, 128, 0), (3, 3, 64, 100), (2, 1, 64, 1), (4, 2, 192, 333)])
 def test_attn_chunk_tcgen05(nh, nkv, P, window):
     """Portions of 2 to 450 tokens at contexts that straddle the 128-key tiles and the pages; whatever lies
