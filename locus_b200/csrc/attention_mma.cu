@@ -21,7 +21,7 @@
 // padded by 16 bytes so that ldmatrix reads no bank twice.
 #include "common.cuh"
 #include "distance.cuh"
-#include "mask.cuh"
+#include "key_tiles.cuh"
 #include "sink.cuh"
 
 #define MQ 64    // queries per block
@@ -46,21 +46,6 @@ struct MmaAttnArgs {
     float* part_o;    // [item][head][split][MQ][hd] unnormalised sums
     float* part_ml;   // [item][head][split][MQ][2] running maximum (base 2, scaled) and denominator
 };
-
-// Key tiles of an item: the first tile's first position and their number (the same in both kernels).
-// With kept first tokens the tiles that hold them and lie in front of the window's first tile come first
-// (kept_tiles of them, from position 0); tile number i of the item starts at tile_pos(i).
-__device__ __forceinline__ void item_tiles(int p0, int nq, int window, int chunk, int keep_first, int& first_tile, int& n_tiles,
-                                           int& kept_tiles) {
-    const int t_hi = p0 + nq - 1;
-    const int t_lo = first_key(window, chunk, p0);
-    first_tile = (t_lo / MK) * MK;
-    kept_tiles = window > 0 ? min(first_tile / MK, (min(keep_first, t_lo) + MK - 1) / MK) : 0;
-    n_tiles = (t_hi - first_tile) / MK + 1 + kept_tiles;
-}
-__device__ __forceinline__ int tile_pos(int i, int first_tile, int kept_tiles) {
-    return i < kept_tiles ? i * MK : first_tile + (i - kept_tiles) * MK;
-}
 
 __device__ __forceinline__ uint32_t sm_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 

@@ -787,6 +787,46 @@ def attn_chunk_mma(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor, *, se
     _check(code, "attn_chunk_mma", f"(heads {n_heads}/{n_kv_heads}, head_dim {head_dim}, {n_splits} key ranges)")
 
 
+F32_ATTN_MAX_HEAD = 128   # larger float32 heads run on attn_chunk
+
+
+def attn_chunk_f32_takes(q: torch.Tensor, head_dim: int) -> bool:
+    """Whether the float32 kernel of 64-query tiles takes this case; otherwise :func:`attn_chunk` does (16-query tiles)."""
+    return (q.is_cuda and q.dtype == torch.float32 and head_dim % 16 == 0 and head_dim <= F32_ATTN_MAX_HEAD
+            and q.data_ptr() % 16 == 0)
+
+
+def attn_chunk_f32(q: torch.Tensor, pool: torch.Tensor, out: torch.Tensor, *, seg_q0: torch.Tensor,
+                   seg_qn: torch.Tensor, seg_ctx: torch.Tensor, block_table: torch.Tensor,
+                   items: torch.Tensor, n_items: int, n_heads: int, n_kv_heads: int, head_dim: int,
+                   page_tokens: int, window: int, scale: float, n_splits: int = 1,
+                   part_o: Optional[torch.Tensor] = None, part_ml: Optional[torch.Tensor] = None,
+                   keep_first: int = 0, sink=False, chunk: int = 0, slopes: Optional[torch.Tensor] = None) -> None:
+    """Attention of portions of prompts in float32 on the CUDA cores: ``items`` [n_items, 2] = (segment, first query of a
+    64-query tile); otherwise as :func:`attn_chunk`.  ``n_splits`` and its scratch as in :func:`attn_chunk_mma`
+    (:func:`attn_chunk_mma_splits`, :func:`attn_chunk_mma_scratch`)."""
+    _cuda_c(q, "q")
+    _cuda_c(out, "out")
+    _cuda_c(pool, "pool")
+    _i32(block_table, "block_table")
+    _i32(items, "items")
+    _need(q.dtype == pool.dtype == out.dtype == torch.float32, "attn_chunk_f32: float32 only")
+    if n_splits > 1:
+        units = n_items * n_heads * n_splits
+        _need(part_o is not None and part_ml is not None and part_o.dtype == part_ml.dtype == torch.float32
+              and part_o.numel() >= units * MMA_QUERY_TILE * head_dim and part_ml.numel() >= units * MMA_QUERY_TILE * 2,
+              "attn_chunk_f32: scratch too small for these ranges")
+    code = _lib("attention_f32").locus_attn_chunk_f32(
+        _p(q), _p(pool), _p(out), _p(seg_q0), _p(seg_qn), _p(seg_ctx), _p(block_table), I(block_table.shape[1]),
+        _p(items), I(n_items), I(n_heads), I(n_kv_heads), I(head_dim), I(page_tokens), I(window), I(chunk), F(scale),
+        I(n_splits), _p(part_o if n_splits > 1 else None), _p(part_ml if n_splits > 1 else None), I(keep_first),
+        *_sink_args(sink, n_heads), _slopes_arg(slopes, n_heads), _stream()
+    )
+    if n_splits > 1 and code == 0:
+        _count_launches(1)
+    _check(code, "attn_chunk_f32", f"(heads {n_heads}/{n_kv_heads}, head_dim {head_dim}, {n_splits} key ranges)")
+
+
 TC_ATTN_HEAD_DIM = 128   # the tcgen05 attention kernel: this head size, pages of a multiple of 64 tokens
 TC_ATTN_MIN_TOKENS = 256  # from this many new tokens in a step on, the tcgen05 kernel takes every portion
 

@@ -305,7 +305,8 @@ class Attention(Mixer):
     def kernel_modules(self, dtype):
         special = bool(self.keep_first or self.sink)   # such an attention runs on the kernels that know of both
         return (["elementwise", "gemm_simt", "gemv", "attention"] + (["short_conv"] if self.shaped else [])
-                + (["gemm_skinny", "gemm_tc", "attention_mma", "attention_tc", "attention_gqa"] if dtype == torch.bfloat16 else []))
+                + (["gemm_skinny", "gemm_tc", "attention_mma", "attention_tc", "attention_gqa"] if dtype == torch.bfloat16
+                   else ["attention_f32"]))
 
     def cache_needs(self):
         state = None
@@ -412,15 +413,16 @@ class Attention(Mixer):
                     part_ml = rt.buf("attention.chunk_tc_part_ml", (n_ml,), torch.float32)
                 K.attn_chunk_tc(q, cache.pool, o, items=tiles["chunk_items64"], n_items=tiles["n_chunk_items64"],
                                 n_splits=n_splits, part_o=part_o, part_ml=part_ml, **extra, **common)
-            elif K.attn_chunk_mma_takes(q, self.head_dim):
+            elif K.attn_chunk_mma_takes(q, self.head_dim) or K.attn_chunk_f32_takes(q, self.head_dim):
                 n_splits = K.attn_chunk_mma_splits(tiles["n_chunk_items64"], self.n_heads, keys)
                 part_o = part_ml = None
                 if n_splits > 1:
                     n_o, n_ml = K.attn_chunk_mma_scratch(self.head_dim)
                     part_o = rt.buf("attention.chunk_part_o", (n_o,), torch.float32)
                     part_ml = rt.buf("attention.chunk_part_ml", (n_ml,), torch.float32)
-                K.attn_chunk_mma(q, cache.pool, o, items=tiles["chunk_items64"], n_items=tiles["n_chunk_items64"],
-                                 n_splits=n_splits, part_o=part_o, part_ml=part_ml, **extra, **common)
+                call = K.attn_chunk_f32 if q.dtype == torch.float32 else K.attn_chunk_mma
+                call(q, cache.pool, o, items=tiles["chunk_items64"], n_items=tiles["n_chunk_items64"],
+                     n_splits=n_splits, part_o=part_o, part_ml=part_ml, **extra, **common)
             else:
                 K.attn_chunk(q, cache.pool, o, items=tiles["chunk_items"], n_items=tiles["n_chunk_items"], **extra, **common)
         if tiles["n_decode_items"]:
