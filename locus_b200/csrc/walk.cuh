@@ -45,16 +45,19 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
     return d;
 }
 
-// v[0 .. N - 1] (N 16 or 32): values to be summed over the warp.  Half of the values change hands at every step: N - 1 (16: 16)
-// exchanges instead of 5 N.  Returns the sum of value walk_sum_index<N>(lane).
+// v[0 .. N - 1] (N 8, 16 or 32): values to be summed over the warp.  Half of the values change hands at every step until each
+// lane has one: 31 exchanges for 32 values instead of 160.  Returns the sum of value walk_sum_index<N>(lane).
 template <int N>
 __device__ __forceinline__ int walk_sum_index(int lane) {
-    return N == 32 ? static_cast<int>(__brev(lane) >> 27) : static_cast<int>(__brev(lane & 15) >> 28);
+    return static_cast<int>(__brev(lane & (N - 1)) >> (N == 32 ? 27 : N == 16 ? 28 : 29));
 }
 template <int N, int MASK = 1>
 __device__ __forceinline__ float walk_sum(const float* v, int lane) {
     if constexpr (N == 1) {
-        return MASK < 32 ? v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16) : v[0];
+        float s = v[0];
+#pragma unroll
+        for (int m = MASK; m < 32; m <<= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+        return s;
     } else {
         float w[N / 2];
         const bool upper = lane & MASK;

@@ -364,13 +364,15 @@ def tensor_cores_take(x: torch.Tensor, w: torch.Tensor, x_rows: Optional[torch.T
 
 
 FEW_ROWS = 8  # rows of x per tile of the row-streaming kernel
+F32_STREAM_ROWS = 32  # most rows of a plain float32 product that go to it, in tiles of 8 that share the weights through L2
 
 
 def few_rows_take(x: torch.Tensor, w: torch.Tensor, m: int, layout: Optional["ExpertLayout"] = None) -> bool:
     """Whether :func:`linear` runs this product with the row-streaming kernel: at most 8 rows
-    (per expert tile when grouped), width a multiple of 8, 32-byte aligned rows."""
+    (per expert tile when grouped; ``F32_STREAM_ROWS`` of a plain float32 product), width a multiple of 8, 32-byte aligned rows."""
     K = x.shape[-1]
-    rows_ok = layout.tile_m <= FEW_ROWS if layout is not None else m <= FEW_ROWS
+    most = F32_STREAM_ROWS if x.dtype == torch.float32 and w.dtype == torch.float32 else FEW_ROWS
+    rows_ok = layout.tile_m <= FEW_ROWS if layout is not None else m <= most
     return (rows_ok and K % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 32 == 0 and w.data_ptr() % 32 == 0)
 
 
