@@ -55,7 +55,7 @@ struct GqaArgs {
 
 // Warps of a block (one block per SM) and chunks of 16 keys whose copies are in flight per warp.  Shared memory
 // (8 KB per chunk at head size 128) allows 8 x 3, 10 x 2, 12 x 2 or 6 x 4; measured at 28 heads on 4 and 8,192 keys,
-// 64 / 8 requests: 202 / 52 us, 184 / 56, 190 / 58, 231 / 47.  More warps hide the latency of a chunk's chain of
+// 64 / 8 requests, before the merge took its heads together: 202 / 52 us, 184 / 56, 190 / 58, 231 / 47.  More warps hide the latency of a chunk's chain of
 // dependent instructions better than a deeper ring does.
 #ifndef GQ_WARPS
 #define GQ_WARPS 10
@@ -402,53 +402,78 @@ __global__ void __launch_bounds__(32 * GQW, 1) attn_decode_gqa_kernel(GqaArgs a,
         last = __shfl_sync(0xffffffffu, last, 0);
         if (!last) continue;
         __threadfence();
-        // two heads at a time, so that twice as many loads are in flight (the merge is a chain of loads)
+        // The group's heads together, up to eight at a time: a lane forms the weights of one range for all of them, and every
+        // range's rows of the heads are asked for at once.  (Two heads after two, each a chain of its own over the ranges, the
+        // merge of 28 ranges of 7 heads was a fifth of the call: 28 heads on 4 behind 8,191 keys, 8 requests 47.5 -> 41.4 us, 16
+        // 66 -> 61, 64 185 -> 180.)
+        constexpr int GM = GQW > 6 ? 4 : 8;   // (ten warps leave registers for four)
         const size_t ustep = static_cast<size_t>(a.nkv) * G;
-        for (int g = 0; g < G; g += 2) {
-            const bool two = g + 1 < G;
-            // range s of head g: slot ((pref + s) * nkv + kvh) * G + g
-            const size_t u0 = (static_cast<size_t>(kr.pref[item]) * a.nkv + kvh) * G + g, u1 = u0 + (two ? 1 : 0);
-            float M0 = -INFINITY, M1 = -INFINITY;
-            for (int sidx = lane; sidx < n_splits; sidx += 32) {
-                M0 = fmaxf(M0, __ldcg(a.part_ml + 2 * (u0 + sidx * ustep)));
-                M1 = fmaxf(M1, __ldcg(a.part_ml + 2 * (u1 + sidx * ustep)));
+        const int d = lane * 4;
+        for (int g0 = 0; g0 < G; g0 += GM) {
+            const int n_g = min(GM, G - g0);
+            // range s of head g0 + g: slot ((pref + s) * nkv + kvh) * G + g0 + g
+            const size_t u0 = (static_cast<size_t>(kr.pref[item]) * a.nkv + kvh) * G + g0;
+            float M[GM], L[GM];
+            float4 acc[GM];
+#pragma unroll
+            for (int g = 0; g < GM; ++g) {
+                M[g] = -INFINITY;
+                L[g] = 0.f;
+                acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            M0 = warp_max(M0);
-            M1 = warp_max(M1);
-            for (int d = lane * 4; d < HD; d += 128) {
-                float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
-                float L0 = 0.f, L1 = 0.f;
-#pragma unroll 8
-                for (int sidx = 0; sidx < n_splits; ++sidx) {
-                    const size_t us0 = u0 + sidx * ustep, us1 = u1 + sidx * ustep;
-                    const float2 ml0 = __ldcg(reinterpret_cast<const float2*>(a.part_ml + 2 * us0));
-                    const float2 ml1 = __ldcg(reinterpret_cast<const float2*>(a.part_ml + 2 * us1));
-                    const float4 v0 = __ldcg(reinterpret_cast<const float4*>(a.part_o + us0 * HD + d));
-                    const float4 v1 = __ldcg(reinterpret_cast<const float4*>(a.part_o + us1 * HD + d));
-                    const float w0 = ml0.x == -INFINITY ? 0.f : exp2f(ml0.x - M0);
-                    const float w1 = ml1.x == -INFINITY ? 0.f : exp2f(ml1.x - M1);
-                    L0 = fmaf(ml0.y, w0, L0);
-                    L1 = fmaf(ml1.y, w1, L1);
-                    acc0.x = fmaf(v0.x, w0, acc0.x); acc0.y = fmaf(v0.y, w0, acc0.y);
-                    acc0.z = fmaf(v0.z, w0, acc0.z); acc0.w = fmaf(v0.w, w0, acc0.w);
-                    acc1.x = fmaf(v1.x, w1, acc1.x); acc1.y = fmaf(v1.y, w1, acc1.y);
-                    acc1.z = fmaf(v1.z, w1, acc1.z); acc1.w = fmaf(v1.w, w1, acc1.w);
+            for (int sidx = lane; sidx < n_splits; sidx += 32)
+#pragma unroll
+                for (int g = 0; g < GM; ++g)
+                    if (g < n_g) M[g] = fmaxf(M[g], __ldcg(a.part_ml + 2 * (u0 + g + sidx * ustep)));
+#pragma unroll
+            for (int g = 0; g < GM; ++g) M[g] = warp_max(M[g]);
+            for (int s0 = 0; s0 < n_splits; s0 += 32) {
+                float w[GM], l[GM];   // of range s0 + lane
+#pragma unroll
+                for (int g = 0; g < GM; ++g) {
+                    w[g] = l[g] = 0.f;
+                    if (g < n_g && s0 + lane < n_splits) {
+                        const float2 ml = __ldcg(reinterpret_cast<const float2*>(a.part_ml + 2 * (u0 + g + (s0 + lane) * ustep)));
+                        w[g] = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M[g]);
+                        l[g] = ml.y;
+                    }
                 }
+                const int n = min(32, n_splits - s0);
+                const float* po = a.part_o + (u0 + s0 * ustep) * HD + (d < HD ? d : 0);
+                for (int j = 0; j < n; j += 4) {   // the rows of four ranges are on their way together
+                    float4 v[4][GM];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int g = 0; g < GM; ++g)
+                            v[k][g] = j + k < n && g < n_g ? __ldcg(reinterpret_cast<const float4*>(po + ((j + k) * ustep + g) * HD))
+                                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (j + k >= n) break;
+#pragma unroll
+                        for (int g = 0; g < GM; ++g) {
+                            const float wj = __shfl_sync(0xffffffffu, w[g], j + k);
+                            L[g] = fmaf(__shfl_sync(0xffffffffu, l[g], j + k), wj, L[g]);
+                            acc[g].x = fmaf(v[k][g].x, wj, acc[g].x);
+                            acc[g].y = fmaf(v[k][g].y, wj, acc[g].y);
+                            acc[g].z = fmaf(v[k][g].z, wj, acc[g].z);
+                            acc[g].w = fmaf(v[k][g].w, wj, acc[g].w);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < GM; ++g) {
+                if (g >= n_g || d >= HD) break;
                 // (the sink: one more term of score 0; scores are in base 2 here)
-                const int h0 = kvh * G + g, h1 = h0 + (two ? 1 : 0);
-                const float inv0 = 1.0f / (a.sink ? L0 + sink_term2(a.sink_val, h0, M0) : L0);
-                const float inv1 = 1.0f / (a.sink ? L1 + sink_term2(a.sink_val, h1, M1) : L1);
-                bf16* dst = a.out + (static_cast<size_t>(row) * a.nh + static_cast<size_t>(kvh) * G + g) * HD + d;
-                dst[0] = from_f<bf16>(acc0.x * inv0);
-                dst[1] = from_f<bf16>(acc0.y * inv0);
-                dst[2] = from_f<bf16>(acc0.z * inv0);
-                dst[3] = from_f<bf16>(acc0.w * inv0);
-                if (two) {
-                    dst[HD] = from_f<bf16>(acc1.x * inv1);
-                    dst[HD + 1] = from_f<bf16>(acc1.y * inv1);
-                    dst[HD + 2] = from_f<bf16>(acc1.z * inv1);
-                    dst[HD + 3] = from_f<bf16>(acc1.w * inv1);
-                }
+                const int h = kvh * G + g0 + g;
+                const float inv = 1.0f / (a.sink ? L[g] + sink_term2(a.sink_val, h, M[g]) : L[g]);
+                bf16* dst = a.out + (static_cast<size_t>(row) * a.nh + h) * HD + d;
+                dst[0] = from_f<bf16>(acc[g].x * inv);
+                dst[1] = from_f<bf16>(acc[g].y * inv);
+                dst[2] = from_f<bf16>(acc[g].z * inv);
+                dst[3] = from_f<bf16>(acc[g].w * inv);
             }
         }
     }
