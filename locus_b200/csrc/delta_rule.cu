@@ -11,18 +11,20 @@
 // k . q, u = beta (v - g a) and o = g b + u (k . q).  So a token costs one round of sums across lanes, not two in a row.
 //
 //   delta_walk   for portions.  A block of eight warps owns 16 columns of one head's state for one request and walks the
-//                request's new tokens eight at a time, the state in registers (walk.cuh says which lane holds what).  The
-//                sums a_t and b_t of eight tokens are all taken against the state in front of the eight, so that they cross
+//                request's new tokens four at a time, the state in registers (walk.cuh says which lane holds what).  The
+//                sums a_t and b_t of four tokens are all taken against the state in front of the four, so that they cross
 //                the row groups together, once, and what a token's write adds to the later ones is a number per pair of
-//                tokens: with G_t = g_0 .. g_t within the eight,
+//                tokens: with G_t = g_0 .. g_t within the four,
 //                    u_t = beta_t v_t - beta_t G_t a_t - beta_t sum_(j < t) (g_(j+1) .. g_t) (k_j . k_t) u_j
 //                    o_t = G_t b_t + sum_(j <= t) (g_(j+1) .. g_t) (k_j . q_t) u_j
-//                    S  <- G_7 S + sum_j (g_(j+1) .. g_7) k_j u_j^T
+//                    S  <- G_3 S + sum_j (g_(j+1) .. g_3) k_j u_j^T
 //                (products of decays only, nothing is divided).  The pairs' numbers are formed once per block for 16
 //                tokens, two threads to a pair; q, k, v, beta and the decays of 16 tokens are copied into shared memory
 //                together, asynchronously, two tiles ahead.  One token at a time with a warp's own fetch one token ahead,
 //                a token took 385 ns (one request of 2,048 tokens, 16 heads of 128 x 128: 788 us, eight such requests 4,470 us): a
-//                chain of fetch, sums, three exchanges and update that the next token waited for.  Now 454 and 2,400 us.
+//                chain of fetch, sums, three exchanges and update that the next token waited for.  Now 440 and 2,030 us, three
+//                requests of 700 tokens 308.  (Eight tokens together: 454, 2,400 and 379 us: fewer crossings, but two
+//                blocks an SM instead of three.)
 //   delta_tokens for steps of few tokens a request (decoding): 16 columns of a head and 8 groups of rows to a block, so that
 //                a row of the state is read and written in whole sectors (64 requests: 51 -> 28 us).
 //   delta_out    a head's read-out divided by its root mean square, times a weight, times silu(gate).
@@ -47,8 +49,8 @@ struct DeltaArgs {
 
 #define DR_STAGES 3
 #define DR_TT 16       // tokens of a tile
-#define DR_G 8         // tokens that are worked on together
-// numbers of eight tokens: beta G, G, E, beta (8 each); then rows 1 .. 7 of L, then rows 0 .. 7 of P (8 each)
+#define DR_G 4         // tokens that are worked on together
+// numbers of four tokens: beta G, G, E, beta (4 each); then rows 1 .. 3 of L, then rows 0 .. 3 of P (4 each)
 #define DR_L (4 * DR_G)
 #define DR_P (DR_L + DR_G * (DR_G - 1))
 #define DR_COEF (DR_P + DR_G * DR_G)
@@ -56,12 +58,12 @@ struct DeltaArgs {
 // RPL: rows of a column that a lane keeps, of two columns (d <= 32 RPL).  VEC: q's and k's rows of a head start on 16-byte
 // boundaries and d is a multiple of 4, so four rows are one copy.
 template <int RPL, bool VEC>
-__global__ void __launch_bounds__(32 * WALK_WARPS) delta_walk_kernel(const DeltaArgs a, int col_blocks) {
+__global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) delta_walk_kernel(const DeltaArgs a, int col_blocks) {
     constexpr int DP = 32 * RPL, LD = DP + 8, TT = DR_TT, CB = WALK_CW * WALK_WARPS, NT = 32 * WALK_WARPS;
     constexpr int RV = RPL < 4 ? RPL : 4;          // rows of a load
     constexpr int TILE = TT * (2 * LD + CB + 2);   // q, k: [TT][LD]; v: [TT][CB]; beta, decay: [TT]
     extern __shared__ __align__(16) float walk_smem[];   // [DR_STAGES][TILE], then [TT / DR_G][DR_COEF]
-    __shared__ __align__(16) f2 writes[WALK_WARPS][DR_G][WALK_CW];   // a warp's u of eight tokens, each twice
+    __shared__ __align__(16) f2 writes[WALK_WARPS][DR_G][WALK_CW];   // a warp's u of four tokens, each twice
     float* coef = walk_smem + DR_STAGES * TILE;
     pdl_entry();
     pdl_trigger();
@@ -127,15 +129,17 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) delta_walk_kernel(const Delta
             s[j][i] = f2_pack((r < d && col + j < dv) ? S[static_cast<size_t>(r) * dv + col + j] : 0.f,
                               (r + 1 < d && col + j < dv) ? S[static_cast<size_t>(r + 1) * dv + col + j] : 0.f);
         }
-    // The pair of tokens j <= t of the eight that this thread's half of a sum belongs to: of the 64 pairs of a group, 28
-    // k_j . k_t (j < t) and 36 k_j . q_t; pair p is (row p & 7, column p >> 3): j and t of k_j . q_t where row <= column, and
-    // elsewhere t and j of k_j . k_t.
-    const int half = tid & 1, pair = (tid >> 1) & 63, group = tid >> 7;
-    const bool with_q = (pair & 7) <= (pair >> 3);
-    const int pj = with_q ? pair & 7 : pair >> 3, pt = with_q ? pair >> 3 : pair & 7;
-    // of the 32 sums (a or b, token, column) of eight tokens, the one that this lane ends up with
-    const int mine = walk_sum_index<32>(lane), my_t = (mine >> 1) & 7, my_c = mine & 1;
-    const bool my_b = mine & 16;
+    // The pair of tokens j <= t of the four that this thread's half of a sum belongs to: of the 16 pairs of a group, 6
+    // k_j . k_t (j < t) and 10 k_j . q_t; a pair is (row, column): j and t of k_j . q_t where row <= column, and elsewhere t
+    // and j of k_j . k_t.
+    constexpr int PAIRS = DR_G * DR_G;
+    const int half = tid & 1, pair = (tid >> 1) % PAIRS, group = tid / (2 * PAIRS);
+    const int pr = pair % DR_G, pc = pair / DR_G;
+    const bool with_q = pr <= pc;
+    const int pj = with_q ? pr : pc, pt = with_q ? pc : pr;
+    // of the 16 sums (a or b, token, column) of four tokens, the one that this lane ends up with
+    const int mine = walk_sum_index<4 * DR_G>(lane), my_t = (mine >> 1) % DR_G, my_c = mine & 1;
+    const bool my_b = mine >= 2 * DR_G;
     for (int tile = 0; tile < n_tiles; ++tile) {
         walk_wait<DR_STAGES - 2>();
         __syncthreads();   // the tile is there for all warps, and nobody reads the buffer and the numbers that are written next
@@ -145,7 +149,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) delta_walk_kernel(const Delta
         const float* ks = qs + TT * LD;
         const float* vs = ks + TT * LD;
         const float* bs = vs + TT * CB;
-        {   // (rows LD = DP + 8 floats apart and the halves of a sum four floats apart meet in no bank)
+        if (group < TT / DR_G) {   // (rows LD = DP + 8 floats apart and the halves of a sum four floats apart meet in no bank)
             const float* x = ks + (DR_G * group + pj) * LD + 4 * half;
             const float* y = (with_q ? qs : ks) + (DR_G * group + pt) * LD + 4 * half;
             float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) delta_walk_kernel(const Delta
             }
             float dot = (d0 + d1) + (d2 + d3);
             dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-            float w = 1.f, before = 1.f, behind = 1.f;   // g_(j+1) .. g_t; g_0 .. g_t; g_(t+1) .. g_7
+            float w = 1.f, before = 1.f, behind = 1.f;   // g_(j+1) .. g_t; g_0 .. g_t; g_(t+1) .. g_3
 #pragma unroll
             for (int i = 0; i < DR_G; ++i) {
                 const float gi = tile * TT + DR_G * group + i < qn ? bs[TT + DR_G * group + i] : 1.f;
@@ -218,28 +222,30 @@ __global__ void __launch_bounds__(32 * WALK_WARPS) delta_walk_kernel(const Delta
                     sums[2 * DR_G + 2 * t + j] = e + f;
                 }
             }
-            const float sum = walk_sum<32>(sums, lane);
-            // u of the eight tokens, of this lane's column, by every lane: a of token t comes from the lane that ended up with it
+            const float sum = walk_sum<4 * DR_G>(sums, lane);
+            // u of the four tokens, of this lane's column, by every lane: a of token t comes from the lane that ended up with it
             auto four = [&](int at) { return *reinterpret_cast<const float4*>(c + at); };
             float u[DR_G];
             const float* vp = vs + t0 * CB + wc + my_c;
 #pragma unroll
             for (int t = 0; t < DR_G; t += 4) {
                 const float4 bG = four(t), be = four(3 * DR_G + t);
-                auto a_of = [&](int i) { return __shfl_sync(0xffffffffu, sum, walk_sum_index<32>(2 * (t + i) + my_c)); };
+                auto a_of = [&](int i) { return __shfl_sync(0xffffffffu, sum, walk_sum_index<4 * DR_G>(2 * (t + i) + my_c)); };
                 u[t] = fmaf(-bG.x, a_of(0), be.x * vp[t * CB]);
                 u[t + 1] = fmaf(-bG.y, a_of(1), be.y * vp[(t + 1) * CB]);
                 u[t + 2] = fmaf(-bG.z, a_of(2), be.z * vp[(t + 2) * CB]);
                 u[t + 3] = fmaf(-bG.w, a_of(3), be.w * vp[(t + 3) * CB]);
             }
-            const float4 p0 = four(DR_P + DR_G * my_t), p1 = four(DR_P + DR_G * my_t + 4);
-            const float p[DR_G] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            float p[DR_G];
+#pragma unroll
+            for (int t = 0; t < DR_G; t += 4) *reinterpret_cast<float4*>(p + t) = four(DR_P + DR_G * my_t + t);
             float o = c[DR_G + my_t] * sum;
 #pragma unroll
             for (int t = 0; t < DR_G; ++t) {
                 if (t > 0) {
-                    const float4 l0 = four(DR_L + DR_G * (t - 1)), l1 = t > 4 ? four(DR_L + DR_G * (t - 1) + 4) : l0;
-                    const float l[DR_G] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+                    float l[DR_G];
+#pragma unroll
+                    for (int j = 0; j < t; j += 4) *reinterpret_cast<float4*>(l + j) = four(DR_L + DR_G * (t - 1) + j);
 #pragma unroll
                     for (int j = 0; j < t; ++j) u[t] = fmaf(l[j], u[j], u[t]);
                 }
@@ -363,7 +369,7 @@ template <int RPL>
 static int delta_walk(const DeltaArgs& a, bool vec, int n_seg, cudaStream_t stream) {
     constexpr int CB = WALK_CW * WALK_WARPS;
     constexpr size_t smem = sizeof(float) * (DR_STAGES * DR_TT * (2 * (32 * RPL + 8) + CB + 2) + DR_TT / DR_G * DR_COEF);
-    static_assert(DR_TT / DR_G * 128 == 32 * WALK_WARPS, "two threads to a pair of tokens");
+    static_assert(DR_TT / DR_G * 2 * DR_G * DR_G <= 32 * WALK_WARPS, "two threads to a pair of tokens");
     const int col_blocks = (a.dv + CB - 1) / CB;
     auto* kernel = vec ? delta_walk_kernel<RPL, true> : delta_walk_kernel<RPL, false>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

@@ -16,7 +16,7 @@
 //               a walk is not the recurrence -- two dependent multiply-adds a token -- but its operands: with each warp
 //               fetching a token ahead by itself a token took 700 ns behind a product that had left the operands in
 //               DRAM and the far L2 (2,048 tokens of 16 heads of 128 x 128: 1,433 us inside the mixer).  So 16 tokens
-//               of q, k and the decays are copied into shared memory together, asynchronously, two tiles ahead, by all
+//               of q, k and the decays are copied into shared memory together, asynchronously, a tile ahead, by all
 //               warps for all, and the read-outs of eight tokens cross the lanes together: 259 us alone (745 before, the operands
 //               in L2) and about as long inside the mixer, whose pass went from 1,613 to 428 us.
 //   gla_tokens  for steps of few tokens a request (decoding): 16 columns of a head and 8 groups of rows to a block, so that
@@ -44,13 +44,13 @@ struct GlaArgs {
     float q_scale;
 };
 
-#define GL_STAGES 3
+#define GL_STAGES 2   // (three: two blocks an SM instead of three, 1,390 us for eight requests of 2,048 tokens, not 1,290)
 #define GL_TT 16   // tokens of a tile
 
 // RPL: rows of a column that a lane keeps, of two columns (d <= 32 RPL).  VEC: the rows of q, k and a of a head start on
 // 16-byte boundaries and d is a multiple of 4, so four rows are one copy.
 template <int RPL, bool VEC>
-__global__ void __launch_bounds__(32 * WALK_WARPS, 2) gla_walk_kernel(const GlaArgs a, int col_blocks) {
+__global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) gla_walk_kernel(const GlaArgs a, int col_blocks) {
     constexpr int DP = 32 * RPL, CB = WALK_CW * WALK_WARPS, TT = GL_TT, TILE = TT * (3 * DP + 2 * CB), NT = 32 * WALK_WARPS;
     constexpr int RV = RPL < 4 ? RPL : 4;                // rows of a load
     extern __shared__ __align__(16) float walk_smem[];   // [GL_STAGES][q, k, a: [TT][DP]; v: [TT][CB], every value twice]
