@@ -18,7 +18,8 @@
 // lanes x 2 x 1.965 GHz = 74.4 TFLOP/s), so everything else is kept off their issue slots: 32 columns of k of 64 rows
 // and 128 weight rows are copied into shared memory asynchronously, two stages ahead, k contiguous as they lie in memory (rows
 // 36 floats apart meet in no bank), a thread owns 8 x 8 outputs, and a multiply-add works on two k at once, so each
-// output has a sum over the even k and one over the odd k, added at the end -- in the same order whatever the tile.  A
+// output has a sum over the even k and one over the odd k, added at the end -- in the same order whatever the tile; a product
+// whose blocks would leave SMs idle is cut along k, its parts added up in order by a second kernel.  A
 // tile's rows are worked on in eights, so that an expert's 34 rows cost 40 and not 64.  gemm_simt: every other type,
 // width and alignment.  Measured: 2,048 x
 // 6,144 x 2,048 1.18 ms = 43.8 TFLOP/s (20 before, with the 64 x 64 x 16 tiles of gemm_simt), 512 x 6,144 x 2,048 343 us, the
@@ -58,6 +59,9 @@ struct GemmArgs {
     const int* tile_rows;
     const int* n_tiles;
     long long w_expert_stride;
+    // gemm_f32, plain products cut along K: [splits][M][N] sums that gemm_f32_sum adds up in order (null: not cut)
+    float* part;
+    int splits;
 };
 
 // One output: activation, bias, row scale (rs), softcap, store.  v2: the second weight's sum.
@@ -238,10 +242,11 @@ __global__ void __launch_bounds__(8 * TX) gemm_f32_kernel(GemmArgs a) {
         const int r = row0 + lrow + i * PER;
         xrow[i] = lrow + i * PER >= rows ? -1 : a.x_rows ? a.x_rows[r] / a.x_row_div : r;
     }
-    const int n_k = (a.K + FK - 1) / FK, live_rows = (rows + 7) & ~7;
+    const int n_all = (a.K + FK - 1) / FK, per_split = (n_all + a.splits - 1) / a.splits;
+    const int kb0 = blockIdx.z * per_split, n_k = min(per_split, n_all - kb0), live_rows = (rows + 7) & ~7;
     auto fetch = [&](int kb) {   // columns behind K and rows that are not there are zeros
         float* st = f32_smem + (kb % F_STAGES) * STAGE + lrow * FLD + chunk;
-        const int k = kb * FK + chunk;
+        const int k = (kb0 + kb) * FK + chunk;
         const bool in = k < a.K;
 #pragma unroll
         for (int i = 0; i < FM / PER; ++i)
@@ -296,21 +301,33 @@ __global__ void __launch_bounds__(8 * TX) gemm_f32_kernel(GemmArgs a) {
             float even, odd, even2 = 0.f, odd2 = 0.f;
             f2_unpack(acc[i][j], even, odd);
             if (SWIGLU) f2_unpack(acc[i][j + 4], even2, odd2);
-            epilogue<SWIGLU>(a, r, n, rs, even + odd, even2 + odd2);
+            if (!SWIGLU && a.part) a.part[(static_cast<size_t>(blockIdx.z) * a.M + r) * a.N + n] = even + odd;
+            else epilogue<SWIGLU>(a, r, n, rs, even + odd, even2 + odd2);
         }
     }
+}
+
+// The sums of a product cut along K, in order, and its epilogue.
+__global__ void __launch_bounds__(256) gemm_f32_sum_kernel(GemmArgs a) {
+    const int n = blockIdx.x * 256 + threadIdx.x, r = blockIdx.y;
+    if (n >= a.N) return;
+    float v = 0.f;
+    for (int z = 0; z < a.splits; ++z) v += a.part[(static_cast<size_t>(z) * a.M + r) * a.N + n];
+    const float rs = a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
+    epilogue<false>(a, r, n, rs, v, 0.f);
 }
 
 template <int TX>
 static int launch_f32(const GemmArgs& a, int tiles, bool swiglu, cudaStream_t stream) {
     constexpr size_t smem = sizeof(float) * F_STAGES * (FM + 8 * TX) * FLD;
-    const dim3 grid(ceil_div(a.N, swiglu ? 4 * TX : 8 * TX), tiles);
+    const dim3 grid(ceil_div(a.N, swiglu ? 4 * TX : 8 * TX), tiles, a.splits);
     if (grid.y == 0 || grid.x == 0) return 0;
     if (grid.y > 65535) return LOCUS_ERR_UNSUPPORTED;
     auto* kernel = swiglu ? gemm_f32_kernel<TX, true> : gemm_f32_kernel<TX, false>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     kernel<<<grid, 8 * TX, smem, stream>>>(a);
+    if (a.part) gemm_f32_sum_kernel<<<dim3(ceil_div(a.N, 256), a.M), 256, 0, stream>>>(a);
     return locus_launch_status();
 }
 
@@ -331,7 +348,8 @@ static int launch(const GemmArgs& a, int max_tiles, bool swiglu, cudaStream_t st
 // bits 1-3 = the activation: 1 squared ReLU (not with W2), 2 the clamped gated unit with limit act_param (with W2),
 // 3 act_param tanh(act_scale v / act_param) (not with W2), 4 relu(x . W + b) (x . W2 + b2) (with W2; bias is then [2N], b and
 // behind it b2, or null).  max_tiles: number of 64-row tiles
-// to launch; for a grouped product an upper bound (tiles past *n_tiles return at once).
+// to launch; for a grouped product an upper bound (tiles past *n_tiles return at once).  part, splits: a plain product of
+// one weight that gemm_f32 takes may be cut along K into splits (2 .. 8) whose sums, splits * M * N floats, part holds; else null, 1.
 extern "C" int locus_gemm_simt(const void* x, int x_dt, const void* w, const void* w2, int w_dt,
                                const void* bias, int bias_dt, void* out, int out_dt,
                                int flags, float act_param, float act_scale, const float* row_scale, const int* scale_rows,
@@ -339,7 +357,7 @@ extern "C" int locus_gemm_simt(const void* x, int x_dt, const void* w, const voi
                                int x_row_div, int M, int N, int K, long long ldx, long long ldo,
                                const int* tile_expert, const int* tile_row0,
                                const int* tile_rows, const int* n_tiles, int max_tiles,
-                               long long w_expert_stride, cudaStream_t stream) {
+                               long long w_expert_stride, float* part, int splits, cudaStream_t stream) {
     if (N <= 0 || K <= 0) return LOCUS_ERR_UNSUPPORTED;
     const int accumulate = flags & 1, act = (flags >> 1) & 7;
     if ((act == 1 && w2 != nullptr) || ((act == 2 || act == 4) && w2 == nullptr) || act > 4 || (act == 3 && (w2 != nullptr || !(act_param > 0.f)))) return LOCUS_ERR_UNSUPPORTED;
@@ -350,16 +368,18 @@ extern "C" int locus_gemm_simt(const void* x, int x_dt, const void* w, const voi
     a.out_dt = out_dt; a.accumulate = accumulate; a.act = act; a.act_param = act_param; a.act_scale = act_scale; a.row_scale = row_scale; a.scale_rows = scale_rows; a.x_rows = x_rows;
     a.x_row_div = x_row_div; a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldo = ldo;
     a.tile_expert = tile_expert; a.tile_row0 = tile_row0; a.tile_rows = tile_rows;
-    a.n_tiles = n_tiles; a.w_expert_stride = w_expert_stride;
+    a.n_tiles = n_tiles; a.w_expert_stride = w_expert_stride; a.part = splits > 1 ? part : nullptr; a.splits = splits > 1 ? splits : 1;
     const int tiles = tile_expert ? max_tiles : ceil_div(M, BM);
     const bool swiglu = w2 != nullptr;
     static_assert(FM == BM, "the grouped tile lists serve both kernels");
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32 && ((K | ldx) & 3) == 0 &&
         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w2)) & 15) == 0) {
+        if (splits > 1 && (part == nullptr || splits > 8 || swiglu || tile_expert != nullptr || M > 65535)) return LOCUS_ERR_UNSUPPORTED;
         // tiles of 64 weight rows where tiles of 128 would leave SMs without one
-        const long long wide = static_cast<long long>(ceil_div(N, swiglu ? 64 : 128)) * tiles;
+        const long long wide = static_cast<long long>(ceil_div(N, swiglu ? 64 : 128)) * tiles * a.splits;
         return wide < 148 ? launch_f32<8>(a, tiles, swiglu, stream) : launch_f32<16>(a, tiles, swiglu, stream);
     }
+    if (splits > 1) return LOCUS_ERR_UNSUPPORTED;
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32) return launch<float, float>(a, tiles, swiglu, stream);
     if (x_dt == LOCUS_DT_BF16 && w_dt == LOCUS_DT_BF16) return launch<bf16, bf16>(a, tiles, swiglu, stream);
     if (x_dt == LOCUS_DT_BF16 && w_dt == LOCUS_DT_F32) return launch<bf16, float>(a, tiles, swiglu, stream);

@@ -464,6 +464,26 @@ def tc_plan(m: int, n: int, k: int, dual: bool) -> Tuple[int, int]:
     return best
 
 
+def f32_splits(m: int, n: int, k: int) -> int:
+    """Parts along K of a plain float32 product on tiles of 64 rows x 128 weight rows, two blocks an SM.  A round of blocks in
+    which an SM has two takes about 3.6 us for every 32 columns of k, one of at most a block an SM 2.0, and a second kernel
+    adds the parts up, so what counts is how full the last round is.  Measured, whole and as cut: 512 rows of 2,048 x 5,632 360
+    and 302 us in 8, of 6,144 x 2,048 369 and 335 in 3; 64 rows of it 139 and 63 in 6; 100 rows of 2,048 x 2,048 137 and 49 in 8."""
+    n_sm = _sm_count()
+    tiles, stages = -(-m // 64) * -(-n // 128), -(-k // 32)
+    best, best_cost = 1, None
+    for s in range(1, 9):
+        if s > 1 and (stages < 8 * s or 4 * s * m * n > SPLIT_SCRATCH_BYTES or m > 65535):
+            break
+        full, rest = divmod(tiles * s, 2 * n_sm)
+        cost = -(-stages // s) * (3.6 * full + (0.0 if rest == 0 else 2.0 if rest <= n_sm else 3.6))
+        if s > 1:
+            cost += 6.0 + s * m * n * 8 / 5e6
+        if best_cost is None or cost < 0.98 * best_cost:
+            best, best_cost = s, cost
+    return best
+
+
 def _split_scratch(device) -> torch.Tensor:
     """The partial sums' buffer of the stream that launches: products on different streams (the shared expert
     beside the routed ones) must not share one.  Made at a stream's first split product, which is never inside
@@ -639,14 +659,20 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         te = t0 = tr = nt = None
         max_tiles = 0
         stride = 0
+    splits = 1
+    if (layout is None and w2 is None and x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
+            and (x.data_ptr() | w.data_ptr()) % 16 == 0):
+        splits = f32_splits(M, N, K)
     code = _lib("gemm_simt").locus_gemm_simt(
         _p(x), I(dtype_code(x.dtype)), _p(w), _p(w2), I(dtype_code(w.dtype)), _p(bias),
         I(dtype_code(bias.dtype) if bias is not None else 0), _p(out), I(dtype_code(out.dtype)),
         flags, F(act_limit), F(act_scale), _p(row_scale), _p(scale_rows), _p(x_rows), I(x_row_div), I(M), I(N), I(K),
         LL(x.stride(0)), LL(out.stride(0)), _p(te), _p(t0), _p(tr), _p(nt), I(max_tiles), LL(stride),
-        _stream()
+        _p(_split_scratch(x.device) if splits > 1 else None), I(splits), _stream()
     )
-    _check(code, "linear", f"(M={M}, N={N}, K={K}, x {x.dtype}, w {w.dtype})")
+    if splits > 1 and code == 0:
+        _count_launches(1)   # the kernel that adds the parts up
+    _check(code, "linear", f"(M={M}, N={N}, K={K}, x {x.dtype}, w {w.dtype}, {splits} splits)")
 
 
 def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor],

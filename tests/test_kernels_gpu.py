@@ -565,6 +565,19 @@ def test_linear_float32_tiles(M, N, K_, dual):
     close(out, ref, torch.float32, f"linear {M} x {N} x {K_} dual={dual}")
 
 
+@pytest.mark.parametrize("splits", [2, 3, 8])
+def test_linear_float32_cut_along_k(splits, monkeypatch):
+    """Parts of unequal length (the last one shorter, or without a column), and the epilogue behind their sum."""
+    monkeypatch.setattr(K, "f32_splits", lambda m, n, k: splits)
+    for M, N, K_ in ((70, 133, 2052), (40, 64, 32 * 9), (33, 20, 4)):
+        x, w, b, old, rs = rnd(M, K_, seed=1), rnd(N, K_, seed=2), rnd(N, seed=3), rnd(M, N, seed=4), rnd(M, seed=5)
+        out = old.to(DEV)
+        before = K.launches
+        K.linear(x.to(DEV), w.to(DEV), out, bias=b.to(DEV), accumulate=True, row_scale=rs.to(DEV))
+        assert K.launches - before == 2
+        close(out, old.double() + (x.double() @ w.double().T + b.double()) * rs.double()[:, None], torch.float32, f"{splits} parts of {K_}")
+
+
 @pytest.mark.parametrize("nh,nkv,P,window", [(2, 2, 64, 0), (4, 1, 128, 0), (3, 3, 64, 100), (2, 1, 64, 1), (4, 2, 192, 333)])
 def test_attn_chunk_tcgen05(nh, nkv, P, window):
     """Portions of 2 to 450 tokens at contexts that straddle the 128-key tiles and the pages; whatever lies
