@@ -183,7 +183,8 @@ def bench_attn_chunk(args) -> None:
     T, ctx = args.tokens, args.ctx
     pool, q, out, meta, kw, i32 = _paged(args, 1, ctx, T)
     mma = K.attn_chunk_mma_takes(q, args.head_dim) and not args.cuda_cores
-    tile = K.MMA_QUERY_TILE if mma else 16
+    f32 = K.attn_chunk_f32_takes(q, args.head_dim)
+    tile = K.MMA_QUERY_TILE if mma or f32 else 16
     items = torch.tensor([(0, o) for o in range(0, T, tile)], dtype=torch.int32, device="cuda:0")
 
     tc = mma and not args.mma_sync and K.attn_chunk_tc_takes(q, args.head_dim, args.page_tokens, T, ctx + T)
@@ -195,14 +196,14 @@ def bench_attn_chunk(args) -> None:
         if n_splits > 1:
             n_o, n_ml = T * args.heads * n_splits * args.head_dim, T * args.heads * n_splits * 2
             extra = dict(n_splits=n_splits, part_o=torch.empty(n_o, device="cuda:0"), part_ml=torch.empty(n_ml, device="cuda:0"))
-    elif mma:
+    elif mma or f32:
         n_splits = K.attn_chunk_mma_splits(items.shape[0], args.heads, ctx + T) if args.key_ranges < 0 else args.key_ranges
         if n_splits > 1:
             n_o, n_ml = K.attn_chunk_mma_scratch(args.head_dim)
             extra = dict(n_splits=n_splits, part_o=torch.empty(n_o, device="cuda:0"), part_ml=torch.empty(n_ml, device="cuda:0"))
 
     def fn():
-        call = K.attn_chunk_tc if tc else (K.attn_chunk_mma if mma else K.attn_chunk)
+        call = K.attn_chunk_tc if tc else (K.attn_chunk_mma if mma else K.attn_chunk_f32 if f32 else K.attn_chunk)
         call(q, pool, out, items=items, n_items=items.shape[0], **meta, **kw, **extra)
 
     us = _time(fn, args.iters, args.graph)
@@ -212,7 +213,7 @@ def bench_attn_chunk(args) -> None:
     flops = 4.0 * args.heads * args.head_dim * seen
     print(f"attn_chunk tokens={T} ctx={ctx} heads={args.heads}/{args.kv_heads} head_dim={args.head_dim} window={args.window} "
           f"keep_first={args.keep_first} sink={args.sink} slopes={args.slopes} "
-          f"{f'tcgen05, {n_splits} key ranges' if tc else (f'mma.sync, {n_splits} key ranges' if mma else 'cuda cores')}: {us:.1f} us/call  {flops / us / 1e6:.1f} TFLOP/s (causal flops)")
+          f"{f'tcgen05, {n_splits} key ranges' if tc else (f'mma.sync, {n_splits} key ranges' if mma else f'float32 tiles, {n_splits} key ranges' if f32 else 'cuda cores')}: {us:.1f} us/call  {flops / us / 1e6:.1f} TFLOP/s (causal flops)")
 
 
 def bench_recurrence(args) -> None:
