@@ -18,7 +18,8 @@
 // number following from N and K alone.  Measured at 8 rows: 151,936 x 2,048 264 us = 4.7 TB/s, 6,144 x 2,048 19.4 us (39.7
 // before), the routed experts of 8 tokens 141 us = 5.9 TB/s (192 before); 16 / 32 rows of 6,144 x 2,048 in tiles of 8, which
 // find the weights in L2, 36 / 71 us (163 on 64-row tiles).  One or two rows stay on the warp-per-row kernel (11.0 us
-// against 13.4 at one row).
+// against 13.4 at one row), and so do grouped products of up to 8 rows, whose few tiles hold a row each (a decode step of
+// one request, 24 layers of 60 experts with 4 picks: 3.20 ms against 3.49).
 #include "common.cuh"
 #include "walk.cuh"
 
@@ -379,7 +380,7 @@ extern "C" int locus_gemv(const void* x, int x_dt, const void* w, const void* w2
     const int tiles = tile_expert ? max_tiles : ceil_div(M, GV_ROWS);
     const bool dual = w2 != nullptr;
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32)
-        return tile_expert == nullptr && M <= 2 ? launch<float, float>(a, tiles, dual, stream) : launch_f32(a, tiles, dual, stream);
+        return M <= (tile_expert == nullptr ? 2 : 8) ? launch<float, float>(a, tiles, dual, stream) : launch_f32(a, tiles, dual, stream);
     if (x_dt == LOCUS_DT_BF16 && w_dt == LOCUS_DT_BF16) return launch<bf16, bf16>(a, tiles, dual, stream);
     if (x_dt == LOCUS_DT_BF16 && w_dt == LOCUS_DT_F32) return launch<bf16, float>(a, tiles, dual, stream);
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_BF16) return launch<float, bf16>(a, tiles, dual, stream);
