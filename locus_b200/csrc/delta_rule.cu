@@ -50,7 +50,7 @@ struct DeltaArgs {
 #define DR_STAGES 3
 #define DR_TT 16       // tokens of a tile
 #define DR_G 4         // tokens that are worked on together
-// numbers of four tokens: beta G, G, E, beta (4 each); then rows 1 .. 3 of L, then rows 0 .. 3 of P (4 each)
+// numbers of four tokens: beta G, G, E, beta (4 each); then rows 1 .. 3 of L, then rows 0 .. 3 of P (4 each, of row t the first t + 1)
 #define DR_L (4 * DR_G)
 #define DR_P (DR_L + DR_G * (DR_G - 1))
 #define DR_COEF (DR_P + DR_G * DR_G)
@@ -181,7 +181,6 @@ __global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) delta_walk_k
                 c[DR_G + pt] = before;
                 c[2 * DR_G + pt] = behind;
                 c[3 * DR_G + pt] = beta;
-                for (int j = pt + 1; j < DR_G; ++j) c[DR_P + DR_G * pt + j] = 0.f;
             }
         }
         __syncthreads();
@@ -250,7 +249,7 @@ __global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) delta_walk_k
                     for (int j = 0; j < t; ++j) u[t] = fmaf(l[j], u[j], u[t]);
                 }
                 if (t >= live) u[t] = 0.f;   // (a token that is not there writes nothing, whatever the state holds)
-                o = fmaf(p[t], u[t], o);
+                if (t <= my_t) o = fmaf(p[t], u[t], o);   // (not 0 * u behind it: a u that is not finite stays with its token and later ones)
             }
             if (my_b) {
                 const int tok = tile * TT + t0 + my_t;

@@ -253,6 +253,35 @@ def test_delta_rule_of_few_tokens_and_of_tiles_edges(heads, per_group, dim, v_di
         assert _close(out, out_w, 3e-5) and _close(state, st_w, 3e-5)
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("dim,v_dim", [(24, 16), (128, 20), (200, 16)])
+def test_delta_rule_keeps_what_is_not_finite_behind_its_token(dim, v_dim, bad):
+    """A value that is not finite reaches its own column from its token on: the tokens in front of it, also those that are
+    worked on together with it, and the other columns and requests have the bits that they have without it."""
+    import locus_b200.kernels as K
+
+    segs = [23, 40]
+    T, q0, qn = sum(segs), _dev([0, 23]), _dev(segs)
+    rows = _rand((T, 2 * dim + v_dim), 5, 0.3)
+    beta = torch.rand(T, 1, generator=torch.Generator().manual_seed(2)).cuda()
+    decay = torch.rand(T, 1, generator=torch.Generator().manual_seed(1)).cuda()
+
+    def run(r):
+        state, out = torch.zeros(2, dim * v_dim, device="cuda"), torch.zeros(T, v_dim, device="cuda")
+        K.delta_rule(r, 0, r, dim, r, 2 * dim, beta, decay, state, 0, _dev([0, 1]), q0, qn, 2, out, n_heads=1,
+                     heads_per_group=1, dim=dim, v_dim=v_dim)
+        return out
+
+    want = run(rows)
+    for t in (1, 2, 3, 6, 18):
+        r = rows.clone()
+        r[t, 2 * dim + 5] = bad
+        got = run(r)
+        assert not torch.isfinite(got[t:23, 5]).any()
+        got[t:23, 5] = want[t:23, 5]
+        assert torch.equal(got, want), t
+
+
 @pytest.mark.parametrize("odt", DTYPES, ids=IDS)
 @pytest.mark.parametrize("heads,v_dim,shared", [(2, 8, True), (3, 10, False), (1, 40, True), (4, 128, True)])
 def test_delta_output_stage_and_gate_rows_against_their_twins(heads, v_dim, shared, odt):
