@@ -297,18 +297,19 @@ __device__ __forceinline__ void f32_stream_body(const GemvArgs& a, const float* 
     gemv_store<DUAL>(a, r, n, rs, v, u);
 }
 
-// grid (tiles of 8 rows, blocks of weight rows): the tiles of the same weights run together, so that a second tile finds them in L2.
+// A flat grid, the tiles of 8 rows its fast index: the tiles of the same weights run together, so that a second tile finds them in
+// L2, and the blocks of weight rows have no limit of their own (65,535 of a second grid index would be 2.1 million rows).
 template <bool DUAL>
-__global__ void __launch_bounds__(32 * GV_WARPS, 2) f32_stream_kernel(GemvArgs a, int split) {
+__global__ void __launch_bounds__(32 * GV_WARPS, 2) f32_stream_kernel(GemvArgs a, int tiles, int split) {
     extern __shared__ __align__(16) float ring_smem[];   // [warp][stage][weight row][128]
     __shared__ float shares[GV_WARPS][GV_NC * GV_ROWS];
     const float* W = static_cast<const float*>(a.w);
     const float* W2 = static_cast<const float*>(a.w2);
     int row0, rows;
     const bool grouped = a.tile_expert != nullptr;
+    const int tile = blockIdx.x % tiles, block = blockIdx.x / tiles;
     if (grouped) {
         pdl_entry();   // (the lists come from the kernels in front)
-        const int tile = blockIdx.x;
         if (tile >= *a.n_tiles) return;
         const long long e = a.tile_expert[tile];
         row0 = a.tile_row0[tile];
@@ -316,11 +317,11 @@ __global__ void __launch_bounds__(32 * GV_WARPS, 2) f32_stream_kernel(GemvArgs a
         W += e * a.w_expert_stride;
         if (DUAL) W2 += e * a.w_expert_stride;
     } else {
-        row0 = blockIdx.x * GV_ROWS;
+        row0 = tile * GV_ROWS;
         rows = min(GV_ROWS, a.M - row0);
     }
     const int wid = threadIdx.x >> 5;
-    const int n0 = (blockIdx.y * (GV_WARPS / split) + wid / split) * (DUAL ? GV_NC / 2 : GV_NC);
+    const int n0 = (block * (GV_WARPS / split) + wid / split) * (DUAL ? GV_NC / 2 : GV_NC);
     float* ring = ring_smem + wid * GV_STAGES * GV_NC * 128 + (threadIdx.x & 31) * 4;
     if (rows <= 2) f32_stream_body<2, DUAL>(a, W, W2, row0, rows, n0, wid % split, split, !grouped, ring, shares);
     else if (rows <= 4) f32_stream_body<4, DUAL>(a, W, W2, row0, rows, n0, wid % split, split, !grouped, ring, shares);
@@ -331,14 +332,14 @@ static int launch_f32(const GemvArgs& a, int tiles, bool dual, cudaStream_t stre
     const int groups = ceil_div(a.N, dual ? GV_NC / 2 : GV_NC);   // four weight rows each
     int split = 1;
     while (a.tile_expert == nullptr && split < GV_WARPS && groups * split < 5000 && a.K >= 256 * split) split *= 2;
-    const dim3 grid(tiles, ceil_div(groups, GV_WARPS / split));
-    if (grid.x == 0 || grid.y == 0) return 0;
-    if (grid.y > 65535) return LOCUS_ERR_UNSUPPORTED;
+    const long long blocks = static_cast<long long>(tiles) * ceil_div(groups, GV_WARPS / split);
+    if (blocks == 0) return 0;
+    if (blocks > 0x7fffffffLL) return LOCUS_ERR_UNSUPPORTED;
     constexpr size_t smem = sizeof(float) * GV_WARPS * GV_STAGES * GV_NC * 128;
     auto* kernel = dual ? f32_stream_kernel<true> : f32_stream_kernel<false>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    locus_launch(kernel, grid, dim3(32 * GV_WARPS), smem, stream, a, split);
+    locus_launch(kernel, dim3(static_cast<unsigned>(blocks)), dim3(32 * GV_WARPS), smem, stream, a, tiles, split);
     return locus_launch_status();
 }
 

@@ -565,6 +565,18 @@ def test_linear_float32_tiles(M, N, K_, dual):
     close(out, ref, torch.float32, f"linear {M} x {N} x {K_} dual={dual}")
 
 
+@pytest.mark.parametrize("dual", [False, True])
+def test_linear_float32_of_few_rows_and_millions_of_weight_rows(dual):
+    """More weight rows than 65,535 blocks of the row-streaming kernel hold (2,097,120, of a pair half as many)."""
+    N, K_ = (2_097_120 >> dual) + 5, 8
+    x = rnd(3, K_, seed=1).to(DEV)
+    w, w2 = (torch.randn(N, K_, generator=torch.Generator(DEV).manual_seed(s), device=DEV) for s in (2, 3))
+    out = torch.full((3, N), float("nan"), device=DEV)
+    K.linear(x, w, out, w2=w2 if dual else None)
+    g = x.double() @ w.double().T
+    close(out, torch.nn.functional.silu(g) * (x.double() @ w2.double().T) if dual else g, torch.float32, f"{N} weight rows")
+
+
 @pytest.mark.parametrize("splits", [2, 3, 8])
 def test_linear_float32_cut_along_k(splits, monkeypatch):
     """Parts of unequal length (the last one shorter, or without a column), and the epilogue behind their sum."""
