@@ -73,6 +73,18 @@ class Runtime:
         """First ``n`` rows of a [max_tokens * per_token, width] buffer."""
         return self.buf(key, (self.max_tokens * per_token, width), dtype)[:n]
 
+    def split_scratch(self) -> torch.Tensor:
+        """Partial sums of the main chain's products that are cut along K."""
+        from .. import kernels as K
+
+        return self.buf("linear.split", (K.SPLIT_SCRATCH_BYTES // 4,), torch.float32)
+
+    def side_split_scratch(self) -> torch.Tensor:
+        """The same for the side stream, whose products run beside the main chain's."""
+        from .. import kernels as K
+
+        return self.buf("linear.split_side", (K.SPLIT_SCRATCH_BYTES // 4,), torch.float32)
+
     def shared_object(self, key: Tuple, factory):
         """One object per key for the whole model (for instance a routing layout that every
         layer with the same expert count shares)."""
@@ -100,7 +112,7 @@ class _SideScope:
         rt.side_stream.wait_event(rt._fork_event)
         self._ctx = torch.cuda.stream(rt.side_stream)
         self._ctx.__enter__()
-        self._scope = K.stream_scope()
+        self._scope = K.stream_scope(rt.side_split_scratch)
         self._scope.__enter__()
         K.timing_restart()
         return self

@@ -269,12 +269,12 @@ class ModelRunner:
             key = len(entries)
             g = self._graphs.get(key)
             if g is None:
-                with K.stream_scope():
+                with K.stream_scope(self.rt.split_scratch):
                     logits = self.model.forward(batch, self.layer_caches)  # also allocates every buffer
                 self._graph_launches[key] = K.launches - before
                 torch.cuda.synchronize(self.device)
                 g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g), K.stream_scope(), K.pdl_scope():
+                with torch.cuda.graph(g), K.stream_scope(self.rt.split_scratch), K.pdl_scope():
                     out = self.model.forward(batch, self.layer_caches)
                 self._graphs[key] = g
                 self._graph_logits[key] = out
@@ -285,7 +285,7 @@ class ModelRunner:
                 logits = self._graph_logits[key]
                 self.launch_counter += self._graph_launches[key]
         else:
-            with K.stream_scope():
+            with K.stream_scope(self.rt.split_scratch):
                 logits = self.model.forward(batch, self.layer_caches)
             self.launch_counter += K.launches - before
         for e in entries:

@@ -48,6 +48,7 @@ def _p(t: Optional[torch.Tensor]):
 
 
 _stream_override = None
+_scratch_override = None
 
 
 def _stream():
@@ -76,17 +77,22 @@ class pdl_scope:
 
 class stream_scope:
     """Within the scope every launch goes to the stream that is torch's current stream when
-    the scope is entered (looked up once instead of once per launch)."""
+    the scope is entered (looked up once instead of once per launch).  ``scratch``: gives the partial sums' buffer of the
+    chain of launches that the scope holds (:func:`_split_scratch`)."""
+
+    def __init__(self, scratch=None) -> None:
+        self._scratch = scratch
 
     def __enter__(self):
-        global _stream_override
-        self._saved = _stream_override
+        global _stream_override, _scratch_override
+        self._saved = _stream_override, _scratch_override
+        _scratch_override = self._scratch
         _stream_override = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream) if torch.cuda.is_available() else None
         return self
 
     def __exit__(self, *exc):
-        global _stream_override
-        _stream_override = self._saved
+        global _stream_override, _scratch_override
+        _stream_override, _scratch_override = self._saved
         return False
 
 
@@ -484,10 +490,16 @@ def f32_splits(m: int, n: int, k: int) -> int:
     return best
 
 
-def _split_scratch(device) -> torch.Tensor:
-    """The partial sums' buffer of the stream that launches: products on different streams (the shared expert
-    beside the routed ones) must not share one.  Made at a stream's first split product, which is never inside
-    a graph capture: a step is run once in the open before it is captured."""
+def _split_scratch(device, floats: int) -> torch.Tensor:
+    """A buffer for at least ``floats`` partial sums that no other chain of launches writes meanwhile.  The steps of a runner use
+    the runner's own, one for its main chain and one for its side stream's (:class:`stream_scope`), so that the graphs of two
+    runners may be replayed at the same time.  A product that is captured outside a runner gets memory of its graph's
+    own pool, which the same stream of the same capture finds again when the caller has let go of it.  All other calls share
+    a buffer per stream."""
+    if _scratch_override is not None:
+        return _scratch_override()
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(floats, dtype=torch.float32, device=device)
     key = (device, _stream().value)
     t = _SPLIT_SCRATCH.get(key)
     if t is None:
@@ -636,7 +648,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
                 # the activation belongs behind the whole sum: such a product is not cut along K
                 TN, splits = tc_plan(M, N, K, True)[0], 1
             if splits > 1:
-                scratch = _split_scratch(x.device)
+                scratch = _split_scratch(x.device, splits * M * N)
             te = t0 = tr = nt = None
             max_tiles = 0
         code = _lib("gemm_tc").locus_gemm_tc(
@@ -659,16 +671,18 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         te = t0 = tr = nt = None
         max_tiles = 0
         stride = 0
-    splits = 1
+    splits, scratch = 1, None
     if (layout is None and w2 is None and x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
             and (x.data_ptr() | w.data_ptr()) % 16 == 0):
         splits = f32_splits(M, N, K)
+        if splits > 1:
+            scratch = _split_scratch(x.device, splits * M * N)
     code = _lib("gemm_simt").locus_gemm_simt(
         _p(x), I(dtype_code(x.dtype)), _p(w), _p(w2), I(dtype_code(w.dtype)), _p(bias),
         I(dtype_code(bias.dtype) if bias is not None else 0), _p(out), I(dtype_code(out.dtype)),
         flags, F(act_limit), F(act_scale), _p(row_scale), _p(scale_rows), _p(x_rows), I(x_row_div), I(M), I(N), I(K),
         LL(x.stride(0)), LL(out.stride(0)), _p(te), _p(t0), _p(tr), _p(nt), I(max_tiles), LL(stride),
-        _p(_split_scratch(x.device) if splits > 1 else None), I(splits), _stream()
+        _p(scratch), I(splits), _stream()
     )
     if splits > 1 and code == 0:
         _count_launches(1)   # the kernel that adds the parts up

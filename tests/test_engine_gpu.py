@@ -702,6 +702,58 @@ def test_released_midway_and_fed_again_from_the_start(case, dtype):
         assert float(err.mean()) <= tol_mean * scale, name
 
 
+def test_partial_sums_of_captured_products_belong_to_their_runner_or_graph(tmp_path_factory, monkeypatch):
+    """Products cut along K leave partial sums behind.  Graphs of two runners may be replayed on two streams at once, so no
+    two runners may share the buffer, nor may two captures of plain products."""
+    import locus_b200.kernels as K
+    from locus_b200.engine.step import StepEntry
+
+    monkeypatch.setattr(K, "f32_splits", lambda m, n, k: 2)
+    few = K.few_rows_take
+    monkeypatch.setattr(K, "few_rows_take", lambda x, w, m, layout=None: layout is not None and few(x, w, m, layout))
+    seen, real = [], K._split_scratch
+
+    def recording(*a):
+        t = real(*a)
+        seen.append((t.data_ptr(), t.data_ptr() + 4 * t.numel()))
+        return t
+
+    monkeypatch.setattr(K, "_split_scratch", recording)
+    case = Case("A", tmp_path_factory.mktemp("models_scratch"))
+    places, kept = [], []
+    for _ in range(2):
+        runner, cache = make_runner(case, torch.float32, use_graphs=True)
+        seq = cache.open("a")
+        seen.clear()
+        for t in case.tokens["r5"][:3]:
+            assert cache.ensure_capacity(seq, 1)
+            runner.step([StepEntry(seq, [t], [0])])
+        assert runner.stats["graph_replays"] > 0 and seen
+        places.append(set(seen))
+        kept.append((runner, cache))
+    x, w = torch.randn(64, 512, device="cuda:0"), torch.randn(256, 512, device="cuda:0")
+    for _ in range(2):
+        out = torch.zeros(64, 256, device="cuda:0")
+        K.linear(x, w, out)
+        torch.cuda.synchronize()
+        seen.clear()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            K.linear(x, w, out)
+        assert seen
+        places.append(set(seen))
+        kept.append((g, out))
+    for i, a in enumerate(places):
+        for b in places[:i]:
+            assert all(p[1] <= q[0] or q[1] <= p[0] for p in a for q in b)
+    for g, out in kept[2:]:
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        ref = x.double() @ w.double().T
+        assert float((out.double() - ref).abs().max()) < 2e-5 * float(ref.abs().max())
+
+
 def test_expert_counters_through_graphs_and_the_kernel_time_table(tmp_path_factory):
     """The expert counters count once per executed step, also when decode steps are replayed from their CUDA graph
     (the counting is one more launch of the graph); the opt-in kernel time table makes steps run eagerly, names the
