@@ -475,6 +475,10 @@ def f32_splits(m: int, n: int, k: int) -> int:
     which an SM has two takes about 3.6 us for every 32 columns of k, one of at most a block an SM 2.0, and a second kernel
     adds the parts up, so what counts is how full the last round is.  Measured, whole and as cut: 512 rows of 2,048 x 5,632 360
     and 302 us in 8, of 6,144 x 2,048 369 and 335 in 3; 64 rows of it 139 and 63 in 6; 100 rows of 2,048 x 2,048 137 and 49 in 8."""
+    key = ("f32", m, n, k)
+    best = _PLANS.get(key)
+    if best is not None:
+        return best
     n_sm = _sm_count()
     tiles, stages = -(-m // 64) * -(-n // 128), -(-k // 32)
     best, best_cost = 1, None
@@ -487,6 +491,7 @@ def f32_splits(m: int, n: int, k: int) -> int:
             cost += 6.0 + s * m * n * 8 / 5e6
         if best_cost is None or cost < 0.98 * best_cost:
             best, best_cost = s, cost
+    _PLANS[key] = best
     return best
 
 

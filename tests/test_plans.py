@@ -32,6 +32,15 @@ def test_product_plans_are_ones_the_kernel_takes():
     assert K.tc_plan(2048, 6144, 2048, False) == (256, 1) and K.tc_plan(2048, 5632, 2048, True) == (128, 1)
 
 
+def test_float32_products_are_cut_into_parts_the_kernel_takes():
+    for m in list(range(1, 70)) + [100, 127, 128, 129, 500, 512, 513, 2048, 4096, 65535, 65536, 100000]:
+        for n, k in ((1, 4), (8, 8), (61, 2048), (2048, 2048), (6144, 2048), (2048, 5632), (151936, 2048), (130, 120)):
+            s = K.f32_splits(m, n, k)
+            assert 1 <= s <= 8 and s == K.f32_splits(m, n, k)
+            if s > 1:
+                assert m <= 65535 and s * m * n * 4 <= K.SPLIT_SCRATCH_BYTES and k >= 32 * 8 * s - 31
+
+
 def test_expert_tiles_and_attention_ranges():
     assert all(K.expert_tile(p, e) == 128 for p in (9, 64, 8192, 10 ** 6) for e in (1, 60, 512))
     for items in (1, 2, 4, 9, 10, 64, 200):
