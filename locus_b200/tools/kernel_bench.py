@@ -183,7 +183,7 @@ def bench_attn_chunk(args) -> None:
     T, ctx = args.tokens, args.ctx
     pool, q, out, meta, kw, i32 = _paged(args, 1, ctx, T)
     mma = K.attn_chunk_mma_takes(q, args.head_dim) and not args.cuda_cores
-    f32 = K.attn_chunk_f32_takes(q, args.head_dim)
+    f32 = K.attn_chunk_f32_takes(q, args.head_dim) and not args.cuda_cores
     tile = K.MMA_QUERY_TILE if mma or f32 else 16
     items = torch.tensor([(0, o) for o in range(0, T, tile)], dtype=torch.int32, device="cuda:0")
 
@@ -554,7 +554,7 @@ def main(argv=None) -> int:
                     help="linear: token tile of the tcgen05 kernel instead of the engine's choice")
     ap.add_argument("--splits", type=int, default=0,
                     help="linear: with --token-tile, parts along K (0 = not split)")
-    ap.add_argument("--cuda-cores", action="store_true", help="attn_chunk: the CUDA-core kernel")
+    ap.add_argument("--cuda-cores", action="store_true", help="attn_chunk: the kernel of 16-query tiles on the CUDA cores")
     ap.add_argument("--key-ranges", type=int, default=-1,
                     help="attn_chunk, latent, tensor-core kernels: ranges the keys are cut into (default: the engine's choice)")
     ap.add_argument("--mma-sync", action="store_true", help="attn_chunk: the mma.sync kernel where tcgen05 would run")

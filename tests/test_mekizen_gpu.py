@@ -224,7 +224,7 @@ def test_delta_rule_against_its_twin(heads, per_group, dim, v_dim, aligned):
 @pytest.mark.parametrize("heads,per_group,dim,v_dim", [(2, 1, 24, 16), (1, 1, 7, 5), (4, 2, 72, 40), (2, 1, 128, 128), (1, 1, 256, 17)])
 def test_delta_rule_of_few_tokens_and_of_tiles_edges(heads, per_group, dim, v_dim):
     """Steps whose rows are few a segment go to a kernel of their own (none, one and two tokens), longer ones end on, in
-    front of and behind a tile of 16 tokens and a group of 8."""
+    front of and behind a tile of 16 tokens and a group of four."""
     import locus_b200.kernels as K
 
     G = heads // per_group
