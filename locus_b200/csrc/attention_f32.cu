@@ -42,6 +42,14 @@ struct F32AttnArgs {
     float* part_ml;           // [item][head][split][FQ][2]
 };
 
+// The weight of a key that a query must not see: a pair of -0, which no exponential is.  Its value takes no part in the sum, so
+// that one that is not finite reaches nobody who does not see it (as a weight of 0 it would: 0 * inf).
+static constexpr f2 HIDDEN = 0x8000000080000000ull;
+template <bool B>
+struct Flag {
+    static constexpr bool value = B;
+};
+
 // HD: the head size that the tiles are laid out for (hd <= HD; dimensions behind hd are zeros).
 template <int HD>
 __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
@@ -140,6 +148,7 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
         for (int i = 0; i < 8; ++i) {
             const int p = p0 + ty + 8 * i;
             float s[4], mx = m[i];
+            bool hid[4];
             const int lo = first_key(a.window, a.chunk, p);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -147,7 +156,8 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
                 float e, f;
                 f2_unpack(s2[i][j], e, f);
                 s[j] = fmaf(slope, static_cast<float>(t - p), (e + f) * a.scale);
-                if (need_mask && !(t <= p && (t >= lo || t < a.keep_first))) s[j] = -INFINITY;
+                hid[j] = need_mask && !(t <= p && (t >= lo || t < a.keep_first));
+                if (hid[j]) s[j] = -INFINITY;
                 mx = fmaxf(mx, s[j]);
             }
 #pragma unroll
@@ -159,7 +169,7 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
             for (int j = 0; j < 4; ++j) {
                 const float e = expf(s[j] - base);
                 sum += e;
-                sp[(ty + 8 * i) * KEY_TILE + tx + 16 * j] = f2_pack(e, e);
+                sp[(ty + 8 * i) * KEY_TILE + tx + 16 * j] = hid[j] ? HIDDEN : f2_pack(e, e);
             }
             m[i] = mx;
             l[i] = l[i] * alpha + sum;   // (this thread's keys; the row's sixteen meet at the end)
@@ -169,32 +179,39 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
         }
         walk_wait<0>();
         __syncthreads();   // the values are there for all warps
+        auto weigh = [&](auto masked) {
+            constexpr bool MASKED = decltype(masked)::value;
 #pragma unroll 2
-        for (int k = 0; k < KEY_TILE; k += 2) {
-            f2 v[2][DP];
+            for (int k = 0; k < KEY_TILE; k += 2) {
+                f2 v[2][DP];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const float* vr = sv + (k + u) * HD;
-                if constexpr (DP == 1) {
-                    v[u][0] = *reinterpret_cast<const f2*>(vr + 2 * tx);
-                } else {
+                for (int u = 0; u < 2; ++u) {
+                    const float* vr = sv + (k + u) * HD;
+                    if constexpr (DP == 1) {
+                        v[u][0] = *reinterpret_cast<const f2*>(vr + 2 * tx);
+                    } else {
 #pragma unroll
-                    for (int d = 0; d < DP / 2; ++d) {
-                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vr + 64 * d + 4 * tx);
-                        v[u][2 * d] = w.x;
-                        v[u][2 * d + 1] = w.y;
+                        for (int d = 0; d < DP / 2; ++d) {
+                            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vr + 64 * d + 4 * tx);
+                            v[u][2 * d] = w.x;
+                            v[u][2 * d + 1] = w.y;
+                        }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(sp + (ty + 8 * i) * KEY_TILE + k);
+                    if (!MASKED || w.x != HIDDEN)
+#pragma unroll
+                        for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.x, v[0][d], o[i][d]);
+                    if (!MASKED || w.y != HIDDEN)
+#pragma unroll
+                        for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.y, v[1][d], o[i][d]);
+                }
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(sp + (ty + 8 * i) * KEY_TILE + k);
-#pragma unroll
-                for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.x, v[0][d], o[i][d]);
-#pragma unroll
-                for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.y, v[1][d], o[i][d]);
-            }
-        }
+        };
+        if (need_mask) weigh(Flag<true>());
+        else weigh(Flag<false>());
         __syncthreads();   // nobody reads the weights and the values any more
     }
     const size_t unit = (static_cast<size_t>(item) * a.nh + h) * a.n_splits + split;

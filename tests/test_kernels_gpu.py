@@ -551,6 +551,35 @@ def test_attn_chunk_float32_tiles(nh, nkv, hd, P, more):
         close(out, ref, torch.float32, f"attn_chunk_f32 in {n_splits} key ranges")
 
 
+@pytest.mark.parametrize("hd,more", [(16, {}), (64, dict(window=20)), (128, {}), (128, dict(window=9, keep_first=3)), (48, dict(chunk=40))])
+def test_attn_chunk_float32_keeps_what_is_not_finite_from_who_does_not_see_it(hd, more):
+    """A value or key of the portion that is not finite reaches the queries that see it and no other: those in front of it and
+    those whose window or chunk begins behind it have the bits that they have without it."""
+    ctx, n, P, bad = 30, 150, 64, 75
+    pool, q, meta, T = _paged_case(torch.float32, 1, 1, hd, P, [(ctx, n)], seed=hd, n_pages=8)
+    items = torch.tensor([(0, o) for o in range(0, n, 64)], dtype=torch.int32, device=DEV)
+    kw = dict(dict(n_heads=1, n_kv_heads=1, head_dim=hd, page_tokens=P, window=0, scale=0.1), **more)
+    pos = torch.arange(ctx, ctx + n)
+    sees = (pos >= bad) & (pos - bad < more.get("window", 10 ** 6)) & (pos // more.get("chunk", 10 ** 6) == bad // more.get("chunk", 10 ** 6))
+    for n_splits in (1, 3):
+        part_o, part_ml = torch.empty(3 * n_splits * 64 * hd, device=DEV), torch.empty(3 * n_splits * 128, device=DEV)
+
+        def run(where, value):
+            dpool = pool.to(DEV)
+            if where is not None:
+                dpool[int(meta["block_table"][0, bad // P]), where, 0, bad % P, hd // 2] = value
+            out = torch.zeros(T, hd, device=DEV)
+            K.attn_chunk_f32(q.to(DEV), dpool, out, items=items, n_items=3, n_splits=n_splits, part_o=part_o, part_ml=part_ml,
+                             **_dev(meta), **kw)
+            return out.cpu()
+
+        want = run(None, 0.0)
+        for where, value in ((1, float("inf")), (1, float("nan")), (0, float("nan"))):
+            got = run(where, value)
+            assert torch.equal(got[~sees], want[~sees]), (where, value, n_splits)
+            assert not torch.isfinite(got[sees]).all(1).any()
+
+
 @pytest.mark.parametrize("dual", [False, True])
 @pytest.mark.parametrize("M,N,K_", [(9, 64, 36), (64, 129, 60), (65, 200, 4), (17, 1000, 2052), (40, 33, 100), (130, 300, 128)])
 def test_linear_float32_tiles(M, N, K_, dual):
