@@ -8,8 +8,9 @@
 // weights go from the one product to the other through rows that a warp writes and reads by itself -- each twice, as the
 // pairs want them, in the buffer that held the keys.  K and V are copied asynchronously (rows of keys 4 floats longer, so
 // that 8 of them meet in no bank); two blocks of 100 KB share an SM and hide each other's copies.
-// Measured: 512 tokens behind 1,500 others, 16 heads of 128: 372 us in two ranges (20 TFLOP/s) where the kernel of 16-query
-// tiles with scalar loads took 1,859 us.
+// Measured: 512 tokens behind 1,500 others, 16 heads of 128: 274 us in two ranges (27 TFLOP/s) where the kernel of 16-query
+// tiles with scalar loads took 1,563 to 1,859 us; with every warp working out its rows' places by itself 372.  A portion of 2 / 16
+// tokens behind none 7.0 / 7.8 us (13.5 / 22.7 with 16-query tiles; 17.8 / 19.1 when all 64 rows of a tile were worked on).
 //
 // Mask, window with kept first tokens, chunks, sink and distance bias as in attention.cu; keys outside a tile's range are
 // zeros, never what the pages hold.  A step with few tiles cuts the keys into n_splits ranges (grid z) whose unnormalised
@@ -45,9 +46,9 @@ struct F32AttnArgs {
 // The weight of a key that a query must not see: a pair of -0, which no exponential is.  Its value takes no part in the sum, so
 // that one that is not finite reaches nobody who does not see it (as a weight of 0 it would: 0 * inf).
 static constexpr f2 HIDDEN = 0x8000000080000000ull;
-template <bool B>
-struct Flag {
-    static constexpr bool value = B;
+template <int N>
+struct Int {
+    static constexpr int value = N;
 };
 
 // HD: the head size that the tiles are laid out for (hd <= HD; dimensions behind hd are zeros).
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
     static_assert(DP == 1 || DP == 2 || DP == 4, "heads of 32, 64 or 128");
     constexpr int KROWS = KEY_TILE * LD > KEY_TILE * KEY_TILE * 2 ? KEY_TILE * LD : KEY_TILE * KEY_TILE * 2;
     extern __shared__ __align__(16) float f32a_smem[];
+    __shared__ long long rows_at[2][KEY_TILE];   // of a tile's keys in the pool, by the tile's parity; -1: not there
     float* sq = f32a_smem;         // [FQ][LD]
     float* sk = sq + FQ * LD;      // [KEY_TILE][LD]; then the weights, [FQ][KEY_TILE] pairs
     float* sv = sk + KROWS;        // [KEY_TILE][HD]
@@ -84,26 +86,40 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
             (r < FQ ? sq + r * LD : sv + (r - FQ) * HD)[d] = 0.f;
         }
     }
-    const int chunks = hd >> 2;   // 16-byte pieces of a row; a warp copies 32 / chunks rows or one in several steps
-    for (int i = tid; i < FQ * chunks; i += 128) {
-        const int r = i / chunks, c = (i % chunks) * 4;
-        const bool live = r < nq;
-        walk_copy<16>(sq + r * LD + c, a.q + (static_cast<size_t>(row0 + (live ? r : 0)) * a.nh + h) * hd + c, live);
-    }
+    // Copies: HD / 4 lanes to a row, of 16 bytes each.  Where the rows of a tile's keys lie is worked out by a thread a row, a tile ahead
+    // (by every warp for its own rows, one row after the other, a tile waited 4 us for two divisions and a table read a row).
+    constexpr int RL = HD / 4, RW = 32 / RL, RI = KEY_TILE / (4 * RW);   // lanes of a row, rows of a warp's copy, copies of a warp
+    const int cl = (lane % RL) * 4, rl = warp * RW + lane / RL;
     const size_t v_off = static_cast<size_t>(a.nkv) * P * hd;
-    auto key_row = [&](int t) {
-        return a.pool + (static_cast<size_t>(table[t / P]) * 2 * a.nkv + kvh) * P * hd + static_cast<size_t>(t % P) * hd;
+    auto place = [&](int it) {
+        if (tid >= KEY_TILE || it >= n_tiles) return;
+        const int t = tile_pos(first_idx + it, first_tile, kept_tiles) + tid;
+        long long at = -1;
+        if ((t >= t_lo || t < kept) && t <= t_hi)
+            at = (static_cast<long long>(table[t / P]) * 2 * a.nkv + kvh) * P * hd + static_cast<long long>(t % P) * hd;
+        rows_at[it & 1][tid] = at;
     };
-    auto copy_tile = [&](int tile0, int which) {   // 0: keys, 1: values
-        for (int r = warp; r < KEY_TILE; r += 4) {
-            const int t = tile0 + r;
-            const bool live = (t >= t_lo || t < kept) && t <= t_hi;
-            const float* src = live ? key_row(t) + (which ? v_off : 0) : a.pool;
-            float* dst = which ? sv + r * HD : sk + r * LD;
-            for (int c = 4 * lane; c < hd; c += 128) walk_copy<16>(dst + c, src + (live ? c : 0), live);
-            if (!which)   // (the weights of the last tile lay here)
-                for (int c = hd + lane; c < HD; c += 32) dst[c] = 0.f;
+    place(0);
+    if (cl < hd)
+        for (int r = rl; r < FQ; r += 4 * RW) {
+            const bool live = r < nq;
+            walk_copy<16>(sq + r * LD + cl, a.q + (static_cast<size_t>(row0 + (live ? r : 0)) * a.nh + h) * hd + cl, live);
         }
+    __syncthreads();
+    auto copy_tile = [&](int it) {
+        long long at[RI];
+#pragma unroll
+        for (int i = 0; i < RI; ++i) at[i] = rows_at[it & 1][rl + 4 * RW * i];
+#pragma unroll
+        for (int i = 0; i < RI; ++i) {
+            float* dst = sk + (rl + 4 * RW * i) * LD + cl;
+            if (cl < hd) walk_copy<16>(dst, a.pool + (at[i] < 0 ? 0 : at[i] + cl), at[i] >= 0);
+            else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);   // (the weights of the last tile lay here)
+        }
+        walk_commit();
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+            if (cl < hd) walk_copy<16>(sv + (rl + 4 * RW * i) * HD + cl, a.pool + (at[i] < 0 ? 0 : at[i] + v_off + cl), at[i] >= 0);
         walk_commit();
     };
     const float slope = slope_of(a.slopes, h);
@@ -117,103 +133,112 @@ __global__ void __launch_bounds__(128, 2) attn_chunk_f32_kernel(F32AttnArgs a) {
         for (int d = 0; d < DP; ++d) o[i][d] = 0;
     }
     const int n_rows = (nq - ty + 7) >> 3;   // (of this thread's queries ty, ty + 8, .. those that are there)
-    for (int it = 0; it < n_tiles; ++it) {
-        const int tile0 = tile_pos(first_idx + it, first_tile, kept_tiles);
-        copy_tile(tile0, 0);
-        copy_tile(tile0, 1);
-        walk_wait<1>();
-        __syncthreads();
-        f2 s2[8][4];
+    // NI: the eights of queries that are worked on.  (A lone tile takes as long as its instructions: a portion of up to 16 queries would
+    // otherwise pay for 64.)
+    auto walk_tiles = [&](auto eights) {
+        constexpr int NI = decltype(eights)::value;
+        for (int it = 0; it < n_tiles; ++it) {
+            const int tile0 = tile_pos(first_idx + it, first_tile, kept_tiles);
+            copy_tile(it);
+            place(it + 1);
+            walk_wait<1>();
+            __syncthreads();
+            f2 s2[NI][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < NI; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s2[i][j] = 0;
+                for (int j = 0; j < 4; ++j) s2[i][j] = 0;
 #pragma unroll 4
-        for (int d = 0; d < HD; d += 4) {
-            ulonglong2 x[8];
+            for (int d = 0; d < HD; d += 4) {
+                ulonglong2 x[NI];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(sq + (ty + 8 * i) * LD + d);
+                for (int i = 0; i < NI; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(sq + (ty + 8 * i) * LD + d);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(sk + (tx + 16 * j) * LD + d);
+                for (int j = 0; j < 4; ++j) {
+                    const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(sk + (tx + 16 * j) * LD + d);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) s2[i][j] = f2_fma(x[i].x, k.x, s2[i][j]);
+                    for (int i = 0; i < NI; ++i) s2[i][j] = f2_fma(x[i].x, k.x, s2[i][j]);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) s2[i][j] = f2_fma(x[i].y, k.y, s2[i][j]);
+                    for (int i = 0; i < NI; ++i) s2[i][j] = f2_fma(x[i].y, k.y, s2[i][j]);
+                }
             }
-        }
-        __syncthreads();   // nobody reads the keys any more: the weights take their place
-        const bool need_mask = tile0 + KEY_TILE - 1 > p0 || tile0 < lo_last;
+            __syncthreads();   // nobody reads the keys any more: the weights take their place
+            const bool need_mask = tile0 + KEY_TILE - 1 > p0 || tile0 < lo_last;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int p = p0 + ty + 8 * i;
-            float s[4], mx = m[i];
-            bool hid[4];
-            const int lo = first_key(a.window, a.chunk, p);
+            for (int i = 0; i < NI; ++i) {
+                const int p = p0 + ty + 8 * i;
+                float s[4], mx = m[i];
+                bool hid[4];
+                const int lo = first_key(a.window, a.chunk, p);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int t = tile0 + tx + 16 * j;
-                float e, f;
-                f2_unpack(s2[i][j], e, f);
-                s[j] = fmaf(slope, static_cast<float>(t - p), (e + f) * a.scale);
-                hid[j] = need_mask && !(t <= p && (t >= lo || t < a.keep_first));
-                if (hid[j]) s[j] = -INFINITY;
-                mx = fmaxf(mx, s[j]);
+                for (int j = 0; j < 4; ++j) {
+                    const int t = tile0 + tx + 16 * j;
+                    float e, f;
+                    f2_unpack(s2[i][j], e, f);
+                    s[j] = fmaf(slope, static_cast<float>(t - p), (e + f) * a.scale);
+                    hid[j] = need_mask && !(t <= p && (t >= lo || t < a.keep_first));
+                    if (hid[j]) s[j] = -INFINITY;
+                    mx = fmaxf(mx, s[j]);
+                }
+#pragma unroll
+                for (int b = 1; b < 16; b <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, b));
+                const float base = mx == -INFINITY ? 0.f : mx;   // (no key seen yet: the weights are exp(-inf) = 0)
+                const float alpha = expf(m[i] - base);           // exp(-inf) = 0 on the first live tile
+                float sum = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float e = expf(s[j] - base);
+                    sum += e;
+                    sp[(ty + 8 * i) * KEY_TILE + tx + 16 * j] = hid[j] ? HIDDEN : f2_pack(e, e);
+                }
+                m[i] = mx;
+                l[i] = l[i] * alpha + sum;   // (this thread's keys; the row's sixteen meet at the end)
+                const f2 al = f2_pack(alpha, alpha);
+#pragma unroll
+                for (int d = 0; d < DP; ++d) o[i][d] = f2_mul(o[i][d], al);
             }
-#pragma unroll
-            for (int b = 1; b < 16; b <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, b));
-            const float base = mx == -INFINITY ? 0.f : mx;   // (no key seen yet: the weights are exp(-inf) = 0)
-            const float alpha = expf(m[i] - base);           // exp(-inf) = 0 on the first live tile
-            float sum = 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float e = expf(s[j] - base);
-                sum += e;
-                sp[(ty + 8 * i) * KEY_TILE + tx + 16 * j] = hid[j] ? HIDDEN : f2_pack(e, e);
-            }
-            m[i] = mx;
-            l[i] = l[i] * alpha + sum;   // (this thread's keys; the row's sixteen meet at the end)
-            const f2 al = f2_pack(alpha, alpha);
-#pragma unroll
-            for (int d = 0; d < DP; ++d) o[i][d] = f2_mul(o[i][d], al);
-        }
-        walk_wait<0>();
-        __syncthreads();   // the values are there for all warps
-        auto weigh = [&](auto masked) {
-            constexpr bool MASKED = decltype(masked)::value;
+            walk_wait<0>();
+            __syncthreads();   // the values are there for all warps
+            auto weigh = [&](auto masked) {
+                constexpr bool MASKED = decltype(masked)::value != 0;
+                const int end = MASKED ? min(KEY_TILE, t_hi - tile0 + 1) : KEY_TILE;   // (behind it every key is hidden from every query)
 #pragma unroll 2
-            for (int k = 0; k < KEY_TILE; k += 2) {
-                f2 v[2][DP];
+                for (int k = 0; k < end; k += 2) {
+                    f2 v[2][DP];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const float* vr = sv + (k + u) * HD;
-                    if constexpr (DP == 1) {
-                        v[u][0] = *reinterpret_cast<const f2*>(vr + 2 * tx);
-                    } else {
+                    for (int u = 0; u < 2; ++u) {
+                        const float* vr = sv + (k + u) * HD;
+                        if constexpr (DP == 1) {
+                            v[u][0] = *reinterpret_cast<const f2*>(vr + 2 * tx);
+                        } else {
 #pragma unroll
-                        for (int d = 0; d < DP / 2; ++d) {
-                            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vr + 64 * d + 4 * tx);
-                            v[u][2 * d] = w.x;
-                            v[u][2 * d + 1] = w.y;
+                            for (int d = 0; d < DP / 2; ++d) {
+                                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vr + 64 * d + 4 * tx);
+                                v[u][2 * d] = w.x;
+                                v[u][2 * d + 1] = w.y;
+                            }
                         }
                     }
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(sp + (ty + 8 * i) * KEY_TILE + k);
+                        if (!MASKED || w.x != HIDDEN)
+#pragma unroll
+                            for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.x, v[0][d], o[i][d]);
+                        if (!MASKED || w.y != HIDDEN)
+#pragma unroll
+                            for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.y, v[1][d], o[i][d]);
+                    }
                 }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(sp + (ty + 8 * i) * KEY_TILE + k);
-                    if (!MASKED || w.x != HIDDEN)
-#pragma unroll
-                        for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.x, v[0][d], o[i][d]);
-                    if (!MASKED || w.y != HIDDEN)
-#pragma unroll
-                        for (int d = 0; d < DP; ++d) o[i][d] = f2_fma(w.y, v[1][d], o[i][d]);
-                }
-            }
-        };
-        if (need_mask) weigh(Flag<true>());
-        else weigh(Flag<false>());
-        __syncthreads();   // nobody reads the weights and the values any more
-    }
+            };
+            if (need_mask) weigh(Int<1>());
+            else weigh(Int<0>());
+            __syncthreads();   // nobody reads the weights and the values any more
+        }
+    };
+    if (nq <= 16) walk_tiles(Int<2>());
+    else if (nq <= 32) walk_tiles(Int<4>());
+    else walk_tiles(Int<8>());
     const size_t unit = (static_cast<size_t>(item) * a.nh + h) * a.n_splits + split;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
