@@ -1,11 +1,15 @@
 // Matrix products on CUDA cores with float32 FMA: out = x . W^T with fused epilogues.
 //
 // This is the true-32-bit path of every linear layer (no tensor cores, no TF32) and the
-// general fallback of the bfloat16 path for shapes the tensor-core kernels refuse.  Each
-// output element is accumulated by one thread over k = 0..K-1 in ascending order, so its
-// value does not depend on M, on the other rows of the batch or on the tile it falls in.
+// general fallback of the bfloat16 path for shapes the tensor-core kernels refuse.  In
+// gemm_simt one thread accumulates an output over k = 0..K-1 in ascending order, so its value
+// does not depend on M, on the other rows of the batch or on the tile it falls in.  In gemm_f32
+// an output is a sum over the even k and one over the odd k, and a plain product may be cut
+// along K, by M, N and K: the other rows' values never matter, but a row of M rows may round
+// otherwise than the same row among more or fewer, whose product is cut otherwise or runs on
+// gemv.cu.
 //
-// One kernel covers:
+// Both kernels cover:
 //   * plain      out[m, n]  = sum_k x[m, k] W[n, k]          (+ bias[n]) (* row_scale[m])
 //   * SwiGLU     out[m, n]  = silu(x . Wg[n]) * (x . Wu[n])   (two accumulators)
 //   * gathered   x row of logical row m is x_rows[m] / x_row_div
@@ -18,13 +22,12 @@
 // lanes x 2 x 1.965 GHz = 74.4 TFLOP/s), so everything else is kept off their issue slots: 32 columns of k of 64 rows
 // and 128 weight rows are copied into shared memory asynchronously, two stages ahead, k contiguous as they lie in memory (rows
 // 36 floats apart meet in no bank), a thread owns 8 x 8 outputs, and a multiply-add works on two k at once, so each
-// output has a sum over the even k and one over the odd k, added at the end -- in the same order whatever the tile; a product
-// whose blocks would leave SMs idle is cut along k, its parts added up in order by a second kernel.  A
-// tile's rows are worked on in eights, so that an expert's 34 rows cost 40 and not 64.  gemm_simt: every other type,
-// width and alignment.  Measured: 2,048 x
-// 6,144 x 2,048 1.18 ms = 43.8 TFLOP/s (20 before, with the 64 x 64 x 16 tiles of gemm_simt), 512 x 6,144 x 2,048 343 us, the
-// routed experts of 512 tokens (60 x (2,048 -> 1,408 -> 2,048), 4 picks) 1.02 ms; one multiply-add at a time instead of
-// two, with up to twice the warps, 1.26 to 1.5 ms on the first.
+// output has a sum over the even k and one over the odd k, added at the end; a product whose blocks would leave SMs idle is
+// cut along k, its parts added up in order by a second kernel.  A tile's rows are worked on in eights, so that an expert's 34
+// rows cost 40 and not 64.  gemm_simt: every other type, width and alignment.  Measured: 2,048 x 6,144 x 2,048 1.16 ms = 44.6
+// TFLOP/s (2.0 ms with the 64 x 64 x 16 tiles of gemm_simt), 512 x 6,144 x 2,048 302 us, 64 x 512 x 512 10 us, the routed experts
+// of 512 tokens (60 x (2,048 -> 1,408 -> 2,048), 4 picks) 1.01 ms; one multiply-add at a time instead of two, with up to twice the
+// warps, 1.26 to 1.5 ms on the first.
 #include "common.cuh"
 #include "walk.cuh"
 
@@ -64,26 +67,37 @@ struct GemmArgs {
     int splits;
 };
 
-// One output: activation, bias, row scale (rs), softcap, store.  v2: the second weight's sum.
+// One output: activation, bias (b; of the second weight b2), row scale (rs), softcap.  v2: the second weight's sum.
 template <bool SWIGLU>
-__device__ __forceinline__ void epilogue(const GemmArgs& a, int r, int n, float rs, float v, float v2) {
+__device__ __forceinline__ float finish(const GemmArgs& a, float rs, float v, float v2, float b, float b2) {
     if (SWIGLU && a.act == 2) {
         const float g = fminf(v * rs, a.act_param);
         const float u = fminf(fmaxf(v2 * rs, -a.act_param), a.act_param);
         v = g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
     } else if (SWIGLU && a.act == 4) {
-        v = fmaxf(v + pair_bias(a.bias, a.bias_dt, n), 0.f) * (v2 + pair_bias(a.bias, a.bias_dt, a.N + n));
+        v = fmaxf(v + b, 0.f) * (v2 + b2);
     } else if (SWIGLU) {
         const float g = v;
         v = g / (1.0f + expf(-g)) * v2;
     }
-    if (a.bias && a.act != 4) v += ld_dyn(a.bias, a.bias_dt, n);
+    if (a.bias && a.act != 4) v += b;
     if (a.act == 1) {
         v = fmaxf(v, 0.f);
         v *= v;
     }
     if (a.row_scale && a.act != 2) v *= rs;
     if (a.act == 3) v = a.act_param * tanhf(v * a.act_scale / a.act_param);
+    return v;
+}
+__device__ __forceinline__ float bias_of(const GemmArgs& a, int n) { return pair_bias(a.bias, a.bias_dt, n); }
+__device__ __forceinline__ float scale_of(const GemmArgs& a, int r) {
+    return a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
+}
+
+// The same, stored or added.
+template <bool SWIGLU>
+__device__ __forceinline__ void epilogue(const GemmArgs& a, int r, int n, float rs, float v, float v2) {
+    v = finish<SWIGLU>(a, rs, v, v2, bias_of(a, n), a.act == 4 ? bias_of(a, a.N + n) : 0.f);
     const size_t o = static_cast<size_t>(r) * a.ldo + n;
     if (a.accumulate) {
         static_cast<float*>(a.out)[o] += v;
@@ -179,7 +193,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs a) {
         const int lrow = ty * 4 + i;
         if (lrow >= rows) continue;
         const int r = row0 + lrow;
-        const float rs = a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
+        const float rs = scale_of(a, r);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = col0 + tx * 4 + j;
@@ -272,6 +286,9 @@ __global__ void __launch_bounds__(8 * TX) gemm_f32_kernel(GemmArgs a) {
         if (i < n_k) fetch(i);
         walk_commit();
     }
+    // An instance each for 2, 4, 5, 6 and 8 eights of rows, the next larger one for the others.  With three more, for 1, 3 and 7, two
+    // registers spilled: 24 rows of 6,144 x 2,048 28.1 -> 24.5 us, the experts of 240 tokens 800 -> 748, but those of 512 1,005 ->
+    // 1,024 and 2,048 rows 1,155 -> 1,181.
     const int groups = (rows + 7) >> 3;
     auto walk_k = [&](auto stage) {
         for (int kb = 0; kb < n_k; ++kb) {
@@ -288,22 +305,47 @@ __global__ void __launch_bounds__(8 * TX) gemm_f32_kernel(GemmArgs a) {
     else if (groups == 5) walk_k([&](const float* x, const float* w) { f32_stage<5, TX>(x, w, acc); });
     else if (groups == 6) walk_k([&](const float* x, const float* w) { f32_stage<6, TX>(x, w, acc); });
     else walk_k([&](const float* x, const float* w) { f32_stage<8, TX>(x, w, acc); });
+    // The tile's sums go through shared memory to a loop that holds the epilogue once: unrolled over a thread's 64 outputs its code
+    // had to be fetched for a single use, 20 cycles to an instruction (64 x 16 x 64 23 -> 11 us, 512 x 512 x 512 35 -> 21, the
+    // routed experts of 300 tokens, 8 x (512 -> 256 -> 512), 89 -> 64).  Old values of an added-to output are fetched together.
+    __syncthreads();   // nobody reads the stages any more
+    constexpr int LD = BNW + TX;   // (a warp's rows of TX sums meet in no bank)
+    float* sums = f32_smem;
+    float* olds = sums + FM * LD;
+    float* scales = olds + FM * COLS;
+    static_assert(FM * (LD + COLS + 1) <= F_STAGES * STAGE, "the epilogue's tile takes the place of the stages");
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = ty + 8 * i;
-        if (m >= rows) continue;
-        const int r = row0 + m;
-        const float rs = a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < (SWIGLU ? 4 : 8); ++j) {
-            const int n = col0 + tx + TX * j;
-            if (n >= a.N) continue;
-            float even, odd, even2 = 0.f, odd2 = 0.f;
+        for (int j = 0; j < 8; ++j) {
+            float even, odd;
             f2_unpack(acc[i][j], even, odd);
-            if (SWIGLU) f2_unpack(acc[i][j + 4], even2, odd2);
-            if (!SWIGLU && a.part) a.part[(static_cast<size_t>(blockIdx.z) * a.M + r) * a.N + n] = even + odd;
-            else epilogue<SWIGLU>(a, r, n, rs, even + odd, even2 + odd2);
+            sums[(ty + 8 * i) * LD + tx + TX * j] = even + odd;
         }
+    const int c = tid % COLS, n = col0 + c;
+    const bool whole = SWIGLU || a.part == nullptr;
+    if (whole && a.accumulate)
+        for (int m = tid / COLS; m < rows; m += NT / COLS) {
+            const bool live = n < a.N;
+            walk_copy<4>(olds + m * COLS + c, static_cast<const float*>(a.out) + static_cast<size_t>(row0 + m) * a.ldo + (live ? n : 0), live);
+        }
+    walk_commit();
+    for (int m = tid; m < rows; m += NT) scales[m] = scale_of(a, row0 + m);
+    const float b = n < a.N ? bias_of(a, n) : 0.f, b2 = a.act == 4 && n < a.N ? bias_of(a, a.N + n) : 0.f;
+    walk_wait<0>();
+    __syncthreads();
+    if (n >= a.N) return;
+#pragma unroll 2
+    for (int m = tid / COLS; m < rows; m += NT / COLS) {
+        const float v = sums[m * LD + c];
+        if (!whole) {
+            a.part[(static_cast<size_t>(blockIdx.z) * a.M + row0 + m) * a.N + n] = v;
+            continue;
+        }
+        const float y = finish<SWIGLU>(a, scales[m], v, SWIGLU ? sums[m * LD + COLS + c] : 0.f, b, b2);
+        const size_t o = static_cast<size_t>(row0 + m) * a.ldo + n;
+        if (a.accumulate) static_cast<float*>(a.out)[o] = olds[m * COLS + c] + y;
+        else st_dyn(a.out, a.out_dt, o, y);
     }
 }
 
@@ -313,8 +355,7 @@ __global__ void __launch_bounds__(256) gemm_f32_sum_kernel(GemmArgs a) {
     if (n >= a.N) return;
     float v = 0.f;
     for (int z = 0; z < a.splits; ++z) v += a.part[(static_cast<size_t>(z) * a.M + r) * a.N + n];
-    const float rs = a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
-    epilogue<false>(a, r, n, rs, v, 0.f);
+    epilogue<false>(a, r, n, scale_of(a, r), v, 0.f);
 }
 
 template <int TX>
@@ -372,12 +413,21 @@ extern "C" int locus_gemm_simt(const void* x, int x_dt, const void* w, const voi
     const int tiles = tile_expert ? max_tiles : ceil_div(M, BM);
     const bool swiglu = w2 != nullptr;
     static_assert(FM == BM, "the grouped tile lists serve both kernels");
+    static int n_sm = 0;
+    if (n_sm == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0) {
+            n_sm = 0;
+            return static_cast<int>(cudaGetLastError());
+        }
+    }
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32 && ((K | ldx) & 3) == 0 &&
         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w2)) & 15) == 0) {
         if (splits > 1 && (part == nullptr || splits > 8 || swiglu || tile_expert != nullptr || M > 65535)) return LOCUS_ERR_UNSUPPORTED;
         // tiles of 64 weight rows where tiles of 128 would leave SMs without one
         const long long wide = static_cast<long long>(ceil_div(N, swiglu ? 64 : 128)) * tiles * a.splits;
-        return wide < 148 ? launch_f32<8>(a, tiles, swiglu, stream) : launch_f32<16>(a, tiles, swiglu, stream);
+        return wide < n_sm ? launch_f32<8>(a, tiles, swiglu, stream) : launch_f32<16>(a, tiles, swiglu, stream);
     }
     if (splits > 1) return LOCUS_ERR_UNSUPPORTED;
     if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32) return launch<float, float>(a, tiles, swiglu, stream);
