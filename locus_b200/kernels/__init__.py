@@ -472,9 +472,11 @@ def tc_plan(m: int, n: int, k: int, dual: bool) -> Tuple[int, int]:
 
 def f32_splits(m: int, n: int, k: int) -> int:
     """Parts along K of a plain float32 product on tiles of 64 rows x 128 weight rows, two blocks an SM.  A round of blocks in
-    which an SM has two takes about 3.6 us for every 32 columns of k, one of at most a block an SM 2.0, and a second kernel
-    adds the parts up, so what counts is how full the last round is.  Measured, whole and as cut: 512 rows of 2,048 x 5,632 360
-    and 302 us in 8, of 6,144 x 2,048 369 and 335 in 3; 64 rows of it 139 and 63 in 6; 100 rows of 2,048 x 2,048 137 and 49 in 8."""
+    which an SM has two takes about 3.3 us for every 32 columns of k, one of at most a block an SM 2.0, and a second kernel
+    adds the parts up, so what counts is how full the last round is; a part has at least 64 columns.  Measured, whole and as
+    cut: 512 rows of 2,048 x 5,632 299 and 268 us in 8, of 6,144 x 2,048 328 and 302 in 3; 64 rows of it 115 and 46 in 6; 100 rows
+    of 2,048 x 2,048 115 and 35 in 8, of 512 x 512 34 and 10 in 8, of 1,024 x 256 21 and 10 in 4; over 80 sizes the choice is
+    within 1 % of the best number of parts on average, at worst 17 % behind (65 rows of 6,144 x 2,048)."""
     key = ("f32", m, n, k)
     best = _PLANS.get(key)
     if best is not None:
@@ -483,12 +485,12 @@ def f32_splits(m: int, n: int, k: int) -> int:
     tiles, stages = -(-m // 64) * -(-n // 128), -(-k // 32)
     best, best_cost = 1, None
     for s in range(1, 9):
-        if s > 1 and (stages < 8 * s or 4 * s * m * n > SPLIT_SCRATCH_BYTES or m > 65535):
+        if s > 1 and (stages < 2 * s or 4 * s * m * n > SPLIT_SCRATCH_BYTES or m > 65535):
             break
         full, rest = divmod(tiles * s, 2 * n_sm)
-        cost = -(-stages // s) * (3.6 * full + (0.0 if rest == 0 else 2.0 if rest <= n_sm else 3.6))
+        cost = -(-stages // s) * (3.3 * full + (0.0 if rest == 0 else 2.0 if rest <= n_sm else 3.3))
         if s > 1:
-            cost += 6.0 + s * m * n * 8 / 5e6
+            cost += 2.0 + s * m * n * 8 / 1e7
         if best_cost is None or cost < 0.98 * best_cost:
             best, best_cost = s, cost
     _PLANS[key] = best

@@ -38,7 +38,7 @@ def test_float32_products_are_cut_into_parts_the_kernel_takes():
             s = K.f32_splits(m, n, k)
             assert 1 <= s <= 8 and s == K.f32_splits(m, n, k)
             if s > 1:
-                assert m <= 65535 and s * m * n * 4 <= K.SPLIT_SCRATCH_BYTES and k >= 32 * 8 * s - 31
+                assert m <= 65535 and s * m * n * 4 <= K.SPLIT_SCRATCH_BYTES and k > 32 * (2 * s - 1)
 
 
 def test_expert_tiles_and_attention_ranges():
