@@ -6,8 +6,9 @@
 // runs the epilogue.  Same epilogues and the same gathered / grouped forms as the other
 // products: bias, SwiGLU of two weight rows, per-row scale, store or add into float32.
 //
-// The order of the sum for an element depends on K (f32_stream: and N) only (8-element chunks per lane, lanes
-// combined by a fixed shuffle tree), not on the other rows.
+// The order of an element's sum follows from the kernel and from K (f32_stream: and N) alone (8-element chunks per lane, lanes
+// combined by a fixed shuffle tree); what the other rows hold never matters.  Which kernel runs follows from the number of rows:
+// float32 rows of one or two (grouped: up to 8 pairs), of 3 to 32 and of more round differently from one another.
 //
 // float32 x float32 has a kernel of its own, f32_stream: with a warp per weight row every 16 bytes of a weight row cost the 8
 // rows' 128 bytes of x from L1, which was the bound (2.5 TB/s of weights).  There a warp streams four weight rows, so that a

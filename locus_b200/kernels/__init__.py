@@ -370,15 +370,28 @@ def tensor_cores_take(x: torch.Tensor, w: torch.Tensor, x_rows: Optional[torch.T
 
 
 FEW_ROWS = 8  # rows of x per tile of the row-streaming kernel
-F32_STREAM_ROWS = 32  # most rows of a plain float32 product that go to it, in tiles of 8 that share the weights through L2
+# Plain float32 products of more rows that go to it, in tiles of 8 that share the weights through L2: up to F32_STREAM_ANY whatever
+# the weight, up to F32_STREAM_ROWS where rows x weight elements are at most F32_STREAM_WORK, and with two weights up to
+# F32_STREAM_PAIR.  Measured against the tiles of gemm_f32 (microseconds, streamed / tiles): 9 rows of 151,936 x 2,048 355 / 393, of
+# 2,048 x 5,632 28 / 31, of 6,144 x 2,048 26 / 22; 16 rows 597 / 400, 39 / 31, 37 / 22; 32 rows of 2,048 x 2,048 30 / 17, of 60 x 2,048
+# 4.8 / 14, of 512 x 512 4.1 / 14; pairs of 5,632 x 2,048 (never cut along K) 16 rows 51 / 71, 24 76 / 88, 32 99 / 89.
+F32_STREAM_ANY = 10
+F32_STREAM_PAIR = 24
+F32_STREAM_ROWS = 32
+F32_STREAM_WORK = 40_000_000
 
 
-def few_rows_take(x: torch.Tensor, w: torch.Tensor, m: int, layout: Optional["ExpertLayout"] = None) -> bool:
-    """Whether :func:`linear` runs this product with the row-streaming kernel: at most 8 rows
-    (per expert tile when grouped; ``F32_STREAM_ROWS`` of a plain float32 product), width a multiple of 8, 32-byte aligned rows."""
+def few_rows_take(x: torch.Tensor, w: torch.Tensor, m: int, layout: Optional["ExpertLayout"] = None, dual: bool = False) -> bool:
+    """Whether :func:`linear` runs this product with the row-streaming kernel: at most 8 rows (per expert tile when grouped; of
+    a plain float32 product up to 32, see ``F32_STREAM_ANY``), width a multiple of 8, 32-byte aligned rows."""
     K = x.shape[-1]
-    most = F32_STREAM_ROWS if x.dtype == torch.float32 and w.dtype == torch.float32 else FEW_ROWS
-    rows_ok = layout.tile_m <= FEW_ROWS if layout is not None else m <= most
+    if layout is not None:
+        rows_ok = layout.tile_m <= FEW_ROWS
+    elif x.dtype == torch.float32 and w.dtype == torch.float32:
+        rows_ok = m <= (F32_STREAM_PAIR if dual else F32_STREAM_ANY) or (
+            m <= F32_STREAM_ROWS and m * w.numel() * (2 if dual else 1) <= F32_STREAM_WORK)
+    else:
+        rows_ok = m <= FEW_ROWS
     return (rows_ok and K % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 32 == 0 and w.data_ptr() % 32 == 0)
 
 
@@ -621,7 +634,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         )
         _check(code, "linear", f"(skinny; M={M}, N={N}, K={K}, tile {tile})")
         return
-    if few_rows_take(x, w, M, layout):
+    if few_rows_take(x, w, M, layout, w2 is not None):
         # a handful of rows: bandwidth-bound row-streaming kernel (csrc/gemv.cu)
         if layout is not None:
             te, t0, tr, nt = layout.tile_expert, layout.tile_row0, layout.tile_rows, layout.n_tiles

@@ -595,6 +595,48 @@ def test_linear_float32_tiles(M, N, K_, dual):
 
 
 @pytest.mark.parametrize("dual", [False, True])
+@pytest.mark.parametrize("N,K_", [(331, 136), (5, 520), (331, 2048), (1, 5632), (20004, 136), (20004, 520), (333, 5632)])
+def test_linear_float32_row_streaming(N, K_, dual, monkeypatch):
+    """The float32 row-streaming kernel at its edges: pieces of 128 columns in a ring of three (K that ends within the first, that
+    wraps the ring and that ends within a piece), K whole and shared by two to eight warps (by N and K), weight rows behind
+    the last, tiles of 8 rows with 1 to 8 of them; bias, row scale, added to what is there.  (One and two rows: the
+    warp-per-row kernel.)"""
+    monkeypatch.setattr(K, "F32_STREAM_WORK", 10 ** 12)
+    w, w2, b = rnd(N, K_, seed=2, scale=K_ ** -0.5), rnd(N, K_, seed=3, scale=K_ ** -0.5), rnd(N, seed=4)
+    dw, dw2, db = w.to(DEV), w2.to(DEV), b.to(DEV)
+    for M in (2, 3, 8, 9, 17, 31, 32):
+        x, old, rs = rnd(M, K_, seed=M), rnd(M, N, seed=5), rnd(M, seed=6)
+        dx, out = x.to(DEV), old.to(DEV)
+        assert K.few_rows_take(dx, dw, M)
+        K.linear(dx, dw, out, w2=dw2 if dual else None, bias=db, row_scale=rs.to(DEV), accumulate=True)
+        g = x.double() @ w.double().T
+        v = torch.nn.functional.silu(g) * (x.double() @ w2.double().T) if dual else g
+        close(out, old.double() + (v + b.double()) * rs.double()[:, None], torch.float32, f"{M} x {N} x {K_} dual={dual}")
+
+
+@pytest.mark.parametrize("H,I", [(520, 136), (2048, 264)])
+def test_linear_float32_row_streaming_of_experts(H, I):
+    """The same over experts' tiles of 8 rows, their rows gathered from the tokens'."""
+    T, E, k = 40, 5, 2
+    ids = _route(T, E, k, 3)
+    ids[:20] = 1   # one expert with several tiles
+    h, wg, wu, wd = rnd(T, H, seed=1), rnd(E, I, H, seed=2, scale=H ** -0.5), rnd(E, I, H, seed=3, scale=H ** -0.5), rnd(E, H, I, seed=4)
+    wts = torch.rand(T * k, generator=torch.Generator().manual_seed(5))
+    lay, ref_lay = K.ExpertLayout(T * k, E, 64, DEV), EK.ExpertLayout(T * k, E, 64, "cpu")
+    K.moe_sort(ids.to(DEV), T * k, lay, K.FEW_ROWS)
+    EK.moe_sort(ids, T * k, ref_lay, K.FEW_ROWS)
+    act, ref_act = torch.empty(T * k, I, device=DEV), torch.empty(T * k, I, dtype=torch.float64)
+    assert K.few_rows_take(h.to(DEV), wg.to(DEV), T * k, lay)
+    K.linear(h.to(DEV), wg.to(DEV), act, w2=wu.to(DEV), x_rows=lay.sorted_pair, x_row_div=k, layout=lay, n_rows=T * k)
+    EK.linear(h, wg, ref_act, w2=wu, x_rows=ref_lay.sorted_pair, x_row_div=k, layout=ref_lay, n_rows=T * k)
+    close(act, ref_act, torch.float32, "gate and up")
+    out, ref = torch.empty(T * k, H, device=DEV), torch.empty(T * k, H, dtype=torch.float64)
+    K.linear(act, wd.to(DEV), out, layout=lay, n_rows=T * k, row_scale=wts.to(DEV), scale_rows=lay.sorted_pair)
+    EK.linear(act.cpu(), wd, ref, layout=ref_lay, n_rows=T * k, row_scale=wts, scale_rows=ref_lay.sorted_pair)
+    close(out, ref, torch.float32, "down")
+
+
+@pytest.mark.parametrize("dual", [False, True])
 def test_linear_float32_of_few_rows_and_millions_of_weight_rows(dual):
     """More weight rows than 65,535 blocks of the row-streaming kernel hold (2,097,120, of a pair half as many)."""
     N, K_ = (2_097_120 >> dual) + 5, 8
