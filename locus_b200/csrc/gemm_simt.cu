@@ -94,10 +94,26 @@ __device__ __forceinline__ float scale_of(const GemmArgs& a, int r) {
     return a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
 }
 
-// The same, stored or added.
+// The same, stored or added, for the kernels that unroll it over a thread's outputs (with the biases in hand it ran 2 us longer).
 template <bool SWIGLU>
 __device__ __forceinline__ void epilogue(const GemmArgs& a, int r, int n, float rs, float v, float v2) {
-    v = finish<SWIGLU>(a, rs, v, v2, bias_of(a, n), a.act == 4 ? bias_of(a, a.N + n) : 0.f);
+    if (SWIGLU && a.act == 2) {
+        const float g = fminf(v * rs, a.act_param);
+        const float u = fminf(fmaxf(v2 * rs, -a.act_param), a.act_param);
+        v = g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
+    } else if (SWIGLU && a.act == 4) {
+        v = fmaxf(v + pair_bias(a.bias, a.bias_dt, n), 0.f) * (v2 + pair_bias(a.bias, a.bias_dt, a.N + n));
+    } else if (SWIGLU) {
+        const float g = v;
+        v = g / (1.0f + expf(-g)) * v2;
+    }
+    if (a.bias && a.act != 4) v += ld_dyn(a.bias, a.bias_dt, n);
+    if (a.act == 1) {
+        v = fmaxf(v, 0.f);
+        v *= v;
+    }
+    if (a.row_scale && a.act != 2) v *= rs;
+    if (a.act == 3) v = a.act_param * tanhf(v * a.act_scale / a.act_param);
     const size_t o = static_cast<size_t>(r) * a.ldo + n;
     if (a.accumulate) {
         static_cast<float*>(a.out)[o] += v;
@@ -193,7 +209,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs a) {
         const int lrow = ty * 4 + i;
         if (lrow >= rows) continue;
         const int r = row0 + lrow;
-        const float rs = scale_of(a, r);
+        const float rs = a.row_scale ? a.row_scale[a.scale_rows ? a.scale_rows[r] : r] : 1.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = col0 + tx * 4 + j;
@@ -422,7 +438,11 @@ extern "C" int locus_gemm_simt(const void* x, int x_dt, const void* w, const voi
             return static_cast<int>(cudaGetLastError());
         }
     }
-    if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32 && ((K | ldx) & 3) == 0 &&
+    // Short sums stay on gemm_simt, whose blocks start and end quicker: up to 32 columns, and one weight's up to 127 while its tiles
+    // fit the GPU at once (gemm_simt / gemm_f32: 2,048 x 6,144 x 16 30 / 54 us, x 32 48 / 54, x 64 78 / 70; 64 x 512 x 64
+    // 6.3 / 11.1, x 96 8.5 / 12.8, x 128 10.4 / 9.1 in two parts; pairs of 64 x 512 x 32 9.1 / 9.0, x 64 12.1 / 11.0).
+    const bool is_short = splits <= 1 && (K <= 32 || (K < 128 && !swiglu && static_cast<long long>(ceil_div(N, 128)) * tiles <= 2 * n_sm));
+    if (x_dt == LOCUS_DT_F32 && w_dt == LOCUS_DT_F32 && !is_short && ((K | ldx) & 3) == 0 &&
         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w2)) & 15) == 0) {
         if (splits > 1 && (part == nullptr || splits > 8 || swiglu || tile_expert != nullptr || M > 65535)) return LOCUS_ERR_UNSUPPORTED;
         // tiles of 64 weight rows where tiles of 128 would leave SMs without one
