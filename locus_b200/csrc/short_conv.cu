@@ -295,18 +295,17 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS) head_rows_kernel(const PrepAr
     }
 }
 
-#define CONV_TT 8   // tokens of a warp
-
-// A grid of (groups of CONV_TT tokens, four units each, segments): a unit is a head of q, k or v, the last one the gates.
-template <typename T, int TAPS>
+// TT: tokens of a warp, 8 or 1.  A grid of (groups of TT tokens, four units each, segments): a unit is a head of q, k or v, the last
+// one the gates.
+template <typename T, int TAPS, int TT>
 __global__ void __launch_bounds__(128) conv_rows_kernel(const PrepArgs a) {
     pdl_entry();
     pdl_trigger();
-    const int seg = blockIdx.z, t0 = blockIdx.x * CONV_TT, qn = a.seg_qn[seg];
+    const int seg = blockIdx.z, t0 = blockIdx.x * TT, qn = a.seg_qn[seg];
     if (t0 >= qn) return;
     const int lane = threadIdx.x & 31, unit = blockIdx.y * 4 + (threadIdx.x >> 5);
     const int nq = a.heads[0], nk = a.heads[1], n_heads = nq + nk + a.heads[2];
-    const int t1 = min(t0 + CONV_TT, qn);
+    const int t1 = min(t0 + TT, qn);
     const size_t row0 = static_cast<size_t>(a.seg_q0[seg]);
     if (unit >= n_heads) {
         if (unit > n_heads || a.beta == nullptr) return;
@@ -345,7 +344,15 @@ __global__ void __launch_bounds__(128) conv_rows_kernel(const PrepArgs a) {
     };
     if (t0 > 0) {
 #pragma unroll
-        for (int j = 1; j < TAPS; ++j) input(t0 - TAPS + j, x[j]);   // (CONV_TT >= TAPS - 1: all of this portion)
+        for (int j = 1; j < TAPS; ++j) {
+            const int before = t0 - TAPS + j;   // (with TT >= TAPS - 1 always of this portion, else maybe in front of it)
+            if (TT >= TAPS - 1 || before >= 0) {
+                input(before, x[j]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x[j][k] = own ? old[static_cast<size_t>(ch + k) * (TAPS - 1) + before + TAPS - 1] : 0.f;
+            }
+        }
     }
     T* out = static_cast<T*>(which == 0 ? a.q_out : which == 1 ? a.k_out : a.v_out);
     for (int t = t0; t < t1; ++t) {
@@ -383,7 +390,10 @@ __global__ void __launch_bounds__(128) conv_rows_kernel(const PrepArgs a) {
 
 // Whether conv_rows_kernel takes the call: rows out, no rotation, no weights of a norm, no factor by position, every head's
 // channels in whole pieces of four that lie on 16-byte boundaries, at most 128 of them.
-static bool conv_rows_take(const PrepArgs& a) {
+// Heads of up to 32 channels leave most of a warp without a channel: while a warp a token fits the GPU at once head_prep is the
+// quicker of the two (64 single tokens of 16 heads of 32: 6.8 against 7.2 us).
+static bool conv_rows_take(const PrepArgs& a, bool one_wave) {
+    if (one_wave && a.laid[0] <= 32 && a.laid[1] <= 32 && a.laid[2] <= 32) return false;
     if (a.conv == nullptr || a.taps < 2 || a.taps > 4 || a.pool != nullptr || a.rot > 0 || a.norm == 3 || a.temp_coef != 0.f || a.ld % 4) return false;
     for (int w = 0; w < 3; ++w)
         if (a.heads[w] > 0 && (a.dim[w] % 4 || a.off[w] % 4 || a.laid[w] % 4 || a.laid[w] > 128)) return false;
@@ -391,12 +401,20 @@ static bool conv_rows_take(const PrepArgs& a) {
              reinterpret_cast<uintptr_t>(a.v_out)) & 15) == 0;
 }
 
-template <typename T>
+template <typename T, int TT>
 static void launch_conv_rows(const PrepArgs& a, int n_seg, int longest_new, int units, cudaStream_t stream) {
-    const dim3 grid((longest_new + CONV_TT - 1) / CONV_TT, (units + 3) / 4, n_seg);
-    if (a.taps == 2) locus_launch(conv_rows_kernel<T, 2>, grid, dim3(128), 0, stream, a);
-    else if (a.taps == 3) locus_launch(conv_rows_kernel<T, 3>, grid, dim3(128), 0, stream, a);
-    else locus_launch(conv_rows_kernel<T, 4>, grid, dim3(128), 0, stream, a);
+    const dim3 grid((longest_new + TT - 1) / TT, (units + 3) / 4, n_seg);
+    if (a.taps == 2) locus_launch(conv_rows_kernel<T, 2, TT>, grid, dim3(128), 0, stream, a);
+    else if (a.taps == 3) locus_launch(conv_rows_kernel<T, 3, TT>, grid, dim3(128), 0, stream, a);
+    else locus_launch(conv_rows_kernel<T, 4, TT>, grid, dim3(128), 0, stream, a);
+}
+
+// A warp walks eight tokens; short portions a warp a token while all of them fit the GPU at once (64 warps an SM), since
+// then only a warp's chain counts: 3 tokens of 16 heads of 64 7.7 -> 6.2 us, 16 tokens 13.6 -> 6.3, 8 requests of 16 14.3 -> 10.3.
+template <typename T>
+static void launch_conv_rows(const PrepArgs& a, int n_seg, int longest_new, int units, bool one_wave, cudaStream_t stream) {
+    if (longest_new > 1 && one_wave) launch_conv_rows<T, 1>(a, n_seg, longest_new, units, stream);
+    else launch_conv_rows<T, 8>(a, n_seg, longest_new, units, stream);
 }
 
 template <typename T>
@@ -492,9 +510,10 @@ extern "C" int locus_head_prep(const float* proj, int ld, const int* sizes, cons
     const int units = a.heads[0] + a.heads[1] + a.heads[2] + (beta != nullptr ? 1 : 0);
     const dim3 grid((units + 3) / 4, longest_new, n_seg);
     if (out_dt != LOCUS_DT_F32 && out_dt != LOCUS_DT_BF16) return LOCUS_ERR_UNSUPPORTED;
-    if (conv_rows_take(a)) {
-        if (out_dt == LOCUS_DT_F32) launch_conv_rows<float>(a, n_seg, longest_new, units, stream);
-        else launch_conv_rows<bf16>(a, n_seg, longest_new, units, stream);
+    const bool one_wave = static_cast<long long>(longest_new) * units * n_seg <= 64 * 148;
+    if (conv_rows_take(a, one_wave)) {
+        if (out_dt == LOCUS_DT_F32) launch_conv_rows<float>(a, n_seg, longest_new, units, one_wave, stream);
+        else launch_conv_rows<bf16>(a, n_seg, longest_new, units, one_wave, stream);
     } else if (out_dt == LOCUS_DT_F32) {
         locus_launch(head_prep_kernel<float>, grid, dim3(128), 0, stream, a);
     } else {

@@ -309,30 +309,23 @@ def test_delta_output_stage_and_gate_rows_against_their_twins(heads, v_dim, shar
     assert _close(out, want, tol) and _close(gated, want_rows, tol)
 
 
-@pytest.mark.parametrize("odt", DTYPES, ids=IDS)
-@pytest.mark.parametrize("heads,dims,laid,taps,norm,act,gated", [
-    ((2, 2, 4), (16, 16, 12), (16, 16, 16), 4, "unit", True, True), ((1, 3, 1), (128, 128, 100), (128, 128, 128), 3, "rms", False, False),
-    ((3, 1, 2), (40, 40, 128), (40, 40, 128), 2, None, True, True)])
-def test_convolved_rows_against_their_twin(heads, dims, laid, taps, norm, act, gated, odt):
-    """Channels in 16-byte pieces (a kernel of their own walks eight tokens of a head): portions of one token, of fewer than
-    the convolution's reach, and that end in front of, on and behind eight."""
+def _convolved(heads, dims, laid, taps, norm, act, gated, odt, segs):
     import locus_b200.kernels as K
 
-    segs = [1, 2, 7, 8, 9, 33]
     T, starts = sum(segs), [sum(segs[:i]) for i in range(len(segs))]
     widths = [h * d for h, d in zip(heads, dims)]
     offsets = (4, 4 + widths[0], 8 + widths[0] + widths[1])
     off_b = offsets[2] + widths[2]
     off_a, H, C = off_b + heads[2], heads[2], sum(widths)
     proj = _rand((T, -(-(off_a + H) // 4) * 4), 11, 1.2)
-    conv, state0 = _rand((C, taps), 12, 0.7, torch.bfloat16), _rand((8, 3 + C * (taps - 1)), 13, 0.8)
+    conv, state0 = _rand((C, taps), 12, 0.7, torch.bfloat16), _rand((len(segs) + 2, 3 + C * (taps - 1)), 13, 0.8)
     a_log, dt_bias = _rand((H,), 14, 1.0), _rand((H,), 15, 1.0)
 
     def run(mod, cv, dt):
         rows = [cv(torch.full((T, h * l), 7.0, dtype=dt, device="cuda")) for h, l in zip(heads, laid)]
         state = cv(state0.clone()) if dt == odt else state0.cpu().double()
         gates = [cv(torch.zeros(T, H, dtype=torch.float32, device="cuda")) for _ in range(2)]
-        mod.head_prep(cv(proj), offsets=offsets, heads=heads, dims=dims, laid=laid, state_slots=cv(_dev([3, 0, 5, 2, 7, 1])),
+        mod.head_prep(cv(proj), offsets=offsets, heads=heads, dims=dims, laid=laid, state_slots=cv(_dev([3, 0, 5, 2, 7, 1] + list(range(8, len(segs) + 2)))),
                       seg_q0=cv(_dev(starts)), seg_qn=cv(_dev(segs)), n_seg=len(segs), longest_new=max(segs),
                       positions=cv(_dev(list(range(T)))), q_out=rows[0], k_out=rows[1], v_out=rows[2], conv=cv(conv), state=state,
                       conv_offset=3, act=act, norm=norm, eps=1e-6, q_scale=0.37,
@@ -348,6 +341,24 @@ def test_convolved_rows_against_their_twin(heads, dims, laid, taps, norm, act, g
     tol = 2e-5 if odt == torch.float32 else 6e-3
     for g, w, t in zip(got, want, (tol, tol, tol, 1e-6, 2e-5, 2e-5)):
         assert _close(g, w, t)
+
+
+@pytest.mark.parametrize("odt", DTYPES, ids=IDS)
+@pytest.mark.parametrize("heads,dims,laid,taps,norm,act,gated", [
+    ((2, 2, 4), (16, 16, 12), (16, 16, 16), 4, "unit", True, True), ((1, 3, 1), (128, 128, 100), (128, 128, 128), 3, "rms", False, False),
+    ((3, 1, 2), (40, 40, 128), (40, 40, 128), 2, None, True, True)])
+def test_convolved_rows_against_their_twin(heads, dims, laid, taps, norm, act, gated, odt):
+    """Channels in 16-byte pieces (a kernel of their own walks eight tokens of a head): portions of one token, of fewer than
+    the convolution's reach, and that end in front of, on and behind eight."""
+    _convolved(heads, dims, laid, taps, norm, act, gated, odt, [1, 2, 7, 8, 9, 33])
+
+
+@pytest.mark.parametrize("heads,dims,laid,taps,norm,act,gated", [
+    ((3, 2, 4), (16, 16, 12), (16, 16, 16), 4, "unit", True, True), ((5, 3, 1), (64, 64, 20), (64, 64, 20), 3, "rms", False, False),
+    ((3, 1, 4), (40, 40, 128), (40, 40, 128), 2, None, True, True)])
+def test_convolved_rows_of_many_portions(heads, dims, laid, taps, norm, act, gated):
+    """More warps than the GPU holds at a token each: eight tokens to a warp, portions that end in front of, on and behind eight."""
+    _convolved(heads, dims, laid, taps, norm, act, gated, torch.float32, [1, 2, 7, 8, 9, 33] + [17, 1, 41, 16] * 12)
 
 
 @pytest.mark.parametrize("odt", DTYPES, ids=IDS)
