@@ -44,13 +44,71 @@ struct GlaArgs {
     float q_scale;
 };
 
+// A request of few tokens in a walk's block of 256 threads: 32 columns from col0 on x 8 groups of R consecutive rows (d <= 8 R), the
+// sums of a column as gla_tokens_kernel below takes them (which as an instance of this function ran 7 to 11 % longer).
+// part: [4][16] for either half of the columns.
+template <int R>
+__device__ __forceinline__ void gla_few(const GlaArgs& a, int seg, int h, int col0, float (*ops)[8 * R], float (*part)[16]) {
+    constexpr int DP = 8 * R;
+    const int tid = threadIdx.x, half = tid >> 7, rg = (tid & 127) >> 4, c = tid & 15, wid = (tid & 127) >> 5;
+    const int col = col0 + 16 * half + c;
+    const int qn = a.seg_qn[seg], q0 = a.seg_q0[seg];
+    const int d = a.d, dv = a.dv;
+    const bool col_ok = col < dv;
+    float* S = a.state + static_cast<size_t>(a.state_slots[seg]) * a.slot_stride + static_cast<size_t>(h) * d * dv;
+    part += 4 * half;
+    float s[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = rg * R + i;
+        s[i] = (r < d && col_ok) ? S[static_cast<size_t>(r) * dv + col] : 0.f;
+    }
+    for (int t = 0; t < qn; ++t) {
+        const size_t row = static_cast<size_t>(q0 + t);
+        const float vv = col_ok ? a.v[row * a.ldv + a.off_v + h * dv + col] : 0.f;
+        for (int r = tid; r < DP; r += 256) {
+            ops[0][r] = r < d ? a.q[row * a.ldq + a.off_q + h * d + r] : 0.f;
+            ops[1][r] = r < d ? a.k[row * a.ldk + a.off_k + h * d + r] : 0.f;
+            ops[2][r] = r < d ? a.a[row * a.lda + a.off_a + h * d + r] : 0.f;
+        }
+        __syncthreads();
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; i += 4) {
+            const float4 qv = *reinterpret_cast<const float4*>(&ops[0][rg * R + i]);
+            const float4 kv = *reinterpret_cast<const float4*>(&ops[1][rg * R + i]);
+            const float4 av = *reinterpret_cast<const float4*>(&ops[2][rg * R + i]);
+            s[i] = fmaf(kv.x, vv, fmaf(-av.x, s[i], s[i]));
+            s[i + 1] = fmaf(kv.y, vv, fmaf(-av.y, s[i + 1], s[i + 1]));
+            s[i + 2] = fmaf(kv.z, vv, fmaf(-av.z, s[i + 2], s[i + 2]));
+            s[i + 3] = fmaf(kv.w, vv, fmaf(-av.w, s[i + 3], s[i + 3]));
+            o0 = fmaf(s[i], qv.x, o0);
+            o1 = fmaf(s[i + 1], qv.y, o1);
+            o0 = fmaf(s[i + 2], qv.z, o0);
+            o1 = fmaf(s[i + 3], qv.w, o1);
+        }
+        float o = o0 + o1;
+        o += __shfl_xor_sync(0xffffffffu, o, 16);
+        if ((tid & 31) < 16) part[wid][c] = o;
+        __syncthreads();   // (also: nobody reads the operands any more)
+        if (rg == 0 && col_ok)
+            a.out[row * a.ldo + h * dv + col] = ((part[0][c] + part[1][c]) + (part[2][c] + part[3][c])) * a.q_scale;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = rg * R + i;
+        if (r < d && col_ok) S[static_cast<size_t>(r) * dv + col] = s[i];
+    }
+}
+
 #define GL_STAGES 2   // (three: two blocks an SM instead of three, 1,390 us for eight requests of 2,048 tokens, not 1,290)
 #define GL_TT 16   // tokens of a tile
 
 // RPL: rows of a column that a lane keeps, of two columns (d <= 32 RPL).  VEC: the rows of q, k and a of a head start on
-// 16-byte boundaries and d is a multiple of 4, so four rows are one copy.
-template <int RPL, bool VEC>
-__global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) gla_walk_kernel(const GlaArgs a, int col_blocks) {
+// 16-byte boundaries and d is a multiple of 4, so four rows are one copy.  MIXED: requests of up to `few` tokens are taken token by
+// token.
+template <int RPL, bool VEC, bool MIXED>
+__global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) gla_walk_kernel(const GlaArgs a, int col_blocks, int few) {
     constexpr int DP = 32 * RPL, CB = WALK_CW * WALK_WARPS, TT = GL_TT, TILE = TT * (3 * DP + 2 * CB), NT = 32 * WALK_WARPS;
     constexpr int RV = RPL < 4 ? RPL : 4;                // rows of a load
     extern __shared__ __align__(16) float walk_smem[];   // [GL_STAGES][q, k, a: [TT][DP]; v: [TT][CB], every value twice]
@@ -61,6 +119,14 @@ __global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) gla_walk_ker
     const int seg = blockIdx.y, h = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * CB;
     const int qn = a.seg_qn[seg], q0 = a.seg_q0[seg];
     if (qn <= 0) return;
+    static_assert(NT == 256 && CB == 16, "gla_few takes the columns of two blocks");
+    if (MIXED && qn <= few) {   // a request of few tokens beside portions: every other block does two blocks' columns
+        if ((blockIdx.x % col_blocks) & 1) return;
+        float (*part)[16] = reinterpret_cast<float (*)[16]>(walk_smem + 3 * DP);
+        if (RPL == 2 && a.d <= 32) gla_few<4>(a, seg, h, col0, reinterpret_cast<float (*)[32]>(walk_smem), part);
+        else gla_few<4 * RPL>(a, seg, h, col0, reinterpret_cast<float (*)[DP]>(walk_smem), part);
+        return;
+    }
     const int d = a.d, dv = a.dv, wc = wid * WALK_CW;
     float* S = a.state + static_cast<size_t>(a.state_slots[seg]) * a.slot_stride + static_cast<size_t>(h) * d * dv;
 
@@ -292,21 +358,23 @@ extern "C" int locus_gla_decay(float* z, int ld, int off, int n, int T, float ta
     return locus_launch_status();
 }
 
-template <int RPL>
+template <int RPL, bool MIXED>
 static int gla_walk(const GlaArgs& a, bool vec, int n_seg, cudaStream_t stream) {
     constexpr int CB = WALK_CW * WALK_WARPS;
     constexpr size_t smem = sizeof(float) * GL_STAGES * GL_TT * (3 * 32 * RPL + 2 * CB);
     const int col_blocks = (a.dv + CB - 1) / CB;
-    auto* kernel = vec ? gla_walk_kernel<RPL, true> : gla_walk_kernel<RPL, false>;
+    auto* kernel = vec ? gla_walk_kernel<RPL, true, MIXED> : gla_walk_kernel<RPL, false, MIXED>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    locus_launch(kernel, dim3(a.H * col_blocks, n_seg), dim3(32 * WALK_WARPS), smem, stream, a, col_blocks);
+    locus_launch(kernel, dim3(a.H * col_blocks, n_seg), dim3(32 * WALK_WARPS), smem, stream, a, col_blocks,
+                 walk_few(static_cast<long long>(a.H) * col_blocks * n_seg));
     return locus_launch_status();
 }
 
-// n_rows: the rows of `out`, which bound the tokens of all segments together.  Where they are at most GL_FEW a segment the
-// walk's copies would mostly be of tokens that are not there.
-#define GL_FEW 2
+// n_rows: the rows of `out`, which bound the tokens of all segments together.  At most two a segment (decoding), or no
+// more than a lone request of few tokens: the tokens kernel.  Where portions may stand beside single tokens each block of the walk
+// looks at its own request: a prompt portion of 100 tokens beside 32 decoding requests, 16 heads of 128, takes 30 us;
+// all of it in tiles took 96, all of it token by token 52.
 extern "C" int locus_gla_scan(const float* q, int ldq, int off_q, const float* k, int ldk, int off_k, const float* v, int ldv,
                               int off_v, const float* dec, int lda, int off_a, float* state, long long slot_stride,
                               const int* state_slots, const int* seg_q0, const int* seg_qn, int n_seg, int n_rows, float* out,
@@ -317,7 +385,7 @@ extern "C" int locus_gla_scan(const float* q, int ldq, int off_q, const float* k
     a.q = q; a.k = k; a.v = v; a.a = dec; a.state = state; a.state_slots = state_slots; a.seg_q0 = seg_q0; a.seg_qn = seg_qn;
     a.out = out; a.slot_stride = slot_stride; a.ldq = ldq; a.off_q = off_q; a.ldk = ldk; a.off_k = off_k; a.ldv = ldv;
     a.off_v = off_v; a.lda = lda; a.off_a = off_a; a.ldo = ldo; a.H = H; a.d = d; a.dv = dv; a.q_scale = q_scale;
-    if (n_rows <= static_cast<long long>(GL_FEW) * n_seg) {
+    if (walk_not_needed(n_rows, n_seg, d)) {
         const int col_blocks = (dv + 15) / 16;
         const dim3 grid(H * col_blocks, n_seg);
         if (d <= 32) locus_launch(gla_tokens_kernel<4>, grid, dim3(128), 0, stream, a, col_blocks);
@@ -326,9 +394,10 @@ extern "C" int locus_gla_scan(const float* q, int ldq, int off_q, const float* k
         else locus_launch(gla_tokens_kernel<32>, grid, dim3(128), 0, stream, a, col_blocks);
         return locus_launch_status();
     }
+    const bool mixed = walk_may_be_mixed(n_rows, n_seg);
     const bool vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(dec)) & 15) == 0 &&
                      ((ldq | off_q | ldk | off_k | lda | off_a | d) & 3) == 0;
-    if (d <= 64) return gla_walk<2>(a, vec, n_seg, stream);
-    if (d <= 128) return gla_walk<4>(a, vec, n_seg, stream);
-    return gla_walk<8>(a, vec, n_seg, stream);
+    if (d <= 64) return mixed ? gla_walk<2, true>(a, vec, n_seg, stream) : gla_walk<2, false>(a, vec, n_seg, stream);
+    if (d <= 128) return mixed ? gla_walk<4, true>(a, vec, n_seg, stream) : gla_walk<4, false>(a, vec, n_seg, stream);
+    return mixed ? gla_walk<8, true>(a, vec, n_seg, stream) : gla_walk<8, false>(a, vec, n_seg, stream);
 }

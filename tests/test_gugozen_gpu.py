@@ -186,6 +186,40 @@ def test_gla_scan_of_few_tokens_and_of_tiles_edges(H, d, dv, precise):
         _cmp(st, ref_state, 2e-5)
 
 
+@pytest.mark.parametrize("H,d,dv", [(2, 24, 33), (3, 72, 40), (2, 130, 17)])
+def test_gla_scan_of_portions_beside_single_tokens(H, d, dv, precise):
+    """A step of portions and decoding requests: every block looks at its own request (few blocks: up to 4 tokens one by one, more
+    than three an SM: up to 20; odd numbers of sixteens of columns); a single token has the bits that it has in a decode step."""
+    import locus_b200.kernels as K
+
+    g = torch.Generator().manual_seed(d)
+    for qn in ([4, 5, 1, 40, 1], [20, 21, 1, 12, 17] * 40, [190, 64, 33, 1]):   # (the last: long enough not to be asked)
+        T, W, n_seg = sum(qn), 2 * H * d + H * dv, len(qn)
+        proj, z = torch.randn(T, W, generator=g), torch.rand(T, H * d, generator=g) * 0.3
+        state = torch.randn(n_seg, H * d * dv, generator=g)
+        slots = torch.arange(n_seg, dtype=torch.int32).flip(0).contiguous()
+        n = torch.tensor(qn, dtype=torch.int32)
+        q0 = (n.cumsum(0) - n).to(torch.int32)
+        kw = dict(n_heads=H, dim=d, v_dim=dv, q_scale=d ** -0.5)
+        ref_state, ref = state.double(), torch.zeros(T, H * dv, dtype=torch.float64)
+        EK.gla_scan(proj.double(), 0, proj.double(), H * d, proj.double(), 2 * H * d, z.double(), 0, ref_state, 0, slots, q0, n, n_seg, ref, **kw)
+        p, dz = proj.to(DEV), z.to(DEV)
+        st, out = state.to(DEV), torch.zeros(T, H * dv, device=DEV)
+        K.gla_scan(p, 0, p, H * d, p, 2 * H * d, dz, 0, st, 0, slots.to(DEV), q0.to(DEV), n.to(DEV), n_seg, out, **kw)
+        _cmp(out, ref, 2e-5)
+        _cmp(st, ref_state, 2e-5)
+        if len(qn) == 4:
+            continue
+        one = [i for i, c in enumerate(qn) if c == 1]
+        st1 = state.to(DEV)
+        pick = torch.tensor([int(q0[i]) for i in one])
+        p1, z1, o1 = proj[pick].to(DEV), z[pick].to(DEV), torch.zeros(len(one), H * dv, device=DEV)
+        K.gla_scan(p1, 0, p1, H * d, p1, 2 * H * d, z1, 0, st1, 0, slots[one].to(DEV), torch.arange(len(one), dtype=torch.int32, device=DEV),
+                   torch.ones(len(one), dtype=torch.int32, device=DEV), len(one), o1, **kw)
+        at = slots[one].long().to(DEV)
+        assert torch.equal(o1, out[pick.to(DEV)]) and torch.equal(st1[at], st[at])
+
+
 @pytest.mark.parametrize("H,d,dv", [(2, 24, 16), (1, 7, 5), (3, 72, 40), (2, 128, 64), (1, 200, 12)])
 def test_gla_scan_and_decay_against_twin(H, d, dv, precise):
     import locus_b200.kernels as K
