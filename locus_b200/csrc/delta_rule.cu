@@ -47,6 +47,76 @@ struct DeltaArgs {
     int H, heads_per_group, d, dv;
 };
 
+// A request of few tokens in a walk's block of 256 threads: 32 columns from col0 on x 8 groups of R consecutive rows (d <= 8 R), the
+// sums of a column as delta_tokens_kernel below takes them (which as an instance of this function ran 7 to 11 % longer).
+// part: [3][4][16] for either half of the columns.
+template <int R>
+__device__ __forceinline__ void delta_few(const DeltaArgs& a, int seg, int h, int col0, float (*ops)[8 * R], float (*part)[4][16]) {
+    constexpr int DP = 8 * R;
+    const int tid = threadIdx.x, half = tid >> 7, rg = (tid & 127) >> 4, c = tid & 15, wid = (tid & 127) >> 5;
+    const int col = col0 + 16 * half + c;
+    const int qn = a.seg_qn[seg], q0 = a.seg_q0[seg];
+    const int d = a.d, dv = a.dv, g = h / a.heads_per_group;
+    part += 3 * half;
+    const bool col_ok = col < dv;
+    float* S = a.state + static_cast<size_t>(a.state_slots[seg]) * a.slot_stride + static_cast<size_t>(h) * d * dv;
+    float s[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = rg * R + i;
+        s[i] = (r < d && col_ok) ? S[static_cast<size_t>(r) * dv + col] : 0.f;
+    }
+    for (int t = 0; t < qn; ++t) {
+        const size_t row = static_cast<size_t>(q0 + t);
+        const float vv = col_ok ? a.v[row * a.ldv + a.off_v + h * dv + col] : 0.f;
+        const float beta = a.beta[row * a.H + h], gd = a.decay[row * a.H + h];
+        for (int r = tid; r < DP; r += 256) {
+            ops[0][r] = r < d ? a.q[row * a.ldq + a.off_q + g * d + r] : 0.f;
+            ops[1][r] = r < d ? a.k[row * a.ldk + a.off_k + g * d + r] : 0.f;
+        }
+        __syncthreads();
+        float sk0 = 0.f, sk1 = 0.f, sq0 = 0.f, sq1 = 0.f, kq0 = 0.f, kq1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; i += 2) {
+            const float2 qv = *reinterpret_cast<const float2*>(&ops[0][rg * R + i]);
+            const float2 kv = *reinterpret_cast<const float2*>(&ops[1][rg * R + i]);
+            sk0 = fmaf(s[i], kv.x, sk0);
+            sq0 = fmaf(s[i], qv.x, sq0);
+            kq0 = fmaf(kv.x, qv.x, kq0);
+            sk1 = fmaf(s[i + 1], kv.y, sk1);
+            sq1 = fmaf(s[i + 1], qv.y, sq1);
+            kq1 = fmaf(kv.y, qv.y, kq1);
+        }
+        float sk = sk0 + sk1, sq = sq0 + sq1, kq = kq0 + kq1;
+        sk += __shfl_xor_sync(0xffffffffu, sk, 16);
+        sq += __shfl_xor_sync(0xffffffffu, sq, 16);
+        kq += __shfl_xor_sync(0xffffffffu, kq, 16);
+        if ((tid & 31) < 16) {
+            part[0][wid][c] = sk;
+            part[1][wid][c] = sq;
+            part[2][wid][c] = kq;
+        }
+        __syncthreads();
+        sk = (part[0][0][c] + part[0][1][c]) + (part[0][2][c] + part[0][3][c]);
+        sq = (part[1][0][c] + part[1][1][c]) + (part[1][2][c] + part[1][3][c]);
+        kq = (part[2][0][c] + part[2][1][c]) + (part[2][2][c] + part[2][3][c]);
+        const float u = beta * (vv - gd * sk);
+#pragma unroll
+        for (int i = 0; i < R; i += 2) {
+            const float2 kv = *reinterpret_cast<const float2*>(&ops[1][rg * R + i]);
+            s[i] = fmaf(gd, s[i], kv.x * u);
+            s[i + 1] = fmaf(gd, s[i + 1], kv.y * u);
+        }
+        if (rg == 0 && col_ok) a.out[row * a.ldo + h * dv + col] = fmaf(u, kq, gd * sq);
+        if (t + 1 < qn) __syncthreads();   // nobody reads this token's operands and sums any more
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = rg * R + i;
+        if (r < d && col_ok) S[static_cast<size_t>(r) * dv + col] = s[i];
+    }
+}
+
 #define DR_STAGES 3
 #define DR_TT 16       // tokens of a tile
 #define DR_G 4         // tokens that are worked on together
@@ -56,9 +126,9 @@ struct DeltaArgs {
 #define DR_COEF (DR_P + DR_G * DR_G)
 
 // RPL: rows of a column that a lane keeps, of two columns (d <= 32 RPL).  VEC: q's and k's rows of a head start on 16-byte
-// boundaries and d is a multiple of 4, so four rows are one copy.
-template <int RPL, bool VEC>
-__global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) delta_walk_kernel(const DeltaArgs a, int col_blocks) {
+// boundaries and d is a multiple of 4, so four rows are one copy.  MIXED: requests of up to `few` tokens are taken token by token.
+template <int RPL, bool VEC, bool MIXED>
+__global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) delta_walk_kernel(const DeltaArgs a, int col_blocks, int few) {
     constexpr int DP = 32 * RPL, LD = DP + 8, TT = DR_TT, CB = WALK_CW * WALK_WARPS, NT = 32 * WALK_WARPS;
     constexpr int RV = RPL < 4 ? RPL : 4;          // rows of a load
     constexpr int TILE = TT * (2 * LD + CB + 2);   // q, k: [TT][LD]; v: [TT][CB]; beta, decay: [TT]
@@ -71,6 +141,14 @@ __global__ void __launch_bounds__(32 * WALK_WARPS, RPL > 4 ? 2 : 3) delta_walk_k
     const int seg = blockIdx.y, h = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * CB;
     const int qn = a.seg_qn[seg], q0 = a.seg_q0[seg];
     if (qn <= 0) return;
+    static_assert(NT == 256 && CB == 16, "delta_few takes the columns of two blocks");
+    if (MIXED && qn <= few) {   // a request of few tokens beside portions: every other block does two blocks' columns
+        if ((blockIdx.x % col_blocks) & 1) return;
+        float (*part)[4][16] = reinterpret_cast<float (*)[4][16]>(walk_smem + 2 * DP);
+        if (RPL == 2 && a.d <= 32) delta_few<4>(a, seg, h, col0, reinterpret_cast<float (*)[32]>(walk_smem), part);
+        else delta_few<4 * RPL>(a, seg, h, col0, reinterpret_cast<float (*)[DP]>(walk_smem), part);
+        return;
+    }
     const int d = a.d, dv = a.dv, wc = wid * WALK_CW, col = col0 + wc;
     float* S = a.state + static_cast<size_t>(a.state_slots[seg]) * a.slot_stride + static_cast<size_t>(h) * d * dv;
     const int g = h / a.heads_per_group;
@@ -364,22 +442,24 @@ __global__ void __launch_bounds__(128) delta_tokens_kernel(const DeltaArgs a, in
     }
 }
 
-template <int RPL>
+template <int RPL, bool MIXED>
 static int delta_walk(const DeltaArgs& a, bool vec, int n_seg, cudaStream_t stream) {
     constexpr int CB = WALK_CW * WALK_WARPS;
     constexpr size_t smem = sizeof(float) * (DR_STAGES * DR_TT * (2 * (32 * RPL + 8) + CB + 2) + DR_TT / DR_G * DR_COEF);
     static_assert(DR_TT / DR_G * 2 * DR_G * DR_G <= 32 * WALK_WARPS, "two threads to a pair of tokens");
     const int col_blocks = (a.dv + CB - 1) / CB;
-    auto* kernel = vec ? delta_walk_kernel<RPL, true> : delta_walk_kernel<RPL, false>;
+    auto* kernel = vec ? delta_walk_kernel<RPL, true, MIXED> : delta_walk_kernel<RPL, false, MIXED>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    locus_launch(kernel, dim3(a.H * col_blocks, n_seg), dim3(32 * WALK_WARPS), smem, stream, a, col_blocks);
+    locus_launch(kernel, dim3(a.H * col_blocks, n_seg), dim3(32 * WALK_WARPS), smem, stream, a, col_blocks,
+                 walk_few(static_cast<long long>(a.H) * col_blocks * n_seg));
     return locus_launch_status();
 }
 
-// n_rows: the rows of `out`, which bound the tokens of all segments together.  Where they are at most DR_FEW a segment the
-// walk's copies and pairs would mostly be of tokens that are not there.
-#define DR_FEW 2
+// n_rows: the rows of `out`, which bound the tokens of all segments together.  At most two a segment (decoding), or no
+// more than a lone request of few tokens: the tokens kernel.  Where portions may stand beside single tokens each block of the walk
+// looks at its own request: a prompt portion of 100 tokens beside 32 decoding requests, 16 heads of 128, takes 41 us;
+// all of it in tiles took 107, all of it token by token 55.
 extern "C" int locus_delta_scan(const float* q, int ldq, int off_q, const float* k, int ldk, int off_k, const float* v, int ldv,
                                 int off_v, const float* beta, const float* decay, float* state, long long slot_stride,
                                 const int* state_slots, const int* seg_q0, const int* seg_qn, int n_seg, int n_rows, float* out,
@@ -392,7 +472,7 @@ extern "C" int locus_delta_scan(const float* q, int ldq, int off_q, const float*
     a.seg_q0 = seg_q0; a.seg_qn = seg_qn; a.out = out; a.slot_stride = slot_stride; a.ldq = ldq; a.off_q = off_q;
     a.ldk = ldk; a.off_k = off_k; a.ldv = ldv; a.off_v = off_v; a.ldo = ldo; a.H = H; a.heads_per_group = heads_per_group;
     a.d = d; a.dv = dv;
-    if (n_rows <= static_cast<long long>(DR_FEW) * n_seg) {
+    if (walk_not_needed(n_rows, n_seg, d)) {
         const int col_blocks = (dv + 15) / 16;
         const dim3 grid(H * col_blocks, n_seg);
         if (d <= 32) locus_launch(delta_tokens_kernel<4>, grid, dim3(128), 0, stream, a, col_blocks);
@@ -401,11 +481,12 @@ extern "C" int locus_delta_scan(const float* q, int ldq, int off_q, const float*
         else locus_launch(delta_tokens_kernel<32>, grid, dim3(128), 0, stream, a, col_blocks);
         return locus_launch_status();
     }
+    const bool mixed = walk_may_be_mixed(n_rows, n_seg);
     const bool vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) == 0 &&
                      ((ldq | off_q | ldk | off_k | d) & 3) == 0;
-    if (d <= 64) return delta_walk<2>(a, vec, n_seg, stream);
-    if (d <= 128) return delta_walk<4>(a, vec, n_seg, stream);
-    return delta_walk<8>(a, vec, n_seg, stream);
+    if (d <= 64) return mixed ? delta_walk<2, true>(a, vec, n_seg, stream) : delta_walk<2, false>(a, vec, n_seg, stream);
+    if (d <= 128) return mixed ? delta_walk<4, true>(a, vec, n_seg, stream) : delta_walk<4, false>(a, vec, n_seg, stream);
+    return mixed ? delta_walk<8, true>(a, vec, n_seg, stream) : delta_walk<8, false>(a, vec, n_seg, stream);
 }
 
 __device__ __forceinline__ float dr_silu(float x) { return x / (1.0f + expf(-x)); }

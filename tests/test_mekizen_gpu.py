@@ -253,6 +253,48 @@ def test_delta_rule_of_few_tokens_and_of_tiles_edges(heads, per_group, dim, v_di
         assert _close(out, out_w, 3e-5) and _close(state, st_w, 3e-5)
 
 
+@pytest.mark.parametrize("heads,per_group,dim,v_dim", [(2, 1, 24, 33), (4, 2, 72, 40), (2, 1, 130, 17)])
+def test_delta_rule_of_portions_beside_single_tokens(heads, per_group, dim, v_dim):
+    """A step of portions and decoding requests: every block looks at its own request (few blocks: up to 4 tokens one by one, more
+    than three an SM: up to 20; odd numbers of sixteens of columns); a single token has the bits that it has in a decode step."""
+    import locus_b200.kernels as K
+
+    G = heads // per_group
+    kw = dict(n_heads=heads, heads_per_group=per_group, dim=dim, v_dim=v_dim)
+    for qn in ([4, 5, 1, 40, 1], [20, 21, 1, 12, 17] * 40, [190, 64, 33, 1]):   # (the last: long enough not to be asked)
+        T, n_seg = sum(qn), len(qn)
+        starts = [sum(qn[:i]) for i in range(n_seg)]
+        rows = _rand((T, 2 * G * dim + heads * v_dim), 5, 0.6)
+        k = rows[:, G * dim:2 * G * dim].view(T, G, dim)
+        k /= k.norm(dim=-1, keepdim=True)
+        beta = torch.rand(T, heads, generator=torch.Generator().manual_seed(2)).cuda()
+        decay = torch.rand(T, heads, generator=torch.Generator().manual_seed(1)).cuda()
+        state0 = _rand((n_seg, heads * dim * v_dim), 6, 0.3)
+        slots = list(range(n_seg))[::-1]
+
+        def run(fn, r, b, g, s, o, sl, q0, n, to):
+            fn(r, 0, r, G * dim, r, 2 * G * dim, b, g, s, 0, to(_dev(sl)), to(_dev(q0)), to(_dev(n)), len(n), o, **kw)
+
+        st_w, out_w = state0.cpu().double(), torch.zeros(T, heads * v_dim, dtype=torch.float64)
+        EK.PRECISE = True
+        try:
+            run(EK.delta_rule, rows.cpu(), beta.cpu(), decay.cpu(), st_w, out_w, slots, starts, qn, lambda x: x.cpu())
+        finally:
+            EK.PRECISE = False
+        state, out = state0.clone(), torch.zeros(T, heads * v_dim, device="cuda")
+        run(K.delta_rule, rows, beta, decay, state, out, slots, starts, qn, lambda x: x)
+        assert _close(out, out_w, 3e-5) and _close(state, st_w, 3e-5)
+        if len(qn) == 4:
+            continue
+        one = [i for i, c in enumerate(qn) if c == 1]
+        pick = [starts[i] for i in one]
+        state1, out1 = state0.clone(), torch.zeros(len(one), heads * v_dim, device="cuda")
+        run(K.delta_rule, rows[pick].contiguous(), beta[pick].contiguous(), decay[pick].contiguous(), state1, out1,
+            [slots[i] for i in one], list(range(len(one))), [1] * len(one), lambda x: x)
+        at = [slots[i] for i in one]
+        assert torch.equal(out1, out[pick]) and torch.equal(state1[at], state[at])
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("dim,v_dim", [(24, 16), (128, 20), (200, 16)])
 def test_delta_rule_keeps_what_is_not_finite_behind_its_token(dim, v_dim, bad):
