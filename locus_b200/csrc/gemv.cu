@@ -17,8 +17,8 @@
 // second piece spilled: 3.8 TB/s on the head).  Where a plain product has few weight rows (fewer than 20,000: 5,000 warps, two
 // rounds of the 16 that an SM holds) two, four or eight warps share K in pieces and their shares are added in order, the
 // number following from N and K alone.  Measured at 8 rows: 151,936 x 2,048 264 us = 4.7 TB/s, 6,144 x 2,048 19.4 us (39.7
-// before), the routed experts of 8 tokens 141 us = 5.9 TB/s (192 before); 16 / 32 rows of 6,144 x 2,048 in tiles of 8, which
-// find the weights in L2, 36 / 71 us (163 on 64-row tiles).  One or two rows stay on the warp-per-row kernel (11.0 us
+// before), the routed experts of 8 tokens 141 us = 5.9 TB/s (192 before).  More rows run in tiles of 8 that find the weights in
+// L2, where that is quicker than gemm_simt.cu (kernels/__init__.py: F32_STREAM_ANY).  One or two rows stay on the warp-per-row kernel (11.0 us
 // against 13.4 at one row), and so do grouped products of up to 8 rows, whose few tiles hold a row each (a decode step of
 // one request, 24 layers of 60 experts with 4 picks: 3.20 ms against 3.49).
 #include "common.cuh"
@@ -298,17 +298,17 @@ __device__ __forceinline__ void f32_stream_body(const GemvArgs& a, const float* 
     gemv_store<DUAL>(a, r, n, rs, v, u);
 }
 
-// A flat grid, the tiles of 8 rows its fast index: the tiles of the same weights run together, so that a second tile finds them in
-// L2, and the blocks of weight rows have no limit of their own (65,535 of a second grid index would be 2.1 million rows).
+// Grid (tiles of 8 rows, blocks of weight rows, and again): the tiles of the same weights run together, so that a second tile finds them
+// in L2; the blocks go on along the third index, since 65,535 along the second hold 2.1 million rows.
 template <bool DUAL>
-__global__ void __launch_bounds__(32 * GV_WARPS, 2) f32_stream_kernel(GemvArgs a, int tiles, int split) {
+__global__ void __launch_bounds__(32 * GV_WARPS, 2) f32_stream_kernel(GemvArgs a, int split) {
     extern __shared__ __align__(16) float ring_smem[];   // [warp][stage][weight row][128]
     __shared__ float shares[GV_WARPS][GV_NC * GV_ROWS];
     const float* W = static_cast<const float*>(a.w);
     const float* W2 = static_cast<const float*>(a.w2);
     int row0, rows;
     const bool grouped = a.tile_expert != nullptr;
-    const int tile = blockIdx.x % tiles, block = blockIdx.x / tiles;
+    const int tile = blockIdx.x, block = blockIdx.z * gridDim.y + blockIdx.y;
     if (grouped) {
         pdl_entry();   // (the lists come from the kernels in front)
         if (tile >= *a.n_tiles) return;
@@ -333,14 +333,14 @@ static int launch_f32(const GemvArgs& a, int tiles, bool dual, cudaStream_t stre
     const int groups = ceil_div(a.N, dual ? GV_NC / 2 : GV_NC);   // four weight rows each
     int split = 1;
     while (a.tile_expert == nullptr && split < GV_WARPS && groups * split < 5000 && a.K >= 256 * split) split *= 2;
-    const long long blocks = static_cast<long long>(tiles) * ceil_div(groups, GV_WARPS / split);
-    if (blocks == 0) return 0;
-    if (blocks > 0x7fffffffLL) return LOCUS_ERR_UNSUPPORTED;
+    const int blocks = ceil_div(groups, GV_WARPS / split), layers = ceil_div(blocks, 65535);
+    const dim3 grid(tiles, layers > 0 ? ceil_div(blocks, layers) : 0, layers);
+    if (grid.x == 0 || grid.y == 0) return 0;
     constexpr size_t smem = sizeof(float) * GV_WARPS * GV_STAGES * GV_NC * 128;
     auto* kernel = dual ? f32_stream_kernel<true> : f32_stream_kernel<false>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
-    locus_launch(kernel, dim3(static_cast<unsigned>(blocks)), dim3(32 * GV_WARPS), smem, stream, a, tiles, split);
+    locus_launch(kernel, grid, dim3(32 * GV_WARPS), smem, stream, a, split);
     return locus_launch_status();
 }
 
