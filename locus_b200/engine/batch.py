@@ -112,7 +112,8 @@ class _SideScope:
         rt.side_stream.wait_event(rt._fork_event)
         self._ctx = torch.cuda.stream(rt.side_stream)
         self._ctx.__enter__()
-        self._scope = K.stream_scope(rt.side_split_scratch)
+        # (a runner's step; parts that are called by themselves take the stream's buffer, which the next runtime finds again)
+        self._scope = K.stream_scope(rt.side_split_scratch if K.scratch_is_owned() else None)
         self._scope.__enter__()
         K.timing_restart()
         return self

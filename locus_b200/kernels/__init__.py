@@ -96,6 +96,11 @@ class stream_scope:
         return False
 
 
+def scratch_is_owned() -> bool:
+    """Whether the scope that launches go to (:class:`stream_scope`) brings partial sums' buffers of its own."""
+    return _scratch_override is not None
+
+
 class kernel_times:
     """Opt-in table of where the time of eager steps goes, by entry point of this module (the reference has no
     profiler of its own: it prints counters at exit and is timed from outside).  Inside the scope an event is
