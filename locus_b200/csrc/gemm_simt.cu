@@ -1,7 +1,8 @@
 // Matrix products on CUDA cores with float32 FMA: out = x . W^T with fused epilogues.
 //
-// This is the true-32-bit path of every linear layer (no tensor cores, no TF32) and the
-// general fallback of the bfloat16 path for shapes the tensor-core kernels refuse.  In
+// This is the true-32-bit path of the linear layers whose work is too small for gemm_f32_tc.cuh (float32 on the tensor cores, no
+// TF32: the choice is f32_tc_takes in kernels/__init__.py) and the general fallback of the bfloat16 path for shapes the
+// tensor-core kernels refuse.  In
 // gemm_simt one thread accumulates an output over k = 0..K-1 in ascending order, so its value
 // does not depend on M, on the other rows of the batch or on the tile it falls in.  In gemm_f32
 // an output is a sum over the even k and one over the odd k, and a plain product may be cut
@@ -373,6 +374,8 @@ __global__ void __launch_bounds__(256) gemm_f32_sum_kernel(GemmArgs a) {
     for (int z = 0; z < a.splits; ++z) v += a.part[(static_cast<size_t>(z) * a.M + r) * a.N + n];
     epilogue<false>(a, r, n, scale_of(a, r), v, 0.f);
 }
+
+#include "gemm_f32_tc.cuh"
 
 template <int TX>
 static int launch_f32(const GemmArgs& a, int tiles, bool swiglu, cudaStream_t stream) {

@@ -515,6 +515,53 @@ def f32_splits(m: int, n: int, k: int) -> int:
     return best
 
 
+F32_TC_WORK = 64_000_000   # multiply-adds from which a float32 product goes to the tensor cores (see f32_tc_takes)
+
+
+def f32_tc_takes(x: torch.Tensor, w: torch.Tensor, m: int, dual: bool = False) -> bool:
+    """Whether :func:`linear` runs a float32 product that is none of the row-streaming kernel's on the tensor cores, every value
+    cut into three bfloat16 (csrc/gemm_f32_tc.cuh): rows that 16-byte loads and TMA can address, enough work for its two
+    launches and its pipeline's start (about 9 us), and scratch for the parts of x.  Measured, on CUDA cores / there: 33 rows of
+    2,048 x 512 9.6 / 10.1 us, 64 11.6 / 11.3, of 4,096 x 256 11.1 / 11.2, 128 14.9 / 11.4, 256 rows of 512 x 512 11.4 / 11.3; 33 rows
+    of 2,048 x 2,048 17.9 / 13.8, 512 110 / 33; 512 rows of 6,144 x 2,048 301 / 82, 2,048 rows 1,156 / 246."""
+    K, n = x.shape[-1], w.shape[-2]
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
+            and (x.data_ptr() | w.data_ptr()) % 16 == 0 and m * n * K * (2 if dual else 1) >= F32_TC_WORK
+            and 4 * f32_tc_floats(m, K) <= SPLIT_SCRATCH_BYTES)
+
+
+def f32_tc_floats(rows: int, k: int) -> int:
+    """Scratch for the parts of x of such a product, in floats: three bfloat16 for every column, in whole stages of 32."""
+    return rows * (-(-k // 32) * 32) * 3 // 2 + 4
+
+
+def f32_tc_plan(m: int, n: int, k: int, dual: bool) -> Tuple[int, int]:
+    """(rows of a tile, parts along K) of such a plain product: blocks of one an SM walk over tiles of 128 weight rows (of a pair
+    64 of each) and 64 or 128 rows of x.  A stage of 32 columns takes 0.32 us + 1.2 ns a row in tiles of 64, 0.38 + 1.4 in
+    tiles of 128, a tile's last sums and epilogue 1.2 us for 64 rows; over 96 sizes the least estimate is the quickest plan or within 5 %
+    of it.  Pairs are not cut along K."""
+    key = ("f32_tc", m, n, k, dual)
+    best = _PLANS.get(key)
+    if best is not None:
+        return best
+    n_sm, stages, best_cost = _sm_count(), -(-k // 32), None
+    for tn in (64, 128):
+        rows = min(tn, m)
+        tiles = -(-m // tn) * -(-n // (64 if dual else 128))
+        per = (0.32 + 0.0012 * rows) if tn == 64 else (0.38 + 0.0014 * rows)
+        for s in range(1, 9):
+            if s > 1 and (dual or stages < 4 * s or tiles * (s - 1) > 2 * n_sm or m > 65535
+                          or 4 * (s * m * n + f32_tc_floats(m, k)) > SPLIT_SCRATCH_BYTES):
+                break
+            cost = 6.9 + -(-tiles * s // n_sm) * (-(-stages // s) * per + 1.2 * rows / 64)
+            if s > 1:
+                cost += 1.4 + s * m * n * 8 / 7.2e6
+            if best_cost is None or cost < best_cost:
+                best, best_cost = (tn, s), cost
+    _PLANS[key] = best
+    return best
+
+
 def _split_scratch(device, floats: int) -> torch.Tensor:
     """A buffer for at least ``floats`` partial sums that no other chain of launches writes meanwhile.  The steps of a runner use
     the runner's own, one for its main chain and one for its side stream's (:class:`stream_scope`), so that the graphs of two
@@ -522,14 +569,16 @@ def _split_scratch(device, floats: int) -> torch.Tensor:
     own pool, which the same stream of the same capture finds again when the caller has let go of it.  All other calls share
     a buffer per stream."""
     if _scratch_override is not None:
-        return _scratch_override()
-    if torch.cuda.is_current_stream_capturing():
-        return torch.empty(floats, dtype=torch.float32, device=device)
-    key = (device, _stream().value)
-    t = _SPLIT_SCRATCH.get(key)
-    if t is None:
-        t = torch.empty(SPLIT_SCRATCH_BYTES // 4, dtype=torch.float32, device=device)
-        _SPLIT_SCRATCH[key] = t
+        t = _scratch_override()
+    elif torch.cuda.is_current_stream_capturing():
+        t = torch.empty(floats, dtype=torch.float32, device=device)
+    else:
+        key = (device, _stream().value)
+        t = _SPLIT_SCRATCH.get(key)
+        if t is None:
+            t = torch.empty(SPLIT_SCRATCH_BYTES // 4, dtype=torch.float32, device=device)
+            _SPLIT_SCRATCH[key] = t
+    _need(floats <= t.numel(), f"a product's partial sums and parts take {floats} floats, their buffer holds {t.numel()}")
     return t
 
 
@@ -560,6 +609,11 @@ def tc_error() -> int:
     """Error word of the tensor-core module (0 = fine); reading it synchronises the device.
     Non-zero: a bounded wait inside a kernel ran out (1 producer, 2 MMA, 3 epilogue)."""
     return int(_lib("gemm_tc").locus_gemm_tc_error())
+
+
+def f32_tc_error() -> int:
+    """The same of the float32 products on the tensor cores."""
+    return int(_lib("gemm_simt").locus_gemm_f32_tc_error())
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[torch.Tensor] = None,
@@ -696,6 +750,22 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         te = t0 = tr = nt = None
         max_tiles = 0
         stride = 0
+    if f32_tc_takes(x, w, M, w2 is not None):
+        # float32 x float32 in three bfloat16 parts each: tcgen05 kernel (csrc/gemm_f32_tc.cuh)
+        tn, splits = (64, 1) if layout is not None else f32_tc_plan(M, N, K, w2 is not None)
+        parts = splits * M * N if splits > 1 else 0        # floats; the parts of x lie behind the partial sums
+        parts += -parts % 4
+        scratch = _split_scratch(x.device, parts + f32_tc_floats(M, K))
+        code = _lib("gemm_simt").locus_gemm_f32_tc(
+            _p(x), _p(w), _p(w2), LL(w.numel() // K), _p(bias), I(dtype_code(bias.dtype) if bias is not None else 0), _p(out),
+            I(dtype_code(out.dtype)), flags, F(act_limit), F(act_scale), _p(row_scale), _p(scale_rows), _p(x_rows), I(x_row_div),
+            I(M), I(N), I(K), LL(x.stride(0)), LL(out.stride(0)), I(tn), _p(te), _p(t0), _p(tr), _p(nt), I(max_tiles),
+            ctypes.c_void_p(scratch.data_ptr() + 4 * parts), _p(scratch) if splits > 1 else None, I(splits), _stream()
+        )
+        if code == 0:
+            _count_launches(2 if splits > 1 else 1)   # the kernel that cuts x up, the kernel that adds the parts up
+        _check(code, "linear", f"(float32 on the tensor cores; M={M}, N={N}, K={K}, {tn} rows a tile, {splits} splits)")
+        return
     splits, scratch = 1, None
     if (layout is None and w2 is None and x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
             and (x.data_ptr() | w.data_ptr()) % 16 == 0):

@@ -113,6 +113,10 @@ SHARED_OVERLAP_FROM = 1024   # steps of at least this many tokens ...
 SHARED_OVERLAP_ROWS = 192    # ... and at most this many rows per routed expert run the shared expert on the side stream
 
 
+# Rows per expert, on average, up to which float32 experts that the tensor cores would take stay on the row-streaming kernel (see forward).
+FEW_PAIRS_F32_TC = 2.75
+
+
 # tensor names below a routed feed-forward's prefix ({e}: the expert's number)
 MOE_NAMES = {"router": "gate.weight", "router_bias": "gate.bias", "selection_bias": "gate.selection_bias",
              "expert_gate": "experts.{e}.gate_proj.weight", "expert_up": "experts.{e}.up_proj.weight",
@@ -280,12 +284,15 @@ class SparseMoe(FeedForward):
         on_input = (wts, lay.sorted_pair) if self.weight_on_input else None
         all_bf16 = (K.tensor_cores_take(h, self.params["up_exps"]) and widths_ok
                     and self.params["down_exps"].dtype == torch.bfloat16)
-        if not all_bf16 and widths_ok and n_pairs <= K.FEW_ROWS * self.E:
-            # No tensor-core form (float32) and a handful of rows per expert: tiles of 8 rows on the row-streaming
-            # kernel read an expert's weights once per tile, where the CUDA-core product would compute a 64-row
-            # tile for every expert that has a row.  Measured, tiles of 8 / of 64: 60 x (2,048 -> 1,408 -> 2,048), 4 picks, 93 tokens
-            # 603 / 700 us, 119 tokens 733 / 703; 64 experts, 8 picks, 60 tokens 734 / 720; small experts, which L2 holds, would gain
-            # further on (8 x (512 -> 256 -> 512), 2 picks, 120 tokens 28 / 47 us, 300 56 / 64, 512 87 / 66).
+        on_tc = (K.f32_tc_takes(h, self.params["up_exps"], n_pairs, self.activation in GATED) and widths_ok
+                 and self.params["down_exps"].dtype == torch.float32)
+        if not all_bf16 and widths_ok and n_pairs <= (FEW_PAIRS_F32_TC if on_tc else K.FEW_ROWS) * self.E:
+            # No bfloat16 form (float32) and a handful of rows per expert: tiles of 8 rows on the row-streaming kernel read an
+            # expert's weights once per tile, where the other products compute a 64-row tile for every expert that has a row: on the
+            # tensor cores soon the quicker way, on CUDA cores (products too small for those) past 8 rows an expert.  Measured, tiles of
+            # 8 / of 64 on the tensor cores: 60 x (2,048 -> 1,408 -> 2,048), 4 picks, 24 tokens 284 / 318 us, 40 364 / 364, 64 448 / 369,
+            # 96 608 / 373; 128 x (2,048 -> 768 -> 2,048), 8 picks, 40 tokens 406 / 388; 16 x (1,024 -> 512 -> 1,024), 2 picks, 24 tokens
+            # 30 / 30, 48 40 / 31; of 8 / of 64 on CUDA cores: 8 x (512 -> 256 -> 512), 2 picks, 40 tokens 15 / 30 us.
             tile = K.FEW_ROWS
         streamed = (all_bf16 and tile <= K.SKINNY_TILE_ROWS) or (widths_ok and tile <= K.FEW_ROWS)
         if not streamed and not all_bf16:

@@ -648,6 +648,82 @@ def test_linear_float32_of_few_rows_and_millions_of_weight_rows(dual):
     close(out, torch.nn.functional.silu(g) * (x.double() @ w2.double().T) if dual else g, torch.float32, f"{N} weight rows")
 
 
+@pytest.mark.parametrize("dual", [False, True])
+@pytest.mark.parametrize("tn,splits", [(64, 1), (128, 1), (64, 3), (128, 8)])
+def test_linear_float32_tensor_cores(tn, splits, dual, monkeypatch):
+    """float32 products in three bfloat16 parts at their edges: rows in sixteens, quarters of a tile and tiles, 64 (of a pair) and
+    128 weight rows, stages of 32 columns (K within one, that ends within one, an odd number of them), parts of K of unequal
+    length or without a stage, more tiles than SMs; bias, row scale, added to what is there.  The bound on the error against 64
+    bits holds for a sum of K products that is rounded (or cut off) at most K / 16 times by 2^-23 of its largest partial sum."""
+    monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    monkeypatch.setattr(K, "few_rows_take", lambda *a, **k: False)
+    monkeypatch.setattr(K, "f32_tc_plan", lambda m, n, k, d: (tn, 1 if d or m * n > 10 ** 6 else splits))   # (what the scratch holds)
+    for M, N, K_ in ((1, 1, 4), (16, 64, 32), (33, 129, 36), (65, 200, 100), (130, 65, 2052), (300, 1000, 160), (1500, 2300, 72)):
+        x, w, w2 = rnd(M, K_ + 4, seed=1)[:, :K_], rnd(N, K_, seed=2, scale=K_ ** -0.5), rnd(N, K_, seed=3, scale=K_ ** -0.5)
+        b, old, rs = rnd(N, seed=4), rnd(M, N, seed=5), rnd(M, seed=6)
+        dx, out = torch.zeros(M, K_ + 4, device=DEV)[:, :K_], old.to(DEV)   # (rows wider than the product's)
+        dx.copy_(x)
+        K.linear(dx, w.to(DEV), out, w2=w2.to(DEV) if dual else None, bias=b.to(DEV), row_scale=rs.to(DEV), accumulate=True)
+        g = x.double() @ w.double().T
+        v = torch.nn.functional.silu(g) * (x.double() @ w2.double().T) if dual else g
+        close(out, old.double() + (v + b.double()) * rs.double()[:, None], torch.float32, f"{M} x {N} x {K_} dual={dual}")
+        if not dual:
+            out = torch.full((M, N), float("nan"), device=DEV)
+            K.linear(dx, w.to(DEV), out)
+            bound = (K_ / 16 + 4) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+            assert bool(((out.cpu().double() - g).abs() <= bound).all())
+    assert K.f32_tc_error() == 0
+
+
+def test_linear_float32_tensor_cores_of_experts(monkeypatch):
+    """The same over experts' tiles of 64 rows, gathered from the tokens': experts with no row, one, a few, and several tiles."""
+    monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    T, E, k, H, I = 150, 5, 2, 520, 136
+    ids = _route(T, E, k, 3)
+    ids[ids == 4] = 0      # nobody picks 4
+    ids[:90] = 1           # several tiles
+    h, wg, wu, wd = rnd(T, H, seed=1), rnd(E, I, H, seed=2, scale=H ** -0.5), rnd(E, I, H, seed=3, scale=H ** -0.5), rnd(E, H, I, seed=4)
+    wts = torch.rand(T * k, generator=torch.Generator().manual_seed(5))
+    lay, ref_lay = K.ExpertLayout(T * k, E, 64, DEV), EK.ExpertLayout(T * k, E, 64, "cpu")
+    K.moe_sort(ids.to(DEV), T * k, lay, 64)
+    EK.moe_sort(ids, T * k, ref_lay, 64)
+    act, ref_act = torch.empty(T * k, I, device=DEV), torch.empty(T * k, I, dtype=torch.float64)
+    before = K.launches
+    K.linear(h.to(DEV), wg.to(DEV), act, w2=wu.to(DEV), x_rows=lay.sorted_pair, x_row_div=k, layout=lay, n_rows=T * k)
+    assert K.launches - before == 2   # (x cut up, the product)
+    EK.linear(h, wg, ref_act, w2=wu, x_rows=ref_lay.sorted_pair, x_row_div=k, layout=ref_lay, n_rows=T * k)
+    close(act, ref_act, torch.float32, "gate and up")
+    out, ref = torch.empty(T * k, H, device=DEV), torch.empty(T * k, H, dtype=torch.float64)
+    K.linear(act, wd.to(DEV), out, layout=lay, n_rows=T * k, row_scale=wts.to(DEV), scale_rows=lay.sorted_pair)
+    EK.linear(act.cpu(), wd, ref, layout=ref_lay, n_rows=T * k, row_scale=wts, scale_rows=ref_lay.sorted_pair)
+    close(out, ref, torch.float32, "down")
+    assert K.f32_tc_error() == 0
+
+
+@pytest.mark.parametrize("tn", [64, 128])
+def test_linear_float32_tensor_cores_keep_what_is_not_finite_and_the_range(tn, monkeypatch):
+    """Infinities, NaN, the largest and the smallest values: what plain multiply-adds give, in their outputs and in no others."""
+    monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    monkeypatch.setattr(K, "few_rows_take", lambda *a, **k: False)
+    monkeypatch.setattr(K, "f32_tc_plan", lambda m, n, k, d: (tn, 1))
+    M, N, K_ = 70, 140, 64
+    x, w = rnd(M, K_, seed=1), rnd(N, K_, seed=2)
+    x[3, 5], x[40, 0], x[66, 63], w[7, 9], w[130, 5] = float("inf"), float("nan"), float("-inf"), float("inf"), 0.0
+    x[10], w[20] = 0.0, 0.0
+    x[10, 2], w[20, 2] = 3.4e38, 0.99
+    x[11], x[12] = x[11] * 1e-30, x[12] * 1e30
+    out = torch.empty(M, N, device=DEV)
+    K.linear(x.to(DEV), w.to(DEV), out)
+    got, ref = out.cpu().double(), x.double() @ w.double().T
+    ref[ref.abs() > 3.4028235677973366e38] = float("inf") * ref[ref.abs() > 3.4028235677973366e38].sign()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref))
+    assert torch.equal(got[torch.isinf(ref)], ref[torch.isinf(ref)])
+    fin = torch.isfinite(ref)
+    scale = x.double().nan_to_num(0, 0, 0).abs() @ w.double().nan_to_num(0, 0, 0).abs().T
+    assert bool(((got - ref).abs()[fin] <= (8 * 2.0 ** -23 * scale)[fin]).all())
+    assert K.f32_tc_error() == 0
+
+
 @pytest.mark.parametrize("splits", [2, 3, 8])
 def test_linear_float32_cut_along_k(splits, monkeypatch):
     """Parts of unequal length (the last one shorter, or without a column), and the epilogue behind their sum."""
