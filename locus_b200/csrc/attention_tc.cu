@@ -4,23 +4,28 @@
 // A block takes 128 consecutive new tokens of one request and one head.  Keys and values come in
 // tiles of 128 positions through the request's block table: TMA boxes of 64 rows x 64 elements
 // (pages are a multiple of 64 tokens, so a box never straddles pages; a box whose page does not
-// exist is fetched from outside the tensor and arrives as zeros), two stages each for K and V.
+// exist is fetched from outside the tensor and arrives as zeros), three tiles of either on
+// their way or in use.
 //
 //   MMA 1:  S[q, t] = sum_d Q[q, d] K[t, d]        (A = Q, B = K, both K-major; 128 x 128 in TMEM)
-//   softmax warps: the threads of a query row read its row of S (tcgen05.ld), mask (causal, window,
-//           end of the sequence), keep the running maximum and denominator (base 2), write
-//           P = exp2(s - m) as bfloat16 into shared memory in the swizzled K-major operand layout
-//   MMA 2:  O[q, d] += sum_t P[q, t] V[t, d]      (A = P, B = V read MN-major: V lies [t][d] in the
+//   softmax: the thread of a query row reads its row of S (tcgen05.ld), masks (causal, window, end of the sequence), keeps
+//           the running maximum and denominator (base 2), writes P = exp2(s - m) as bfloat16 over S in tensor memory
+//   MMA 2:  O[q, d] += sum_t P[q, t] V[t, d]      (A = P from tensor memory, B = V read MN-major: V lies [t][d] in the
 //           cache, which is the transposed operand; 128 x 128 in TMEM, ONE sum from the first tile to the last)
-//   The row's threads rescale O in tensor memory (tcgen05.ld, multiply, tcgen05.st) only when the row's maximum
-//   has run ahead of the reference its probabilities are formed against by more than 2^8, and read it once at
-//   the end: O / denominator.  (Adding every tile's P V into registers cost 400 cycles a tile.)
+//   The row's thread rescales O in tensor memory (tcgen05.ld, multiply, tcgen05.st) only when the row's maximum
+//   has run ahead of the reference its probabilities are formed against by more than 2^8.
 //
-// S is double-buffered in tensor memory (2 x 128 columns beside the 128 of O), so the tensor pipe computes the
-// scores of the next tile while the softmax warps work on this one; P has two buffers in shared memory.
-// Warp 0: TMA; warp 1: MMA issue (one thread);
-// warps 2-9: softmax and output, two threads per query row (64 keys and 64 output dimensions each).  Head size 128 only (other sizes and pages that are not a multiple
-// of 64 tokens go to the mma.sync kernel).
+// A tile costs the tensor cores 1,024 cycles and its exponentials as many of the special-function units, so the two have to work
+// at the same time.  Two groups of four warps take the even and the odd key tiles, and three buffers of scores (with the sum of V
+// all of tensor memory) let the tensor cores form scores two tiles ahead: while one group is at its exponentials the other loads
+// scores and looks for maxima, and neither waits for a product.  All tiles add to one sum, against one reference maximum a row,
+// which is handed from each tile's thread to the next tile's, in the other group, as soon as it is known.
+// Measured, 2,048 tokens behind 8,192, 28 heads on 4: 253 us; one group of eight warps, two threads to a row, P through
+// shared memory 368 (all warps in the same phase at the same time); a sum and a buffer of scores for either group 307 (each
+// tile's scores waited for the group's sum before).
+// Warp 0: TMA; warps 1 and 2: MMA issue (one thread each); warps 4-11: softmax and output, a thread per query row.  Head size
+// 128 only (other
+// sizes and pages that are not a multiple of 64 tokens go to the mma.sync kernel).
 //
 // Keys and values may also lie in plain rows instead of pages (rows form): two matrices [rows][kv heads * 128] in which a
 // segment's keys are consecutive rows from kv_row0[segment] on (latent attention expands its heads' keys and values of a
@@ -107,8 +112,8 @@ __device__ __forceinline__ bool at_try_wait(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity, int code) {
     if (at_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
-    while (!at_try_wait(bar, parity)) {
-        if (*reinterpret_cast<volatile int*>(&g_at_error) != 0) return false;
+    for (int i = 1; !at_try_wait(bar, parity); ++i) {
+        if ((i & 63) == 0 && *reinterpret_cast<volatile int*>(&g_at_error) != 0) return false;   // (a trip to L2)
         if (clock64() - t0 > AT_WAIT_LIMIT) {
             atomicCAS(&g_at_error, 0, code);
             return false;
@@ -151,6 +156,15 @@ __device__ __forceinline__ void at_mma(uint32_t tmem_d, uint64_t da, uint64_t db
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc)
         : "memory");
 }
+// The same with A in tensor memory (lane: row; a column two elements of k).
+__device__ __forceinline__ void at_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc)
+        : "memory");
+}
 __device__ __forceinline__ void at_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -170,12 +184,6 @@ __device__ __forceinline__ float at_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-// Two probabilities (finite, in [0, 1]) as bfloat16, rounded to nearest (ties upward) with integer
-// arithmetic: the conversion instruction runs on the same narrow pipe as ex2 and would add half as
-// much again to what already takes as long as the tile's MMAs.
-__device__ __forceinline__ uint32_t at_pack_prob(float lo, float hi) {
-    return __byte_perm(__float_as_uint(lo) + 0x8000u, __float_as_uint(hi) + 0x8000u, 0x7632);
 }
 __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -230,9 +238,11 @@ __device__ __forceinline__ void at_st32(uint32_t taddr, const uint32_t* v) {
 // sum / denominator is the same number whatever reference it was formed with.
 #define AT_LAG_LOG2 8.0f
 
+#define AT_S 3   // tiles of K, of V (shared memory) and of scores (tensor memory): tile j's in place j % 3
+
 // BIAS: a distance bias; an instance of its own (the softmax warps are bound by instruction issue).
 template <bool BIAS>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(384, 1)
 attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, TcAttnArgs a) {
     extern __shared__ __align__(1024) uint8_t at_raw[];
@@ -263,7 +273,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     };
     const int* table = a.kv_row0 ? nullptr : a.block_table + static_cast<size_t>(seg) * a.table_stride;
 
-    // shared memory: Q, K[2], V[2], P[2] (each a tile of two swizzled halves), then the barriers.  That is
+    // shared memory: Q, K[3], V[3] (each a tile of two swizzled halves), then the barriers.  That is nearly
     // all the shared memory a block can have, so the tiles start at the very base, which must be
     // 1024-byte aligned for the swizzle (checked: a block that finds it otherwise reports and leaves).
     const uint32_t base = at_smem(at_raw);
@@ -271,25 +281,20 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (threadIdx.x == 0) atomicCAS(&g_at_error, 0, 12);
         return;
     }
-    const uint32_t sQ = base, sK = sQ + AT_TILE_BYTES, sV = sK + 2 * AT_TILE_BYTES, sP = sV + 2 * AT_TILE_BYTES;
-    const uint32_t bars = sP + 2 * AT_TILE_BYTES;
-    const uint32_t q_full = bars, k_full = bars + 8, v_full = bars + 24, k_free = bars + 40, v_free = bars + 56;
-    const uint32_t s_full = bars + 72, s_free = bars + 88, pv_done = bars + 104, p_ready = bars + 136;
-    const uint32_t slot = bars + 144;
-    volatile uint32_t* slot_ptr = reinterpret_cast<volatile uint32_t*>(at_raw + (slot - at_smem(at_raw)));
+    const uint32_t sQ = base, sK = sQ + AT_TILE_BYTES, sV = sK + AT_S * AT_TILE_BYTES, bars = sV + AT_S * AT_TILE_BYTES;
+    const uint32_t q_full = bars, k_full = bars + 8, k_free = k_full + 8 * AT_S, v_full = k_free + 8 * AT_S, v_free = v_full + 8 * AT_S;
+    const uint32_t s_full = v_free + 8 * AT_S, p_ready = s_full + 8 * AT_S, slot = p_ready + 8 * AT_S + 8;
 
     if (threadIdx.x == 0) {
         at_bar_init(q_full, 1);
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < AT_S; ++b) {
             at_bar_init(k_full + 8 * b, 1);
-            at_bar_init(v_full + 8 * b, 1);
             at_bar_init(k_free + 8 * b, 1);
-            at_bar_init(v_free + 8 * b, 1);
+            at_bar_init(v_full + 8 * b, 1);
+            at_bar_init(v_free + 8 * b, 1);     // the tile's P V is finished: V's place and that of the scores are free
             at_bar_init(s_full + 8 * b, 1);
-            at_bar_init(s_free + 8 * b, 8);    // one arrival per softmax warp
-            at_bar_init(pv_done + 8 * b, 1);
+            at_bar_init(p_ready + 8 * b, 4);    // one arrival per softmax warp of the group
         }
-        at_bar_init(p_ready, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -300,92 +305,126 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *slot_ptr;
-    const uint32_t tS = tmem, tO = tmem + 2 * AT_MK;  // S0, S1, O: 128 columns each
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(at_raw + (slot - base));
+    const uint32_t tS = tmem, tO = tmem + AT_S * AT_MK;  // three S (and P over it), O: 128 columns each
 
-    if (warp == 0) {
-        if (lane == 0) {
-            // Q: two halves of 64 elements, rows row0 .. row0 + 127 (rows past the portion are never stored)
-            at_expect_tx(q_full, AT_TILE_BYTES);
-            at_tma_2d(sQ, &map_q, h * AT_HD, row0, q_full);
-            at_tma_2d(sQ + AT_HALF_BYTES, &map_q, h * AT_HD + 64, row0, q_full);
+    // Registers by role: of the 168 a thread that the block was launched with, what the first four warps give back goes to the
+    // softmax (56 + 2 x 224 <= 3 x 168).
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == 0) {
+            uint32_t elected;
+            asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+            if (elected) {
+                // Q: two halves of 64 elements, rows row0 .. row0 + 127 (rows past the portion are never stored)
+                at_expect_tx(q_full, AT_TILE_BYTES);
+                at_tma_2d(sQ, &map_q, h * AT_HD, row0, q_full);
+                at_tma_2d(sQ + AT_HALF_BYTES, &map_q, h * AT_HD + 64, row0, q_full);
+            }
             const long long rows_per_page = 2LL * a.nkv * P;
             const int v_shift = a.kv_row0 ? 0 : a.nkv * P;  // V rows of a page lie nkv * P rows behind its K rows
             const int col0 = a.kv_row0 ? kvh * AT_HD : 0;
             const int rows0 = a.kv_row0 ? a.kv_row0[seg] : 0;
-            for (int j = 0; j < n_tiles; ++j) {
-                const int b = j & 1;
-                const uint32_t par = ((j >> 1) & 1) ^ 1;
-                const int tile0 = tile_at(j);
-                // rows of the pool (viewed as [pages * 2 * nkv * P][hd]) of the two 64-key halves; a half with
-                // no page, or wholly outside the keys this block may see, is fetched from outside the tensor
-                int krow[2];
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int t = tile0 + 64 * hh;
-                    const bool seen = t <= t_hi && (t + 63 >= t_lo || t < keep);
-                    if (a.kv_row0) {
-                        krow[hh] = seen ? rows0 + t : -64;
-                    } else {
-                        const int page = seen ? table[t / P] : -1;
-                        krow[hh] = page < 0 ? -64 : static_cast<int>(page * rows_per_page + static_cast<long long>(kvh) * P + t % P);
-                    }
+            // Row of the pool (viewed as [pages * 2 * nkv * P][hd]) of the 64-key half hh of tile j; a half with no page, or wholly
+            // outside the keys this block may see, is fetched from outside the tensor.  The lanes look up sixteen tiles at a time, sixteen
+            // ahead: with a trip to the table and back before every tile the loader was what a long context waited for.
+            auto look_up = [&](int j, int hh) -> int {
+                const int t = tile_at(j) + 64 * hh;
+                const bool seen = j < n_tiles && t <= t_hi && (t + 63 >= t_lo || t < keep);
+                if (!seen) return -64;
+                if (a.kv_row0) return rows0 + t;
+                const int page = table[t / P];
+                return page < 0 ? -64 : static_cast<int>(page * rows_per_page + static_cast<long long>(kvh) * P + t % P);
+            };
+            int now = look_up(lane >> 1, lane & 1), ahead = look_up(16 + (lane >> 1), lane & 1);
+            auto rows_of = [&](int j) -> int2 {   // (asked for in ascending order)
+                if (j > 0 && (j & 15) == 0) {
+                    now = ahead;
+                    ahead = look_up(j + 16 + (lane >> 1), lane & 1);
                 }
-                if (!at_wait(k_free + 8 * b, par, 1)) break;
-                at_expect_tx(k_full + 8 * b, AT_TILE_BYTES);
-                for (int hh = 0; hh < 2; ++hh)
-                    for (int ch = 0; ch < 2; ++ch)
-                        at_tma_2d(sK + b * AT_TILE_BYTES + ch * AT_HALF_BYTES + hh * (64 * 128), &map_k, col0 + 64 * ch, krow[hh],
-                                  k_full + 8 * b);
-                if (!at_wait(v_free + 8 * b, par, 2)) break;
-                at_expect_tx(v_full + 8 * b, AT_TILE_BYTES);
-                for (int hh = 0; hh < 2; ++hh)
-                    for (int ch = 0; ch < 2; ++ch)
-                        at_tma_2d(sV + b * AT_TILE_BYTES + ch * AT_HALF_BYTES + hh * (64 * 128), &map_v, col0 + 64 * ch,
-                                  krow[hh] < 0 ? -64 : krow[hh] + v_shift, v_full + 8 * b);
+                return make_int2(__shfl_sync(0xffffffffu, now, 2 * (j & 15)), __shfl_sync(0xffffffffu, now, 2 * (j & 15) + 1));
+            };
+            auto load = [&](const CUtensorMap* map, int2 rows, int shift, int j, uint32_t to, uint32_t full, uint32_t free_) {
+                const int turn = j / AT_S, b = j - turn * AT_S;
+                at_wait(free_ + 8 * b, (turn & 1) ^ 1, 1);
+                if (elected) {
+                    const uint32_t dst = to + b * AT_TILE_BYTES, bar = full + 8 * b;
+                    const int ra = rows.x < 0 ? -64 : rows.x + shift, rb = rows.y < 0 ? -64 : rows.y + shift;
+                    at_expect_tx(bar, AT_TILE_BYTES);
+                    at_tma_2d(dst, map, col0, ra, bar);
+                    at_tma_2d(dst + AT_HALF_BYTES, map, col0 + 64, ra, bar);
+                    at_tma_2d(dst + 64 * 128, map, col0, rb, bar);
+                    at_tma_2d(dst + AT_HALF_BYTES + 64 * 128, map, col0 + 64, rb, bar);
+                }
+                __syncwarp();
+            };
+            int2 r[AT_S + 1];   // the rows of tiles j .. j + 3
+    #pragma unroll
+            for (int j = 0; j < AT_S; ++j) {
+                r[j] = make_int2(-64, -64);
+                if (j < n_tiles) {
+                    r[j] = rows_of(j);
+                    load(&map_k, r[j], 0, j, sK, k_full, k_free);
+                }
             }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
+            for (int j = 0; j < n_tiles; ++j) {
+                load(&map_v, r[0], v_shift, j, sV, v_full, v_free);
+                if (j + AT_S < n_tiles) {
+                    r[AT_S] = rows_of(j + AT_S);
+                    load(&map_k, r[AT_S], 0, j + AT_S, sK, k_full, k_free);
+                }
+    #pragma unroll
+                for (int i = 0; i < AT_S; ++i) r[i] = r[i + 1];
+            }
+        } else if (warp < 3) {
+            // Warp 1 issues the scores, warp 2 the sums of V: a thread that did both would leave the tensor cores idle while it waits
+            // for one tile's weights and gives its places back.  (The whole warp walks, one thread issues: what does not depend on
+            // the lane stays in uniform registers.)
+            uint32_t elected;
+            asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
             // f32 accumulate, bf16 x bf16, M = 128, N = 128; MMA 2 reads its B operand MN-major
             const uint32_t idesc1 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(AT_MK >> 3) << 17) |
                                     (static_cast<uint32_t>(AT_MQ >> 4) << 24);
             const uint32_t idesc2 = idesc1 | (1u << 16);
-            auto scores = [&](int j) -> bool {  // S_j = Q K_j^T
-                const int b = j & 1;
-                if (!at_wait(k_full + 8 * b, (j >> 1) & 1, 3)) return false;
-                if (!at_wait(s_free + 8 * b, ((j >> 1) & 1) ^ 1, 4)) return false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                for (int ks = 0; ks < AT_HD / 16; ++ks) {
-                    const uint32_t off = (ks >> 2) * AT_HALF_BYTES + (ks & 3) * 32;
-                    at_mma(tS + b * AT_MK, at_desc_k(sQ + off), at_desc_k(sK + b * AT_TILE_BYTES + off), idesc1, ks > 0);
+            int b = 0;
+            uint32_t turn = 0;
+            if (warp == 1) at_wait(q_full, 0, 5);
+            for (int j = 0; j < n_tiles; ++j) {
+                if (warp == 1) {
+                    at_wait(k_full + 8 * b, turn & 1, 3);
+                    at_wait(v_free + 8 * b, (turn & 1) ^ 1, 4);   // the tile before in this place has been weighted and added up
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elected) {
+    #pragma unroll
+                        for (int ks = 0; ks < AT_HD / 16; ++ks) {  // S = Q K^T
+                            const uint32_t off = (ks >> 2) * AT_HALF_BYTES + (ks & 3) * 32;
+                            at_mma(tS + b * AT_MK, at_desc_k(sQ + off), at_desc_k(sK + b * AT_TILE_BYTES + off), idesc1, ks > 0);
+                        }
+                        at_commit(s_full + 8 * b);
+                        at_commit(k_free + 8 * b);
+                    }
+                } else {
+                    at_wait(v_full + 8 * b, turn & 1, 7);
+                    at_wait(p_ready + 8 * b, turn & 1, 6);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (elected) {
+    #pragma unroll
+                        for (int ks = 0; ks < AT_MK / 16; ++ks)  // O += P V
+                            at_mma_ts(tO, tS + b * AT_MK + 8 * ks, at_desc_mn(sV + b * AT_TILE_BYTES + ks * (16 * 128), AT_HALF_BYTES), idesc2,
+                                      (j > 0 || ks > 0) ? 1u : 0u);
+                        at_commit(v_free + 8 * b);
+                    }
                 }
-                at_commit(s_full + 8 * b);
-                at_commit(k_free + 8 * b);
-                return true;
-            };
-            bool ok = at_wait(q_full, 0, 5) && scores(0);
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                const int b = j & 1;
-                if (j + 1 < n_tiles && !scores(j + 1)) break;
-                // O += P_j V_j: the sum stays in tensor memory from the first tile to the last
-                if (!at_wait(p_ready, j & 1, 6)) break;
-                if (!at_wait(v_full + 8 * b, (j >> 1) & 1, 7)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                for (int ks = 0; ks < AT_MK / 16; ++ks) {
-                    const uint64_t dp = at_desc_k(sP + b * AT_TILE_BYTES + (ks >> 2) * AT_HALF_BYTES + (ks & 3) * 32);
-                    const uint64_t dv = at_desc_mn(sV + b * AT_TILE_BYTES + ks * (16 * 128), AT_HALF_BYTES);
-                    at_mma(tO, dp, dv, idesc2, (j > 0 || ks > 0) ? 1u : 0u);  // O += P_j V_j
+                __syncwarp();
+                if (++b == AT_S) {
+                    b = 0;
+                    ++turn;
                 }
-                at_commit(pv_done + 8 * b);  // tells the softmax warps (P's buffer is free, the sum may be touched) ...
-                at_commit(v_free + 8 * b);   // ... and the loader (the stage's V is free)
             }
         }
     } else {
-        // Softmax and output: two threads per query row (warps w and w + 4 reach the same quarter of the
-        // lanes of tensor memory); each takes 64 of the tile's 128 keys and 64 of the 128 output dimensions.
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        const int quarter = warp & 3, x = (warp - 4) >> 2;   // quarter of tensor memory's lanes; even or odd tiles
         const int r = quarter * 32 + lane;  // this thread's query row
         const int pq = p0 + r;              // its position
         const uint32_t lane_bits = static_cast<uint32_t>(quarter * 32) << 16;
@@ -394,181 +433,176 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const float mult = BIAS ? 1.0f : scale_log2;
         const unsigned long long scale2 = at_pair(mult, mult);
         const float slope = BIAS ? slope_log2(a.slopes, h) : 0.f;
-        float m_run = -INFINITY, l_run = 0.f;  // the row's reference maximum (base 2, scaled); this thread's part of the denominator
-        uint8_t* at_generic = at_raw + (base - at_smem(at_raw));
-        uint8_t* gP0 = at_generic + (sP - base) + half * AT_HALF_BYTES + r * 128;
-        float* xch = reinterpret_cast<float*>(at_generic + (slot + 16 - base));  // [2 tile parities][2 halves][128 rows]
+        float m_run = -INFINITY, l_run = 0.f;  // the row's reference maximum (base 2, scaled); this group's part of the denominator
         bool ok = true;
         const int lo = first_key(a.window, a.chunk, pq);                    // first key this row sees ...
         const int lo_last = first_key(a.window, a.chunk, p0 + AT_MQ - 1);   // ... and the block's last row
-        const uint32_t tOmine = tO + lane_bits + 64 * half;           // this thread's 64 columns of the row's sum
+        const uint32_t tOmine = tO + lane_bits;
+        float2* ml = reinterpret_cast<float2*>(at_raw + (slot + 16 - base));   // [2][128]: what the groups' threads tell each other
 
-        // the two threads of a row exchange a value through shared memory (a barrier of their two warps)
-        auto with_partner = [&](int parity, float mine) -> float {
-            float* slot_f = xch + parity * 256;
-            slot_f[half * 128 + r] = mine;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
-            return slot_f[(half ^ 1) * 128 + r];
-        };
-
-        // (When a wait gives up, this loop still runs to its end -- every later wait returns at once -- so that
-        // the two warps of a row meet at every one of their barriers.)
-        for (int j = 0; j < n_tiles; ++j) {
-            const int b = j & 1;
-            const int tile_first = tile_at(j);
-            const int tile0 = tile_first + 64 * half;  // first key of this thread's half of the tile
-            if (!at_wait(s_full + 8 * b, (j >> 1) & 1, 10)) ok = false;
+        for (int j = x; j < n_tiles; j += 2) {
+            const int tile0 = tile_at(j), turn = j / AT_S, b = j - turn * AT_S;
+            const uint32_t tSx = tS + b * AT_MK + lane_bits;
+            if (!at_wait(s_full + 8 * b, turn & 1, 10)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t s0[32], s1[32];
-            at_ld32(tS + b * AT_MK + lane_bits + 64 * half, s0);
-            at_ld32(tS + b * AT_MK + lane_bits + 64 * half + 32, s1);
+            uint32_t s[4][32];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) at_ld32(tSx + 32 * c, s[c]);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             // a key t counts for this row when lo <= t <= pq, or when it is one of the kept first tokens; only tiles
             // at an edge need the test (a tile of kept tokens lies in front of t_lo, so it is always tested)
-            const bool need_mask = tile_first + AT_MK - 1 > p0 || tile_first < lo_last;
-            float mx = -INFINITY;
+            const bool need_mask = tile0 + AT_MK - 1 > p0 || tile0 < lo_last;
             if constexpr (BIAS) {
-                // s <- s scale + slope (t - pq), two keys at a time: the tile's first key's share (t - pq is an exact float32),
+                // s <- s scale + slope (t - pq), two keys at a time: the first key's share (t - pq is an exact float32),
                 // then a multiple of the slope per key
                 const unsigned long long k2 = at_pair(scale_log2, scale_log2), sl2 = at_pair(slope, slope);
-                const float d0 = slope * static_cast<float>(tile0 - pq), d1 = slope * static_cast<float>(tile0 + 32 - pq);
-                const unsigned long long b0 = at_pair(d0, d0), b1 = at_pair(d1, d1);
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float x, y;
-                    const unsigned long long at2 = at_pair(static_cast<float>(i), static_cast<float>(i + 1));
-                    at_unpair(at_fma2(at_pair(__uint_as_float(s0[i]), __uint_as_float(s0[i + 1])), k2, at_fma2(sl2, at2, b0)), x, y);
-                    s0[i] = __float_as_uint(x);
-                    s0[i + 1] = __float_as_uint(y);
-                    at_unpair(at_fma2(at_pair(__uint_as_float(s1[i]), __uint_as_float(s1[i + 1])), k2, at_fma2(sl2, at2, b1)), x, y);
-                    s1[i] = __float_as_uint(x);
-                    s1[i + 1] = __float_as_uint(y);
+                for (int c = 0; c < 4; ++c) {
+                    const float d0 = slope * static_cast<float>(tile0 + 32 * c - pq);
+                    const unsigned long long b0 = at_pair(d0, d0);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float u, v;
+                        const unsigned long long at2 = at_pair(static_cast<float>(i), static_cast<float>(i + 1));
+                        at_unpair(at_fma2(at_pair(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), k2, at_fma2(sl2, at2, b0)), u, v);
+                        s[c][i] = __float_as_uint(u);
+                        s[c][i + 1] = __float_as_uint(v);
+                    }
                 }
             }
             if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int t = tile0 + i;
-                    if (!(t <= pq && (t >= lo || t < keep))) s0[i] = 0xff800000u;            // -inf
-                    if (!(t + 32 <= pq && (t + 32 >= lo || t + 32 < keep))) s1[i] = 0xff800000u;
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const int t = tile0 + 32 * c + i;
+                        if (!(t <= pq && (t >= lo || t < keep))) s[c][i] = 0xff800000u;            // -inf
+                    }
+            }
+            float mx[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                mx[c] = fmaxf(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]));
+#pragma unroll
+                for (int i = 2; i < 32; i += 2) mx[c] = at_max3(mx[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+            }
+            // the reference maximum as the tile before left it, from the other group's thread of the row
+            if (j > 0) {
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter + 4 * (x ^ 1)) : "memory");
+                const float before = ml[(x ^ 1) * 128 + r].x;
+                if (before != m_run) {
+                    l_run *= m_run == -INFINITY ? 1.f : at_exp2(m_run - before);
+                    m_run = before;
                 }
             }
-#pragma unroll
-            for (int i = 0; i < 32; ++i) mx = at_max3(mx, __uint_as_float(s0[i]), __uint_as_float(s1[i]));
-            mx = fmaxf(mx, with_partner(b, mx)) * mult;  // the scale is positive: the maximum can be scaled last
-            const float m_new = fmaxf(mx, m_run);               // the same in both threads of the row
-            // The buffer of P_{j-2} is free when its product is finished (the same barrier frees the stage's V).
-            if (j > 1 && !at_wait(pv_done + 8 * b, ((j >> 1) & 1) ^ 1, 9)) ok = false;
+            const float m_new = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mult, m_run);   // (the scale is positive)
             // Does the reference maximum follow?  Only when some row of the warp has run ahead of its reference by
             // more than 2^AT_LAG_LOG2 (always at a row's first key: -inf is infinitely far; -inf - -inf is not a
-            // number and compares false, so a row without a key yet keeps -inf).  Both warps of a row hold the same
-            // rows and the same maxima, so they decide alike.  Then every row of the warp moves its reference and
-            // rescales its sum, which needs the product of the tile before this one finished.
+            // number and compares false, so a row without a key yet keeps -inf).  Then every row of the warp moves its reference
+            // and rescales its sum, once the product of the tile before is in it.
             if (__any_sync(0xffffffffu, m_new - m_run > AT_LAG_LOG2)) {
                 if (j > 0) {
-                    if (!at_wait(pv_done + 8 * (b ^ 1), ((j - 1) >> 1) & 1, 12)) ok = false;
+                    if (!at_wait(v_free + 8 * ((j - 1) % AT_S), ((j - 1) / AT_S) & 1, 12)) ok = false;
                     const float f = m_run == -INFINITY ? 1.f : at_exp2(m_run - m_new);
                     const unsigned long long f2 = at_pair(f, f);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
+#pragma unroll 1
+                    for (int c = 0; c < AT_HD; c += 32) {
                         uint32_t v[32];
-                        at_ld32(tOmine + 32 * c, v);
+                        at_ld32(tOmine + c, v);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int d = 0; d < 32; d += 2) {
-                            float x, y;
-                            at_unpair(at_mul2(at_pair(__uint_as_float(v[d]), __uint_as_float(v[d + 1])), f2), x, y);
-                            v[d] = __float_as_uint(x);
-                            v[d + 1] = __float_as_uint(y);
+                            float u, w;
+                            at_unpair(at_mul2(at_pair(__uint_as_float(v[d]), __uint_as_float(v[d + 1])), f2), u, w);
+                            v[d] = __float_as_uint(u);
+                            v[d + 1] = __float_as_uint(w);
                         }
-                        at_st32(tOmine + 32 * c, v);
+                        at_st32(tOmine + c, v);
                     }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     l_run *= f;
                 }
                 m_run = m_new;
             }
+            ml[x * 128 + r].x = m_run;
+            if (j + 1 < n_tiles) asm volatile("bar.arrive %0, 64;" ::"r"(1 + quarter + 4 * x) : "memory");
             const float m_ref = m_run == -INFINITY ? 0.f : m_run;  // exp2(-inf - 0) = 0 for a row without keys so far
             const unsigned long long neg_m2 = at_pair(-m_ref, -m_ref);
-            // P = exp2(s * scale - m_ref) as bfloat16 into shared memory (K-major operand, 128-byte swizzle)
-            uint8_t* gP = gP0 + b * AT_TILE_BYTES;
-            unsigned long long sum2 = at_pair(0.f, 0.f);
+            // P = exp2(s * scale - m_ref) as bfloat16 over S
+            unsigned long long sum2[2] = {at_pair(0.f, 0.f), at_pair(0.f, 0.f)};
 #pragma unroll
-            for (int q8 = 0; q8 < 8; ++q8) {  // 16-byte pieces of 8 probabilities
-                float pr[8];
+            for (int c = 0; c < 4; c += 2) {
+                uint32_t pk[32];
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    const uint32_t r0 = q8 < 4 ? s0[8 * q8 + i] : s1[8 * (q8 - 4) + i];
-                    const uint32_t r1 = q8 < 4 ? s0[8 * q8 + i + 1] : s1[8 * (q8 - 4) + i + 1];
-                    float x, y;
-                    at_unpair(at_fma2(at_pair(__uint_as_float(r0), __uint_as_float(r1)), scale2, neg_m2), x, y);
-                    pr[i] = at_exp2(x);
-                    pr[i + 1] = at_exp2(y);
-                    sum2 = at_add2(sum2, at_pair(pr[i], pr[i + 1]));
+                for (int i = 0; i < 32; ++i) {
+                    float u, v;
+                    at_unpair(at_fma2(at_pair(__uint_as_float(s[c + (i >> 4)][2 * i & 31]), __uint_as_float(s[c + (i >> 4)][(2 * i & 31) + 1])),
+                                      scale2, neg_m2), u, v);
+                    u = at_exp2(u);
+                    v = at_exp2(v);
+                    sum2[i & 1] = at_add2(sum2[i & 1], at_pair(u, v));
+                    pk[i] = at_pack(u, v);   // (the conversion is not on the pipe of the exponentials: integer rounding took 1 % longer)
                 }
-                uint4 pk;
-                pk.x = at_pack_prob(pr[0], pr[1]);
-                pk.y = at_pack_prob(pr[2], pr[3]);
-                pk.z = at_pack_prob(pr[4], pr[5]);
-                pk.w = at_pack_prob(pr[6], pr[7]);
-                *reinterpret_cast<uint4*>(gP + ((q8 ^ (r & 7)) << 4)) = pk;
+                at_st32(tSx + 16 * c, pk);
             }
             {
-                float x, y;
-                at_unpair(sum2, x, y);
-                l_run += x + y;
+                float u, v;
+                at_unpair(at_add2(sum2[0], sum2[1]), u, v);
+                l_run += u + v;
             }
             // the last tile may hold rows of V behind the sequence's end (never written, any bit pattern): zero them
-            if (tile_first + AT_MK - 1 > t_hi) {
-                if (!at_wait(v_full + 8 * b, (j >> 1) & 1, 11)) ok = false;
-                if (tile_first + r > t_hi) {
-                    uint8_t* gV = at_generic + (sV - base) + b * AT_TILE_BYTES + half * AT_HALF_BYTES + r * 128;
+            if (tile0 + AT_MK - 1 > t_hi) {
+                if (!at_wait(v_full + 8 * b, turn & 1, 11)) ok = false;
+                if (tile0 + r > t_hi)
 #pragma unroll
-                    for (int q8 = 0; q8 < 8; ++q8) *reinterpret_cast<uint4*>(gV + q8 * 16) = make_uint4(0, 0, 0, 0);
-                }
+                    for (int q8 = 0; q8 < 16; ++q8)
+                        *reinterpret_cast<uint4*>(at_raw + (sV - base) + b * AT_TILE_BYTES + (q8 >> 3) * AT_HALF_BYTES + r * 128 + (q8 & 7) * 16) =
+                            make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
-            // S_j is read, P_j is written, the sum is where the MMAs may add to it: tell the MMA warp
+            // P is written, the sum is where the MMAs may add to it: tell the MMA warp
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-                at_arrive(s_free + 8 * b);
-                at_arrive(p_ready);
-            }
+            if (lane == 0) at_arrive(p_ready + 8 * b);
         }
-        // the sum is complete when the last product is
-        if (!at_wait(pv_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 13)) ok = false;
+        // The last tile's reference is the larger one and that of the sum; a group writes half of the columns of its rows.  (A group
+        // without a tile counts for nothing.)
+        ml[x * 128 + r] = make_float2(m_run, l_run);
+        // (the wait counts in the group of the last tile, whose scores came behind the sum before in this place; the other meets it)
+        if (!at_wait(v_free + 8 * ((n_tiles - 1) % AT_S), ((n_tiles - 1) / AT_S) & 1, 13)) ok = false;
+        asm volatile("bar.sync 9, 256;" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        {
-            const float l = l_run + with_partner(n_tiles & 1, l_run);
-            // the sink: one more term of score 0 (the sums are relative to 2^m_run); with ranges, the merge adds it
-            const float inv = 1.0f / (a.sink && a.n_splits == 1 ? l + sink_term2(a.sink_val, h, m_run) : l);
+        const float2 e = ml[r], o2 = ml[128 + r];
+        const float m = fmaxf(e.x, o2.x);
+        const float l = (e.x == -INFINITY ? 0.f : e.y * at_exp2(e.x - m)) + (o2.x == -INFINITY ? 0.f : o2.y * at_exp2(o2.x - m));
+        // the sink: one more term of score 0 (the sums are relative to 2^m); with ranges, the merge adds it
+        const float inv = 1.0f / (a.sink && a.n_splits == 1 ? l + sink_term2(a.sink_val, h, m) : l);
+#pragma unroll 1
+        for (int c = 64 * x; c < 64 * x + 64; c += 32) {
+            uint32_t v[32];
+            at_ld32(tOmine + c, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float o[32];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint32_t v[32];
-                at_ld32(tOmine + 32 * c, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (a.n_splits > 1) {
-                    if (ok && r < nq) {
-                        const size_t unit = (static_cast<size_t>(row0 + r) * a.nh + h) * a.n_splits + split;
-                        float* po = a.part_o + unit * AT_HD + 64 * half + 32 * c;
+            for (int d = 0; d < 32; ++d) o[d] = __uint_as_float(v[d]);
+            if (!ok || r >= nq) continue;
+            if (a.n_splits > 1) {
+                const size_t unit = (static_cast<size_t>(row0 + r) * a.nh + h) * a.n_splits + split;
+                float* po = a.part_o + unit * AT_HD + c;
 #pragma unroll
-                        for (int d = 0; d < 32; d += 4)
-                            *reinterpret_cast<uint4*>(po + d) = make_uint4(v[d], v[d + 1], v[d + 2], v[d + 3]);
-                        if (half == 0 && c == 0) *reinterpret_cast<float2*>(a.part_ml + unit * 2) = make_float2(m_run, l);
-                    }
-                } else if (ok && r < nq) {
-                    bf16* dst = a.out + (static_cast<size_t>(row0 + r) * a.nh + h) * AT_HD + 64 * half + 32 * c;
+                for (int d = 0; d < 32; d += 4) *reinterpret_cast<float4*>(po + d) = make_float4(o[d], o[d + 1], o[d + 2], o[d + 3]);
+                if (c == 0) *reinterpret_cast<float2*>(a.part_ml + unit * 2) = make_float2(m, l);
+            } else {
+                bf16* dst = a.out + (static_cast<size_t>(row0 + r) * a.nh + h) * AT_HD + c;
 #pragma unroll
-                    for (int d = 0; d < 32; d += 8) {
-                        uint4 pk;
-                        pk.x = at_pack(__uint_as_float(v[d]) * inv, __uint_as_float(v[d + 1]) * inv);
-                        pk.y = at_pack(__uint_as_float(v[d + 2]) * inv, __uint_as_float(v[d + 3]) * inv);
-                        pk.z = at_pack(__uint_as_float(v[d + 4]) * inv, __uint_as_float(v[d + 5]) * inv);
-                        pk.w = at_pack(__uint_as_float(v[d + 6]) * inv, __uint_as_float(v[d + 7]) * inv);
-                        *reinterpret_cast<uint4*>(dst + d) = pk;
-                    }
+                for (int d = 0; d < 32; d += 8) {
+                    uint4 pk;
+                    pk.x = at_pack(o[d] * inv, o[d + 1] * inv);
+                    pk.y = at_pack(o[d + 2] * inv, o[d + 3] * inv);
+                    pk.z = at_pack(o[d + 4] * inv, o[d + 5] * inv);
+                    pk.w = at_pack(o[d + 6] * inv, o[d + 7] * inv);
+                    *reinterpret_cast<uint4*>(dst + d) = pk;
                 }
             }
         }
@@ -669,7 +703,7 @@ static int at_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const C
                      int n_splits, float* part_o, float* part_ml, cudaStream_t stream) {
     if (n_items > 65535) return LOCUS_ERR_UNSUPPORTED;
     a.n_splits = n_splits; a.part_o = part_o; a.part_ml = part_ml;
-    const size_t smem = 7 * AT_TILE_BYTES + 160 + 2 * 2 * 128 * 4;
+    const size_t smem = (1 + 2 * AT_S) * AT_TILE_BYTES + 8 * (6 * AT_S + 2) + 16 + 2 * 128 * 8;
     static bool set = false;
     if (!set) {
         if (cudaFuncSetAttribute(attn_chunk_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -678,8 +712,8 @@ static int at_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const C
         set = true;
     }
     dim3 grid(a.nh, n_items, n_splits);
-    if (a.slopes != nullptr) attn_chunk_tc_kernel<true><<<grid, 320, smem, stream>>>(map_q, map_k, map_v, a);
-    else attn_chunk_tc_kernel<false><<<grid, 320, smem, stream>>>(map_q, map_k, map_v, a);
+    if (a.slopes != nullptr) attn_chunk_tc_kernel<true><<<grid, 384, smem, stream>>>(map_q, map_k, map_v, a);
+    else attn_chunk_tc_kernel<false><<<grid, 384, smem, stream>>>(map_q, map_k, map_v, a);
     if (n_splits > 1)
         attn_chunk_tc_merge_kernel<<<dim3(AT_MQ * (AT_HD / 4) / 128, n_items, a.nh), 128, 0, stream>>>(a);
     return locus_launch_status();
