@@ -19,10 +19,10 @@
 // memory so that stores are 16 or 32 bytes wide.  Grouped products (experts) take the tile list
 // that moe_sort built.
 //
-// What sets the pace (measured with clock stamps in the kernel, taken out again): the thread
-// that issues the MMAs -- an MMA is accepted only when the tensor pipe has room, 4 MMAs of a
-// k-block take about 560 cycles to issue and the whole loop about 700 -- and the epilogue, which
-// must stay well below the main loop of a tile to hide behind it.  Hence the lean issue loop,
+// What sets the pace: the warp that issues the MMAs -- an MMA is accepted only when the tensor pipe has room, 4 MMAs of a
+// k-block of 256 tokens are 512 cycles -- the shared memory, which the operands' arrival and the MMAs' reading of them (768
+// cycles a k-block for one block, 512 for each of a pair), and the epilogue, which
+// must stay well below the main loop of a tile to hide behind it.  Hence the lean issue loop, the pairs of blocks,
 // and the SwiGLU switch as a template parameter: as a run-time flag the compiler evaluated the
 // SwiGLU arithmetic for every product and selected afterwards, which made the epilogue as long
 // as the main loop.
@@ -52,6 +52,8 @@ struct XMaps {
 };
 __host__ __device__ __forceinline__ int x_box_index(int rows) { return rows <= 16 ? 0 : (rows + 31) / 32; }
 __host__ __device__ __forceinline__ int x_box_rows(int index) { return index == 0 ? 16 : 32 * index; }
+// Token rows of a pair's MMA: an even number of sixteens (either block holds half of them).
+__host__ __device__ __forceinline__ int pair_rows(int rows) { return (rows + 31) & ~31; }
 
 struct TileGeom {
     int x_row0, rows_valid, tx, w_row0;  // first token row, live token rows, weight tile, first weight row
@@ -109,6 +111,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// A look that never waits (try_wait may suspend the warp for a few microseconds, which a small product's end would wait for).
+__device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait: false (and the error word set to `code`) when the limit runs out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -127,6 +142,38 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
         : "memory");
+}
+
+// A pair of blocks: the address of the same place in the first block's shared memory, ...
+__device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+// ... a load into this block's shared memory that is counted by a barrier of either block, ...
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+// ... the MMA of both (issued by the first: 128 rows of A from either block, half of B's rows from either, the sums in the
+// tensor memory of the block that A came from), its commit to the same barrier of both, and a barrier of all their threads.
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
@@ -168,7 +215,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
 // warps drain this one.
 // (ALT: an epilogue with an instance of its own, so that the other products' unrolled epilogue does not carry it: the tanh
 // of activation 3 with one weight matrix, the rectified gate of activation 4 with two.)
-template <bool DUAL, bool ALT = false>
+// PAIR: two blocks on neighbouring SMs (a cluster) work on a tile of 256 weight rows together, 128 rows each; either fetches
+// half of the tile's tokens, and the MMAs of the pair read them from both.
+template <bool DUAL, bool ALT, bool PAIR>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                const __grid_constant__ XMaps maps_x, TcArgs a) {
@@ -181,7 +230,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const long long n_total = static_cast<long long>(a.tiles_x) * n_y * a.splits;
 
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzled tiles need 1024-byte alignment
-    const uint32_t x_bytes = static_cast<uint32_t>(a.TN) * TILE_K * 2;
+    const uint32_t x_bytes = static_cast<uint32_t>(a.TN) * TILE_K * 2 / (PAIR ? 2 : 1);
+    const int rank = PAIR ? static_cast<int>(blockIdx.x & 1) : 0;   // (a cluster is two neighbours along x)
+    constexpr int ROWS = PAIR ? 2 * TILE_W : TILE_W;                // weight rows of a tile
     const uint32_t stage_bytes = A_BYTES * (1 + DUAL) + x_bytes;
     const uint32_t bars = base + a.stages * stage_bytes;
     // barriers: full[s], empty[s], accumulator full[2], accumulator empty[2], then the TMEM slot
@@ -198,17 +249,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_acc_full + 8 * b, 1);
-            mbar_init(bar_acc_empty + 8 * b, 4);  // one arrival per epilogue warp
+            mbar_init(bar_acc_empty + 8 * b, PAIR ? 8 : 4);  // one arrival per epilogue warp (of both blocks, at the first's)
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(a.tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(a.tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(a.tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) pair_sync();   // the other block's barriers are there too
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *slot_ptr;
     const int nkb = (a.K + TILE_K - 1) / TILE_K;
@@ -235,7 +292,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         g.kb1 = min(nkb, g.kb0 + a.kb_per_split);
         const int ty = ti / a.tiles_x;  // blocks that run together share a token tile
         g.tx = ti - ty * a.tiles_x;
-        g.w_row0 = g.tx * TILE_W;
+        g.w_row0 = g.tx * ROWS + rank * TILE_W;
         if (a.tile_expert != nullptr) {
             g.x_row0 = a.tile_row0[ty];
             g.rows_valid = a.tile_rows[ty];
@@ -247,20 +304,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         g.out_row0 = g.x_row0 + split * a.M;
         return g;
     };
-    const long long t_step = gridDim.x;
+    const long long t_step = gridDim.x / (PAIR ? 2 : 1), t_first = blockIdx.x / (PAIR ? 2 : 1);
 
     if (warp == 0) {
         if (lane == 0) {
             int s = 0;          // stage of the ring, running over all tiles
             uint32_t round = 0;  // how often the ring has wrapped (its low bit is the barriers' phase)
             bool ok = true;      // false once a bounded wait ran out: the role stops
-            TileGeom g = tile_geom(blockIdx.x);
-            for (long long t = blockIdx.x; t < n_total && ok; t += t_step) {
+            TileGeom g = tile_geom(t_first);
+            for (long long t = t_first; t < n_total && ok; t += t_step) {
                 const TileGeom g_next = tile_geom(t + t_step);
                 const int x_row0 = g.x_row0, w_row0 = g.w_row0;
-                const int box = x_box_index(g.rows_valid);
+                const int box = x_box_index(PAIR ? pair_rows(g.rows_valid) / 2 : g.rows_valid);
                 const CUtensorMap* map_x = &maps_x.m[box];
-                const uint32_t bytes = A_BYTES * (1 + DUAL) + static_cast<uint32_t>(min(x_box_rows(box), a.TN)) * (TILE_K * 2);
+                const uint32_t bytes = A_BYTES * (1 + DUAL) + static_cast<uint32_t>(min(x_box_rows(box), PAIR ? a.TN / 2 : a.TN)) * (TILE_K * 2);
+                const int x_mine = PAIR ? x_row0 + rank * (pair_rows(g.rows_valid) / 2) : x_row0;
                 const int kb_end = g.kb1;
                 for (int kb = g.kb0; kb < kb_end; ++kb) {
                     if (!mbar_wait(bar_empty + 8 * s, (round & 1) ^ 1, 1)) {
@@ -268,10 +326,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         break;
                     }
                     const uint32_t st = base + s * stage_bytes;
-                    mbar_expect_tx(bar_full + 8 * s, bytes);
-                    tma_load_2d(st, &map_w, kb * TILE_K, w_row0, bar_full + 8 * s);
-                    if (DUAL) tma_load_2d(st + A_BYTES, &map_w2, kb * TILE_K, w_row0, bar_full + 8 * s);
-                    tma_load_2d(st + A_BYTES * (1 + DUAL), map_x, kb * TILE_K, x_row0, bar_full + 8 * s);
+                    if (PAIR) {   // the first block's barrier counts what arrives in both
+                        const uint32_t bar = in_leader(bar_full + 8 * s);
+                        if (rank == 0) mbar_expect_tx(bar_full + 8 * s, 2 * bytes);
+                        tma_load_2d_pair(st, &map_w, kb * TILE_K, w_row0, bar);
+                        if (DUAL) tma_load_2d_pair(st + A_BYTES, &map_w2, kb * TILE_K, w_row0, bar);
+                        tma_load_2d_pair(st + A_BYTES * (1 + DUAL), map_x, kb * TILE_K, x_mine, bar);
+                    } else {
+                        mbar_expect_tx(bar_full + 8 * s, bytes);
+                        tma_load_2d(st, &map_w, kb * TILE_K, w_row0, bar_full + 8 * s);
+                        if (DUAL) tma_load_2d(st + A_BYTES, &map_w2, kb * TILE_K, w_row0, bar_full + 8 * s);
+                        tma_load_2d(st + A_BYTES * (1 + DUAL), map_x, kb * TILE_K, x_mine, bar_full + 8 * s);
+                    }
                     if (++s == a.stages) {
                         s = 0;
                         ++round;
@@ -281,12 +347,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // This thread sets the pace of the block: an MMA is accepted only when the tensor pipe has room,
-            // so what the thread does between the last MMA of one k-block and the first of the next is time
-            // the pipe may stand idle.  Hence no divisions, descriptors advanced by addition, and a look at
-            // the next stage's barrier right after this stage's MMAs went out.
-            unsigned n_done = 0;
+        if (rank == 0) {
+            // This warp sets the pace of the block: an MMA is accepted only when the tensor pipe has room,
+            // so what it does between the last MMA of one k-block and the first of the next is time
+            // the pipe may stand idle.  Hence no divisions, descriptors advanced by addition, a look at
+            // the next stage's barrier right after this stage's MMAs went out -- and the whole warp walks while one elected thread
+            // issues: with all of the loop inside a branch for one thread, 4 MMAs, a commit and a wait took 540 cycles
+            // however small the MMAs, this way 280.
+            uint32_t elected;
+            asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
             int s = 0, buf = 0;
             uint32_t round = 0, acc_round = 0;
             bool ok = true;
@@ -294,8 +363,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const uint64_t stage_units = stage_bytes >> 4;  // descriptors count in 16-byte units
             const uint64_t w2_units = A_BYTES >> 4, x_units = (A_BYTES * (1 + DUAL)) >> 4;
             bool ready = false;
-            TileGeom g = tile_geom(blockIdx.x);
-            for (long long t = blockIdx.x; t < n_total && ok; t += t_step) {
+            TileGeom g = tile_geom(t_first);
+            for (long long t = t_first; t < n_total && ok; t += t_step) {
                 const TileGeom g_next = tile_geom(t + t_step);
                 const int rows_valid = g.rows_valid, kb_first = g.kb0, kb_end = g.kb1;
                 g = g_next;
@@ -305,9 +374,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 // instruction descriptor: f32 accumulate, bf16 x bf16, both operands K-major, M = 128; N covers
                 // only the valid token rows of this tile, rounded up to 16: a ragged tile (or an expert with
                 // few rows) costs MMA time for its rows, not for the whole tile
-                const int n_mma = min(a.TN, (rows_valid + 15) & ~15);
+                const int n_mma = PAIR ? pair_rows(rows_valid) : min(a.TN, (rows_valid + 15) & ~15);
                 const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n_mma >> 3) << 17) |
-                                       (static_cast<uint32_t>(TILE_W >> 4) << 24);
+                                       (static_cast<uint32_t>(ROWS >> 4) << 24);
                 const uint32_t d0 = tmem + buf * acc_cols;
                 for (int kb = kb_first; kb < kb_end; ++kb) {
                     if (!ready && !mbar_wait(bar_full + 8 * s, round & 1, 2)) {
@@ -316,22 +385,35 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t dw = desc0 + s * stage_units, dw2 = dw + w2_units, dx = dw + x_units;
+                    if (elected) {
 #pragma unroll
-                    for (int k4 = 0; k4 < TILE_K / 16; ++k4) {
-                        const uint32_t acc = (kb > kb_first || k4 > 0) ? 1u : 0u;
-                        umma_bf16(d0, dw + 2 * k4, dx + 2 * k4, idesc, acc);  // 16 elements = 32 bytes = 2 units
-                        if (DUAL) umma_bf16(d0 + a.TN, dw2 + 2 * k4, dx + 2 * k4, idesc, acc);
+                        for (int k4 = 0; k4 < TILE_K / 16; ++k4) {  // 16 elements = 32 bytes = 2 units
+                            const uint32_t acc = (kb > kb_first || k4 > 0) ? 1u : 0u;
+                            if (PAIR) {
+                                umma_bf16_pair(d0, dw + 2 * k4, dx + 2 * k4, idesc, acc);
+                                if (DUAL) umma_bf16_pair(d0 + a.TN, dw2 + 2 * k4, dx + 2 * k4, idesc, acc);
+                            } else {
+                                umma_bf16(d0, dw + 2 * k4, dx + 2 * k4, idesc, acc);
+                                if (DUAL) umma_bf16(d0 + a.TN, dw2 + 2 * k4, dx + 2 * k4, idesc, acc);
+                            }
+                        }
+                        // the stage is free when these MMAs have read it, the accumulators complete when the last ones are done
+                        if (PAIR) {
+                            umma_commit_pair(bar_empty + 8 * s);
+                            if (kb == kb_end - 1) umma_commit_pair(bar_acc_full + 8 * buf);
+                        } else {
+                            umma_commit(bar_empty + 8 * s);
+                            if (kb == kb_end - 1) umma_commit(bar_acc_full + 8 * buf);
+                        }
                     }
-                    umma_commit(bar_empty + 8 * s);  // the stage is free when these MMAs have read it
+                    __syncwarp();
                     if (++s == a.stages) {
                         s = 0;
                         ++round;
                     }
-                    ready = mbar_try_wait(bar_full + 8 * s, round & 1);  // (past the last stage: simply not ready)
+                    ready = __all_sync(0xffffffffu, mbar_peek(bar_full + 8 * s, round & 1));  // (past the last stage: not ready)
                 }
                 if (!ok) break;
-                umma_commit(bar_acc_full + 8 * buf);
-                ++n_done;
                 if (++buf == a.acc_bufs) {
                     buf = 0;
                     ++acc_round;
@@ -348,14 +430,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const int esize = a.out_dt == LOCUS_DT_F32 ? 4 : 2;
         const bool rows_aligned = (a.ldo * esize) % 16 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
         float* outf = static_cast<float*>(a.out);
-        unsigned n_done = 0;
         int buf = 0;
         uint32_t acc_round = 0;
         // Row scales come through two dependent loads (row index, then scale) behind the tile list: the
         // lane holds the scales of this tile, the row indices of the next and the geometry of the two
         // after it, each fetched one tile before it is needed.
         constexpr int NS = 256 / 32;  // token rows of a tile per lane
-        TileGeom g = tile_geom(blockIdx.x), g1 = tile_geom(blockIdx.x + t_step), g2 = tile_geom(blockIdx.x + 2 * t_step);
+        TileGeom g = tile_geom(t_first), g1 = tile_geom(t_first + t_step), g2 = tile_geom(t_first + 2 * t_step);
         auto scale_index = [&](const TileGeom& q, int k) -> int {
             const int c = lane + 32 * k;
             if (c >= q.rows_valid) return -1;
@@ -371,11 +452,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 idx1[k] = scale_index(g1, k);
             }
         }
-        for (long long t = blockIdx.x; t < n_total; t += t_step) {
+        for (long long t = t_first; t < n_total; t += t_step) {
             const TileGeom g3 = tile_geom(t + 3 * t_step);
             const int rows_valid = g.rows_valid, tx = g.tx;
             const int x_row0 = g.out_row0;  // rows of out; the row scales go by the token rows (scale_index)
-            const long long n = static_cast<long long>(tx) * TILE_W + row;  // output column of this lane
+            const long long n = static_cast<long long>(tx) * ROWS + rank * TILE_W + row;  // output column of this lane
             const bool n_ok = n < a.N;
             if (a.row_scale) {
 #pragma unroll
@@ -396,7 +477,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const float bias2 = (ALT && DUAL && n_ok) ? pair_bias(a.bias, a.bias_dt, a.N + n) : 0.f;
             // Wide stores: the warp's 32 output columns x 16 token rows go through a small transpose in
             // shared memory so that a lane writes 8 consecutive columns of one token (16 or 32 bytes).
-            const long long n_warp = static_cast<long long>(tx) * TILE_W + quarter * 32;
+            const long long n_warp = static_cast<long long>(tx) * ROWS + rank * TILE_W + quarter * 32;
             const bool wide = rows_aligned && n_warp + 32 <= a.N;
             // Add-into with wide stores reads the old values of out: those loads do not depend on the
             // accumulators, so they are issued one 16-row step ahead (the first before the accumulators
@@ -525,8 +606,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             // this warp has read everything it needs from the buffer: hand it back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty + 8 * buf) : "memory");
-            ++n_done;
+            if (lane == 0) {
+                if (PAIR) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_leader(bar_acc_empty + 8 * buf)) : "memory");
+                else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty + 8 * buf) : "memory");
+            }
             if (++buf == a.acc_bufs) {
                 buf = 0;
                 ++acc_round;
@@ -535,9 +618,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) pair_sync();   // the other block is done with this one's memory and barriers
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
     }
 }
 
@@ -641,6 +726,26 @@ extern "C" int locus_gemm_tc(const void* x, long long x_rows_total, long long ld
         return LOCUS_ERR_UNSUPPORTED;
     if (accumulate && out_dt != LOCUS_DT_F32) return LOCUS_ERR_UNSUPPORTED;
     if (w_rows_total >= (1LL << 31) || x_rows_total >= (1LL << 31)) return LOCUS_ERR_UNSUPPORTED;
+    static int n_sm = 0;
+    if (n_sm == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0)
+            return static_cast<int>(cudaGetLastError());
+    }
+    // Pairs of blocks on tiles of 256 weight rows: where the tensor cores set the pace (token tiles of 128 and more), where a last
+    // half tile does not cost a thirtieth of the weights, and, of a plain product, where an SM's tiles have at least 48 k-blocks
+    // together (a pair starts and ends about 1 us later).  Measured, one block / pairs: 2,048 x 6,144 x 2,048 44.2 / 41.0 us, pairs of
+    // 5,632 x 2,048 80.1 / 71.4, 2,048 x 3,584 x 3,584 51.3 / 44.9, 2,048 x 2,048 x 5,632 39.3 / 38.0 and x 2,048 19.2 / 19.9; experts of
+    // 2,048 tokens, 60 x (1,408 -> 2,048) 77.6 / 70.6, 60 x (2,048 -> 2 x 1,408) 139 / 147 (eleven tiles of 128 rows).  Pairs of
+    // experts' weights with few rows each wait for memory, where one block is 2 % quicker: 64 x (3,584 -> 2 x 2,560), 64 rows an
+    // expert 394 / 402 us, 256 697 / 665.
+    const int one_rows = ceil_div(N, TILE_W) * TILE_W, pair_w_rows = ceil_div(N, 2 * TILE_W) * 2 * TILE_W;
+    const long long sm_blocks = tile_expert ? (1LL << 30)
+                                            : (static_cast<long long>(ceil_div(N, TILE_W)) * ceil_div(M, TN) * (splits > 1 ? splits : 1) + n_sm - 1) /
+                                                  n_sm * ceil_div(K, TILE_K) / (splits > 1 ? splits : 1);
+    const bool pair = TN >= 128 && TN % 32 == 0 && (pair_w_rows - one_rows) * 30 <= one_rows && sm_blocks >= 48 &&
+                      !(dual && tile_expert != nullptr && M < 96 * (w_rows_total / N));
     CUtensorMap map_w, map_w2;
     XMaps maps_x;
     memset(&maps_x, 0, sizeof(maps_x));
@@ -649,18 +754,19 @@ extern "C" int locus_gemm_tc(const void* x, long long x_rows_total, long long ld
     {
         // boxes that tiles of this call can ask for: every size up to TN for a grouped product (the rows of
         // a tile are known on the device only), the full tile and the last, ragged one for a plain product
-        const int full = x_box_index(TN), last = x_box_index(M % TN == 0 ? TN : M % TN);
+        const int rest = M % TN == 0 ? TN : M % TN, most = pair ? TN / 2 : TN;
+        const int full = x_box_index(most), last = x_box_index(pair ? pair_rows(rest) / 2 : rest);
         for (int i = 0; i <= full; ++i) {
             if (tile_expert == nullptr && i != full && i != last) continue;
-            const int rows = x_box_rows(i) < TN ? x_box_rows(i) : TN;
+            const int rows = x_box_rows(i) < most ? x_box_rows(i) : most;
             if (!make_map(&maps_x.m[i], x, x_rows_total, K, ldx, rows)) return LOCUS_ERR_UNSUPPORTED;
         }
     }
     TcArgs a;
     a.M = M; a.N = N; a.K = K; a.TN = TN; a.dual = dual;
-    const int stage_bytes = A_BYTES * (1 + dual) + TN * TILE_K * 2;
+    const int stage_bytes = A_BYTES * (1 + dual) + TN * TILE_K * 2 / (pair ? 2 : 1);
     const int tiles_y = tile_expert ? max_tiles : ceil_div(M, TN);
-    const int tiles_x = ceil_div(N, TILE_W);
+    const int tiles_x = ceil_div(N, pair ? 2 * TILE_W : TILE_W);
     const long long n_tiles_all = static_cast<long long>(tiles_x) * tiles_y;
     // one block per SM with the whole shared memory as its pipeline
     const int budget = (g_budget_kb > 0 ? g_budget_kb : 200) * 1024;
@@ -700,29 +806,27 @@ extern "C" int locus_gemm_tc(const void* x, long long x_rows_total, long long ld
     a.scale_rows = split ? nullptr : scale_rows; a.tile_expert = tile_expert; a.tile_row0 = tile_row0;
     a.tile_rows = tile_rows; a.n_tiles = n_tiles;
     const size_t smem = static_cast<size_t>(stages) * stage_bytes + 16 * stages + 96 + 16 * TN + 4 * 16 * 36 * 4 + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-            cudaFuncSetAttribute(gemm_tc_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-            cudaFuncSetAttribute(gemm_tc_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-            cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
-            return static_cast<int>(cudaGetLastError());
-        attr_set = true;
-    }
+    auto* kernel = dual ? (act == 4 ? (pair ? gemm_tc_kernel<true, true, true> : gemm_tc_kernel<true, true, false>)
+                                    : (pair ? gemm_tc_kernel<true, false, true> : gemm_tc_kernel<true, false, false>))
+                        : (act == 3 ? (pair ? gemm_tc_kernel<false, true, true> : gemm_tc_kernel<false, true, false>)
+                                    : (pair ? gemm_tc_kernel<false, false, true> : gemm_tc_kernel<false, false, false>));
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return static_cast<int>(e);
     if (tiles_y <= 0) return 0;
-    static int n_sm = 0;
-    if (n_sm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0)
-            return static_cast<int>(cudaGetLastError());
-    }
-    const long long n_units = n_tiles_all * a.splits;
-    const unsigned grid = static_cast<unsigned>(n_units < n_sm ? n_units : n_sm);
-    if (dual && act == 4) gemm_tc_kernel<true, true><<<grid, 192, smem, stream>>>(map_w, map_w2, maps_x, a);
-    else if (dual) gemm_tc_kernel<true><<<grid, 192, smem, stream>>>(map_w, map_w2, maps_x, a);
-    else if (act == 3) gemm_tc_kernel<false, true><<<grid, 192, smem, stream>>>(map_w, map_w2, maps_x, a);
-    else gemm_tc_kernel<false><<<grid, 192, smem, stream>>>(map_w, map_w2, maps_x, a);
+    const long long n_units = n_tiles_all * a.splits, most_blocks = pair ? n_sm / 2 : n_sm;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(n_units < most_blocks ? n_units : most_blocks) * (pair ? 2 : 1));
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pair ? 1 : 0;
+    const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, map_w, map_w2, maps_x, a);
+    if (le != cudaSuccess) return static_cast<int>(le);
     if (split) {
         const long long n_threads = static_cast<long long>(M) * (N / 4);
         locus_launch(splitk_reduce_kernel, static_cast<unsigned>((n_threads + 255) / 256), 256, 0, stream,

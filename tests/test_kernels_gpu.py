@@ -1184,6 +1184,47 @@ def test_linear_tensor_cores_large_tiles(M, N, K_):
     assert K.tc_error() == 0
 
 
+@pytest.mark.parametrize("M,N,dual", [(2125, 924, False), (2048, 512, True), (2333, 1300, True)])
+def test_linear_tensor_cores_pairs_of_blocks(M, N, dual):
+    """Products of enough k-blocks for pairs of blocks on tiles of 256 weight rows: a last token tile of a few rows (an odd number of
+    sixteens), weight rows that end within either block of a pair, and exactly; the same rows as bfloat16 and added to float32."""
+    dt, K_ = torch.bfloat16, 3208
+    x, w, w2 = rnd(M, K_, dtype=dt, seed=3), rnd(N, K_, dtype=dt, seed=4, scale=0.02), rnd(N, K_, dtype=dt, seed=5, scale=0.02)
+    old = rnd(M, N, seed=7)
+    g = (x.float() @ w.float().T).double()   # (float32 sums, far inside bfloat16's tolerance)
+    ref = torch.nn.functional.silu(g) * (x.float() @ w2.float().T).double() if dual else g
+    out, res = torch.empty(M, N, dtype=dt, device=DEV), old.to(DEV)
+    K.linear(x.to(DEV), w.to(DEV), out, w2=w2.to(DEV) if dual else None)
+    close(out, ref, dt, f"{M} x {N} dual={dual}")
+    K.linear(x.to(DEV), w.to(DEV), res, w2=w2.to(DEV) if dual else None, accumulate=True)
+    close(res, old.double() + ref, dt, f"{M} x {N} dual={dual}, added")
+    assert K.tc_error() == 0
+
+
+def test_linear_tensor_cores_pairs_of_blocks_of_experts():
+    """The same over experts' tiles: no row, a few, one tile and several, of 128 and of 256 rows."""
+    T, E, k, H, I, dt = 330, 5, 2, 256, 512, torch.bfloat16
+    ids = _route(T, E, k, 3)
+    ids[ids == 2] = 1
+    ids[-300:] = 4
+    ids[: 9] = 3
+    h, wts = rnd(T, H, dtype=dt, seed=1), torch.rand(T * k, generator=torch.Generator().manual_seed(5))
+    wg, wu, wd = rnd(E, I, H, dtype=dt, seed=2, scale=0.1), rnd(E, I, H, dtype=dt, seed=3, scale=0.1), rnd(E, H, I, dtype=dt, seed=4, scale=0.1)
+    lay, ref_lay = K.ExpertLayout(T * k, E, 64, DEV), EK.ExpertLayout(T * k, E, 64, "cpu")
+    K.moe_sort(ids.to(DEV), T * k, lay, 128, 256)
+    EK.moe_sort(ids, T * k, ref_lay, 128)
+    xs = h[(ref_lay.sorted_pair.long() // k)].contiguous()
+    act, ref_act = torch.empty(T * k, I, dtype=dt, device=DEV), torch.empty(T * k, I, dtype=torch.float64)
+    K.linear(xs.to(DEV), wg.to(DEV), act, w2=wu.to(DEV), layout=lay, n_rows=T * k)
+    EK.linear(xs, wg, ref_act, w2=wu, layout=ref_lay, n_rows=T * k)
+    close(act, ref_act, dt, "gate and up")
+    out, ref = torch.empty(T * k, H, device=DEV), torch.empty(T * k, H, dtype=torch.float64)
+    K.linear(act, wd.to(DEV), out, layout=lay, n_rows=T * k, row_scale=wts.to(DEV), scale_rows=lay.sorted_pair, second_tiles=True)
+    EK.linear(act.cpu(), wd, ref, layout=ref_lay, n_rows=T * k, row_scale=wts, scale_rows=ref_lay.sorted_pair)
+    close(out, ref, dt, "down")
+    assert K.tc_error() == 0
+
+
 @pytest.mark.parametrize("M,N,K_,tile,splits", [(64, 2048, 2048, 64, 8), (70, 132, 5632, 32, 16), (257, 64, 200, 128, 3),
                                                 (512, 2048, 1408, 256, 4), (40, 260, 72, 64, 2)])
 def test_linear_tensor_cores_split_along_k(M, N, K_, tile, splits, monkeypatch):
