@@ -22,11 +22,24 @@
 //   gla_tokens  for steps of few tokens a request (decoding): 16 columns of a head and 8 groups of rows to a block, so that
 //               a row of the state is read and written in whole sectors (64 requests: 46 -> 24 us).
 //
-// The order of every sum is fixed by d and by the kernel.  (A chunked form -- per chunk of 16 tokens the products with
-// e^(L_i - L_j), L the running sum of log a, every exponent <= 0 -- needs an exponential per pair of tokens and channel and
-// was slower than a walk.)
+//   gla_chunk   for long portions of heads of 128 channels: sixteen tokens together, as matrix products.  With C_i = 1 - a_0 .. a_i and
+//               R_j = 1 - a_(j+1) .. a_15 within the sixteen (formed from the c by C <- C + c - C c, so that a slow channel
+//               keeps its rate),
+//                   o_i = ((1 - C_i) q_i) . S + sum_(j <= i) A_ij v_j,   A_ij = sum_d q_id k_jd a_(j+1)d .. a_id,
+//                   S  <- S - C_15 S + sum_j ((1 - R_j) k_j) v_j^T.
+//               Everything but the last product's sum and the reading of S is the same for all columns of a head and for all tokens
+//               at once: gla_chunk_prep forms it, in three bfloat16 parts (chunk_mma.cuh).  What remains of the walk is a state in
+//               the registers of eight warps, sixteen channels each, 24 MMAs a warp for sixteen tokens (36 of one), and sums
+//               over the warps, which nothing waits for: the chain from chunk to chunk is one multiply-add.
+//               Bound by the latency of a chunk's chain of loads, cuts and MMAs, 1,500 cycles with two warps a scheduler.  Measured,
+//               2,048 tokens of 16 heads of 128 x 128: 255 -> 132 us (26 of them gla_chunk_prep), eight requests of 256 181 -> 113,
+//               one of 64 13.5 -> 13.2 (of 32 9.4 / 11.1: the walk's); the error against 64 bits 4.3e-7 -> 2.0e-7 of the
+//               read-outs' norm, of the state 4.4e-7 -> 1.3e-7.  Two chunks to a turn, one block an SM: 134 and 135 us.
+//
+// The order of every sum is fixed by d and by the kernel.
 #include "common.cuh"
 #include "walk.cuh"
+#include "chunk_mma.cuh"
 
 struct GlaArgs {
     const float* q;
@@ -335,6 +348,290 @@ __global__ void __launch_bounds__(128) gla_tokens_kernel(const GlaArgs a, int co
     }
 }
 
+#define GC_D 128                 // channels of a head
+#define GC_LD (GC_D + 8)         // bfloat16 from row to row of a chunk's operands (rows meet in no bank)
+#define GC_ALD 24                // the same of a chunk's 16 x 16 matrices
+#define GC_PART (CH * GC_LD)     // a part of q or k
+#define GC_STAGE (2 * (6 * GC_PART + 3 * CH * GC_ALD) + 4 * GC_D)   // bytes: q, k, A, C
+#define GC_STAGES 3
+
+// What gla_chunk_prep leaves for rows w0 .. w1 of the step: a stage's bytes for every chunk and head, as they lie in shared memory.
+struct GlaChunks {
+    uint8_t* at;
+    int w0, w1;
+};
+// A segment's rows within the window and the place of its first chunk: behind those of the rows in front of it, of which every
+// segment may have left one unfilled (segments need not come in the order of their rows).
+__device__ __forceinline__ void gla_window(const GlaArgs& a, const GlaChunks& s, int seg, int n_seg, int& q0, int& qn, int& chunk0) {
+    const int first = a.seg_q0[seg], last = min(first + a.seg_qn[seg], s.w1);
+    q0 = max(first, s.w0);
+    qn = last - q0;
+    if (qn <= 0) return;
+    chunk0 = (q0 - s.w0) / CH;
+    for (int j = 0; j < n_seg; ++j) chunk0 += a.seg_q0[j] < first && a.seg_qn[j] > 0 ? 1 : 0;
+}
+
+// 64 threads to a chunk and head, two channels each; a block takes four heads of a chunk.
+__global__ void __launch_bounds__(256) gla_chunk_prep(const GlaArgs a, const GlaChunks s) {
+    __shared__ float sums[4][2][160];
+    pdl_entry();
+    pdl_trigger();
+    int q0, qn, chunk0 = 0;
+    gla_window(a, s, blockIdx.y, gridDim.y, q0, qn, chunk0);
+    const int t0 = blockIdx.x * CH, live = min(CH, qn - t0);
+    if (live <= 0) return;
+    const int hl = threadIdx.x >> 6, h = blockIdx.z * 4 + hl, tid = threadIdx.x & 63, lane = tid & 31, half = tid >> 5;
+    const bool on = h < a.H;
+    const int d0 = 2 * tid, hh = on ? h : 0;
+    float2 q[CH], k[CH], c[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+        q[i] = k[i] = c[i] = make_float2(0.f, 0.f);
+        if (i < live) {
+            const size_t row = static_cast<size_t>(q0 + t0 + i);
+            q[i] = *reinterpret_cast<const float2*>(a.q + row * a.ldq + a.off_q + hh * GC_D + d0);
+            k[i] = *reinterpret_cast<const float2*>(a.k + row * a.ldk + a.off_k + hh * GC_D + d0);
+            c[i] = *reinterpret_cast<const float2*>(a.a + row * a.lda + a.off_a + hh * GC_D + d0);
+        }
+    }
+    auto grow = [](float& x, float rate) { x += fmaf(-x, rate, rate); };   // 1 - (1 - x)(1 - rate)
+    uint8_t* st = s.at + (static_cast<size_t>(chunk0 + blockIdx.x) * a.H + hh) * GC_STAGE;
+    bf16* parts = reinterpret_cast<bf16*>(st);
+    bf16* amat = parts + 6 * GC_PART;
+    float* rates = reinterpret_cast<float*>(amat + 3 * CH * GC_ALD);
+    auto leave = [&](int i, int which, float x, float y) {   // (rows that are not there: zeros)
+        if (!on) return;
+        uint32_t p[3];
+        ch_cut(x, y, p);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(parts + (3 * which + j) * GC_PART + i * GC_LD + d0) = p[j];
+    };
+    {
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            grow(x, c[i].x);
+            grow(y, c[i].y);
+            leave(i, 0, fmaf(-x, q[i].x, q[i].x), fmaf(-y, q[i].y, q[i].y));
+        }
+        if (on) *reinterpret_cast<float2*>(rates + d0) = make_float2(x, y);
+    }
+    {
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int j = CH - 1; j >= 0; --j) {
+            leave(j, 1, fmaf(-x, k[j].x, k[j].x), fmaf(-y, k[j].y, k[j].y));
+            grow(x, c[j].x);
+            grow(y, c[j].y);
+        }
+    }
+    // A: pair (j, i), i = j .. 15, is value 16 j - j (j - 1) / 2 + i - j; 32 values cross the lanes together
+    float v[32];
+    int n = 0;
+#pragma unroll
+    for (int j = 0; j < CH; ++j) {
+        float x = k[j].x, y = k[j].y;
+#pragma unroll
+        for (int i = j; i < CH; ++i) {
+            if (i > j) {
+                x = fmaf(-x, c[i].x, x);
+                y = fmaf(-y, c[i].y, y);
+            }
+            v[n & 31] = fmaf(q[i].x, x, q[i].y * y);
+            if ((n & 31) == 31) sums[hl][half][(n & ~31) + walk_sum_index<32>(lane)] = walk_sum<32>(v, lane);
+            ++n;
+        }
+    }
+    {
+        const float last = walk_sum<8>(v, lane);   // 136 = 4 x 32 + 8
+        if (lane < 8) sums[hl][half][128 + walk_sum_index<8>(lane)] = last;
+    }
+    __syncthreads();
+    if (!on) return;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int i = (tid + 64 * u) >> 3, j = 2 * (tid & 7);
+        auto at = [&](int jj) -> float {
+            const int x = 16 * jj - jj * (jj - 1) / 2 + i - jj;
+            return jj <= i ? sums[hl][0][x] + sums[hl][1][x] : 0.f;
+        };
+        uint32_t p[3];
+        ch_cut(at(j), at(j + 1), p);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) *reinterpret_cast<uint32_t*>(amat + (m * CH + i) * GC_ALD + j) = p[m];
+    }
+}
+
+// A block: sixteen columns of one head of one request; warp w keeps S^T of its sixteen columns x channels 16 w .. 16 w + 15, two
+// tiles of sums (chunk_mma.cuh).  Two blocks an SM: 228 KB hold 3 stages and 25 KB of each.
+__global__ void __launch_bounds__(256, 2) gla_chunk_kernel(const GlaArgs a, const GlaChunks s, int col_blocks) {
+    extern __shared__ __align__(16) uint8_t gc_smem[];   // [GC_STAGES][GC_STAGE]
+    __shared__ __align__(8) unsigned long long bars[GC_STAGES];
+    __shared__ __align__(16) bf16 vt[2][3][CH][GC_ALD];  // v^T of a chunk: [parity][part][column][token]
+    __shared__ float vf[3][CH][CH];                      // and as it is, copied two chunks ahead: [chunk][token][column]
+    __shared__ float red[2][8][CH][CH + 4];              // read-outs of the warps: [parity][warp][token][column] (a warp's meet in no bank)
+    pdl_entry();
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int h = blockIdx.x / col_blocks, col0 = (blockIdx.x % col_blocks) * CH;
+    int q0, qn, chunk0 = 0;
+    gla_window(a, s, blockIdx.y, gridDim.y, q0, qn, chunk0);
+    if (qn <= 0) return;
+    if (tid == 0) {
+        for (int i = 0; i < GC_STAGES; ++i) ch_bar_init(ch_smem(&bars[i]));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    const int dv = a.dv, n_chunks = (qn + CH - 1) / CH;
+    float* S = a.state + static_cast<size_t>(a.state_slots[blockIdx.y]) * a.slot_stride + static_cast<size_t>(h) * GC_D * dv;
+    const int vc = tid & 15, vtok = tid >> 4;   // this thread's value of v, and the read-out that it sums up
+
+    auto fetch = [&](int c) {
+        const int i = c % GC_STAGES;
+        if (c < n_chunks)
+            ch_bulk(ch_smem(gc_smem + i * GC_STAGE), s.at + (static_cast<size_t>(chunk0 + c) * a.H + h) * GC_STAGE, GC_STAGE, ch_smem(&bars[i]));
+    };
+    auto copy_v = [&](int c) {   // (a thread lays out what it copied itself)
+        const int tok = c * CH + vtok;
+        const bool live = tok < qn && col0 + vc < dv;
+        walk_copy<4>(&vf[c % 3][vtok][vc], live ? a.v + static_cast<size_t>(q0 + tok) * a.ldv + a.off_v + h * dv + col0 + vc : a.v, live);
+        walk_commit();
+    };
+    auto lay = [&](int c) -> bool {   // v into its places; false where it is not finite
+        const float v = vf[c % 3][vtok][vc];
+        uint32_t p[3];
+        ch_cut(v, 0.f, p);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) *reinterpret_cast<unsigned short*>(&vt[c & 1][j][vc][vtok]) = static_cast<unsigned short>(p[j]);
+        return fabsf(v) < INFINITY;
+    };
+    if (tid == 0)
+        for (int i = 0; i < GC_STAGES - 1; ++i) fetch(i);
+    for (int c = 0; c < 2; ++c) copy_v(c);
+    float sv[2][4];   // S^T: column g (+ 8 for the upper two), channel 16 w + 8 tile + 2 t (+ 1)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int col = col0 + g + 8 * (e >> 1), d = 16 * w + 8 * n + 2 * t + (e & 1);
+            sv[n][e] = col < dv ? S[static_cast<size_t>(d) * dv + col] : 0.f;
+        }
+    walk_wait<1>();
+    bool plain = lay(0);   // this thread's value of the chunk is finite
+    auto read_out = [&](int c, bool odd) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += red[c & 1][i][vtok][vc];
+        if (odd) {   // a v that is not finite must not meet the zeros of A in front of it: what the MMAs left out
+            const bf16* A = reinterpret_cast<const bf16*>(gc_smem + (c % GC_STAGES) * GC_STAGE) + 6 * GC_PART + vtok * GC_ALD;
+            for (int j = 0; j <= vtok; ++j) {
+                const float x = __bfloat162float(A[j]) + __bfloat162float(A[CH * GC_ALD + j]) + __bfloat162float(A[2 * CH * GC_ALD + j]);
+                sum = fmaf(x, vf[c % 3][j][vc], sum);
+            }
+        }
+        const int tok = c * CH + vtok;
+        if (tok < qn && col0 + vc < dv) a.out[static_cast<size_t>(q0 + tok) * a.ldo + h * dv + col0 + vc] = sum * a.q_scale;
+    };
+    bool odd_before = false;
+    for (int c = 0; c < n_chunks; ++c) {
+        const bool odd = __syncthreads_or(!plain);   // the chunk before is left by all
+        if (odd_before) {                            // (its A and v are read once more)
+            read_out(c - 1, true);
+            __syncthreads();
+        }
+        if (tid == 0) fetch(c + GC_STAGES - 1);
+        ch_wait(ch_smem(&bars[c % GC_STAGES]), (c / GC_STAGES) & 1);
+        const bf16* Q = reinterpret_cast<const bf16*>(gc_smem + (c % GC_STAGES) * GC_STAGE);
+        const bf16* Kp = Q + 3 * GC_PART;
+        const bf16* A = Q + 6 * GC_PART;
+        const float* C = reinterpret_cast<const float*>(A + 3 * CH * GC_ALD);
+        // the reading of S, o^T[column][token] over this warp's sixteen channels, and v^T k for its channels
+        float o[2][4], u[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[n][e] = u[n][e] = 0.f;
+        uint32_t sp[3][4], vp[3][4], bq[2][3][2], bk[2][3][2];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            uint32_t p[3];
+            ch_cut(sv[e >> 1][2 * (e & 1)], sv[e >> 1][2 * (e & 1) + 1], p);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) sp[j][e] = p[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            ch_ldsm(vp[j], &vt[c & 1][j][(lane & 7) + 8 * ((lane >> 3) & 1)][8 * (lane >> 4)]);   // v^T: 16 columns x 16 tokens
+            uint32_t r[4];
+            ch_ldsm_t(r, Kp + j * GC_PART + (lane & 15) * GC_LD + 16 * w + 8 * (lane >> 4));
+            bk[0][j][0] = r[0]; bk[0][j][1] = r[1]; bk[1][j][0] = r[2]; bk[1][j][1] = r[3];
+            ch_ldsm(r, Q + j * GC_PART + ((lane & 7) + 8 * (lane >> 4)) * GC_LD + 16 * w + 8 * ((lane >> 3) & 1));
+            bq[0][j][0] = r[0]; bq[0][j][1] = r[1]; bq[1][j][0] = r[2]; bq[1][j][1] = r[3];
+        }
+        // (the four sums' products in turn)
+#define GC_STEP(P) ch_mma_part<P>(u[0], vp, bk[0]); ch_mma_part<P>(o[0], sp, bq[0]); ch_mma_part<P>(u[1], vp, bk[1]); ch_mma_part<P>(o[1], sp, bq[1]);
+        GC_STEP(0) GC_STEP(1) GC_STEP(2) GC_STEP(3) GC_STEP(4) GC_STEP(5)
+#undef GC_STEP
+        if (!odd && w == (c & 7)) {   // the chunk's own tokens: one warp's share, in turn
+            uint32_t ba[2][3][2];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                uint32_t r[4];
+                ch_ldsm(r, A + (j * CH + (lane & 7) + 8 * (lane >> 4)) * GC_ALD + 8 * ((lane >> 3) & 1));
+                ba[0][j][0] = r[0]; ba[0][j][1] = r[1]; ba[1][j][0] = r[2]; ba[1][j][1] = r[3];
+            }
+            ch_mma_pair(o, vp, ba);
+        }
+        // while the MMAs run: the chunk before is summed up, the next one's v laid out
+        if (c > 0 && !odd_before) read_out(c - 1, false);
+        copy_v(c + 2);
+        walk_wait<1>();
+        if (c + 1 < n_chunks) plain = lay(c + 1);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const float2 rate = *reinterpret_cast<const float2*>(C + 16 * w + 8 * n + 2 * t);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                red[c & 1][w][8 * n + 2 * t + (e & 1)][g + 8 * (e >> 1)] = o[n][e];
+                sv[n][e] = fmaf(-((e & 1) ? rate.y : rate.x), sv[n][e], sv[n][e]) + u[n][e];   // S <- S - C S + v^T k
+            }
+        }
+        odd_before = odd;
+    }
+    walk_wait<0>();
+    __syncthreads();
+    read_out(n_chunks - 1, odd_before);
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int col = col0 + g + 8 * (e >> 1), d = 16 * w + 8 * n + 2 * t + (e & 1);
+            if (col < dv) S[static_cast<size_t>(d) * dv + col] = sv[n][e];
+        }
+}
+
+// Rows of a step whose chunks scratch of `bytes` holds, with one unfilled chunk a segment; in whole chunks.
+static long long gla_chunk_rows(int H, int n_seg, long long bytes) {
+    const long long chunks = bytes / (static_cast<long long>(H) * GC_STAGE) - n_seg;
+    return chunks > 0 ? chunks * CH : 0;
+}
+
+static int gla_chunks(const GlaArgs& a, int n_seg, int n_rows, void* scratch, long long scratch_bytes, cudaStream_t stream) {
+    const long long rows = gla_chunk_rows(a.H, n_seg, scratch_bytes);
+    const cudaError_t e = cudaFuncSetAttribute(gla_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_STAGES * GC_STAGE);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    const int col_blocks = ceil_div(a.dv, CH);
+    for (long long w0 = 0; w0 < n_rows; w0 += rows) {
+        GlaChunks s;
+        s.w0 = static_cast<int>(w0);
+        s.w1 = static_cast<int>(w0 + rows < n_rows ? w0 + rows : n_rows);
+        s.at = static_cast<uint8_t*>(scratch);
+        locus_launch(gla_chunk_prep, dim3(ceil_div(s.w1 - s.w0, CH), n_seg, ceil_div(a.H, 4)), dim3(256), 0, stream, a, s);
+        locus_launch(gla_chunk_kernel, dim3(a.H * col_blocks, n_seg), dim3(256), GC_STAGES * GC_STAGE, stream, a, s, col_blocks);
+    }
+    return locus_launch_status();
+}
+
 // z [T, ld] float32, columns [off, off + n): z <- 1 - exp(-softplus(-z) / tau).
 __global__ void __launch_bounds__(256) gla_decay_kernel(float* __restrict__ z, int ld, int off, int n, float inv_tau,
                                                         long long total) {
@@ -378,7 +675,8 @@ static int gla_walk(const GlaArgs& a, bool vec, int n_seg, cudaStream_t stream) 
 extern "C" int locus_gla_scan(const float* q, int ldq, int off_q, const float* k, int ldk, int off_k, const float* v, int ldv,
                               int off_v, const float* dec, int lda, int off_a, float* state, long long slot_stride,
                               const int* state_slots, const int* seg_q0, const int* seg_qn, int n_seg, int n_rows, float* out,
-                              int ldo, int H, int d, int dv, float q_scale, cudaStream_t stream) {
+                              int ldo, int H, int d, int dv, float q_scale, void* scratch, long long scratch_bytes,
+                              cudaStream_t stream) {
     if (n_seg <= 0) return 0;
     if (H <= 0 || d <= 0 || d > 256 || dv <= 0 || n_seg > 65535 || H > 65535) return LOCUS_ERR_UNSUPPORTED;
     GlaArgs a;
@@ -397,6 +695,8 @@ extern "C" int locus_gla_scan(const float* q, int ldq, int off_q, const float* k
     const bool mixed = walk_may_be_mixed(n_rows, n_seg);
     const bool vec = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(dec)) & 15) == 0 &&
                      ((ldq | off_q | ldk | off_k | lda | off_a | d) & 3) == 0;
+    if (scratch != nullptr && vec && d == GC_D && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 && gla_chunk_rows(H, n_seg, scratch_bytes) > 0)
+        return gla_chunks(a, n_seg, n_rows, scratch, scratch_bytes, stream);
     if (d <= 64) return mixed ? gla_walk<2, true>(a, vec, n_seg, stream) : gla_walk<2, false>(a, vec, n_seg, stream);
     if (d <= 128) return mixed ? gla_walk<4, true>(a, vec, n_seg, stream) : gla_walk<4, false>(a, vec, n_seg, stream);
     return mixed ? gla_walk<8, true>(a, vec, n_seg, stream) : gla_walk<8, false>(a, vec, n_seg, stream);

@@ -2296,6 +2296,18 @@ def gla_decay(z: torch.Tensor, off: int, n: int, tau: float) -> None:
     _check(code, "gla_decay")
 
 
+CHUNK_DIM = 128          # channels of a head that gla_scan takes sixteen tokens together (csrc/gla.cu, gla_chunk)
+CHUNK_MIN_TOKENS = 64    # ... of steps of at least so many tokens a segment (64 tokens 13.5 us walked, 13.2 in chunks; 32 9.4, 11.1)
+CHUNK_BYTES = 2 * (6 * 16 * (CHUNK_DIM + 8) + 3 * 16 * 24) + 4 * CHUNK_DIM   # scratch by chunk and head
+
+
+def _chunk_scratch(out: torch.Tensor, n_heads: int, n_seg: int):
+    """(scratch for the chunks of all rows of ``out``, or of as many as the split products' buffer holds; how many rows)."""
+    per, most = n_heads * CHUNK_BYTES, -(-out.shape[0] // 16)
+    chunks = min(most, SPLIT_SCRATCH_BYTES // per - n_seg)
+    return (_split_scratch(out.device, (chunks + n_seg) * per // 4), 16 * chunks) if chunks > 0 else (None, 0)
+
+
 def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.Tensor, off_v: int, decay: torch.Tensor,
              off_a: int, state: torch.Tensor, state_offset: int, state_slots: torch.Tensor, seg_q0: torch.Tensor,
              seg_qn: torch.Tensor, n_seg: int, out: torch.Tensor, *, n_heads: int, dim: int, v_dim: int, q_scale: float) -> None:
@@ -2310,11 +2322,18 @@ def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.
     _need(state.is_cuda and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
           and state_offset + n_heads * dim * v_dim <= state.shape[1], "gla_scan: the state does not hold the heads")
     _need(out.shape[1] == n_heads * v_dim and dim <= GLA_MAX_DIM, "gla_scan: out [T, n_heads * v_dim], dim <= 256")
+    scratch, rows = None, 0
+    if (dim == CHUNK_DIM and n_seg > 0 and out.shape[0] >= CHUNK_MIN_TOKENS * n_seg
+            and (q.data_ptr() | k.data_ptr() | decay.data_ptr()) % 16 == 0
+            and (q.stride(0) | off_q | k.stride(0) | off_k | decay.stride(0) | off_a) % 4 == 0):
+        scratch, rows = _chunk_scratch(out, n_heads, n_seg)
     code = _lib("gla").locus_gla_scan(
         _p(q), I(q.stride(0)), I(off_q), _p(k), I(k.stride(0)), I(off_k), _p(v), I(v.stride(0)), I(off_v), _p(decay),
         I(decay.stride(0)), I(off_a), ctypes.c_void_p(state.data_ptr() + 4 * state_offset), LL(state.stride(0)),
         _p(state_slots), _p(seg_q0), _p(seg_qn), I(n_seg), I(out.shape[0]), _p(out), I(out.stride(0)), I(n_heads), I(dim),
-        I(v_dim), F(q_scale), _stream())
+        I(v_dim), F(q_scale), _p(scratch), LL((rows // 16 + n_seg) * n_heads * CHUNK_BYTES if rows else 0), _stream())
+    if rows and code == 0:
+        _count_launches(2 * -(-out.shape[0] // rows) - 1)   # two for every stretch of rows that the scratch holds
     _check(code, "gla_scan", f"(heads {n_heads}, dim {dim}, v_dim {v_dim})")
 
 

@@ -220,6 +220,60 @@ def test_gla_scan_of_portions_beside_single_tokens(H, d, dv, precise):
         assert torch.equal(o1, out[pick.to(DEV)]) and torch.equal(st1[at], st[at])
 
 
+@pytest.mark.parametrize("H,dv,small", [(5, 128, False), (2, 40, True), (3, 17, False)])
+def test_gla_scan_in_chunks(H, dv, small, precise, monkeypatch):
+    """Heads of 128 channels sixteen tokens together: chunks that are whole, of one token and of fifteen, requests of no token, in
+    another order than their rows, rows that belong to nobody between them, numbers of heads that are no multiple of four and of
+    columns that are none of sixteen, decays of 1 and of nearly 0; and the same where the scratch holds only a part of the rows
+    (requests that go on from one part to the next)."""
+    import locus_b200.kernels as K
+
+    d = 128
+    monkeypatch.setattr(K, "CHUNK_MIN_TOKENS", 0)
+    g = torch.Generator().manual_seed(H)
+    qn, q0 = [65, 0, 1, 47, 16, 95], [130, 7, 4, 5, 52, 200]   # rows 68 .. 129 and 195 .. 199 are nobody's
+    n_seg, T, W = len(qn), 295, 2 * H * d + H * dv + 3
+    W += -W % 4
+    proj, z = torch.randn(T, W, generator=g), torch.rand(T, H * d, generator=g) * 0.3
+    z[:, 0], z[:, 1], z[140, 2] = 0.0, 1.0, 1.0
+    z[:, 3] = 1e-6
+    state = torch.randn(n_seg + 1, H * d * dv, generator=g)
+    slots = torch.tensor([3, 0, 6, 5, 1, 2], dtype=torch.int32)
+    n, q0 = torch.tensor(qn, dtype=torch.int32), torch.tensor(q0, dtype=torch.int32)
+    kw = dict(n_heads=H, dim=d, v_dim=dv, q_scale=d ** -0.5)
+    args = (0, H * d, 2 * H * d + 3)
+    ref_state, ref = state.double(), torch.zeros(T, H * dv, dtype=torch.float64)
+    EK.gla_scan(proj.double(), args[0], proj.double(), args[1], proj.double(), args[2], z.double(), 0, ref_state, 0, slots, q0, n, n_seg, ref, **kw)
+    if small:
+        monkeypatch.setattr(K, "SPLIT_SCRATCH_BYTES", H * K.CHUNK_BYTES * (n_seg + 5))   # five chunks beside the unfilled ones
+        monkeypatch.setattr(K, "_SPLIT_SCRATCH", {})
+    before = K.launches
+
+    def run(p):
+        st, out = state.to(DEV), torch.zeros(T, H * dv, device=DEV)
+        dp = p.to(DEV)
+        K.gla_scan(dp, args[0], dp, args[1], dp, args[2], z.to(DEV), 0, st, 0, slots.to(DEV), q0.to(DEV), n.to(DEV), n_seg, out, **kw)
+        return out, st
+
+    out, st = run(proj)
+    assert K.launches - before == (2 * 4 if small else 2)
+    _cmp(out, ref, 2e-5)
+    _cmp(st, ref_state, 2e-5)
+    assert torch.equal(st[4].cpu(), state[4])   # nobody's slot
+    # a value that is not finite reaches its own column from its token on, and no token in front of it
+    for bad in (float("nan"), float("inf")):
+        odd = proj.clone()
+        odd[141, args[2] + 5] = bad   # request 0, its twelfth token: the middle of a chunk
+        got, gst = run(odd)
+        # (the sixteen columns that share a block with it sum up this chunk's own tokens in another order, with the same bound)
+        assert torch.equal(got[:, 16:], out[:, 16:])
+        clean = torch.ones(T, H * dv, dtype=torch.bool)
+        clean[141:195, 5] = False
+        _cmp(got.cpu()[clean], ref[clean], 2e-5)
+        assert not torch.isfinite(got[141:195, 5]).any()
+        assert not torch.isfinite(gst[3].view(H, d, dv)[0, 3, 5])
+
+
 @pytest.mark.parametrize("H,d,dv", [(2, 24, 16), (1, 7, 5), (3, 72, 40), (2, 128, 64), (1, 200, 12)])
 def test_gla_scan_and_decay_against_twin(H, d, dv, precise):
     import locus_b200.kernels as K
