@@ -29,7 +29,11 @@
 //
 // Keys and values may also lie in plain rows instead of pages (rows form): two matrices [rows][kv heads * 128] in which a
 // segment's keys are consecutive rows from kv_row0[segment] on (latent attention expands its heads' keys and values of a
-// long portion's context that way); only the coordinates of the loads differ.
+// long portion's context that way); only the coordinates of the loads differ.  Queries and keys may then have a rotated part of
+// 64 more dimensions, the keys' one row for all heads: a third 64 columns of Q and K in shared memory, two tiles of K and V
+// instead of three (208 KB).  A latent mixer's portion of 1,000 tokens, 16 heads: 16.0 us, with the gather and the product that
+// expands the keys 23, where the two per-head products and the attention over 576-wide latents took 178; 1,500 tokens behind 3,000:
+// the whole mixer 1,660 -> 196 us, with no larger error against 64 bits (3.3e-3, 3.1e-3).
 //
 // Every wait on an mbarrier is bounded; when one runs out the kernel sets the module's error word,
 // and every later wait of every role returns at once, so the kernel ends quickly instead of hanging.
@@ -238,13 +242,17 @@ __device__ __forceinline__ void at_st32(uint32_t taddr, const uint32_t* v) {
 // sum / denominator is the same number whatever reference it was formed with.
 #define AT_LAG_LOG2 8.0f
 
-#define AT_S 3   // tiles of K, of V (shared memory) and of scores (tensor memory): tile j's in place j % 3
+#define AT_S 3   // tiles of scores in tensor memory: tile j's in place j % 3
 
 // BIAS: a distance bias; an instance of its own (the softmax warps are bound by instruction issue).
-template <bool BIAS>
+// ROT: a rotated part (rows form).
+template <bool BIAS, bool ROT>
 __global__ void __launch_bounds__(384, 1)
 attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                     const __grid_constant__ CUtensorMap map_v, TcAttnArgs a) {
+                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_qr,
+                     const __grid_constant__ CUtensorMap map_kr, TcAttnArgs a) {
+    constexpr int AT_D = ROT ? 2 : 3;                               // tiles of K and of V in shared memory
+    constexpr int AT_QK_BYTES = (ROT ? 3 : 2) * AT_HALF_BYTES;      // a tile of Q or K
     extern __shared__ __align__(1024) uint8_t at_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the late tiles of a prompt see the most keys: the grid takes them first, for all heads (the heads are the
@@ -281,17 +289,19 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (threadIdx.x == 0) atomicCAS(&g_at_error, 0, 12);
         return;
     }
-    const uint32_t sQ = base, sK = sQ + AT_TILE_BYTES, sV = sK + AT_S * AT_TILE_BYTES, bars = sV + AT_S * AT_TILE_BYTES;
-    const uint32_t q_full = bars, k_full = bars + 8, k_free = k_full + 8 * AT_S, v_full = k_free + 8 * AT_S, v_free = v_full + 8 * AT_S;
-    const uint32_t s_full = v_free + 8 * AT_S, p_ready = s_full + 8 * AT_S, slot = p_ready + 8 * AT_S + 8;
+    const uint32_t sQ = base, sK = sQ + AT_QK_BYTES, sV = sK + AT_D * AT_QK_BYTES, bars = sV + AT_D * AT_TILE_BYTES;
+    const uint32_t q_full = bars, k_full = bars + 8, k_free = k_full + 8 * AT_D, v_full = k_free + 8 * AT_D, v_free = v_full + 8 * AT_D;
+    const uint32_t s_full = v_free + 8 * AT_D, p_ready = s_full + 8 * AT_S, slot = p_ready + 8 * AT_S + 8;
 
     if (threadIdx.x == 0) {
         at_bar_init(q_full, 1);
-        for (int b = 0; b < AT_S; ++b) {
+        for (int b = 0; b < AT_D; ++b) {
             at_bar_init(k_full + 8 * b, 1);
             at_bar_init(k_free + 8 * b, 1);
             at_bar_init(v_full + 8 * b, 1);
             at_bar_init(v_free + 8 * b, 1);     // the tile's P V is finished: V's place and that of the scores are free
+        }
+        for (int b = 0; b < AT_S; ++b) {
             at_bar_init(s_full + 8 * b, 1);
             at_bar_init(p_ready + 8 * b, 4);    // one arrival per softmax warp of the group
         }
@@ -316,10 +326,12 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             uint32_t elected;
             asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
             if (elected) {
-                // Q: two halves of 64 elements, rows row0 .. row0 + 127 (rows past the portion are never stored)
-                at_expect_tx(q_full, AT_TILE_BYTES);
-                at_tma_2d(sQ, &map_q, h * AT_HD, row0, q_full);
-                at_tma_2d(sQ + AT_HALF_BYTES, &map_q, h * AT_HD + 64, row0, q_full);
+                // Q: pieces of 64 elements, rows row0 .. row0 + 127 (rows past the portion are never stored)
+                const int col = h * (ROT ? AT_HD + 64 : AT_HD);
+                at_expect_tx(q_full, AT_QK_BYTES);
+                at_tma_2d(sQ, &map_q, col, row0, q_full);
+                at_tma_2d(sQ + AT_HALF_BYTES, &map_q, col + 64, row0, q_full);
+                if (ROT) at_tma_2d(sQ + 2 * AT_HALF_BYTES, &map_qr, h * 64, row0, q_full);
             }
             const long long rows_per_page = 2LL * a.nkv * P;
             const int v_shift = a.kv_row0 ? 0 : a.nkv * P;  // V rows of a page lie nkv * P rows behind its K rows
@@ -344,37 +356,43 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 }
                 return make_int2(__shfl_sync(0xffffffffu, now, 2 * (j & 15)), __shfl_sync(0xffffffffu, now, 2 * (j & 15) + 1));
             };
-            auto load = [&](const CUtensorMap* map, int2 rows, int shift, int j, uint32_t to, uint32_t full, uint32_t free_) {
-                const int turn = j / AT_S, b = j - turn * AT_S;
-                at_wait(free_ + 8 * b, (turn & 1) ^ 1, 1);
+            auto load = [&](bool key, int2 rows, int j) {
+                const int turn = j / AT_D, b = j - turn * AT_D;
+                const uint32_t bar = (key ? k_full : v_full) + 8 * b;
+                at_wait((key ? k_free : v_free) + 8 * b, (turn & 1) ^ 1, 1);
                 if (elected) {
-                    const uint32_t dst = to + b * AT_TILE_BYTES, bar = full + 8 * b;
-                    const int ra = rows.x < 0 ? -64 : rows.x + shift, rb = rows.y < 0 ? -64 : rows.y + shift;
-                    at_expect_tx(bar, AT_TILE_BYTES);
+                    const uint32_t dst = key ? sK + b * AT_QK_BYTES : sV + b * AT_TILE_BYTES;
+                    const CUtensorMap* map = key ? &map_k : &map_v;
+                    const int shift = key ? 0 : v_shift, ra = rows.x < 0 ? -64 : rows.x + shift, rb = rows.y < 0 ? -64 : rows.y + shift;
+                    at_expect_tx(bar, key ? AT_QK_BYTES : AT_TILE_BYTES);
                     at_tma_2d(dst, map, col0, ra, bar);
                     at_tma_2d(dst + AT_HALF_BYTES, map, col0 + 64, ra, bar);
                     at_tma_2d(dst + 64 * 128, map, col0, rb, bar);
                     at_tma_2d(dst + AT_HALF_BYTES + 64 * 128, map, col0 + 64, rb, bar);
+                    if (ROT && key) {
+                        at_tma_2d(dst + 2 * AT_HALF_BYTES, &map_kr, 0, ra, bar);
+                        at_tma_2d(dst + 2 * AT_HALF_BYTES + 64 * 128, &map_kr, 0, rb, bar);
+                    }
                 }
                 __syncwarp();
             };
-            int2 r[AT_S + 1];   // the rows of tiles j .. j + 3
-    #pragma unroll
-            for (int j = 0; j < AT_S; ++j) {
+            int2 r[AT_D + 1];   // the rows of tiles j .. j + AT_D
+#pragma unroll
+            for (int j = 0; j < AT_D; ++j) {
                 r[j] = make_int2(-64, -64);
                 if (j < n_tiles) {
                     r[j] = rows_of(j);
-                    load(&map_k, r[j], 0, j, sK, k_full, k_free);
+                    load(true, r[j], j);
                 }
             }
             for (int j = 0; j < n_tiles; ++j) {
-                load(&map_v, r[0], v_shift, j, sV, v_full, v_free);
-                if (j + AT_S < n_tiles) {
-                    r[AT_S] = rows_of(j + AT_S);
-                    load(&map_k, r[AT_S], 0, j + AT_S, sK, k_full, k_free);
+                load(false, r[0], j);
+                if (j + AT_D < n_tiles) {
+                    r[AT_D] = rows_of(j + AT_D);
+                    load(true, r[AT_D], j + AT_D);
                 }
-    #pragma unroll
-                for (int i = 0; i < AT_S; ++i) r[i] = r[i + 1];
+#pragma unroll
+                for (int i = 0; i < AT_D; ++i) r[i] = r[i + 1];
             }
         } else if (warp < 3) {
             // Warp 1 issues the scores, warp 2 the sums of V: a thread that did both would leave the tensor cores idle while it waits
@@ -386,40 +404,36 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t idesc1 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(AT_MK >> 3) << 17) |
                                     (static_cast<uint32_t>(AT_MQ >> 4) << 24);
             const uint32_t idesc2 = idesc1 | (1u << 16);
-            int b = 0;
-            uint32_t turn = 0;
             if (warp == 1) at_wait(q_full, 0, 5);
             for (int j = 0; j < n_tiles; ++j) {
+                const int turn_d = j / AT_D, d = j - turn_d * AT_D, turn_s = j / AT_S, b = j - turn_s * AT_S;   // places of K and V, of the scores
                 if (warp == 1) {
-                    at_wait(k_full + 8 * b, turn & 1, 3);
-                    at_wait(v_free + 8 * b, (turn & 1) ^ 1, 4);   // the tile before in this place has been weighted and added up
+                    at_wait(k_full + 8 * d, turn_d & 1, 3);
+                    // the tile before in this place of the scores has been weighted and added up
+                    if (j >= AT_S) at_wait(v_free + 8 * ((j - AT_S) % AT_D), ((j - AT_S) / AT_D) & 1, 4);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elected) {
-    #pragma unroll
-                        for (int ks = 0; ks < AT_HD / 16; ++ks) {  // S = Q K^T
+#pragma unroll
+                        for (int ks = 0; ks < (ROT ? AT_HD + 64 : AT_HD) / 16; ++ks) {  // S = Q K^T
                             const uint32_t off = (ks >> 2) * AT_HALF_BYTES + (ks & 3) * 32;
-                            at_mma(tS + b * AT_MK, at_desc_k(sQ + off), at_desc_k(sK + b * AT_TILE_BYTES + off), idesc1, ks > 0);
+                            at_mma(tS + b * AT_MK, at_desc_k(sQ + off), at_desc_k(sK + d * AT_QK_BYTES + off), idesc1, ks > 0);
                         }
                         at_commit(s_full + 8 * b);
-                        at_commit(k_free + 8 * b);
+                        at_commit(k_free + 8 * d);
                     }
                 } else {
-                    at_wait(v_full + 8 * b, turn & 1, 7);
-                    at_wait(p_ready + 8 * b, turn & 1, 6);
+                    at_wait(v_full + 8 * d, turn_d & 1, 7);
+                    at_wait(p_ready + 8 * b, turn_s & 1, 6);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elected) {
-    #pragma unroll
+#pragma unroll
                         for (int ks = 0; ks < AT_MK / 16; ++ks)  // O += P V
-                            at_mma_ts(tO, tS + b * AT_MK + 8 * ks, at_desc_mn(sV + b * AT_TILE_BYTES + ks * (16 * 128), AT_HALF_BYTES), idesc2,
+                            at_mma_ts(tO, tS + b * AT_MK + 8 * ks, at_desc_mn(sV + d * AT_TILE_BYTES + ks * (16 * 128), AT_HALF_BYTES), idesc2,
                                       (j > 0 || ks > 0) ? 1u : 0u);
-                        at_commit(v_free + 8 * b);
+                        at_commit(v_free + 8 * d);
                     }
                 }
                 __syncwarp();
-                if (++b == AT_S) {
-                    b = 0;
-                    ++turn;
-                }
             }
         }
     } else {
@@ -502,7 +516,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             // and rescales its sum, once the product of the tile before is in it.
             if (__any_sync(0xffffffffu, m_new - m_run > AT_LAG_LOG2)) {
                 if (j > 0) {
-                    if (!at_wait(v_free + 8 * ((j - 1) % AT_S), ((j - 1) / AT_S) & 1, 12)) ok = false;
+                    if (!at_wait(v_free + 8 * ((j - 1) % AT_D), ((j - 1) / AT_D) & 1, 12)) ok = false;
                     const float f = m_run == -INFINITY ? 1.f : at_exp2(m_run - m_new);
                     const unsigned long long f2 = at_pair(f, f);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -552,11 +566,12 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             }
             // the last tile may hold rows of V behind the sequence's end (never written, any bit pattern): zero them
             if (tile0 + AT_MK - 1 > t_hi) {
-                if (!at_wait(v_full + 8 * b, turn & 1, 11)) ok = false;
+                const int d = j % AT_D;
+                if (!at_wait(v_full + 8 * d, (j / AT_D) & 1, 11)) ok = false;
                 if (tile0 + r > t_hi)
 #pragma unroll
                     for (int q8 = 0; q8 < 16; ++q8)
-                        *reinterpret_cast<uint4*>(at_raw + (sV - base) + b * AT_TILE_BYTES + (q8 >> 3) * AT_HALF_BYTES + r * 128 + (q8 & 7) * 16) =
+                        *reinterpret_cast<uint4*>(at_raw + (sV - base) + d * AT_TILE_BYTES + (q8 >> 3) * AT_HALF_BYTES + r * 128 + (q8 & 7) * 16) =
                             make_uint4(0, 0, 0, 0);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
@@ -569,8 +584,11 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // The last tile's reference is the larger one and that of the sum; a group writes half of the columns of its rows.  (A group
         // without a tile counts for nothing.)
         ml[x * 128 + r] = make_float2(m_run, l_run);
-        // (the wait counts in the group of the last tile, whose scores came behind the sum before in this place; the other meets it)
-        if (!at_wait(v_free + 8 * ((n_tiles - 1) % AT_S), ((n_tiles - 1) / AT_S) & 1, 13)) ok = false;
+        // (The last sum, and before it the one before in its place, so that its barrier is not one turn further back than the wait takes
+        // it to be: that of the last tile but three is complete, its scores' place was used again.  The group of the last tile counts;
+        // the other meets it.)
+        for (int j = max(n_tiles - 1 - AT_D, (n_tiles - 1) % AT_D); j < n_tiles; j += AT_D)
+            if (!at_wait(v_free + 8 * (j % AT_D), (j / AT_D) & 1, 13)) ok = false;
         asm volatile("bar.sync 9, 256;" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float2 e = ml[r], o2 = ml[128 + r];
@@ -700,20 +718,18 @@ static bool at_make_map(CUtensorMap* map, const void* ptr, long long rows, long 
 
 // The launch shared by the entry points below: `a` carries everything but the scratch of the ranges.
 static int at_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, TcAttnArgs a, int n_items,
-                     int n_splits, float* part_o, float* part_ml, cudaStream_t stream) {
+                     int n_splits, float* part_o, float* part_ml, cudaStream_t stream, const CUtensorMap* map_qr = nullptr,
+                     const CUtensorMap* map_kr = nullptr) {
     if (n_items > 65535) return LOCUS_ERR_UNSUPPORTED;
     a.n_splits = n_splits; a.part_o = part_o; a.part_ml = part_ml;
-    const size_t smem = (1 + 2 * AT_S) * AT_TILE_BYTES + 8 * (6 * AT_S + 2) + 16 + 2 * 128 * 8;
-    static bool set = false;
-    if (!set) {
-        if (cudaFuncSetAttribute(attn_chunk_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_chunk_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return static_cast<int>(cudaGetLastError());
-        set = true;
-    }
+    const bool rot = map_qr != nullptr;
+    const size_t smem = (rot ? 3 * 3 + 2 * 2 : 2 + 3 * 4) * AT_HALF_BYTES + 8 * (6 * AT_S + 2) + 16 + 2 * 128 * 8;
+    auto* kernel = a.slopes != nullptr ? (rot ? attn_chunk_tc_kernel<true, true> : attn_chunk_tc_kernel<true, false>)
+                                       : (rot ? attn_chunk_tc_kernel<false, true> : attn_chunk_tc_kernel<false, false>);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
     dim3 grid(a.nh, n_items, n_splits);
-    if (a.slopes != nullptr) attn_chunk_tc_kernel<true><<<grid, 384, smem, stream>>>(map_q, map_k, map_v, a);
-    else attn_chunk_tc_kernel<false><<<grid, 384, smem, stream>>>(map_q, map_k, map_v, a);
+    kernel<<<grid, 384, smem, stream>>>(map_q, map_k, map_v, rot ? *map_qr : map_q, rot ? *map_kr : map_k, a);
     if (n_splits > 1)
         attn_chunk_tc_merge_kernel<<<dim3(AT_MQ * (AT_HD / 4) / 128, n_items, a.nh), 128, 0, stream>>>(a);
     return locus_launch_status();
@@ -758,14 +774,19 @@ extern "C" int locus_attn_chunk_tc(const void* q, long long T, const void* pool,
 }
 
 // The rows form: k and v [rows, >= nkv * 128] bfloat16 with row strides ldk, ldv (elements, multiples of 8, 16-byte aligned
-// bases); segment s's key at position t is row kv_row0[s] + t of both.  Otherwise as above.
+// bases); segment s's key at position t is row kv_row0[s] + t of both.  With k_rot [rows, 64] (row stride ldkr) keys have 64 more
+// dimensions, the same for all heads, and queries those of q_rot [T, nh * 64]; a head's first 128 of q then lie 192 elements
+// apart (its last 64 there are not read).  Otherwise as above.
 extern "C" int locus_attn_chunk_tc_rows(const void* q, long long T, const void* k, long long ldk, const void* v, long long ldv,
                                         long long rows, void* out, const int* seg_q0, const int* seg_qn, const int* seg_ctx,
                                         const int* kv_row0, const int* items, int n_items, int nh, int nkv, int hd, int window,
                                         int chunk, float scale, int n_splits, float* part_o, float* part_ml, int keep_first,
-                                        int sink, const float* sink_val, const float* slopes, cudaStream_t stream) {
+                                        int sink, const float* sink_val, const float* slopes, const void* q_rot, const void* k_rot,
+                                        long long ldkr, cudaStream_t stream) {
     if (n_items <= 0) return 0;
     if (!at_scratch_ok(n_splits, part_o, part_ml)) return LOCUS_ERR_UNSUPPORTED;
+    if ((q_rot != nullptr) != (k_rot != nullptr) || (k_rot != nullptr && (ldkr < 64 || ldkr % 8 != 0))) return LOCUS_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(q_rot) | reinterpret_cast<uintptr_t>(k_rot)) & 15) return LOCUS_ERR_UNSUPPORTED;
     if (hd != AT_HD || kv_row0 == nullptr || !mask_ok(window, chunk, keep_first)) return LOCUS_ERR_UNSUPPORTED;
     if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || nh > 65535) return LOCUS_ERR_UNSUPPORTED;
     if (T <= 0 || T >= (1LL << 31) || rows <= 0 || rows >= (1LL << 31)) return LOCUS_ERR_UNSUPPORTED;
@@ -773,8 +794,12 @@ extern "C" int locus_attn_chunk_tc_rows(const void* q, long long T, const void* 
     if (ldk < cols || ldv < cols || ldk % 8 != 0 || ldv % 8 != 0) return LOCUS_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15)
         return LOCUS_ERR_UNSUPPORTED;
-    CUtensorMap map_q, map_k, map_v;
-    if (!at_make_map(&map_q, q, T, static_cast<long long>(nh) * hd, static_cast<long long>(nh) * hd, AT_MQ) ||
+    CUtensorMap map_q, map_k, map_v, map_qr, map_kr;
+    const long long q_cols = static_cast<long long>(nh) * (k_rot ? hd + 64 : hd);
+    if (k_rot && (!at_make_map(&map_qr, q_rot, T, static_cast<long long>(nh) * 64, static_cast<long long>(nh) * 64, AT_MQ) ||
+                  !at_make_map(&map_kr, k_rot, rows, 64, ldkr, 64)))
+        return LOCUS_ERR_UNSUPPORTED;
+    if (!at_make_map(&map_q, q, T, q_cols, q_cols, AT_MQ) ||
         !at_make_map(&map_k, k, rows, cols, ldk, 64) || !at_make_map(&map_v, v, rows, cols, ldv, 64))
         return LOCUS_ERR_UNSUPPORTED;
     TcAttnArgs a;
@@ -783,7 +808,7 @@ extern "C" int locus_attn_chunk_tc_rows(const void* q, long long T, const void* 
     a.page_tokens = 64; a.window = window; a.chunk = chunk; a.scale = scale;
     a.keep_first = window > 0 ? keep_first : 0; a.sink = sink ? 1 : 0; a.sink_val = sink ? sink_val : nullptr;
     a.slopes = slopes;
-    return at_launch(map_q, map_k, map_v, a, n_items, n_splits, part_o, part_ml, stream);
+    return at_launch(map_q, map_k, map_v, a, n_items, n_splits, part_o, part_ml, stream, k_rot ? &map_qr : nullptr, k_rot ? &map_kr : nullptr);
 }
 
 // Reads and clears the module's error word (0 = no bounded wait ran out).  Synchronises.

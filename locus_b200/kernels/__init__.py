@@ -1050,11 +1050,13 @@ def attn_chunk_tc_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: t
                        seg_qn: torch.Tensor, seg_ctx: torch.Tensor, kv_row0: torch.Tensor, items: torch.Tensor, n_items: int,
                        n_heads: int, n_kv_heads: int, head_dim: int, window: int, scale: float, n_splits: int = 1,
                        part_o: Optional[torch.Tensor] = None, part_ml: Optional[torch.Tensor] = None, keep_first: int = 0,
-                       sink=False, chunk: int = 0, slopes: Optional[torch.Tensor] = None) -> None:
+                       sink=False, chunk: int = 0, slopes: Optional[torch.Tensor] = None, q_rot: Optional[torch.Tensor] = None,
+                       k_rot: Optional[torch.Tensor] = None) -> None:
     """:func:`attn_chunk_tc` over keys and values in plain rows instead of pages: ``k`` and ``v`` [rows, n_kv_heads *
     head_dim] (stretches of columns of wider rows are taken), a segment's key at position t in row ``kv_row0[segment]`` + t
     of both.  ``items`` lists tiles of 64 queries of the segments that have such rows; the others' entries of ``kv_row0`` are
-    not read."""
+    not read.  ``k_rot`` [rows, 64]: 64 more dimensions of the keys, the same for all heads, and ``q_rot`` [T, n_heads * 64] of the
+    queries; ``q`` is then [T, n_heads * (head_dim + 64)], of which a head's last 64 are not read."""
     _cuda_c(q, "q")
     _cuda_c(out, "out")
     _i32(items, "items")
@@ -1063,6 +1065,12 @@ def attn_chunk_tc_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: t
     for t in (k, v):
         _need(t.is_cuda and t.stride(1) == 1 and t.shape[0] == k.shape[0] and t.shape[1] == n_kv_heads * head_dim,
               "attn_chunk_tc_rows: k, v rows [rows, n_kv_heads * head_dim]")
+    _need((q_rot is None) == (k_rot is None), "attn_chunk_tc_rows: a rotated part of queries and keys, or of neither")
+    if k_rot is not None:
+        _cuda_c(q_rot, "q_rot")
+        _need(q_rot.dtype == k_rot.dtype == torch.bfloat16 and q_rot.shape == (q.shape[0], n_heads * 64) and k_rot.is_cuda
+              and k_rot.stride(1) == 1 and k_rot.shape == (k.shape[0], 64) and q.shape[1] == n_heads * (head_dim + 64),
+              "attn_chunk_tc_rows: rotated parts of 64")
     _need(1 <= n_splits <= TC_ATTN_MAX_SPLITS, f"attn_chunk_tc_rows: 1 to {TC_ATTN_MAX_SPLITS} key ranges")
     if n_splits > 1:
         units = q.shape[0] * n_heads * n_splits
@@ -1073,7 +1081,8 @@ def attn_chunk_tc_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: t
         _p(q), LL(q.shape[0]), _p(k), LL(k.stride(0)), _p(v), LL(v.stride(0)), LL(k.shape[0]), _p(out), _p(seg_q0), _p(seg_qn),
         _p(seg_ctx), _p(kv_row0), _p(items), I(n_items), I(n_heads), I(n_kv_heads), I(head_dim), I(window), I(chunk), F(scale),
         I(n_splits), _p(part_o if n_splits > 1 else None), _p(part_ml if n_splits > 1 else None),
-        I(keep_first if window > 0 else 0), *_sink_args(sink, n_heads), _slopes_arg(slopes, n_heads), _stream())
+        I(keep_first if window > 0 else 0), *_sink_args(sink, n_heads), _slopes_arg(slopes, n_heads), _p(q_rot), _p(k_rot),
+        LL(k_rot.stride(0) if k_rot is not None else 0), _stream())
     if n_splits > 1 and code == 0:
         _count_launches(1)
     _check(code, "attn_chunk_tc", f"(rows; heads {n_heads}/{n_kv_heads}, head_dim {head_dim}, {n_splits} key ranges)")
@@ -1602,17 +1611,26 @@ def latent_attn(q_abs_hm: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tensor,
 # of two products per context row and is shared by the portion's queries.  Measured at 16 heads of 128 on a latent of 512, all
 # kernels between the queries and the output projection, over the latents / expanded: 2,048 tokens 561 / 55 us; 128 tokens
 # behind 0, 1,024 and 8,192 others 45 / 16, 77 / 34 and 307 / 91 us; 64 tokens over the latents 32, 54 and 157 us.
-LATENT_EXPAND_FROM = 64          # new tokens of a segment from which on it is expanded
+LATENT_EXPAND_FROM = 64          # new tokens of a segment from which on it is expanded (with a rotated part: 69 / 54 us)
 LATENT_EXPAND_ROWS = 16384       # most context rows of a step that are expanded ...
 LATENT_EXPAND_BYTES = 512 << 20  # ... and most bytes of their keys and values; segments beyond run over the latents
 
 
 def latent_expand_rows(dtype: torch.dtype, n_heads: int, nope_dim: int, rot_dim: int, v_dim: int, kv_rank: int) -> int:
     """Context rows of a step that may be expanded for the tcgen05 attention kernel; 0 where it does not take this mixer's sizes
-    (bfloat16, keys without a rotated part and values of the kernel's head size)."""
-    if not (USE_TENSOR_CORES and dtype == torch.bfloat16 and nope_dim == v_dim == TC_ATTN_HEAD_DIM and rot_dim == 0 and kv_rank % 8 == 0):
+    (bfloat16, values and the keys' own part of the kernel's head size, a rotated part of 64 or none)."""
+    if not (USE_TENSOR_CORES and dtype == torch.bfloat16 and nope_dim == v_dim == TC_ATTN_HEAD_DIM and rot_dim in (0, 64) and kv_rank % 8 == 0):
         return 0
     return min(LATENT_EXPAND_ROWS, LATENT_EXPAND_BYTES // (2 * n_heads * (nope_dim + v_dim)))
+
+
+def latent_expand_pays(n_new: int, n_ctx: int, window: int) -> bool:
+    """Whether to expand the whole context of a segment that sees only ``window`` keys of it (0: all): a product over rows
+    that nobody sees (7 us a thousand, 16 heads on a latent of 512) is spent for less work on every pair of a query and a key
+    and for the per-head products.  Device time of the mixer over the latents / expanded, window 128: 64 new tokens behind 2,000
+    82 / 71 us, behind 4,000 82 / 86; 1,000 behind 4,000 164 / 130, behind 8,000 164 / 159; window 2,048: 256 behind 15,000 236 / 189."""
+    behind = n_ctx + 1 - window if window > 0 else 0
+    return behind <= max(2048, n_new * window // 32)
 
 
 def latent_gather(pool: torch.Tensor, out: torch.Tensor, *, segs: torch.Tensor, n_segs: int, row0: torch.Tensor,

@@ -22,8 +22,9 @@ W_uk, W_uv and queries.  The rotated parts' pairs are interleaved, (2i, 2i + 1),
 position encoding says.
 
 Long portions (kernels.LATENT_EXPAND_FROM tokens of a request on) of sizes that the tcgen05 attention kernel takes go the
-other way: the cached latents of the request's context are gathered into plain rows, expanded into every head's keys and
-values by one product with [W_uk; W_uv], and attended to by that kernel.  The pages hold latents either way.
+other way: the cached rows of the request's context are gathered into plain rows, their latents expanded into every head's keys and
+values by one product with [W_uk; W_uv], and attended to by that kernel, which takes the rotated part as it was cached.  The
+pages hold latents either way.
 
 The softmax's denominator may hold a learned sink per head, exp(sink_h), without a key or a value.  A query at
 position p sees the keys j with p - window < j <= p (window 0: all).  Scores, softmax, the norms' statistics,
@@ -44,17 +45,18 @@ class LatentTiles(StepPlan):
     """Work items of the latent attention kernels, for every segment by its new tokens: tiles of ``tile`` queries
     (``items``); with ``singles`` the segments with one new token go to a list of their own (``single_items``), which the
     decode kernel takes; with ``max_rows`` > 0 the segments with at least ``expand_from`` new tokens, as long as the rows of
-    their contexts fit into ``max_rows`` together, go to tiles of 64 queries (``long_items``), with the segments, the first row
+    their contexts fit into ``max_rows`` together and not too many lie behind a ``window``, go to tiles of 64 queries (``long_items``), with the segments, the first row
     of each and the rows of all.  Tiles are ordered by the position of their first query (the kernels walk a list from its
     end, so the tiles with the most keys start first)."""
 
-    def __init__(self, tile: int = K.LATENT_QUERY_TILE, singles: bool = False, max_rows: int = 0, expand_from: int = 0) -> None:
+    def __init__(self, tile: int = K.LATENT_QUERY_TILE, singles: bool = False, max_rows: int = 0, expand_from: int = 0, window: int = 0) -> None:
         from ..cache import native
 
         self._lib = native.lib()
         self.tile, self.singles = int(tile), bool(singles)
         self.max_rows, self.expand_from = int(max_rows), int(expand_from) if max_rows else 0
-        self.key = ("latent_attention.tiles", self.tile, self.singles, self.max_rows, self.expand_from)
+        self.window = int(window) if max_rows else 0
+        self.key = ("latent_attention.tiles", self.tile, self.singles, self.max_rows, self.expand_from, self.window)
 
     def capacity(self, max_tokens: int, max_segments: int) -> int:
         return 2 * (max_tokens // self.tile + max_tokens // K.MMA_QUERY_TILE + 2 * max_segments) + 3 * max_segments
@@ -82,7 +84,7 @@ class LatentTiles(StepPlan):
             row0 = np.full(n_seg, -1, dtype=np.int32)
             for s in np.nonzero(seg_qn >= self.expand_from)[0]:
                 n = int(seg_ctx[s]) + int(seg_qn[s])
-                if rows + n <= self.max_rows:
+                if rows + n <= self.max_rows and K.latent_expand_pays(int(seg_qn[s]), int(seg_ctx[s]), self.window):
                     row0[s] = rows
                     rows += n
                     longest = max(longest, n)
@@ -223,7 +225,7 @@ class LatentAttention(Mixer):
         tile = 64 >> self._head_shift if self._mma else K.LATENT_QUERY_TILE
         self._singles = K.latent_decode_takes(dtype, self.kv_rank, self.dr)
         self._max_rows = self._expand_rows(dtype)
-        return LatentTiles(tile, self._singles, self._max_rows, K.LATENT_EXPAND_FROM)
+        return LatentTiles(tile, self._singles, self._max_rows, K.LATENT_EXPAND_FROM, self.window)
 
     @property
     def _head_tiles(self) -> HeadTiles:
@@ -270,19 +272,22 @@ class LatentAttention(Mixer):
         K.linear(cq if self.q_rank else h, self.params["w_uq"], q)
         o = rt.rows("latent.o", H * self.dv, rt.dtype, T)
         tiles = batch.plans[self._tiles_key]
-        if tiles["n_items"] or tiles.get("n_single_items"):
-            self._attend_latents(q, o, tiles, batch, cache, gb, rt)
-        if tiles.get("n_long_items"):
-            self._attend_expanded(q, o, tiles, batch, cache, gb, rt)
+        latents, expanded = tiles["n_items"] or tiles.get("n_single_items"), tiles.get("n_long_items")
+        split = self._split_queries(q, batch, rt) if latents or self.dr else None
+        if latents:
+            self._attend_latents(*split, o, tiles, batch, cache, gb, rt)
+        if expanded:
+            self._attend_expanded(q, split[1] if self.dr else None, o, tiles, batch, cache, gb, rt)
         if self.out_gate:
             K.gate_rows(o, down, self.n_down, n_heads=H, dim=self.dv, laid=self.dv)
         K.linear(o, self.params["w_o"], residual, accumulate=accumulate)
 
-    def _attend_expanded(self, q, o, tiles, batch, cache, gb, rt) -> None:
+    def _attend_expanded(self, q, q_rot, o, tiles, batch, cache, gb, rt) -> None:
         """The step's long segments: their contexts' keys and values expanded into rows [keys of all heads | values of all heads]."""
         H, n = self.H, tiles["n_rows"]
-        c = rt.buf(f"latent.c_rows{self.kv_rank}", (self._max_rows, self.kv_rank), rt.dtype)[:n]
-        K.latent_gather(cache.pool, c, segs=tiles["long_segs"], n_segs=tiles["n_long"], row0=tiles["row0"], seg_qn=batch.seg_qn,
+        rows = rt.buf(f"latent.c_rows{self.kv_rank}.{self.dr}", (self._max_rows, self.kv_rank + self.dr), rt.dtype)[:n]
+        c, rotated = rows[:, :self.kv_rank], dict(q_rot=q_rot, k_rot=rows[:, self.kv_rank:]) if self.dr else {}
+        K.latent_gather(cache.pool, rows, segs=tiles["long_segs"], n_segs=tiles["n_long"], row0=tiles["row0"], seg_qn=batch.seg_qn,
                         seg_ctx=batch.seg_ctx, block_table=gb.block_table, page_tokens=gb.page_tokens, longest=tiles["longest"])
         kv = rt.buf("latent.kv_rows", (self._max_rows, H * (self.dn + self.dv)), rt.dtype)[:n]
         K.linear(c, self.params["w_ukv"], kv)
@@ -298,20 +303,22 @@ class LatentAttention(Mixer):
         K.attn_chunk_tc_rows(q, kv[:, : H * self.dn], kv[:, H * self.dn:], o, seg_q0=batch.seg_q0, seg_qn=batch.seg_qn, seg_ctx=batch.seg_ctx,
                              kv_row0=tiles["row0"], items=tiles["long_items"], n_items=tiles["n_long_items"], n_heads=H, n_kv_heads=H,
                              head_dim=self.dn, window=self.window, scale=self.scale, n_splits=n_splits, part_o=part_o, part_ml=part_ml,
-                             sink=self._sink if self._sink is not None else False)
+                             sink=self._sink if self._sink is not None else False, **rotated)
 
-    def _attend_latents(self, q, o, tiles, batch, cache, gb, rt) -> None:
-        """The step's short segments over the cached latents themselves (the per-head products run over all rows)."""
+    def _split_queries(self, q, batch, rt):
+        """The queries' own parts by head, [heads x rows, nope_dim], and their rotated parts, [rows, heads x rot_dim]."""
         T, H = batch.T, self.H
         table = self.position.rotary_table()
-        freq = table.freq64 if table is not None else None
-        pairs = table.rot_dim // 2 if table is not None else 0
-        mag = table.magnitude if table is not None else 1.0
-        half = table is not None and not table.interleaved
         q_nope = rt.rows(f"latent.q_nope{self.dn}", self.dn, rt.dtype, H * T, per_token=H)
         q_rot = rt.rows("latent.q_rot", H * self.dr, rt.dtype, T)
-        K.latent_q_split(q, batch.positions, freq, mag, q_nope, q_rot, n_heads=H, nope_dim=self.dn, rot_dim=self.dr,
-                         rot_pairs=pairs, half_split=half)
+        K.latent_q_split(q, batch.positions, table.freq64 if table is not None else None, table.magnitude if table is not None else 1.0,
+                         q_nope, q_rot, n_heads=H, nope_dim=self.dn, rot_dim=self.dr,
+                         rot_pairs=table.rot_dim // 2 if table is not None else 0, half_split=table is not None and not table.interleaved)
+        return q_nope, q_rot
+
+    def _attend_latents(self, q_nope, q_rot, o, tiles, batch, cache, gb, rt) -> None:
+        """The step's short segments over the cached latents themselves (the per-head products run over all rows)."""
+        T, H = batch.T, self.H
         ht = batch.plans[self._head_tiles.key]
         lay = K.HeadLayout(H, ht["tile"], ht["offsets"], ht["tile_head"], ht["tile_row0"], ht["tile_rows"],
                            ht["n_tiles"], ht["count"])

@@ -525,8 +525,8 @@ def attn_chunk_tc_splits(n_items, n_heads, max_ctx, n_rows=0):
 
 
 def attn_chunk_tc_rows(q, k, v, out, *, seg_q0, seg_qn, seg_ctx, kv_row0, items, n_items, n_heads, n_kv_heads, head_dim, window, scale,
-                       n_splits=1, part_o=None, part_ml=None, keep_first=0, sink=False, chunk=0, slopes=None):
-    assert window == 0 and keep_first == 0 and chunk == 0
+                       n_splits=1, part_o=None, part_ml=None, keep_first=0, sink=False, chunk=0, slopes=None, q_rot=None, k_rot=None):
+    assert keep_first == 0 and chunk == 0
     group = n_heads // n_kv_heads
     for seg in sorted({int(items[i, 0]) for i in range(n_items)}):
         q0, qn, ctx, r0 = int(seg_q0[seg]), int(seg_qn[seg]), int(seg_ctx[seg]), int(kv_row0[seg])
@@ -534,7 +534,12 @@ def attn_chunk_tc_rows(q, k, v, out, *, seg_q0, seg_qn, seg_ctx, kv_row0, items,
             p = ctx + i
             for h in range(n_heads):
                 cols = slice((h // group) * head_dim, (h // group + 1) * head_dim)
-                s = (_f(k[r0:r0 + p + 1, cols]) @ _f(q[q0 + i].view(n_heads, head_dim)[h])) * scale
+                s = _f(k[r0:r0 + p + 1, cols]) @ _f(q[q0 + i].view(n_heads, -1)[h, :head_dim])
+                if k_rot is not None:
+                    s = s + _f(k_rot[r0:r0 + p + 1]) @ _f(q_rot[q0 + i].view(n_heads, -1)[h])
+                s = s * scale
+                if window:
+                    s[: max(0, p + 1 - window)] = -float("inf")
                 if slopes is not None:
                     s = s - _f(slopes)[h] * (p - torch.arange(p + 1, dtype=s.dtype))
                 if sink is not False:

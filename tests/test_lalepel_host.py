@@ -160,3 +160,31 @@ def test_greedy_generation_through_the_scheduler(tmp_path):
                 assert int(torch.argmax(lg[-1])) == tok
             seq.append(tok)
     assert eng.cache.free_pages() == eng.cache.total_pages()
+
+
+def test_long_portions_with_expanded_keys_and_a_rotated_part(tmp_path, monkeypatch):
+    """Portions of at least eight tokens take the rows form with the rotated parts beside it; one that has more context behind its
+    window than the rule allows stays on the latents, beside one in the same step that does not."""
+    import locus_b200.kernels as K
+
+    monkeypatch.setattr(K, "LATENT_EXPAND_FROM", 8)
+    monkeypatch.setattr(K, "latent_expand_rows", lambda dtype, H, dn, dr, dv, rank: 200)
+    monkeypatch.setattr(K, "latent_expand_pays", lambda n, ctx, window: window == 20 and ctx + 1 - window <= 25)
+    calls, rows = [], K.attn_chunk_tc_rows
+    monkeypatch.setattr(K, "attn_chunk_tc_rows", lambda *a, **kw: (calls.append((sorted({int(s) for s, _ in kw["items"].tolist()}),
+                                                                                 tuple(kw["q_rot"].shape), kw["k_rot"].shape[1])), rows(*a, **kw)))
+    case = Case("latent_only", tmp_path, torch.float32, requests=(90, 30))
+    runner, cache = make_runner(case, torch.float32, "cpu", page_tokens=8, n_pages=24, max_tokens=72, slots=2)
+    steps = [[("r0", 44)], [("r0", 10), ("r1", 3)], [("r1", 9), ("r0", 20)], [("r1", 18)], [("r0", 16)]]
+    got, routed = run_steps(runner, cache, case, steps)
+    compare(case, got, routed, *TOL, NEAR_TIE)
+    assert calls == [([0], (44, 64), 16), ([0], (13, 64), 16), ([0], (29, 64), 16), ([0], (18, 64), 16)]
+
+
+def test_how_much_context_behind_a_window_is_expanded():
+    import locus_b200.kernels as K
+
+    # (no window; what is measured beside the rule, 16 heads: 64 new tokens behind 2,000 and 4,000, 1,000 behind 4,000 and 15,000)
+    assert K.latent_expand_pays(64, 16000, 0)
+    for new, ctx, window, pays in ((64, 2000, 128, True), (64, 4000, 128, False), (1000, 4000, 128, True), (1000, 15000, 128, False), (1000, 15000, 512, True)):
+        assert K.latent_expand_pays(new, ctx, window) == pays

@@ -610,6 +610,56 @@ def test_the_tcgen05_attention_over_plain_rows(nh, nkv, how):
         _cmp(out[used], ref[used], 1.5e-2)
 
 
+@pytest.mark.parametrize("nh,how", [(4, "plain"), (1, "sink"), (3, "window"), (2, "slopes")])
+def test_the_tcgen05_attention_with_a_rotated_part(nh, how):
+    """Keys with 64 more dimensions that all heads share, whole and with the keys cut into ranges: portions around the edges of the
+    tiles of 64 queries and 128 keys, one to six tiles.  What no query may see is NaN: rows between the segments, the queries' columns
+    in the place of the rotated part."""
+    import locus_b200.kernels as K
+
+    g = torch.Generator().manual_seed(nh)
+    hd, segs, window = 128, [(0, 64), (0, 129), (60, 68), (3, 1), (500, 200), (127, 257)], 90 if how == "window" else 0
+    T, i32, at, row0 = sum(n for _, n in segs), lambda v: torch.tensor(v, dtype=torch.int32), 3, []
+    for c, n in segs:
+        row0.append(at)
+        at += c + n + 2
+    wide = torch.full((at, 320 + 64), float("nan"), dtype=torch.bfloat16)      # the rotated part behind a latent
+    kv = torch.full((at, 2 * nh * hd), float("nan"), dtype=torch.bfloat16)
+    for (c, n), r0 in zip(segs, row0):
+        wide[r0:r0 + c + n], kv[r0:r0 + c + n] = torch.randn(c + n, 384, generator=g), torch.randn(c + n, 2 * nh * hd, generator=g)
+    q, q_rot = torch.randn(T, nh, hd + 64, generator=g).to(torch.bfloat16), torch.randn(T, nh * 64, generator=g).to(torch.bfloat16)
+    q[:, :, hd:] = float("nan")
+    q = q.view(T, -1)
+    items = i32([[s, o] for s, (_, n) in enumerate(segs) for o in range(0, n, K.MMA_QUERY_TILE)])
+    slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / nh) for h in range(nh)]) if how == "slopes" else None
+    sink = torch.linspace(-1.0, 2.0, nh) if how == "sink" else False
+    meta = dict(seg_q0=i32([sum(n for _, n in segs[:s]) for s in range(len(segs))]), seg_qn=i32([n for _, n in segs]), seg_ctx=i32([c for c, _ in segs]),
+                kv_row0=i32(row0), items=items)
+    W, k_rot, opts = nh * hd, wide[:, 320:], dict(n_items=len(items), n_heads=nh, n_kv_heads=nh, head_dim=hd, scale=0.07, window=window)
+    want = torch.zeros(T, nh, hd, dtype=torch.float64)
+    for (c, n), r0, q0 in zip(segs, row0, meta["seg_q0"].tolist()):
+        pos, t = torch.arange(c, c + n)[:, None], torch.arange(c + n)[None]
+        for h in range(nh):
+            s = (q.double()[q0:q0 + n].view(n, nh, -1)[:, h, :hd] @ kv.double()[r0:r0 + c + n, h * hd:(h + 1) * hd].T
+                 + q_rot.double()[q0:q0 + n].view(n, nh, -1)[:, h] @ k_rot.double()[r0:r0 + c + n].T) * 0.07
+            if slopes is not None:
+                s = s - slopes[h].double() * (pos - t)
+            s = s.masked_fill((t > pos) | ((t <= pos - window) if window else False), -float("inf"))
+            extra = sink[h].double().expand(n, 1) if how == "sink" else s[:, :0]
+            want[q0:q0 + n, h] = torch.softmax(torch.cat([s, extra], 1), 1)[:, :c + n] @ kv.double()[r0:r0 + c + n, W + h * hd:W + (h + 1) * hd]
+    dev, kv, k_rot = {k: v.cuda() for k, v in meta.items()}, kv.cuda(), wide.cuda()[:, 320:]
+    for n_splits in (1, 2, 5):
+        extra = {}
+        if n_splits > 1:
+            extra = dict(n_splits=n_splits, part_o=torch.full((T * nh * n_splits * hd,), float("nan"), device=DEV),
+                         part_ml=torch.full((T * nh * n_splits * 2,), float("nan"), device=DEV))
+        out = torch.full((T, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+        K.attn_chunk_tc_rows(q.cuda(), kv[:, :W], kv[:, W:], out, q_rot=q_rot.cuda(), k_rot=k_rot, sink=sink.cuda() if torch.is_tensor(sink) else sink,
+                             slopes=None if slopes is None else slopes.cuda(), **extra, **dev, **opts)
+        assert K.attn_tc_error() == 0
+        _cmp(out, want.view(T, -1), 1.5e-2)   # (that of the rows form above)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_generation_through_the_engine_and_the_command_line(dtype, cases):
     """Greedy generation with portions and requests side by side: every token is the plain implementation's best one or within
