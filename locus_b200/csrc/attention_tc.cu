@@ -244,6 +244,42 @@ __device__ __forceinline__ void at_st32(uint32_t taddr, const uint32_t* v) {
 
 #define AT_S 3   // tiles of scores in tensor memory: tile j's in place j % 3
 
+// A block's barriers, in the order in which they lie in shared memory, and what is waited for before each of its steps: a barrier
+// and the parity of the turn of its place.  A wait by parity cannot tell a turn from the one two further on, so whoever waits for the
+// end of a turn must know that the one before it has ended, and must itself keep the one behind it from ending.
+// tests/test_attention_tc_waits.py walks through every order of the roles' steps with these waits.
+struct AtWait {
+    int bar;
+    uint32_t parity;
+};
+#define AT_BARS 20   // places for them
+template <bool ROT>
+struct AtBars {
+    static constexpr int D = ROT ? 2 : 3;   // tiles of K and of V in shared memory
+    static constexpr int Q_FULL = 0, K_FULL = 1, K_FREE = K_FULL + D, V_FULL = K_FREE + D, V_FREE = V_FULL + D, S_FULL = V_FREE + D,
+                         P_READY = S_FULL + AT_S;
+    // A place of the scores is free when the tile's P V is finished.  With as many places of V as of scores that is the barrier of V's
+    // place; with fewer, the next tile's but one would end the turn behind on that one, which nothing keeps it from before the
+    // scores are waited for.
+    static constexpr int S_FREE = ROT ? P_READY + AT_S : V_FREE, COUNT = P_READY + AT_S + (ROT ? AT_S : 0);
+    __host__ __device__ static constexpr AtWait full(int first, int places, int j) {
+        return {first + j % places, static_cast<uint32_t>(j / places) & 1};
+    }
+    __host__ __device__ static constexpr AtWait free(int first, int places, int j) {   // of the tile before in tile j's place
+        return {first + j % places, (static_cast<uint32_t>(j / places) & 1) ^ 1};
+    }
+    // the loader, before tile j's K and V; the score warp, for K and for the scores' place; the warp that sums V up, for V and the weights
+    __host__ __device__ static constexpr AtWait k_place(int j) { return free(K_FREE, D, j); }
+    __host__ __device__ static constexpr AtWait v_place(int j) { return free(V_FREE, D, j); }
+    __host__ __device__ static constexpr AtWait k_there(int j) { return full(K_FULL, D, j); }
+    __host__ __device__ static constexpr AtWait s_place(int j) { return free(S_FREE, AT_S, j); }
+    __host__ __device__ static constexpr AtWait v_there(int j) { return full(V_FULL, D, j); }
+    __host__ __device__ static constexpr AtWait p_there(int j) { return full(P_READY, AT_S, j); }
+    // a softmax warp, for tile j's scores and for the sum that the tile before is in
+    __host__ __device__ static constexpr AtWait s_there(int j) { return full(S_FULL, AT_S, j); }
+    __host__ __device__ static constexpr AtWait summed(int j) { return full(V_FREE, D, j); }
+};
+
 // BIAS: a distance bias; an instance of its own (the softmax warps are bound by instruction issue).
 // ROT: a rotated part (rows form).
 template <bool BIAS, bool ROT>
@@ -251,7 +287,8 @@ __global__ void __launch_bounds__(384, 1)
 attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_qr,
                      const __grid_constant__ CUtensorMap map_kr, TcAttnArgs a) {
-    constexpr int AT_D = ROT ? 2 : 3;                               // tiles of K and of V in shared memory
+    using B = AtBars<ROT>;
+    constexpr int AT_D = B::D;
     constexpr int AT_QK_BYTES = (ROT ? 3 : 2) * AT_HALF_BYTES;      // a tile of Q or K
     extern __shared__ __align__(1024) uint8_t at_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -290,8 +327,11 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         return;
     }
     const uint32_t sQ = base, sK = sQ + AT_QK_BYTES, sV = sK + AT_D * AT_QK_BYTES, bars = sV + AT_D * AT_TILE_BYTES;
-    const uint32_t q_full = bars, k_full = bars + 8, k_free = k_full + 8 * AT_D, v_full = k_free + 8 * AT_D, v_free = v_full + 8 * AT_D;
-    const uint32_t s_full = v_free + 8 * AT_D, p_ready = s_full + 8 * AT_S, slot = p_ready + 8 * AT_S + 8;
+    const uint32_t q_full = bars + 8 * B::Q_FULL, k_full = bars + 8 * B::K_FULL, k_free = bars + 8 * B::K_FREE, v_full = bars + 8 * B::V_FULL;
+    const uint32_t v_free = bars + 8 * B::V_FREE, s_full = bars + 8 * B::S_FULL, p_ready = bars + 8 * B::P_READY, s_free = bars + 8 * B::S_FREE;
+    const uint32_t slot = bars + 8 * AT_BARS;
+    static_assert(B::COUNT <= AT_BARS, "barriers");
+    auto wait = [&](AtWait w, int code) { return at_wait(bars + 8 * w.bar, w.parity, code); };
 
     if (threadIdx.x == 0) {
         at_bar_init(q_full, 1);
@@ -299,9 +339,10 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             at_bar_init(k_full + 8 * b, 1);
             at_bar_init(k_free + 8 * b, 1);
             at_bar_init(v_full + 8 * b, 1);
-            at_bar_init(v_free + 8 * b, 1);     // the tile's P V is finished: V's place and that of the scores are free
+            at_bar_init(v_free + 8 * b, 1);     // the tile's P V is finished
         }
         for (int b = 0; b < AT_S; ++b) {
+            if (ROT) at_bar_init(s_free + 8 * b, 1);
             at_bar_init(s_full + 8 * b, 1);
             at_bar_init(p_ready + 8 * b, 4);    // one arrival per softmax warp of the group
         }
@@ -357,9 +398,9 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                 return make_int2(__shfl_sync(0xffffffffu, now, 2 * (j & 15)), __shfl_sync(0xffffffffu, now, 2 * (j & 15) + 1));
             };
             auto load = [&](bool key, int2 rows, int j) {
-                const int turn = j / AT_D, b = j - turn * AT_D;
+                const int b = j % AT_D;
                 const uint32_t bar = (key ? k_full : v_full) + 8 * b;
-                at_wait((key ? k_free : v_free) + 8 * b, (turn & 1) ^ 1, 1);
+                wait(key ? B::k_place(j) : B::v_place(j), 1);
                 if (elected) {
                     const uint32_t dst = key ? sK + b * AT_QK_BYTES : sV + b * AT_TILE_BYTES;
                     const CUtensorMap* map = key ? &map_k : &map_v;
@@ -406,11 +447,10 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             const uint32_t idesc2 = idesc1 | (1u << 16);
             if (warp == 1) at_wait(q_full, 0, 5);
             for (int j = 0; j < n_tiles; ++j) {
-                const int turn_d = j / AT_D, d = j - turn_d * AT_D, turn_s = j / AT_S, b = j - turn_s * AT_S;   // places of K and V, of the scores
+                const int d = j % AT_D, b = j % AT_S;   // places of K and V, of the scores
                 if (warp == 1) {
-                    at_wait(k_full + 8 * d, turn_d & 1, 3);
-                    // the tile before in this place of the scores has been weighted and added up
-                    if (j >= AT_S) at_wait(v_free + 8 * ((j - AT_S) % AT_D), ((j - AT_S) / AT_D) & 1, 4);
+                    wait(B::k_there(j), 3);
+                    wait(B::s_place(j), 4);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elected) {
 #pragma unroll
@@ -422,8 +462,8 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                         at_commit(k_free + 8 * d);
                     }
                 } else {
-                    at_wait(v_full + 8 * d, turn_d & 1, 7);
-                    at_wait(p_ready + 8 * b, turn_s & 1, 6);
+                    wait(B::v_there(j), 7);
+                    wait(B::p_there(j), 6);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elected) {
 #pragma unroll
@@ -431,6 +471,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                             at_mma_ts(tO, tS + b * AT_MK + 8 * ks, at_desc_mn(sV + d * AT_TILE_BYTES + ks * (16 * 128), AT_HALF_BYTES), idesc2,
                                       (j > 0 || ks > 0) ? 1u : 0u);
                         at_commit(v_free + 8 * d);
+                        if (ROT) at_commit(s_free + 8 * b);
                     }
                 }
                 __syncwarp();
@@ -455,9 +496,9 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         float2* ml = reinterpret_cast<float2*>(at_raw + (slot + 16 - base));   // [2][128]: what the groups' threads tell each other
 
         for (int j = x; j < n_tiles; j += 2) {
-            const int tile0 = tile_at(j), turn = j / AT_S, b = j - turn * AT_S;
+            const int tile0 = tile_at(j), b = j % AT_S;
             const uint32_t tSx = tS + b * AT_MK + lane_bits;
-            if (!at_wait(s_full + 8 * b, turn & 1, 10)) ok = false;
+            if (!wait(B::s_there(j), 10)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t s[4][32];
 #pragma unroll
@@ -516,7 +557,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             // and rescales its sum, once the product of the tile before is in it.
             if (__any_sync(0xffffffffu, m_new - m_run > AT_LAG_LOG2)) {
                 if (j > 0) {
-                    if (!at_wait(v_free + 8 * ((j - 1) % AT_D), ((j - 1) / AT_D) & 1, 12)) ok = false;
+                    if (!wait(B::summed(j - 1), 12)) ok = false;
                     const float f = m_run == -INFINITY ? 1.f : at_exp2(m_run - m_new);
                     const unsigned long long f2 = at_pair(f, f);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -723,7 +764,7 @@ static int at_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const C
     if (n_items > 65535) return LOCUS_ERR_UNSUPPORTED;
     a.n_splits = n_splits; a.part_o = part_o; a.part_ml = part_ml;
     const bool rot = map_qr != nullptr;
-    const size_t smem = (rot ? 3 * 3 + 2 * 2 : 2 + 3 * 4) * AT_HALF_BYTES + 8 * (6 * AT_S + 2) + 16 + 2 * 128 * 8;
+    const size_t smem = (rot ? 3 * 3 + 2 * 2 : 2 + 3 * 4) * AT_HALF_BYTES + 8 * AT_BARS + 16 + 2 * 128 * 8;
     auto* kernel = a.slopes != nullptr ? (rot ? attn_chunk_tc_kernel<true, true> : attn_chunk_tc_kernel<true, false>)
                                        : (rot ? attn_chunk_tc_kernel<false, true> : attn_chunk_tc_kernel<false, false>);
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -809,6 +850,18 @@ extern "C" int locus_attn_chunk_tc_rows(const void* q, long long T, const void* 
     a.keep_first = window > 0 ? keep_first : 0; a.sink = sink ? 1 : 0; a.sink_val = sink ? sink_val : nullptr;
     a.slopes = slopes;
     return at_launch(map_q, map_k, map_v, a, n_items, n_splits, part_o, part_ml, stream, k_rot ? &map_qr : nullptr, k_rot ? &map_kr : nullptr);
+}
+
+// What a block waits for before a step of tile j (AtBars; `which` in the order of its functions): 2 * barrier + parity.  Host only.
+extern "C" int locus_attn_tc_wait(int rot, int which, int j) {
+    auto of = [&](auto bars) -> int {
+        using B = decltype(bars);
+        constexpr AtWait (*f[])(int) = {B::k_place, B::v_place, B::k_there, B::s_place, B::v_there, B::p_there, B::s_there, B::summed};
+        if (which < 0 || which >= static_cast<int>(sizeof(f) / sizeof(f[0])) || j < 0) return -1;
+        const AtWait w = f[which](j);
+        return 2 * w.bar + static_cast<int>(w.parity);
+    };
+    return rot ? of(AtBars<true>()) : of(AtBars<false>());
 }
 
 // Reads and clears the module's error word (0 = no bounded wait ran out).  Synchronises.
