@@ -278,6 +278,10 @@ struct AtBars {
     // a softmax warp, for tile j's scores and for the sum that the tile before is in
     __host__ __device__ static constexpr AtWait s_there(int j) { return full(S_FULL, AT_S, j); }
     __host__ __device__ static constexpr AtWait summed(int j) { return full(V_FREE, D, j); }
+    // ... and, before tile j's rows of V are touched, for the sum of the tile before in V's place (that of tile j - 3 is in when the scores
+    // of tile j are there: with three places nothing is left to wait for), then for V
+    static constexpr bool V_CLEAR_WAITS = ROT;
+    __host__ __device__ static constexpr AtWait v_clear(int j) { return full(S_FREE, AT_S, j - D); }
 };
 
 // BIAS: a distance bias; an instance of its own (the softmax warps are bound by instruction issue).
@@ -608,7 +612,8 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             // the last tile may hold rows of V behind the sequence's end (never written, any bit pattern): zero them
             if (tile0 + AT_MK - 1 > t_hi) {
                 const int d = j % AT_D;
-                if (!at_wait(v_full + 8 * d, (j / AT_D) & 1, 11)) ok = false;
+                if (B::V_CLEAR_WAITS && j >= AT_D && !wait(B::v_clear(j), 14)) ok = false;
+                if (!wait(B::v_there(j), 11)) ok = false;
                 if (tile0 + r > t_hi)
 #pragma unroll
                     for (int q8 = 0; q8 < 16; ++q8)
@@ -852,12 +857,14 @@ extern "C" int locus_attn_chunk_tc_rows(const void* q, long long T, const void* 
     return at_launch(map_q, map_k, map_v, a, n_items, n_splits, part_o, part_ml, stream, k_rot ? &map_qr : nullptr, k_rot ? &map_kr : nullptr);
 }
 
-// What a block waits for before a step of tile j (AtBars; `which` in the order of its functions): 2 * barrier + parity.  Host only.
+// What a block waits for before a step of tile j (AtBars; `which` in the order of its functions): 2 * barrier + parity, -1 for
+// nothing.  Host only.
 extern "C" int locus_attn_tc_wait(int rot, int which, int j) {
     auto of = [&](auto bars) -> int {
         using B = decltype(bars);
-        constexpr AtWait (*f[])(int) = {B::k_place, B::v_place, B::k_there, B::s_place, B::v_there, B::p_there, B::s_there, B::summed};
-        if (which < 0 || which >= static_cast<int>(sizeof(f) / sizeof(f[0])) || j < 0) return -1;
+        constexpr AtWait (*f[])(int) = {B::k_place, B::v_place, B::k_there, B::s_place, B::v_there, B::p_there, B::s_there, B::summed, B::v_clear};
+        if (which < 0 || which >= static_cast<int>(sizeof(f) / sizeof(f[0])) || j < 0 || (f[which] == B::v_clear && (!B::V_CLEAR_WAITS || j < B::D)))
+            return -1;
         const AtWait w = f[which](j);
         return 2 * w.bar + static_cast<int>(w.parity);
     };

@@ -11,7 +11,7 @@ import pytest
 
 from locus_b200.csrc import build
 
-WAITS = ("k_place", "v_place", "k_there", "s_place", "v_there", "p_there", "s_there", "summed")
+WAITS = ("k_place", "v_place", "k_there", "s_place", "v_there", "p_there", "s_there", "summed", "v_clear")
 SCORES = 3   # places of the scores
 
 
@@ -22,7 +22,7 @@ class Waits:
         fn.argtypes, fn.restype = [ctypes.c_int] * 3, ctypes.c_int
         self.places = 2 if rot else 3   # of K and of V
         for i, name in enumerate(WAITS):
-            setattr(self, name, lru_cache(None)(lambda j, i=i: (lambda v: (v >> 1, v & 1))(fn(int(rot), i, j))))
+            setattr(self, name, lru_cache(None)(lambda j, i=i: (lambda v: None if v < 0 else (v >> 1, v & 1))(fn(int(rot), i, j))))
 
 
 def walk(w, n):
@@ -35,7 +35,7 @@ def walk(w, n):
         if j + D < n:
             loads.append(("K", j + D))
     # state: loads issued, loads under way, score products issued / done, sums issued / done, per group of warps (tile, step);
-    # step 0: before the scores, 1: scores read, 2: rescales the sum, 3: reference handed on
+    # step 0: before the scores, 1: scores read, 2: rescales the sum, 3: reference handed on, 4 (last tile): V's dead rows are cleared
     start = (0, frozenset(), 0, 0, 0, 0, ((0, 0), (1, 0)))
     seen, todo = {start}, [start]
     while todo:
@@ -43,7 +43,7 @@ def walk(w, n):
         issued, flying, s_out, s_done, v_out, v_done, groups = state
         there = lambda kind, j: (kind, j) in loads[:issued] and (kind, j) not in flying
         ready = lambda j: groups[j & 1][0] > j             # the weights of tile j are written
-        handed = lambda j: ready(j) or groups[j & 1] == (j, 3)
+        handed = lambda j: ready(j) or groups[j & 1] in ((j, 3), (j, 4))
 
         def turns(bar):   # ends of a turn so far: every arrival ends one
             count = sum(1 for kind, j in loads[:issued] if there(kind, j) and (w.k_there if kind == "K" else w.v_there)(j)[0] == bar)
@@ -52,6 +52,8 @@ def walk(w, n):
             return count + sum(w.p_there(j)[0] == bar for j in range(n) if ready(j))
 
         def passes(wait, truth, what):
+            if wait is None:
+                return True
             bar, parity = wait
             if (turns(bar) & 1) == parity:
                 return False
@@ -92,7 +94,11 @@ def walk(w, n):
                     to(j, 2)
             elif step == 2 and passes(w.summed(j - 1), v_done >= j, f"the sum before tile {j} rescaled too early"):
                 to(j, 3)
-            elif step == 3:
+            elif step == 3 and j < last:
+                to(j + 2, 0)
+            elif step == 3 and passes(w.v_clear(j), j < D or v_done > j - D, f"V of tile {j} cleared while tile {j - D} uses its place"):
+                to(j, 4)
+            elif step == 4 and passes(w.v_there(j), there("V", j), f"V of tile {j} cleared before it is there"):
                 to(j + 2, 0)
         if not after:
             assert v_done == n and issued == len(loads) and not flying and min(g[0] for g in groups) > last, f"stuck: {state}"
@@ -115,3 +121,11 @@ def test_the_walk_finds_a_scores_place_that_shares_the_barrier_of_vs_place():
     w.s_place = lambda j: (w.v_place(0)[0] + (j - SCORES) % 2, ((j - SCORES) // 2) & 1) if j >= SCORES else (w.v_place(0)[0], 1)
     with pytest.raises(AssertionError, match="stuck"):
         walk(w, 6)
+
+
+def test_the_walk_finds_rows_of_v_cleared_too_early():
+    """Two places of V: before the sum of the tile before in V's place, a wait for V passes with that tile's turn still to come."""
+    w = Waits(True)
+    w.v_clear = lambda j: None
+    with pytest.raises(AssertionError, match="cleared before it is there"):
+        walk(w, 3)
