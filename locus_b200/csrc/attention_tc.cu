@@ -257,11 +257,11 @@ template <bool ROT>
 struct AtBars {
     static constexpr int D = ROT ? 2 : 3;   // tiles of K and of V in shared memory
     static constexpr int Q_FULL = 0, K_FULL = 1, K_FREE = K_FULL + D, V_FULL = K_FREE + D, V_FREE = V_FULL + D, S_FULL = V_FREE + D,
-                         P_READY = S_FULL + AT_S;
+                         P_READY = S_FULL + AT_S, DONE = P_READY + AT_S;
     // A place of the scores is free when the tile's P V is finished.  With as many places of V as of scores that is the barrier of V's
     // place; with fewer, the next tile's but one would end the turn behind on that one, which nothing keeps it from before the
     // scores are waited for.
-    static constexpr int S_FREE = ROT ? P_READY + AT_S : V_FREE, COUNT = P_READY + AT_S + (ROT ? AT_S : 0);
+    static constexpr int S_FREE = ROT ? DONE + 1 : V_FREE, COUNT = DONE + 1 + (ROT ? AT_S : 0);
     __host__ __device__ static constexpr AtWait full(int first, int places, int j) {
         return {first + j % places, static_cast<uint32_t>(j / places) & 1};
     }
@@ -282,6 +282,9 @@ struct AtBars {
     // of tile j are there: with three places nothing is left to wait for), then for V
     static constexpr bool V_CLEAR_WAITS = ROT;
     __host__ __device__ static constexpr AtWait v_clear(int j) { return full(S_FREE, AT_S, j - D); }
+    // ... and, at the end, for the last sum, by a barrier that is used once (V's place may be a turn further than a late warp's wait takes it
+    // to be)
+    __host__ __device__ static constexpr AtWait done(int) { return {DONE, 0}; }
 };
 
 // BIAS: a distance bias; an instance of its own (the softmax warps are bound by instruction issue).
@@ -332,13 +335,14 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     }
     const uint32_t sQ = base, sK = sQ + AT_QK_BYTES, sV = sK + AT_D * AT_QK_BYTES, bars = sV + AT_D * AT_TILE_BYTES;
     const uint32_t q_full = bars + 8 * B::Q_FULL, k_full = bars + 8 * B::K_FULL, k_free = bars + 8 * B::K_FREE, v_full = bars + 8 * B::V_FULL;
-    const uint32_t v_free = bars + 8 * B::V_FREE, s_full = bars + 8 * B::S_FULL, p_ready = bars + 8 * B::P_READY, s_free = bars + 8 * B::S_FREE;
+    const uint32_t v_free = bars + 8 * B::V_FREE, s_full = bars + 8 * B::S_FULL, p_ready = bars + 8 * B::P_READY, done = bars + 8 * B::DONE, s_free = bars + 8 * B::S_FREE;
     const uint32_t slot = bars + 8 * AT_BARS;
     static_assert(B::COUNT <= AT_BARS, "barriers");
     auto wait = [&](AtWait w, int code) { return at_wait(bars + 8 * w.bar, w.parity, code); };
 
     if (threadIdx.x == 0) {
         at_bar_init(q_full, 1);
+        at_bar_init(done, 1);
         for (int b = 0; b < AT_D; ++b) {
             at_bar_init(k_full + 8 * b, 1);
             at_bar_init(k_free + 8 * b, 1);
@@ -476,6 +480,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                                       (j > 0 || ks > 0) ? 1u : 0u);
                         at_commit(v_free + 8 * d);
                         if (ROT) at_commit(s_free + 8 * b);
+                        if (j == n_tiles - 1) at_commit(done);
                     }
                 }
                 __syncwarp();
@@ -630,11 +635,7 @@ attn_chunk_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         // The last tile's reference is the larger one and that of the sum; a group writes half of the columns of its rows.  (A group
         // without a tile counts for nothing.)
         ml[x * 128 + r] = make_float2(m_run, l_run);
-        // (The last sum, and before it the one before in its place, so that its barrier is not one turn further back than the wait takes
-        // it to be: that of the last tile but three is complete, its scores' place was used again.  The group of the last tile counts;
-        // the other meets it.)
-        for (int j = max(n_tiles - 1 - AT_D, (n_tiles - 1) % AT_D); j < n_tiles; j += AT_D)
-            if (!at_wait(v_free + 8 * (j % AT_D), (j / AT_D) & 1, 13)) ok = false;
+        if (!wait(B::done(n_tiles - 1), 13)) ok = false;
         asm volatile("bar.sync 9, 256;" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float2 e = ml[r], o2 = ml[128 + r];
@@ -862,7 +863,7 @@ extern "C" int locus_attn_chunk_tc_rows(const void* q, long long T, const void* 
 extern "C" int locus_attn_tc_wait(int rot, int which, int j) {
     auto of = [&](auto bars) -> int {
         using B = decltype(bars);
-        constexpr AtWait (*f[])(int) = {B::k_place, B::v_place, B::k_there, B::s_place, B::v_there, B::p_there, B::s_there, B::summed, B::v_clear};
+        constexpr AtWait (*f[])(int) = {B::k_place, B::v_place, B::k_there, B::s_place, B::v_there, B::p_there, B::s_there, B::summed, B::v_clear, B::done};
         if (which < 0 || which >= static_cast<int>(sizeof(f) / sizeof(f[0])) || j < 0 || (f[which] == B::v_clear && (!B::V_CLEAR_WAITS || j < B::D)))
             return -1;
         const AtWait w = f[which](j);

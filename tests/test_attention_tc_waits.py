@@ -11,7 +11,7 @@ import pytest
 
 from locus_b200.csrc import build
 
-WAITS = ("k_place", "v_place", "k_there", "s_place", "v_there", "p_there", "s_there", "summed", "v_clear")
+WAITS = ("k_place", "v_place", "k_there", "s_place", "v_there", "p_there", "s_there", "summed", "v_clear", "done")
 SCORES = 3   # places of the scores
 
 
@@ -21,6 +21,7 @@ class Waits:
         fn = build.load("attention_tc").locus_attn_tc_wait
         fn.argtypes, fn.restype = [ctypes.c_int] * 3, ctypes.c_int
         self.places = 2 if rot else 3   # of K and of V
+        self.end = lambda last: [self.done(last)]
         for i, name in enumerate(WAITS):
             setattr(self, name, lru_cache(None)(lambda j, i=i: (lambda v: None if v < 0 else (v >> 1, v & 1))(fn(int(rot), i, j))))
 
@@ -35,7 +36,7 @@ def walk(w, n):
         if j + D < n:
             loads.append(("K", j + D))
     # state: loads issued, loads under way, score products issued / done, sums issued / done, per group of warps (tile, step);
-    # step 0: before the scores, 1: scores read, 2: rescales the sum, 3: reference handed on, 4 (last tile): V's dead rows are cleared
+    # step 0: before the scores, 1: scores read, 2: rescales the sum, 3: reference handed on, 4 (last tile): V's dead rows are cleared, 5: the whole sum read
     start = (0, frozenset(), 0, 0, 0, 0, ((0, 0), (1, 0)))
     seen, todo = {start}, [start]
     while todo:
@@ -49,6 +50,7 @@ def walk(w, n):
             count = sum(1 for kind, j in loads[:issued] if there(kind, j) and (w.k_there if kind == "K" else w.v_there)(j)[0] == bar)
             count += sum((w.k_place(j)[0] == bar) + (w.s_there(j)[0] == bar) for j in range(s_done))
             count += sum(bar in {w.v_place(j)[0], w.s_place(j)[0]} for j in range(v_done))
+            count += v_done == n and w.done(last)[0] == bar
             return count + sum(w.p_there(j)[0] == bar for j in range(n) if ready(j))
 
         def passes(wait, truth, what):
@@ -85,6 +87,8 @@ def walk(w, n):
                 after.append((issued, flying, s_out, s_done, v_out, v_done, tuple((tile, nxt) if y == x else groups[y] for y in (0, 1))))
 
             if j > last:
+                if step == 0 and all(passes(wait, v_done == n, "the whole sum read too early") for wait in w.end(last)):
+                    to(j, 5)
                 continue
             if step == 0 and passes(w.s_there(j), s_done > j, f"scores {j} read too early"):
                 to(j, 1)
@@ -101,7 +105,7 @@ def walk(w, n):
             elif step == 4 and passes(w.v_there(j), there("V", j), f"V of tile {j} cleared before it is there"):
                 to(j + 2, 0)
         if not after:
-            assert v_done == n and issued == len(loads) and not flying and min(g[0] for g in groups) > last, f"stuck: {state}"
+            assert v_done == n and issued == len(loads) and not flying and groups[0][1] == groups[1][1] == 5, f"stuck: {state}"
         for s in after:
             if s not in seen:
                 seen.add(s)
@@ -129,3 +133,17 @@ def test_the_walk_finds_rows_of_v_cleared_too_early():
     w.v_clear = lambda j: None
     with pytest.raises(AssertionError, match="cleared before it is there"):
         walk(w, 3)
+
+
+@pytest.mark.parametrize("rot", [False, True])
+def test_the_walk_finds_a_last_sum_waited_for_at_vs_place(rot):
+    """The place of V turns twice for the last tile and the one before in its place: a warp that asks for the first turn behind the second
+    is stuck, one that asks for the second alone may pass before the first."""
+    w = Waits(rot)
+    D = w.places
+    w.end = lambda last: [w.summed(last)] if last < D else [w.summed(last - D)]
+    with pytest.raises(AssertionError, match="stuck|too early"):
+        walk(w, D + 1)
+    w.end = lambda last: [w.summed(last)]
+    with pytest.raises(AssertionError, match="too early"):
+        walk(w, 2 * D + 1)
