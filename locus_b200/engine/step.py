@@ -240,6 +240,11 @@ class ModelRunner:
             if code:
                 raise RuntimeError(f"tensor-core kernel fault: a pipeline wait ran out (code {code}: "
                                    "1 = loader, 2 = MMA issuer, 3 = epilogue); results since the last check are invalid")
+        if self.device.type == "cuda" and "gemm_simt" in K._LIBS:
+            code = K.f32_tc_error()
+            if code:
+                raise RuntimeError(f"float32 tensor-core kernel fault: a pipeline wait ran out (code {code}: 1 = loader, 2 to 4 = MMA issuer, "
+                                   "5 = sums, 6 and 7 = weights); results since the last check are invalid")
         if self.device.type == "cuda" and "attention" in K._LIBS:
             code = K.attn_error()
             if code:

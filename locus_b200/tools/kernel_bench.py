@@ -81,7 +81,7 @@ def bench_linear(args) -> None:
     flops = 2.0 * M * N * Kd * (2 if args.dual else 1)
     print(f"linear M={M} N={N} K={Kd} dual={int(args.dual)}{' rectified' if extra else ''} accumulate={int(args.accumulate)} {args.dtype}: "
           f"{us:.1f} us/call  {flops / us / 1e6:.1f} TFLOP/s  weights {wbytes / us / 1e3:.1f} GB/s  "
-          f"(tensor-core error word {K.tc_error() if dt == torch.bfloat16 else 0})")
+          f"(tensor-core error word {K.tc_error() if dt == torch.bfloat16 else K.f32_tc_error()})")
 
 
 def bench_experts(args) -> None:
@@ -133,7 +133,7 @@ def bench_experts(args) -> None:
     wbytes = used * I * H * el * share
     print(f"experts T={T} E={E} top_k={k} hidden={H} inner={I} part={args.part} tile={tile} {args.dtype}: "
           f"{us:.1f} us/call  {flops / us / 1e6:.1f} TFLOP/s  weights of the {used} experts used {wbytes / us / 1e3:.1f} GB/s  "
-          f"(tensor-core error word {K.tc_error() if dt == torch.bfloat16 else 0})")
+          f"(tensor-core error word {K.tc_error() if dt == torch.bfloat16 else K.f32_tc_error()})")
 
 
 def _paged(args, B: int, ctx: int, new: int):

@@ -261,3 +261,18 @@ def test_step_refuses_numbers_that_fit_no_field(tmp_path):
     lg = runner.step([StepEntry(s, [1, 2, 3], [2])])   # and a good step still runs
     ref = plain.forward(cfg, W, [1, 2, 3], torch.float64)
     assert float((lg[0].double() - ref[2]).abs().max()) <= 2e-5 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("module,word", [("gemm_tc", "gemm_tc"), ("gemm_simt", "gemm_f32_tc"), ("attention", "attn"), ("attention_gqa", "attn_gqa"),
+                                         ("attention_tc", "attn_tc")])
+def test_every_error_word_of_a_loaded_kernel_module_is_raised(module, word, monkeypatch):
+    import types
+
+    from locus_b200 import kernels as K
+
+    code, runner = [0], types.SimpleNamespace(device=torch.device("cuda"))
+    monkeypatch.setattr(K, "_LIBS", {module: types.SimpleNamespace(**{f"locus_{word}_error": lambda: code[0]})})
+    ModelRunner.check_device_errors(runner)
+    code[0] = 4
+    with pytest.raises(RuntimeError, match="code 4"):
+        ModelRunner.check_device_errors(runner)
