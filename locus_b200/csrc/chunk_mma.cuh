@@ -48,8 +48,11 @@ __device__ __forceinline__ void ch_ldsm_t(uint32_t (&r)[4], const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(ch_smem(p)) : "memory");
 }
-// Bulk copies into shared memory, counted by an mbarrier, and a bounded wait for them (after the limit the caller goes on with what
-// is there).
+// Bulk copies into shared memory, counted by an mbarrier, and a bounded wait for them (about a second of clock cycles): when it runs out
+// the module's error word is set, all later waits that have to spin return soon, and the caller goes on with what is there, so that the
+// kernel ends.
+#define CH_WAIT_LIMIT 2000000000LL
+__device__ int g_chunk_error = 0;
 __device__ __forceinline__ void ch_bar_init(uint32_t bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar)); }
 __device__ __forceinline__ void ch_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -58,8 +61,19 @@ __device__ __forceinline__ void ch_bulk(uint32_t dst, const void* src, uint32_t 
                  : "memory");
 }
 __device__ __forceinline__ void ch_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok = 0;
-    for (int i = 0; i < 20000000 && !ok; ++i)
+    auto there = [&]() -> bool {
+        uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        return ok != 0;
+    };
+    if (there()) return;
+    const long long t0 = clock64();
+    for (int i = 1; !there(); ++i) {
+        if ((i & 63) == 0 && *reinterpret_cast<volatile int*>(&g_chunk_error) != 0) return;   // (a trip to L2)
+        if (clock64() - t0 > CH_WAIT_LIMIT) {
+            atomicCAS(&g_chunk_error, 0, 1);
+            return;
+        }
+    }
 }

@@ -632,6 +632,14 @@ static int gla_chunks(const GlaArgs& a, int n_seg, int n_rows, void* scratch, lo
     return locus_launch_status();
 }
 
+// Reads and clears the module's error word (0 = no bounded wait ran out).  Synchronises.
+extern "C" int locus_gla_error() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_chunk_error, sizeof(int)) != cudaSuccess) return -1;
+    if (v != 0) cudaMemcpyToSymbol(g_chunk_error, &zero, sizeof(int));
+    return v;
+}
+
 // z [T, ld] float32, columns [off, off + n): z <- 1 - exp(-softplus(-z) / tau).
 __global__ void __launch_bounds__(256) gla_decay_kernel(float* __restrict__ z, int ld, int off, int n, float inv_tau,
                                                         long long total) {

@@ -255,6 +255,11 @@ class ModelRunner:
             if code:
                 raise RuntimeError(f"grouped-query decode attention fault (code {code}): a wait for a bulk copy ran out; "
                                    "results since the last check are invalid")
+        if self.device.type == "cuda" and "gla" in K._LIBS:
+            code = K.gla_error()
+            if code:
+                raise RuntimeError(f"gated linear attention fault (code {code}): a wait for a bulk copy ran out; "
+                                   "results since the last check are invalid")
         if self.device.type == "cuda" and "attention_tc" in K._LIBS:
             code = K.attn_tc_error()
             if code:

@@ -2319,6 +2319,12 @@ CHUNK_MIN_TOKENS = 64    # ... of steps of at least so many tokens a segment (64
 CHUNK_BYTES = 2 * (6 * 16 * (CHUNK_DIM + 8) + 3 * 16 * 24) + 4 * CHUNK_DIM   # scratch by chunk and head
 
 
+def gla_error() -> int:
+    """Error word of gated linear attention in chunks (0 = fine; 1: a wait for a chunk's operands ran out); reading it synchronises
+    the device."""
+    return int(_lib("gla").locus_gla_error())
+
+
 def _chunk_scratch(out: torch.Tensor, n_heads: int, n_seg: int):
     """(scratch for the chunks of all rows of ``out``, or of as many as the split products' buffer holds; how many rows)."""
     per, most = n_heads * CHUNK_BYTES, -(-out.shape[0] // 16)

@@ -264,7 +264,7 @@ def test_step_refuses_numbers_that_fit_no_field(tmp_path):
 
 
 @pytest.mark.parametrize("module,word", [("gemm_tc", "gemm_tc"), ("gemm_simt", "gemm_f32_tc"), ("attention", "attn"), ("attention_gqa", "attn_gqa"),
-                                         ("attention_tc", "attn_tc")])
+                                         ("attention_tc", "attn_tc"), ("gla", "gla")])
 def test_every_error_word_of_a_loaded_kernel_module_is_raised(module, word, monkeypatch):
     import types
 

@@ -272,6 +272,7 @@ def test_gla_scan_in_chunks(H, dv, small, precise, monkeypatch):
         _cmp(got.cpu()[clean], ref[clean], 2e-5)
         assert not torch.isfinite(got[141:195, 5]).any()
         assert not torch.isfinite(gst[3].view(H, d, dv)[0, 3, 5])
+    assert K.gla_error() == 0
 
 
 @pytest.mark.parametrize("H,d,dv", [(2, 24, 16), (1, 7, 5), (3, 72, 40), (2, 128, 64), (1, 200, 12)])
