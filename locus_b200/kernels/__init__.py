@@ -518,15 +518,16 @@ def f32_splits(m: int, n: int, k: int) -> int:
 F32_TC_WORK = 64_000_000   # multiply-adds from which a float32 product goes to the tensor cores (see f32_tc_takes)
 
 
-def f32_tc_takes(x: torch.Tensor, w: torch.Tensor, m: int, dual: bool = False) -> bool:
+def f32_tc_takes(x: torch.Tensor, w: torch.Tensor, m: int, w2: Optional[torch.Tensor] = None) -> bool:
     """Whether :func:`linear` runs a float32 product that is none of the row-streaming kernel's on the tensor cores, every value
-    cut into three bfloat16 (csrc/gemm_f32_tc.cuh): rows that 16-byte loads and TMA can address, enough work for its two
+    cut into three bfloat16 (csrc/gemm_f32_tc.cuh): rows (of ``w2`` too) that 16-byte loads and TMA can address, enough work for its two
     launches and its pipeline's start (about 9 us), and scratch for the parts of x.  Measured, on CUDA cores / there: 33 rows of
     2,048 x 512 9.6 / 10.1 us, 64 11.6 / 11.3, of 4,096 x 256 11.1 / 11.2, 128 14.9 / 11.4, 256 rows of 512 x 512 11.4 / 11.3; 33 rows
     of 2,048 x 2,048 17.9 / 13.8, 512 110 / 33; 512 rows of 6,144 x 2,048 301 / 82, 2,048 rows 1,156 / 246."""
     K, n = x.shape[-1], w.shape[-2]
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
-            and (x.data_ptr() | w.data_ptr()) % 16 == 0 and m * n * K * (2 if dual else 1) >= F32_TC_WORK
+            and (x.data_ptr() | w.data_ptr() | (w2.data_ptr() if w2 is not None else 0)) % 16 == 0
+            and m * n * K * (2 if w2 is not None else 1) >= F32_TC_WORK and w.numel() // K < 1 << 31
             and 4 * f32_tc_floats(m, K) <= SPLIT_SCRATCH_BYTES)
 
 
@@ -750,7 +751,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         te = t0 = tr = nt = None
         max_tiles = 0
         stride = 0
-    if f32_tc_takes(x, w, M, w2 is not None):
+    if f32_tc_takes(x, w, M, w2):
         # float32 x float32 in three bfloat16 parts each: tcgen05 kernel (csrc/gemm_f32_tc.cuh)
         tn, splits = (64, 1) if layout is not None else f32_tc_plan(M, N, K, w2 is not None)
         parts = splits * M * N if splits > 1 else 0        # floats; the parts of x lie behind the partial sums

@@ -284,8 +284,8 @@ class SparseMoe(FeedForward):
         on_input = (wts, lay.sorted_pair) if self.weight_on_input else None
         all_bf16 = (K.tensor_cores_take(h, self.params["up_exps"]) and widths_ok
                     and self.params["down_exps"].dtype == torch.bfloat16)
-        on_tc = (K.f32_tc_takes(h, self.params["up_exps"], n_pairs, self.activation in GATED) and widths_ok
-                 and self.params["down_exps"].dtype == torch.float32)
+        on_tc = (K.f32_tc_takes(h, self.params["up_exps"], n_pairs, self.params["gate_exps"] if self.activation in GATED else None)
+                 and widths_ok and self.params["down_exps"].dtype == torch.float32)
         if not all_bf16 and widths_ok and n_pairs <= (FEW_PAIRS_F32_TC if on_tc else K.FEW_ROWS) * self.E:
             # No bfloat16 form (float32) and a handful of rows per expert: tiles of 8 rows on the row-streaming kernel read an
             # expert's weights once per tile, where the other products compute a 64-row tile for every expert that has a row: on the

@@ -724,6 +724,16 @@ def test_linear_float32_tensor_cores_keep_what_is_not_finite_and_the_range(tn, m
     assert K.f32_tc_error() == 0
 
 
+@pytest.mark.parametrize("which", ["x", "w", "w2"])
+def test_linear_float32_of_unaligned_rows_where_the_work_is_enough_for_the_tensor_cores(which):
+    M, N, K_ = 300, 512, 512
+    on_gpu = lambda t, off: torch.empty(t.numel() + 4, device=DEV)[off:off + t.numel()].view(t.shape).copy_(t)
+    x, w, w2 = rnd(M, K_, seed=1), rnd(N, K_, seed=2, scale=K_ ** -0.5), rnd(N, K_, seed=3, scale=K_ ** -0.5)
+    out = torch.empty(M, N, device=DEV)
+    K.linear(on_gpu(x, which == "x"), on_gpu(w, which == "w"), out, w2=on_gpu(w2, which == "w2"))
+    close(out, torch.nn.functional.silu(x.double() @ w.double().T) * (x.double() @ w2.double().T), torch.float32, which)
+
+
 @pytest.mark.parametrize("splits", [2, 3, 8])
 def test_linear_float32_cut_along_k(splits, monkeypatch):
     """Parts of unequal length (the last one shorter, or without a column), and the epilogue behind their sum."""

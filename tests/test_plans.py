@@ -88,3 +88,25 @@ def test_which_portions_the_tensor_core_attention_takes():
     assert takes(n=2, ctx=4096) and not takes(n=2, ctx=4095)              # fewer: behind 4,096 and more
     assert not takes(n=2048, hd=64) and not takes(n=2048, page=16) and takes(n=2048, page=128)
     assert not K.attn_chunk_tc_takes(torch.empty(1, dtype=torch.float32), 128, 64, 2048, 0)
+
+
+def _floats(*shape, offset=0):
+    """Rows of float32 whose first lies ``offset`` elements behind a 64-byte boundary."""
+    import math
+
+    import torch
+
+    n = math.prod(shape)
+    t = torch.empty(n + 32)
+    at = (-t.data_ptr() // 4) % 16 + offset
+    return t[at:at + n].view(*shape)
+
+
+def test_float32_products_go_to_the_tensor_cores_only_with_rows_that_tma_can_address():
+    """A second weight at an address that TMA cannot take stays where it always ran, as one of x or of the first weight does."""
+    x, w = _floats(512, 512), _floats(512, 512)
+    assert K.f32_tc_takes(x, w, 512) and K.f32_tc_takes(x, w, 512, _floats(512, 512))
+    for offset in (1, 2, 3):
+        assert not K.f32_tc_takes(x, w, 512, _floats(512, 512, offset=offset))
+        assert not K.f32_tc_takes(x, _floats(512, 512, offset=offset), 512) and not K.f32_tc_takes(_floats(512, 512, offset=offset), w, 512)
+    assert K.f32_tc_takes(x, w, 512, _floats(512, 512, offset=4))
