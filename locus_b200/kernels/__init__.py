@@ -11,6 +11,7 @@ plain torch functions of the same signature to exercise the engine's host logic.
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -433,7 +434,22 @@ def _sm_count() -> int:
 
 SPLIT_SCRATCH_BYTES = 64 << 20   # float32 partial sums of a product split along K
 _PLANS: dict = {}
-_SPLIT_SCRATCH: dict = {}
+
+
+class _PerThread(threading.local):
+    """Buffers by key, every thread's its own (given back when the thread ends)."""
+
+    def __init__(self) -> None:
+        self._buffers: dict = {}
+
+    def get(self, key):
+        return self._buffers.get(key)
+
+    def __setitem__(self, key, buffer) -> None:
+        self._buffers[key] = buffer
+
+
+_SPLIT_SCRATCH = _PerThread()
 
 
 def token_tile(m: int, dual: bool = False, n_weight_tiles: int = 0, k: int = 0) -> int:
@@ -567,8 +583,8 @@ def _split_scratch(device, floats: int) -> torch.Tensor:
     """A buffer for at least ``floats`` partial sums that no other chain of launches writes meanwhile.  The steps of a runner use
     the runner's own, one for its main chain and one for its side stream's (:class:`stream_scope`), so that the graphs of two
     runners may be replayed at the same time.  A product that is captured outside a runner gets memory of its graph's
-    own pool, which the same stream of the same capture finds again when the caller has let go of it.  All other calls share
-    a buffer per stream."""
+    own pool, which the same stream of the same capture finds again when the caller has let go of it.  All other calls of
+    a thread share a buffer per stream (two threads may launch on one stream, and the launches of a product are several)."""
     if _scratch_override is not None:
         t = _scratch_override()
     elif torch.cuda.is_current_stream_capturing():

@@ -110,3 +110,29 @@ def test_float32_products_go_to_the_tensor_cores_only_with_rows_that_tma_can_add
         assert not K.f32_tc_takes(x, w, 512, _floats(512, 512, offset=offset))
         assert not K.f32_tc_takes(x, _floats(512, 512, offset=offset), 512) and not K.f32_tc_takes(_floats(512, 512, offset=offset), w, 512)
     assert K.f32_tc_takes(x, w, 512, _floats(512, 512, offset=4))
+
+
+def test_threads_that_share_a_stream_have_scratch_of_their_own(monkeypatch):
+    """A product's launches (its parts cut up, the product, the sum of its parts) meet in the scratch; those of another thread on the
+    same stream may come between them."""
+    import threading
+    import types
+    import weakref
+
+    import torch
+
+    monkeypatch.setattr(K, "_stream", lambda: types.SimpleNamespace(value=7))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(K, "SPLIT_SCRATCH_BYTES", 1024)
+    mine, seen = K._split_scratch("cpu", 100), []
+    assert K._split_scratch("cpu", 256) is mine
+
+    def other():
+        t = K._split_scratch("cpu", 100)
+        seen.extend([t is mine, t.data_ptr() == mine.data_ptr(), K._split_scratch("cpu", 100) is t, weakref.ref(t)])
+
+    thread = threading.Thread(target=other)
+    thread.start()
+    thread.join()
+    assert seen[:3] == [False, False, True] and seen[3]() is None   # ... and it is given back
+    assert K._split_scratch("cpu", 100) is mine
