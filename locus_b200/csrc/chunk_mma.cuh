@@ -1,25 +1,15 @@
 // Portions of a recurrence in chunks of 16 tokens (gla.cu): small float32 matrix products on the tensor cores.
 //
-// Every float32 operand is cut into three bfloat16 whose sum it is exactly (its upper 16 bits, the rest rounded to 8 bits, what is
-// left), and a product of two is the sum of six products of parts, the small ones first: exact but for the rounding of
-// float32 sums.  mma.sync m16n8k16 (a warp's 16 x 16 times 16 x 8): lane 4 g + t holds of A the rows g and g + 8 at columns 2 t,
+// Every float32 operand is cut into three bfloat16 whose sum it is (bf16_parts.cuh), and a product of two is the sum of six products
+// of parts, the small ones first: it lacks at most 2^-24 of itself, and float32 sums round as ever.  mma.sync m16n8k16 (a warp's 16 x 16 times 16 x 8): lane 4 g + t holds of A the rows g and g + 8 at columns 2 t,
 // 2 t + 1, 2 t + 8, 2 t + 9, of B the column g at the same rows, of the sums rows g and g + 8 at columns 2 t, 2 t + 1, so that the
 // sums of two neighbouring tiles of eight columns are the A operand of a product over those sixteen columns.
 #pragma once
+#include "bf16_parts.cuh"
 #include "walk.cuh"
 
 #define CH 16   // tokens of a chunk
 
-// Two float32 as three pairs of bfloat16 (a in the lower half).
-__device__ __forceinline__ void ch_cut(float a, float b, uint32_t (&p)[3]) {
-    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-    p[0] = __byte_perm(ua, ub, 0x7632);
-    const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
-    const uint32_t ta = __float_as_uint(ra) + 0x8000u, tb = __float_as_uint(rb) + 0x8000u;
-    p[1] = __byte_perm(ta, tb, 0x7632);
-    const float sa = ra - __uint_as_float(ta & 0xffff0000u), sb = rb - __uint_as_float(tb & 0xffff0000u);
-    p[2] = __byte_perm(__float_as_uint(sa), __float_as_uint(sb), 0x7632);
-}
 __device__ __forceinline__ void ch_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])

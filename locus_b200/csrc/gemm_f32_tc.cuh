@@ -1,10 +1,6 @@
 // float32 products on the Blackwell tensor cores (included by gemm_simt.cu, whose arguments and epilogue it shares): every
-// float32 is cut into three bfloat16 whose sum it is exactly,
-//
-//   a = a0 + a1 + a2,   a0 = a's upper 16 bits (8 bits of its fraction), a1 = the rest rounded to 8 bits, a2 = what is left,
-//
-// and the product of two float32 is the sum of the six products a0 b0, a0 b1, a1 b0, a1 b1, a0 b2, a2 b0; the three left out
-// are below 2^-25 of it and of either sign.  Products of bfloat16 are exact in the tensor cores; what rounds is their sum: a
+// float32 is cut into three bfloat16 whose sum it is (bf16_parts.cuh, with the bound of what the six products of parts leave out of a
+// product and the range that this holds for).  Products of bfloat16 are exact in the tensor cores; what rounds is their sum: a
 // float32 accumulator is cut off, not rounded, at every 16 columns of k.  So the large products a0 b0 have an accumulator of their own,
 // which is taken out after 64 columns and added up in registers, rounded; the five small ones share another one for
 // the whole sum, where a cut is 2^-8 of what it would be beside the large ones.
@@ -18,8 +14,9 @@
 // out, add them up and do the epilogue while the next tile's MMAs run.  A SwiGLU tile holds 64 weight rows of each
 // matrix.  A block walks over tiles, all roles run ahead across them.
 //
-// An operand that is not finite makes NaN of every sum it enters (its parts are infinity and infinity - infinity), so a NaN is
-// formed again, by plain multiply-adds, from its row and weight row: what comes out is what such operands give.
+// An operand that is not finite makes NaN of every sum it enters, and the rounded first parts of two values may be more than float32
+// holds where their product is not (within 2^-7 of its largest value): a sum that is not finite is formed again, by plain
+// multiply-adds, from its row and weight row, and comes out as such operands give it.
 //
 // What bounds it: the MMAs, six for one (a stage of 128 rows 768 cycles), where there are many rows, and the weights' way from
 // memory where there are few.  Measured, against the CUDA-core kernel: 2,048 x 6,144 x 2,048 1,156 -> 246 us (209 TFLOP/s; cuBLAS's
@@ -34,6 +31,8 @@
 // the kernel ends.
 #pragma once
 #include <cuda.h>
+
+#include "bf16_parts.cuh"
 
 #define FT_W 128              // weight rows of a tile
 #define FT_K 32               // columns of k of a stage: 128 bytes of float32, 64 of bfloat16
@@ -121,17 +120,8 @@ __device__ __forceinline__ void ft_st8(uint32_t taddr, const uint32_t* v) {
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-// Two float32 as the three pairs of bfloat16 (a in the lower half).
-__device__ __forceinline__ void ft_cut(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-    p0 = __byte_perm(ua, ub, 0x7632);
-    const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);   // exact: 16 bits
-    const uint32_t ta = __float_as_uint(ra) + 0x8000u, tb = __float_as_uint(rb) + 0x8000u;
-    p1 = __byte_perm(ta, tb, 0x7632);
-    const float sa = ra - __uint_as_float(ta & 0xffff0000u), sb = rb - __uint_as_float(tb & 0xffff0000u);   // exact: 8 bits
-    p2 = __byte_perm(__float_as_uint(sa), __float_as_uint(sb), 0x7632);
-}
-// A sum that came out as NaN, formed by multiply-adds.
+__device__ __forceinline__ bool ft_odd(float v) { return !(fabsf(v) < INFINITY); }
+// A sum that came out as not finite, formed by multiply-adds.
 __device__ __forceinline__ float ft_plain(const float* x, const float* w, int n) {
     float even = 0.f, odd = 0.f;
 #pragma unroll 1
@@ -156,10 +146,10 @@ __global__ void __launch_bounds__(256) f32_cut_kernel(const float* __restrict__ 
     const float4* p = reinterpret_cast<const float4*>(x + (x_rows ? x_rows[row] / x_row_div : row) * ldx + k);
     const float4 u = k < K ? p[0] : z, v = k + 4 < K ? p[1] : z;
     uint4 q[3];
-    ft_cut(u.x, u.y, q[0].x, q[1].x, q[2].x);
-    ft_cut(u.z, u.w, q[0].y, q[1].y, q[2].y);
-    ft_cut(v.x, v.y, q[0].z, q[1].z, q[2].z);
-    ft_cut(v.z, v.w, q[0].w, q[1].w, q[2].w);
+    bf16_parts(u.x, u.y, q[0].x, q[1].x, q[2].x);
+    bf16_parts(u.z, u.w, q[0].y, q[1].y, q[2].y);
+    bf16_parts(v.x, v.y, q[0].z, q[1].z, q[2].z);
+    bf16_parts(v.z, v.w, q[0].w, q[1].w, q[2].w);
 #pragma unroll
     for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(parts + (static_cast<long long>(j) * rows + row) * Kp + k) = q[j];
 }
@@ -343,8 +333,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float4 wv = *reinterpret_cast<const float4*>(wr + (((4 * half + i) ^ (wrow & 7)) << 4));
-                        ft_cut(wv.x, wv.y, p[half][0][2 * i], p[half][1][2 * i], p[half][2][2 * i]);
-                        ft_cut(wv.z, wv.w, p[half][0][2 * i + 1], p[half][1][2 * i + 1], p[half][2][2 * i + 1]);
+                        bf16_parts(wv.x, wv.y, p[half][0][2 * i], p[half][1][2 * i], p[half][2][2 * i]);
+                        bf16_parts(wv.z, wv.w, p[half][0][2 * i + 1], p[half][1][2 * i + 1], p[half][2][2 * i + 1]);
                     }
                 if (i0 >= SA) ft_wait(free_ + 8 * ((i0 - SA) % SR), ((i0 - SA) / SR) & 1, 6);   // the place of the stage SA before
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -420,7 +410,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         for (int i = 0; i < 8; ++i) {
                             v[i] = sums[(m0 + i) * FT_W + c];
                             if (SWIGLU) v2[i] = sums[(m0 + i) * FT_W + COLS + c];
-                            odd |= v[i] != v[i] || (SWIGLU && v2[i] != v2[i]);
+                            odd |= ft_odd(v[i]) || (SWIGLU && ft_odd(v2[i]));
                         }
                         if (odd)
 #pragma unroll 1
@@ -432,7 +422,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                                 const float s2 = SWIGLU ? ft_plain(xp, static_cast<const float*>(a.w2) + wo, kn) : 0.f;
 #pragma unroll
                                 for (int i = 0; i < 8; ++i)   // (the array stays in registers)
-                                    if (i == q && (v[i] != v[i] || (SWIGLU && v2[i] != v2[i]))) {
+                                    if (i == q && (ft_odd(v[i]) || (SWIGLU && ft_odd(v2[i])))) {
                                         v[i] = s1;
                                         if (SWIGLU) v2[i] = s2;
                                     }

@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(256) gla_chunk_prep(const GlaArgs a, const Gla
     auto leave = [&](int i, int which, float x, float y) {   // (rows that are not there: zeros)
         if (!on) return;
         uint32_t p[3];
-        ch_cut(x, y, p);
+        bf16_parts(x, y, p[0], p[1], p[2]);
 #pragma unroll
         for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(parts + (3 * which + j) * GC_PART + i * GC_LD + d0) = p[j];
     };
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256) gla_chunk_prep(const GlaArgs a, const Gla
             return jj <= i ? sums[hl][0][x] + sums[hl][1][x] : 0.f;
         };
         uint32_t p[3];
-        ch_cut(at(j), at(j + 1), p);
+        bf16_parts(at(j), at(j + 1), p[0], p[1], p[2]);
 #pragma unroll
         for (int m = 0; m < 3; ++m) *reinterpret_cast<uint32_t*>(amat + (m * CH + i) * GC_ALD + j) = p[m];
     }
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_kernel(const GlaArgs a, cons
     auto lay = [&](int c) -> bool {   // v into its places; false where it is not finite
         const float v = vf[c % 3][vtok][vc];
         uint32_t p[3];
-        ch_cut(v, 0.f, p);
+        bf16_parts(v, 0.f, p[0], p[1], p[2]);
 #pragma unroll
         for (int j = 0; j < 3; ++j) *reinterpret_cast<unsigned short*>(&vt[c & 1][j][vc][vtok]) = static_cast<unsigned short>(p[j]);
         return fabsf(v) < INFINITY;
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(256, 2) gla_chunk_kernel(const GlaArgs a, cons
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             uint32_t p[3];
-            ch_cut(sv[e >> 1][2 * (e & 1)], sv[e >> 1][2 * (e & 1) + 1], p);
+            bf16_parts(sv[e >> 1][2 * (e & 1)], sv[e >> 1][2 * (e & 1) + 1], p[0], p[1], p[2]);
 #pragma unroll
             for (int j = 0; j < 3; ++j) sp[j][e] = p[j];
         }

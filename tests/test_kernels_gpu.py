@@ -724,6 +724,32 @@ def test_linear_float32_tensor_cores_keep_what_is_not_finite_and_the_range(tn, m
     assert K.f32_tc_error() == 0
 
 
+def test_linear_float32_tensor_cores_leave_out_no_more_than_they_say(monkeypatch):
+    """Four equal products of operands whose left-out parts are the largest: the sum of the parts' large products is exact, so an output
+    is off by what the six products leave out (2^-24 of each) and by the rounding of its last sum (2^-24), and by nothing else that
+    counts.  With the first part cut off instead of rounded the second kind of operand is off by 2^-22."""
+    monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    monkeypatch.setattr(K, "few_rows_take", lambda *a, **k: False)
+    low = [1 + 2 ** -8 - 2 ** -16 + 2 ** -17 - 2 ** -23, 1 + 2 ** -7 - 2 ** -15 + 2 ** -16 - 2 ** -23, 1 + 2 ** -8 + 2 ** -16, 1 + 2 ** -23, 2 - 2 ** -23]
+    values = torch.tensor([s * v * 2.0 ** e for v in low for s in (1, -1) for e in (0, -9, 40)], dtype=torch.float32)
+    x = w = values[:, None].expand(-1, 4).contiguous()
+    out = torch.empty(len(values), len(values), device=DEV)
+    K.linear(x.to(DEV), w.to(DEV), out)
+    ref = x.double() @ w.double().T
+    assert bool(((out.cpu().double() - ref).abs() <= (2.0 ** -24 + 2.0 ** -24 + 2.0 ** -29) * ref.abs()).all())
+    # a product just below the largest value, whose first parts' product is above it
+    x, w = torch.full((1, 4), 0.0), torch.full((1, 4), 0.0)
+    x[0, 1] = 2.0 ** 127 * (1 + 2 ** -8 + 2 ** -16)    # (first parts 2^127 (1 + 2^-7) and 1.9921875)
+    x[0, 2], w[0, 2] = 2.0 ** 110, 1.0
+    for v in (1.9885, 1.99, 1.992):
+        w[0, 1] = v
+        out = torch.empty(1, 1, device=DEV)
+        K.linear(x.to(DEV), w.to(DEV), out)
+        ref = x.double() @ w.double().T
+        assert float(ref) < 3.4028235e38 and abs(float(out) - float(ref)) <= 2.0 ** -22 * float(ref)
+    assert K.f32_tc_error() == 0
+
+
 @pytest.mark.parametrize("which", ["x", "w", "w2"])
 def test_linear_float32_of_unaligned_rows_where_the_work_is_enough_for_the_tensor_cores(which):
     M, N, K_ = 300, 512, 512
