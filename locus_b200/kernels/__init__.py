@@ -531,7 +531,8 @@ def f32_splits(m: int, n: int, k: int) -> int:
     return best
 
 
-F32_TC_WORK = 64_000_000   # multiply-adds from which a float32 product goes to the tensor cores (see f32_tc_takes)
+F32_TC_WORK = 64_000_000   # multiply-adds from which a float32 product goes to the tensor cores (see f32_tc_takes) ...
+F32_TC_COLUMNS = 32        # ... if its sums have as many columns, those of a pair more
 
 
 def f32_tc_takes(x: torch.Tensor, w: torch.Tensor, m: int, w2: Optional[torch.Tensor] = None) -> bool:
@@ -539,9 +540,12 @@ def f32_tc_takes(x: torch.Tensor, w: torch.Tensor, m: int, w2: Optional[torch.Te
     cut into three bfloat16 (csrc/gemm_f32_tc.cuh): rows (of ``w2`` too) that 16-byte loads and TMA can address, enough work for its two
     launches and its pipeline's start (about 9 us), and scratch for the parts of x.  Measured, on CUDA cores / there: 33 rows of
     2,048 x 512 9.6 / 10.1 us, 64 11.6 / 11.3, of 4,096 x 256 11.1 / 11.2, 128 14.9 / 11.4, 256 rows of 512 x 512 11.4 / 11.3; 33 rows
-    of 2,048 x 2,048 17.9 / 13.8, 512 110 / 33; 512 rows of 6,144 x 2,048 301 / 82, 2,048 rows 1,156 / 246."""
+    of 2,048 x 2,048 17.9 / 13.8, 512 110 / 33; 512 rows of 6,144 x 2,048 301 / 82, 2,048 rows 1,156 / 246.  Sums of less than a stage of
+    32 columns (of a pair: of up to one) stay on gemm_simt, which needs no kernel in front and keeps more blocks at their epilogues: 2,048
+    rows of 2,048 x 16 11.1 / 18.1, x 20 15.1 / 18.8, x 32 18.5 / 18.4, of 6,144 x 16 29.4 / 38.7, x 20 37.9 / 39.0, x 32 47.7 / 38.7; pairs of 2,048 x 16
+    26.3 / 33.6, x 32 37.0 / 33.5, of 6,144 x 16 63 / 103, x 32 92 / 103, x 36 131 / 106."""
     K, n = x.shape[-1], w.shape[-2]
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0 and K >= F32_TC_COLUMNS + (0 if w2 is None else 4)
             and (x.data_ptr() | w.data_ptr() | (w2.data_ptr() if w2 is not None else 0)) % 16 == 0
             and m * n * K * (2 if w2 is not None else 1) >= F32_TC_WORK and w.numel() // K < 1 << 31
             and 4 * f32_tc_floats(m, K) <= SPLIT_SCRATCH_BYTES)

@@ -656,6 +656,7 @@ def test_linear_float32_tensor_cores(tn, splits, dual, monkeypatch):
     length or without a stage, more tiles than SMs; bias, row scale, added to what is there.  The bound on the error against 64
     bits holds for a sum of K products that is rounded (or cut off) at most K / 16 times by 2^-23 of its largest partial sum."""
     monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    monkeypatch.setattr(K, "F32_TC_COLUMNS", 0)
     monkeypatch.setattr(K, "few_rows_take", lambda *a, **k: False)
     monkeypatch.setattr(K, "f32_tc_plan", lambda m, n, k, d: (tn, 1 if d or m * n > 10 ** 6 else splits))   # (what the scratch holds)
     for M, N, K_ in ((1, 1, 4), (16, 64, 32), (33, 129, 36), (65, 200, 100), (130, 65, 2052), (300, 1000, 160), (1500, 2300, 72)):
@@ -704,6 +705,7 @@ def test_linear_float32_tensor_cores_of_experts(monkeypatch):
 def test_linear_float32_tensor_cores_keep_what_is_not_finite_and_the_range(tn, monkeypatch):
     """Infinities, NaN, the largest and the smallest values: what plain multiply-adds give, in their outputs and in no others."""
     monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    monkeypatch.setattr(K, "F32_TC_COLUMNS", 0)
     monkeypatch.setattr(K, "few_rows_take", lambda *a, **k: False)
     monkeypatch.setattr(K, "f32_tc_plan", lambda m, n, k, d: (tn, 1))
     M, N, K_ = 70, 140, 64
@@ -729,6 +731,7 @@ def test_linear_float32_tensor_cores_leave_out_no_more_than_they_say(monkeypatch
     is off by what the six products leave out (2^-24 of each) and by the rounding of its last sum (2^-24), and by nothing else that
     counts.  With the first part cut off instead of rounded the second kind of operand is off by 2^-22."""
     monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    monkeypatch.setattr(K, "F32_TC_COLUMNS", 0)
     monkeypatch.setattr(K, "few_rows_take", lambda *a, **k: False)
     low = [1 + 2 ** -8 - 2 ** -16 + 2 ** -17 - 2 ** -23, 1 + 2 ** -7 - 2 ** -15 + 2 ** -16 - 2 ** -23, 1 + 2 ** -8 + 2 ** -16, 1 + 2 ** -23, 2 - 2 ** -23]
     values = torch.tensor([s * v * 2.0 ** e for v in low for s in (1, -1) for e in (0, -9, 40)], dtype=torch.float32)

@@ -112,6 +112,13 @@ def test_float32_products_go_to_the_tensor_cores_only_with_rows_that_tma_can_add
     assert K.f32_tc_takes(x, w, 512, _floats(512, 512, offset=4))
 
 
+def test_short_float32_sums_stay_on_the_cuda_cores():
+    """Whatever the work: one weight's sums of less than a stage of 32 columns, a pair's of up to one."""
+    for k in (4, 16, 20, 28, 32, 36, 64):
+        x, w, w2 = _floats(4096, k), _floats(4096, k), _floats(4096, k)
+        assert K.f32_tc_takes(x, w, 4096) == (k >= 32) and K.f32_tc_takes(x, w, 4096, w2) == (k > 32)
+
+
 def test_threads_that_share_a_stream_have_scratch_of_their_own(monkeypatch):
     """A product's launches (its parts cut up, the product, the sum of its parts) meet in the scratch; those of another thread on the
     same stream may come between them."""
