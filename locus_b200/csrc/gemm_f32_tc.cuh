@@ -31,6 +31,7 @@
 // the kernel ends.
 #pragma once
 #include <cuda.h>
+#include <string.h>
 
 #include "bf16_parts.cuh"
 
@@ -518,17 +519,25 @@ static bool ft_map_x(CUtensorMap* map, void* ptr, long long rows, long long Kp, 
 template <int TN, bool SWIGLU>
 static int launch_f32_tc(const GemmArgs& a, const CUtensorMap& map_w, const CUtensorMap& map_w2, bf16* parts, int Kp, int tiles_y,
                          cudaStream_t stream) {
+    // the boxes that tiles of this call ask for: a plain product's full tiles and its last one; of experts' any (a map takes the host
+    // about half a microsecond)
     FtXMaps maps_x;
+    memset(&maps_x, 0, sizeof(maps_x));
+    const int rest = a.M % TN, last = rest == 0 ? 3 : (rest + TN / 4 - 1) / (TN / 4) - 1;
     for (int q = 0; q < 4; ++q)
-        if (!ft_map_x(&maps_x.m[q], parts, a.M, Kp, (q + 1) * (TN / 4))) return LOCUS_ERR_UNSUPPORTED;
+        if ((a.tile_expert != nullptr || q == last || (q == 3 && a.M >= TN)) && !ft_map_x(&maps_x.m[q], parts, a.M, Kp, (q + 1) * (TN / 4)))
+            return LOCUS_ERR_UNSUPPORTED;
     auto* kernel = gemm_f32_tc_kernel<TN, SWIGLU>;
     constexpr int smem = FtShape<TN>::SMEM;
     static_assert(smem <= 227 * 1024, "shared memory");
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
-    int dev = 0, n_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return static_cast<int>(cudaGetLastError());
+    static int n_sm = 0;
+    if (n_sm == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return static_cast<int>(cudaGetLastError());
+    }
     const int tiles_x = ceil_div(a.N, SWIGLU ? FT_W / 2 : FT_W);
     const long long n = static_cast<long long>(tiles_x) * tiles_y * a.splits;
     if (n >= (1LL << 31)) return LOCUS_ERR_UNSUPPORTED;
@@ -560,9 +569,9 @@ extern "C" int locus_gemm_f32_tc(const void* x, const void* w, const void* w2, l
     const int tiles_y = tile_expert ? max_tiles : ceil_div(M, tn), Kp = ceil_div(K, FT_K) * FT_K;
     if (M == 0 || tiles_y <= 0) return 0;
     CUtensorMap map_w, map_w2;
-    if (!ft_map_w(&map_w, w, w_rows_total, K, swiglu ? FT_W / 2 : FT_W) ||
-        !ft_map_w(&map_w2, swiglu ? w2 : w, w_rows_total, K, swiglu ? FT_W / 2 : FT_W))
-        return LOCUS_ERR_UNSUPPORTED;
+    if (!ft_map_w(&map_w, w, w_rows_total, K, swiglu ? FT_W / 2 : FT_W)) return LOCUS_ERR_UNSUPPORTED;
+    map_w2 = map_w;
+    if (swiglu && !ft_map_w(&map_w2, w2, w_rows_total, K, FT_W / 2)) return LOCUS_ERR_UNSUPPORTED;
     GemmArgs a;
     a.x = x; a.w = w; a.w2 = w2; a.bias = bias; a.bias_dt = bias_dt; a.out = out; a.out_dt = out_dt; a.accumulate = accumulate;
     a.act = act; a.act_param = act_param; a.act_scale = act_scale; a.row_scale = row_scale; a.scale_rows = scale_rows;

@@ -178,13 +178,16 @@ def _count_launches(n: int) -> None:
     launches += n
 
 
-def _check(code: int, what: str, detail: str = "") -> None:
+def _check(code: int, what: str, detail="") -> None:
+    """Raise if a C entry point returned an error.  ``detail``: a text, or a function that gives it."""
     global launches
     if code == 0:
         launches += _LAUNCHES_OF.get(what, 1)
         if _TIMES is not None:
             _TIMES._mark(what)
         return
+    if callable(detail):
+        detail = detail()
     if code == ERR_UNSUPPORTED:
         raise KernelError(f"{what}: sizes or element types outside what the kernel takes {detail}")
     raise KernelError(f"{what}: CUDA error {code} {detail}")
@@ -196,13 +199,17 @@ def _need(cond: bool, msg: str) -> None:
 
 
 def _cuda_c(t: torch.Tensor, name: str) -> None:
-    _need(t.is_cuda, f"{name} must be a CUDA tensor")
-    _need(t.is_contiguous(), f"{name} must be contiguous")
+    # (messages are put together when they are needed: small steps wait for the host)
+    if not t.is_cuda:
+        raise KernelError(f"{name} must be a CUDA tensor")
+    if not t.is_contiguous():
+        raise KernelError(f"{name} must be contiguous")
 
 
 def _i32(t: torch.Tensor, name: str) -> None:
     _cuda_c(t, name)
-    _need(t.dtype == torch.int32, f"{name} must be int32")
+    if t.dtype != torch.int32:
+        raise KernelError(f"{name} must be int32")
 
 
 LL = ctypes.c_longlong
@@ -544,10 +551,13 @@ def f32_tc_takes(x: torch.Tensor, w: torch.Tensor, m: int, w2: Optional[torch.Te
     32 columns (of a pair: of up to one) stay on gemm_simt, which needs no kernel in front and keeps more blocks at their epilogues: 2,048
     rows of 2,048 x 16 11.1 / 18.1, x 20 15.1 / 18.8, x 32 18.5 / 18.4, of 6,144 x 16 29.4 / 38.7, x 20 37.9 / 39.0, x 32 47.7 / 38.7; pairs of 2,048 x 16
     26.3 / 33.6, x 32 37.0 / 33.5, of 6,144 x 16 63 / 103, x 32 92 / 103, x 36 131 / 106."""
-    K, n = x.shape[-1], w.shape[-2]
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0 and K >= F32_TC_COLUMNS + (0 if w2 is None else 4)
+    if x.dtype != torch.float32:
+        return False
+    K, n = w.shape[-1], w.shape[-2]
+    if m * n * K * (1 if w2 is None else 2) < F32_TC_WORK or K < F32_TC_COLUMNS + (0 if w2 is None else 4):   # (most calls; the quickest test)
+        return False
+    return (w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0 and w.numel() // K < 1 << 31
             and (x.data_ptr() | w.data_ptr() | (w2.data_ptr() if w2 is not None else 0)) % 16 == 0
-            and m * n * K * (2 if w2 is not None else 1) >= F32_TC_WORK and w.numel() // K < 1 << 31
             and 4 * f32_tc_floats(m, K) <= SPLIT_SCRATCH_BYTES)
 
 
@@ -599,7 +609,8 @@ def _split_scratch(device, floats: int) -> torch.Tensor:
         if t is None:
             t = torch.empty(SPLIT_SCRATCH_BYTES // 4, dtype=torch.float32, device=device)
             _SPLIT_SCRATCH[key] = t
-    _need(floats <= t.numel(), f"a product's partial sums and parts take {floats} floats, their buffer holds {t.numel()}")
+    if floats > t.numel():
+        raise KernelError(f"a product's partial sums and parts take {floats} floats, their buffer holds {t.numel()}")
     return t
 
 
@@ -666,8 +677,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
     _cuda_c(out, "out")
     K = x.shape[-1]
     N = w.shape[-2]
-    _need(w.shape[-1] == K, f"linear: x has width {K} but w has {w.shape[-1]}")
-    _need(out.shape[-1] == N, f"linear: out has width {out.shape[-1]} but w has {N} rows")
+    if w.shape[-1] != K:
+        raise KernelError(f"linear: x has width {K} but w has {w.shape[-1]}")
+    if out.shape[-1] != N:
+        raise KernelError(f"linear: out has width {out.shape[-1]} but w has {N} rows")
     M = out.shape[0] if n_rows is None else n_rows
     _need(M <= out.shape[0], "linear: more rows than out holds")
     if x_rows is None and layout is None:
@@ -676,10 +689,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         _need(w2.shape == w.shape and w2.dtype == w.dtype and w2.is_contiguous(), "linear: w2 must match w")
     if accumulate:
         _need(out.dtype == torch.float32, "linear: accumulate needs a float32 out")
-    _need(act in ACTIVATIONS and not (act == "relu2" and w2 is not None) and not (act == "reglu" and w2 is None) and not (act == "glu_clamp" and (w2 is None or not act_limit > 0))
-          and not (act == "softcap" and (w2 is not None or not act_limit > 0)),
-          f"linear: activation {act!r} (known: relu2 without w2; reglu with w2; glu_clamp with w2 and a positive act_limit; softcap without "
-          "w2 and with a positive act_limit)")
+    if act is not None and (act not in ACTIVATIONS or (act == "relu2" and w2 is not None) or (act == "reglu" and w2 is None)
+                            or (act == "glu_clamp" and (w2 is None or not act_limit > 0)) or (act == "softcap" and (w2 is not None or not act_limit > 0))):
+        raise KernelError(f"linear: activation {act!r} (known: relu2 without w2; reglu with w2; glu_clamp with w2 and a positive act_limit; "
+                          "softcap without w2 and with a positive act_limit)")
     flags = I((1 if accumulate else 0) | (ACTIVATIONS[act] << 1))
     if bias is not None:
         _need(bias.numel() == (2 * N if act == "reglu" else N) and bias.is_contiguous(), "linear: bias size")
@@ -712,7 +725,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
             I(x_row_div), I(M), I(N), I(K), LL(x.stride(0)), LL(out.stride(0)), I(tile), _p(te), _p(t0), _p(tr),
             _p(nt), I(max_tiles), LL(stride), I(1 if (lists_ready and layout is not None) else 0), _stream()
         )
-        _check(code, "linear", f"(skinny; M={M}, N={N}, K={K}, tile {tile})")
+        _check(code, "linear", lambda: f"(skinny; M={M}, N={N}, K={K}, tile {tile})")
         return
     if few_rows_take(x, w, M, layout, w2 is not None):
         # a handful of rows: bandwidth-bound row-streaming kernel (csrc/gemv.cu)
@@ -729,7 +742,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
             flags, F(act_limit), F(act_scale), _p(row_scale), _p(scale_rows), _p(x_rows), I(x_row_div), I(M), I(N), I(K),
             LL(x.stride(0)), LL(out.stride(0)), _p(te), _p(t0), _p(tr), _p(nt), I(max_tiles), LL(stride), _stream()
         )
-        _check(code, "linear", f"(few rows; M={M}, N={N}, K={K}, x {x.dtype}, w {w.dtype})")
+        _check(code, "linear", lambda: f"(few rows; M={M}, N={N}, K={K}, x {x.dtype}, w {w.dtype})")
         return
     if tensor_cores_take(x, w, x_rows):
         # bfloat16 x bfloat16: tcgen05 kernel (csrc/gemm_tc.cu)
@@ -759,7 +772,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         )
         if splits > 1 and code == 0:
             _count_launches(1)   # the kernel that adds the splits up
-        _check(code, "linear", f"(tensor cores; M={M}, N={N}, K={K}, token tile {TN}, {splits} splits)")
+        _check(code, "linear", lambda: f"(tensor cores; M={M}, N={N}, K={K}, token tile {TN}, {splits} splits)")
         return
     if layout is not None:
         _need(layout.tile_m == 64, "linear: the CUDA-core product uses 64-row tiles")
@@ -785,7 +798,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
         )
         if code == 0:
             _count_launches(2 if splits > 1 else 1)   # the kernel that cuts x up, the kernel that adds the parts up
-        _check(code, "linear", f"(float32 on the tensor cores; M={M}, N={N}, K={K}, {tn} rows a tile, {splits} splits)")
+        _check(code, "linear", lambda: f"(float32 on the tensor cores; M={M}, N={N}, K={K}, {tn} rows a tile, {splits} splits)")
         return
     splits, scratch = 1, None
     if (layout is None and w2 is None and x.dtype == torch.float32 and w.dtype == torch.float32 and (K | x.stride(0)) % 4 == 0
@@ -802,7 +815,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
     )
     if splits > 1 and code == 0:
         _count_launches(1)   # the kernel that adds the parts up
-    _check(code, "linear", f"(M={M}, N={N}, K={K}, x {x.dtype}, w {w.dtype}, {splits} splits)")
+    _check(code, "linear", lambda: f"(M={M}, N={N}, K={K}, x {x.dtype}, w {w.dtype}, {splits} splits)")
 
 
 def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor],
@@ -2361,8 +2374,8 @@ def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.
     key channel: :func:`gla_decay`) and ``v``: float32 row matrices in which head h's columns start at ``off_*`` + h * dim (``off_v`` + h * v_dim);
     head h's state [dim, v_dim] starts ``state_offset`` + h * dim * v_dim floats into a slot of ``state`` [n_slots,
     floats]; ``out`` [T, n_heads * v_dim] float32."""
-    for t, name in ((q, "q"), (k, "k"), (v, "v"), (decay, "decay"), (out, "out")):
-        _f32c(t, f"gla_scan: {name}")
+    for t, name in ((q, "gla_scan: q"), (k, "gla_scan: k"), (v, "gla_scan: v"), (decay, "gla_scan: decay"), (out, "gla_scan: out")):
+        _f32c(t, name)
     _i32(state_slots, "state_slots")
     _need(state.is_cuda and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
           and state_offset + n_heads * dim * v_dim <= state.shape[1], "gla_scan: the state does not hold the heads")
@@ -2379,7 +2392,7 @@ def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.
         I(v_dim), F(q_scale), _p(scratch), LL((rows // 16 + n_seg) * n_heads * CHUNK_BYTES if rows else 0), _stream())
     if rows and code == 0:
         _count_launches(2 * -(-out.shape[0] // rows) - 1)   # two for every stretch of rows that the scratch holds
-    _check(code, "gla_scan", f"(heads {n_heads}, dim {dim}, v_dim {v_dim})")
+    _check(code, "gla_scan", lambda: f"(heads {n_heads}, dim {dim}, v_dim {v_dim})")
 
 
 def apply_penalties(logits: torch.Tensor, history: torch.Tensor, repeat: torch.Tensor,
