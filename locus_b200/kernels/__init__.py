@@ -2360,10 +2360,13 @@ def gla_error() -> int:
 
 
 def _chunk_scratch(out: torch.Tensor, n_heads: int, n_seg: int):
-    """(scratch for the chunks of all rows of ``out``, or of as many as the split products' buffer holds; how many rows)."""
+    """(scratch for the chunks of all rows of ``out``, or of as many as the split products' buffer holds; how many rows), 0 rows where
+    it holds so few beside the one that every segment may leave unfilled that the many stretches take longer than the walk: 64 heads, walked / in chunks,
+    32 requests of 64 tokens (4 chunks a stretch) 862 / 1,395 us, 24 (12 chunks) 651 / 498; 16 heads, 128 requests (17 chunks) 863 / 1,708, 96
+    (49 chunks) 652 / 512."""
     per, most = n_heads * CHUNK_BYTES, -(-out.shape[0] // 16)
     chunks = min(most, SPLIT_SCRATCH_BYTES // per - n_seg)
-    return (_split_scratch(out.device, (chunks + n_seg) * per // 4), 16 * chunks) if chunks > 0 else (None, 0)
+    return (_split_scratch(out.device, (chunks + n_seg) * per // 4), 16 * chunks) if 2 * chunks >= min(2 * most, n_seg) > 0 else (None, 0)
 
 
 def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.Tensor, off_v: int, decay: torch.Tensor,

@@ -275,6 +275,35 @@ def test_gla_scan_in_chunks(H, dv, small, precise, monkeypatch):
     assert K.gla_error() == 0
 
 
+@pytest.mark.parametrize("n_seg,small", [(33, False), (70, True), (32, False)])
+def test_gla_scan_in_chunks_of_many_requests(n_seg, small, precise, monkeypatch):
+    """More requests than a warp has lanes, some of no token, in any order of their rows; whole and in stretches of rows."""
+    import locus_b200.kernels as K
+
+    H, d, dv = 2, 128, 16
+    monkeypatch.setattr(K, "CHUNK_MIN_TOKENS", 0)
+    g = torch.Generator().manual_seed(n_seg)
+    lens = [[0, 1, 15, 16, 17, 33, 5][i % 7] for i in range(n_seg)]
+    q0, T = [0] * n_seg, 0
+    for i in torch.randperm(n_seg, generator=g).tolist():
+        q0[i], T = T, T + lens[i]
+    proj, z = torch.randn(T, 3 * H * d, generator=g), torch.rand(T, H * d, generator=g) * 0.3
+    state, slots = torch.randn(n_seg, H * d * dv, generator=g), torch.randperm(n_seg, generator=g).to(torch.int32)
+    n, q0 = torch.tensor(lens, dtype=torch.int32), torch.tensor(q0, dtype=torch.int32)
+    kw = dict(n_heads=H, dim=d, v_dim=dv, q_scale=d ** -0.5)
+    ref_state, ref = state.double(), torch.zeros(T, H * dv, dtype=torch.float64)
+    EK.gla_scan(proj.double(), 0, proj.double(), H * d, proj.double(), 2 * H * d, z.double(), 0, ref_state, 0, slots, q0, n, n_seg, ref, **kw)
+    if small:
+        monkeypatch.setattr(K, "SPLIT_SCRATCH_BYTES", H * K.CHUNK_BYTES * (n_seg + n_seg // 2))
+        monkeypatch.setattr(K, "_SPLIT_SCRATCH", {})
+    before, dp, st, out = K.launches, proj.to(DEV), state.to(DEV), torch.zeros(T, H * dv, device=DEV)
+    K.gla_scan(dp, 0, dp, H * d, dp, 2 * H * d, z.to(DEV), 0, st, 0, slots.to(DEV), q0.to(DEV), n.to(DEV), n_seg, out, **kw)
+    assert K.launches - before == 2 * (-(-T // (16 * (n_seg // 2))) if small else 1)
+    _cmp(out, ref, 2e-5)
+    _cmp(st, ref_state, 2e-5)
+    assert K.gla_error() == 0
+
+
 @pytest.mark.parametrize("H,d,dv", [(2, 24, 16), (1, 7, 5), (3, 72, 40), (2, 128, 64), (1, 200, 12)])
 def test_gla_scan_and_decay_against_twin(H, d, dv, precise):
     import locus_b200.kernels as K

@@ -143,3 +143,16 @@ def test_threads_that_share_a_stream_have_scratch_of_their_own(monkeypatch):
     thread.join()
     assert seen[:3] == [False, False, True] and seen[3]() is None   # ... and it is given back
     assert K._split_scratch("cpu", 100) is mine
+
+
+def test_chunks_of_a_recurrence_take_no_stretches_of_a_few_chunks(monkeypatch):
+    """Where the scratch does not hold all rows, a stretch has at least half a chunk for every segment; else the walk runs."""
+    import torch
+
+    monkeypatch.setattr(K, "_split_scratch", lambda device, floats: floats)
+    for heads, n_seg, tokens, takes in ((16, 1, 4096, True), (16, 64, 64, True), (16, 96, 64, True), (16, 128, 64, False), (64, 24, 64, True),
+                                        (64, 32, 64, False), (64, 64, 64, False), (4, 300, 64, True), (2048, 1, 64, False)):
+        floats, rows = K._chunk_scratch(torch.empty(n_seg * tokens, 1), heads, n_seg)
+        assert (floats is not None) == (rows > 0) == takes
+        if takes:
+            assert rows % 16 == 0 and (rows // 16 + n_seg) * heads * K.CHUNK_BYTES == 4 * floats <= K.SPLIT_SCRATCH_BYTES
