@@ -2349,7 +2349,7 @@ def gla_decay(z: torch.Tensor, off: int, n: int, tau: float) -> None:
 
 
 CHUNK_DIM = 128          # channels of a head that gla_scan takes sixteen tokens together (csrc/gla.cu, gla_chunk)
-CHUNK_MIN_TOKENS = 64    # ... of steps of at least so many tokens a segment (64 tokens 13.5 us walked, 13.2 in chunks; 32 9.4, 11.1)
+CHUNK_MIN_TOKENS = 320   # ... in steps of so many tokens (see chunks_pay)
 CHUNK_BYTES = 2 * (6 * 16 * (CHUNK_DIM + 8) + 3 * 16 * 24) + 4 * CHUNK_DIM   # scratch by chunk and head
 
 
@@ -2357,6 +2357,15 @@ def gla_error() -> int:
     """Error word of gated linear attention in chunks (0 = fine; 1: a wait for a chunk's operands ran out); reading it synchronises
     the device."""
     return int(_lib("gla").locus_gla_error())
+
+
+def chunks_pay(n_tokens: int, n_seg: int, n_heads: int) -> bool:
+    """Whether heads of CHUNK_DIM channels take sixteen tokens together instead of walking.  A segment needs enough of them (64 tokens
+    12.1 us walked, 12.4 in chunks; 32 9.4, 11.1), and the walk must take longer than what the second launch costs the host, which is
+    what a step of few tokens waits for: a mixer's pass, 16 heads, walked / in chunks, 64 to 256 tokens 100 / 108 us, 320 113 / 104, 512
+    145 / 118, 3 requests of 231 in all 101 / 109, 4 of 322 117 / 107.  The walk's time goes by the longest segment or, from 16 heads
+    on, by all heads' tokens."""
+    return 5 * n_tokens >= CHUNK_MIN_TOKENS * n_seg and n_tokens * max(16, n_heads * n_seg) >= CHUNK_MIN_TOKENS * 16 * n_seg
 
 
 def _chunk_scratch(out: torch.Tensor, n_heads: int, n_seg: int):
@@ -2384,7 +2393,7 @@ def gla_scan(q: torch.Tensor, off_q: int, k: torch.Tensor, off_k: int, v: torch.
           and state_offset + n_heads * dim * v_dim <= state.shape[1], "gla_scan: the state does not hold the heads")
     _need(out.shape[1] == n_heads * v_dim and dim <= GLA_MAX_DIM, "gla_scan: out [T, n_heads * v_dim], dim <= 256")
     scratch, rows = None, 0
-    if (dim == CHUNK_DIM and n_seg > 0 and out.shape[0] >= CHUNK_MIN_TOKENS * n_seg
+    if (dim == CHUNK_DIM and n_seg > 0 and chunks_pay(out.shape[0], n_seg, n_heads)
             and (q.data_ptr() | k.data_ptr() | decay.data_ptr()) % 16 == 0
             and (q.stride(0) | off_q | k.stride(0) | off_k | decay.stride(0) | off_a) % 4 == 0):
         scratch, rows = _chunk_scratch(out, n_heads, n_seg)

@@ -156,3 +156,10 @@ def test_chunks_of_a_recurrence_take_no_stretches_of_a_few_chunks(monkeypatch):
         assert (floats is not None) == (rows > 0) == takes
         if takes:
             assert rows % 16 == 0 and (rows // 16 + n_seg) * heads * K.CHUNK_BYTES == 4 * floats <= K.SPLIT_SCRATCH_BYTES
+
+
+def test_when_a_recurrence_is_taken_in_chunks():
+    """By the longest segment (on average) or, from sixteen heads on, by all heads' tokens; never with fewer than 64 tokens a segment."""
+    for tokens, n_seg, heads, pays in ((320, 1, 1, True), (319, 1, 16, False), (320, 5, 16, True), (320, 6, 16, False), (80, 1, 64, True), (79, 1, 64, False),
+                                       (128, 2, 64, True), (127, 2, 64, False), (512, 8, 4, False), (2048, 8, 4, True), (1, 1, 16, False)):
+        assert K.chunks_pay(tokens, n_seg, heads) == pays, (tokens, n_seg, heads)
