@@ -1658,13 +1658,20 @@ def latent_expand_rows(dtype: torch.dtype, n_heads: int, nope_dim: int, rot_dim:
     return min(LATENT_EXPAND_ROWS, LATENT_EXPAND_BYTES // (2 * n_heads * (nope_dim + v_dim)))
 
 
-def latent_expand_pays(n_new: int, n_ctx: int, window: int) -> bool:
-    """Whether to expand the whole context of a segment that sees only ``window`` keys of it (0: all): a product over rows
-    that nobody sees (7 us a thousand, 16 heads on a latent of 512) is spent for less work on every pair of a query and a key
-    and for the per-head products.  Device time of the mixer over the latents / expanded, window 128: 64 new tokens behind 2,000
-    82 / 71 us, behind 4,000 82 / 86; 1,000 behind 4,000 164 / 130, behind 8,000 164 / 159; window 2,048: 256 behind 15,000 236 / 189."""
+def latent_expand_pays(n_new: int, n_ctx: int, window: int, n_heads: int = 16, kv_rank: int = 512) -> bool:
+    """Whether to expand the whole context of a segment of keys with a rotated part that sees only ``window`` keys of it (0: all): rows
+    that nobody sees are expanded for less work on every pair of a query and a key and no per-head products.  In microseconds: a
+    thousand rows 1.5 + 0.38 a head; what is gained, fitted from below, on latents of 512.  Device time of the mixer over the
+    latents / expanded: 16 heads, window 128, 64 new tokens behind 2,000 79 / 69, behind 4,000 79 / 83, 1,000 behind 8,000 162 / 157,
+    window 2,048, 64 behind 4,000 106 / 90, 256 behind 15,000 232 / 184; 64 heads, 64 behind 1,000 136 / 129, behind 2,000
+    135 / 157, 1,000 behind 8,000 499 / 497; 128 heads, 64 behind 1,000 207 / 232; 4 heads, behind 8,000 69 / 59; a latent of 256, 16
+    heads, 64 behind 3,000 70 / 71, 1,000 behind 4,000 116 / 120, window 2,048, 256 behind 8,000 168 / 127.  Without a window expanding is
+    the quicker way at all of these (64 new tokens behind none to 15,000: 49 to 186 us for 63 to 309)."""
     behind = n_ctx + 1 - window if window > 0 else 0
-    return behind <= max(2048, n_new * window // 32)
+    if behind <= 0:
+        return True
+    gain = 20 - 0.12 * n_heads + n_heads * ((n_new - 35) * window * 1.3e-5 + n_new * 1.3e-3)
+    return behind * (1.5e-3 + 0.38e-3 * n_heads) <= gain * (kv_rank - 82) / 430
 
 
 def latent_gather(pool: torch.Tensor, out: torch.Tensor, *, segs: torch.Tensor, n_segs: int, row0: torch.Tensor,

@@ -45,18 +45,20 @@ class LatentTiles(StepPlan):
     """Work items of the latent attention kernels, for every segment by its new tokens: tiles of ``tile`` queries
     (``items``); with ``singles`` the segments with one new token go to a list of their own (``single_items``), which the
     decode kernel takes; with ``max_rows`` > 0 the segments with at least ``expand_from`` new tokens, as long as the rows of
-    their contexts fit into ``max_rows`` together and not too many lie behind a ``window``, go to tiles of 64 queries (``long_items``), with the segments, the first row
+    their contexts fit into ``max_rows`` together and, of keys with a rotated part, not too many lie behind the ``window``, go to tiles of 64 queries (``long_items``), with the segments, the first row
     of each and the rows of all.  Tiles are ordered by the position of their first query (the kernels walk a list from its
     end, so the tiles with the most keys start first)."""
 
-    def __init__(self, tile: int = K.LATENT_QUERY_TILE, singles: bool = False, max_rows: int = 0, expand_from: int = 0, window: int = 0) -> None:
+    def __init__(self, tile: int = K.LATENT_QUERY_TILE, singles: bool = False, max_rows: int = 0, expand_from: int = 0, window: int = 0,
+                 n_heads: int = 16, kv_rank: int = 512) -> None:
         from ..cache import native
 
         self._lib = native.lib()
         self.tile, self.singles = int(tile), bool(singles)
         self.max_rows, self.expand_from = int(max_rows), int(expand_from) if max_rows else 0
         self.window = int(window) if max_rows else 0
-        self.key = ("latent_attention.tiles", self.tile, self.singles, self.max_rows, self.expand_from, self.window)
+        self.sizes = (int(n_heads), int(kv_rank)) if self.window else ()   # (what the rule for rows behind the window asks for)
+        self.key = ("latent_attention.tiles", self.tile, self.singles, self.max_rows, self.expand_from, self.window) + self.sizes
 
     def capacity(self, max_tokens: int, max_segments: int) -> int:
         return 2 * (max_tokens // self.tile + max_tokens // K.MMA_QUERY_TILE + 2 * max_segments) + 3 * max_segments
@@ -84,7 +86,7 @@ class LatentTiles(StepPlan):
             row0 = np.full(n_seg, -1, dtype=np.int32)
             for s in np.nonzero(seg_qn >= self.expand_from)[0]:
                 n = int(seg_ctx[s]) + int(seg_qn[s])
-                if rows + n <= self.max_rows and K.latent_expand_pays(int(seg_qn[s]), int(seg_ctx[s]), self.window):
+                if rows + n <= self.max_rows and K.latent_expand_pays(int(seg_qn[s]), int(seg_ctx[s]), self.window, *self.sizes):
                     row0[s] = rows
                     rows += n
                     longest = max(longest, n)
@@ -225,7 +227,7 @@ class LatentAttention(Mixer):
         tile = 64 >> self._head_shift if self._mma else K.LATENT_QUERY_TILE
         self._singles = K.latent_decode_takes(dtype, self.kv_rank, self.dr)
         self._max_rows = self._expand_rows(dtype)
-        return LatentTiles(tile, self._singles, self._max_rows, K.LATENT_EXPAND_FROM, self.window)
+        return LatentTiles(tile, self._singles, self._max_rows, K.LATENT_EXPAND_FROM, self.window if self.dr else 0, self.H, self.kv_rank)
 
     @property
     def _head_tiles(self) -> HeadTiles:

@@ -169,7 +169,7 @@ def test_long_portions_with_expanded_keys_and_a_rotated_part(tmp_path, monkeypat
 
     monkeypatch.setattr(K, "LATENT_EXPAND_FROM", 8)
     monkeypatch.setattr(K, "latent_expand_rows", lambda dtype, H, dn, dr, dv, rank: 200)
-    monkeypatch.setattr(K, "latent_expand_pays", lambda n, ctx, window: window == 20 and ctx + 1 - window <= 25)
+    monkeypatch.setattr(K, "latent_expand_pays", lambda n, ctx, window, *sizes: window == 20 and ctx + 1 - window <= 25)
     calls, rows = [], K.attn_chunk_tc_rows
     monkeypatch.setattr(K, "attn_chunk_tc_rows", lambda *a, **kw: (calls.append((sorted({int(s) for s, _ in kw["items"].tolist()}),
                                                                                  tuple(kw["q_rot"].shape), kw["k_rot"].shape[1])), rows(*a, **kw)))
@@ -188,3 +188,26 @@ def test_how_much_context_behind_a_window_is_expanded():
     assert K.latent_expand_pays(64, 16000, 0)
     for new, ctx, window, pays in ((64, 2000, 128, True), (64, 4000, 128, False), (1000, 4000, 128, True), (1000, 15000, 128, False), (1000, 15000, 512, True)):
         assert K.latent_expand_pays(new, ctx, window) == pays
+    # other numbers of heads and another latent, as measured beside the rule
+    for new, ctx, window, heads, rank, pays in ((64, 2000, 128, 64, 512, False), (64, 1000, 128, 128, 512, False), (64, 5000, 128, 4, 512, True),
+                                                (1000, 4000, 128, 64, 512, True), (256, 15000, 2048, 64, 512, True), (64, 4000, 2048, 128, 512, True),
+                                                (1000, 4000, 128, 16, 256, False), (256, 8000, 2048, 16, 256, True), (64, 2000, 2048, 128, 512, True)):
+        assert K.latent_expand_pays(new, ctx, window, heads, rank) == pays, (new, ctx, window, heads, rank)
+
+
+@pytest.mark.parametrize("rot,rule", [(64, True), (0, False)])
+def test_the_rule_for_rows_behind_a_window_is_for_keys_with_a_rotated_part(rot, rule, monkeypatch):
+    """Without one every long portion whose rows fit is expanded, as before there was a rule."""
+    import numpy as np
+
+    import locus_b200.kernels as K
+    from locus_b200.parts.latent_attention import LatentAttention
+
+    asked, pays = [], K.latent_expand_pays
+    monkeypatch.setattr(K, "latent_expand_pays", lambda *a: (asked.append(a), pays(*a))[1])
+    part = LatentAttention("a", hidden=64, n_heads=8, nope_dim=128, rot_dim=rot, v_dim=128, q_rank=0, kv_rank=512, scale=1.0, eps=1e-6, window=128)
+    part._dtype = torch.bfloat16
+    plan = part._query_tiles
+    seg = lambda *v: np.array(v, dtype=np.int32)
+    got = plan.build(seg(0, 64), seg(64, 64), seg(9000, 100), np.zeros(plan.capacity(128, 2), dtype=np.int32))
+    assert got["n_long"] == (1 if rule else 2) and len(got["long_segs"]) and asked[-1] == ((64, 100, 128, 8, 512) if rule else (64, 100, 0))
