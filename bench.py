@@ -9,7 +9,8 @@ sizes (random weights, bfloat16) at batch 8 and context 4096, with the prefill o
 
 With no options: the headline configuration.  ``--config 57b-a14b``: the Qwen2-57B-A14B layer sizes
 (28 layers, 114.8 GB of weights), decode from 8,192-token contexts and a 32,768-token prefill in portions
-of 2,048.  ``--dtype fp32``: the true 32-bit path (CUDA-core products, float32 cache).  ``--trace``: adds
+of 2,048.  ``--dtype fp32``: the true 32-bit path (float32 weights and cache; products on the
+CUDA cores, large ones on the tensor cores with every value in three bfloat16 parts).  ``--trace``: adds
 a mixed continuous-batching trace through ``Engine`` (32 requests, prompts uniform in [16, 4096], decode
 lengths uniform in [1, 512], one arrival every 4 steps, portions of 512 tokens).
 
@@ -269,8 +270,8 @@ def main() -> int:
     T = PREFILL_TOKENS
     flops = 2.0 * lin * T + 2.0 * V * cfg.hidden_size \
         + args.layers * 2.0 * cfg.num_attention_heads * cfg.head_dim * T * T  # causal QK^T and PV
-    # float32 runs on the CUDA cores: 128 FMA lanes per SM
-    peak_flops = pk["bf16_tflops"] * 1e12 if args.dtype == "bf16" else 148 * 128 * 2 * 1.965e9
+    # large float32 products are six bfloat16 products each
+    peak_flops = pk["bf16_tflops"] * 1e12 / (1 if args.dtype == "bf16" else 6)
     prefill = {"value": T / (pre_ms / 1e3), "tokens": T, "ms": pre_ms, "portions": len(portions),
                "frac": flops / (pre_ms / 1e3) / peak_flops, "tflops": flops / (pre_ms / 1e3) / 1e12,
                "peak_tflops": peak_flops / 1e12}

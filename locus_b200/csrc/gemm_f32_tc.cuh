@@ -21,9 +21,11 @@
 // What bounds it: the MMAs, six for one (a stage of 128 rows 768 cycles), where there are many rows, and the weights' way from
 // memory where there are few.  Measured, against the CUDA-core kernel: 2,048 x 6,144 x 2,048 1,156 -> 246 us (209 TFLOP/s; cuBLAS's
 // bfloat16 rate / 6 is 276), 512 x 6,144 x 2,048 301 -> 83, 64 x 6,144 x 2,048 47 -> 22, 512 x 2,048 x 5,632 268 -> 67, the routed
-// experts of 512 tokens (60 x (2,048 -> 1,408 -> 2,048), 4 picks) 1,004 -> 445 (their weights 4.7 TB/s).  The error of a sum
-// of 2,048 products against 64 bits 5.7e-7 -> 1.7e-7 of its norm (uncut; CUDA cores cut in parts 3.3e-7), of 128 1.5e-7 -> 0.8e-7;
-// with the large products' accumulator taken out after 128 columns 1.9e-7 and 1.25e-7, 3 % quicker.  On the way here: weights and x cut up
+// experts of 512 tokens (60 x (2,048 -> 1,408 -> 2,048), 4 picks) 1,004 -> 445 (their weights 4.7 TB/s).  The error of
+// sums of 2,048 normally distributed products against 64 bits 5.7e-7 -> 1.3e-7 of their norm (uncut; CUDA cores cut in parts
+// 3.3e-7), of 128 1.5e-7 -> 0.75e-7; of one sign 3.5e-7 -> 1.2e-7 and 0.93e-7 -> 0.92e-7, where the CUDA cores' sums are short, though (512
+// in 8 parts, 5,632 in 8), 0.56e-7 -> 0.90e-7 and 0.80e-7 -> 0.90e-7: what the accumulators cut off within 64 columns is of one sign then.
+// With the large products' accumulator taken out after 128 columns 1.9e-7 and 1.25e-7 (the first two, first parts cut off), 3 % quicker.  On the way here: weights and x cut up
 // by the same eight warps 573 us for the first (a chain of waits, loads, conversions and stores for every stage), x cut up
 // first and the sums taken out by the same warps 321.
 //

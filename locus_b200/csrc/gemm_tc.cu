@@ -8,9 +8,9 @@
 //
 //   D[n, t] (tensor memory, lane n, column t) = sum_k W[n0 + n, k] * x[t0 + t, k]
 //
-// A 128 x TN output tile is computed over the whole K by one CTA (no split of K: the order of
-// the sum for an element depends on K only).  The kernel is persistent: one CTA per SM walks
-// over the tiles in a fixed stride.  Warp 0 issues TMA loads (one elected thread) and runs
+// A 128 x TN output tile is computed by one CTA, over the whole K or over one of the parts that the host cut K into, and a
+// 256 x TN tile by a pair of CTAs of one cluster, 128 rows each (the order of the sum for an element is the same).  The
+// kernel is persistent: one CTA per SM walks over the tiles in a fixed stride.  Warp 0 issues TMA loads (one elected thread) and runs
 // ahead across tile boundaries, so the pipeline never drains between tiles; warp 1 allocates
 // tensor memory and issues the MMAs (one elected thread) into one of TWO accumulator buffers;
 // warps 2-5 read the other buffer back (tcgen05.ld, each warp its own 32 lanes) and run the
@@ -29,8 +29,10 @@
 //
 // Every wait on an mbarrier is bounded (about a second of clock cycles); when a wait runs
 // out the kernel records a code in the module's error word, stops waiting and finishes, so
-// a fault in the pipeline shows as an error on the host, never as a hang.  Every TMA load goes
-// to the shared memory of the block that issued it; nothing is sent to other blocks.
+// a fault in the pipeline shows as an error on the host, never as a hang.  Every TMA load goes to the shared memory of
+// the block that issued it.  What crosses between the blocks of a pair: loads of the second are counted by the first's barriers, the
+// first's MMAs read the token rows of both and commit to barriers of both, and the second's epilogue warps give the accumulators
+// back at the first's barriers; neither block leaves before the other (pair_sync).
 #include <cuda.h>
 
 #include "common.cuh"

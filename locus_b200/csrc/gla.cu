@@ -31,10 +31,11 @@
 //               at once: gla_chunk_prep forms it, in three bfloat16 parts (chunk_mma.cuh).  What remains of the walk is a state in
 //               the registers of eight warps, sixteen channels each, 24 MMAs a warp for sixteen tokens (36 of one), and sums
 //               over the warps, which nothing waits for: the chain from chunk to chunk is one multiply-add.
-//               Bound by the latency of a chunk's chain of loads, cuts and MMAs, 1,500 cycles with two warps a scheduler.  Measured,
-//               2,048 tokens of 16 heads of 128 x 128: 255 -> 132 us (26 of them gla_chunk_prep), eight requests of 256 181 -> 113,
-//               one of 64 13.5 -> 13.2 (of 32 9.4 / 11.1: the walk's); the error against 64 bits 4.3e-7 -> 2.0e-7 of the
-//               read-outs' norm, of the state 4.4e-7 -> 1.3e-7.  Two chunks to a turn, one block an SM: 134 and 135 us.
+//               Bound by the latency of a chunk's chain of loads, cuts and MMAs, 1,320 cycles with two warps a scheduler.  Measured,
+//               2,048 tokens of 16 heads of 128 x 128: 254 -> 129 us (26 of them gla_chunk_prep), eight requests of 256 178 -> 100,
+//               64 of 64 437 -> 295, one of 64 12.1 -> 12.4 (of 32 9.4 / 11.1; kernels.chunks_pay draws the line); the error against
+//               64 bits 4.3e-7 -> 2.0e-7 of the read-outs' norm, of the state 4.4e-7 -> 1.3e-7.  Two chunks to a turn, one block an
+//               SM: 134 and 135 us.
 //
 // The order of every sum is fixed by d and by the kernel.
 #include "common.cuh"

@@ -654,7 +654,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w2: Optional[
            x_rows: Optional[torch.Tensor] = None, x_row_div: int = 1, layout: Optional[ExpertLayout] = None,
            n_rows: Optional[int] = None, lists_ready: bool = False, second_tiles: bool = False,
            act: Optional[str] = None, act_limit: float = 0.0, act_scale: float = 1.0) -> None:
-    """out = x . w^T with float32 accumulation on CUDA cores (see csrc/gemm_simt.cu).
+    """out = x . w^T with float32 accumulation, by the kernel that sizes, element types and alignment call for: gemm_skinny and
+    gemm_tc (bfloat16 on the tensor cores), gemv (few rows), gemm_f32_tc (float32 in three bfloat16 parts on the tensor cores) or
+    gemm_simt (CUDA cores, everything else).
 
     ``w2``: out = silu(x . w^T) * (x . w2^T).  ``act`` = "relu2": out = max(x . w^T + bias, 0)^2 (not with ``w2``).
     ``act`` = "glu_clamp" (with ``w2``): the clamped gated unit out = g sigmoid(1.702 g) (u + 1) with g = min(s x . w^T,

@@ -296,6 +296,16 @@ def run(args) -> dict:
     H, R = z["heads"], z["kv_rank"] + z["rot"]
     keys_avg = sum(min(p + 1, z["window"]) for p in range(T)) / T
     fma_tflops = 148 * 128 * 2 * 1.965e9 / 1e12       # float32 FMAs of the CUDA cores at the top clock
+    f32_tc_tflops = pk["bf16_tflops"] / 6             # float32 products as six bfloat16 products
+    expands = K.latent_expand_rows(dtype, H, z["dim"], z["rot"], z["vdim"], z["kv_rank"]) >= T
+
+    def latent_flops(pairs):
+        """Of a portion's latent attention behind the projections: keys and values of all heads expanded, or the absorbed form, which
+        multiplies the cached row (latent and rotated part) per score and the latent per value."""
+        if expands:
+            return 2.0 * H * (pairs * (z["dim"] + z["rot"] + z["vdim"]) + T * (z["dim"] + z["vdim"]) * z["kv_rank"])
+        return 2.0 * H * pairs * (R + z["kv_rank"])
+
     if design == "megovik":
         G, D, Wd, r = max(1, H // 4), z["dim"], z["width"], z["kv_rank"]
         causal = T * (T + 1) / 2
@@ -306,7 +316,7 @@ def run(args) -> dict:
             "attn_decode_us": B * ctx * 2 * G * D * el / (pk["hbm_gbs"] * 1e9) * 1e6,
             "latent_attn_prefill_us": 2.0 * causal * H * 2 * r / (pk["bf16_tflops"] * 1e12) * 1e6,
             "latent_attn_decode_us": B * ctx * r * el / (pk["hbm_gbs"] * 1e9) * 1e6,
-            "gugozen_latent_attn_prefill_us": 2.0 * causal * H * (R + r) / (pk["bf16_tflops"] * 1e12) * 1e6,
+            "gugozen_latent_attn_prefill_us": latent_flops(causal) / (pk["bf16_tflops"] * 1e12) * 1e6,
             "gugozen_latent_attn_decode_us": B * ctx * R * el / (pk["hbm_gbs"] * 1e9) * 1e6,
             "head_prep_prefill_us": row * ((H + G) * D * 4 + (H + 2 * G) * D * el),
             "dense_ff_prefill_us": 2.0 * T * 3 * Wd * z["shared"] / (pk["bf16_tflops"] * 1e12) * 1e6,
@@ -342,15 +352,14 @@ def run(args) -> dict:
         bounds = {
             "attn_prefill_us": 2.0 * T * (T + 1) / 2 * H * 2 * z["dim"] / (pk["bf16_tflops"] * 1e12) * 1e6,
             "attn_decode_us": B * ctx * 2 * G * z["dim"] * el / (pk["hbm_gbs"] * 1e9) * 1e6,
-            # the absorbed form multiplies the cached row (latent and rotated part) per score and the latent per value
-            "latent_attn_prefill_us": 2.0 * T * (T + 1) / 2 * H * (R + z["kv_rank"]) / (pk["bf16_tflops"] * 1e12) * 1e6,
+            "latent_attn_prefill_us": latent_flops(T * (T + 1) / 2) / (pk["bf16_tflops"] * 1e12) * 1e6,
             "latent_attn_decode_us": B * ctx * R * el / (pk["hbm_gbs"] * 1e9) * 1e6,
-            # per token and head the decayed rank-one update and the read-out, float32 FMAs
-            "gla_prefill_us": 2.0 * T * H * 2 * d * dv / (fma_tflops * 1e12) * 1e6,
+            # per token and head the decayed rank-one update and the read-out: walked, or in chunks of tokens as products
+            "gla_prefill_us": 2.0 * T * H * 2 * d * dv / ((f32_tc_tflops if d == K.CHUNK_DIM else fma_tflops) * 1e12) * 1e6,
             "gla_decode_us": B * H * d * dv * 4 * 2 / (pk["hbm_gbs"] * 1e9) * 1e6,
             "retention_decode_us": B * H * d * dv * 4 * 2 / (pk["hbm_gbs"] * 1e9) * 1e6,
             "qwen_attn_decode_us": B * ctx * 2 * H * z["dim"] * el / (pk["hbm_gbs"] * 1e9) * 1e6,
-            "fp32_fma_tflops": fma_tflops,
+            "fp32_fma_tflops": fma_tflops, "fp32_tensor_tflops": f32_tc_tflops,
         }
         return {"metric": f"prefill and decode tokens/s, Gugozen beside Lalepel and Qwen2-MoE at equal layer sizes "
                           f"({args.size}, {args.layers} layers, {args.dtype})",
@@ -404,7 +413,7 @@ def run(args) -> dict:
                 "bounds_per_layer": bounds, "peaks": pk,
                 "l2": "no flush: every step reads its weights, more than the 126 MB L2"}
     bounds = {
-        "latent_attn_prefill_us": 2.0 * T * keys_avg * H * (R + z["kv_rank"]) / (pk["bf16_tflops"] * 1e12) * 1e6,
+        "latent_attn_prefill_us": latent_flops(T * keys_avg) / (pk["bf16_tflops"] * 1e12) * 1e6,
         "qwen_attn_prefill_us": 2.0 * T * (T + 1) / 2 * H * 2 * z["dim"] / (pk["bf16_tflops"] * 1e12) * 1e6,
         "latent_attn_decode_us": B * min(ctx, z["window"]) * R * el / (pk["hbm_gbs"] * 1e9) * 1e6,
         "qwen_attn_decode_us": B * ctx * 2 * H * z["dim"] * el / (pk["hbm_gbs"] * 1e9) * 1e6,
