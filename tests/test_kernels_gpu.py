@@ -753,6 +753,18 @@ def test_linear_float32_tensor_cores_leave_out_no_more_than_they_say(monkeypatch
     assert K.f32_tc_error() == 0
 
 
+@pytest.mark.parametrize("e", [-100, -110, -113, -117, -122, -126])
+def test_linear_float32_tensor_cores_at_the_end_of_the_range(e, monkeypatch):
+    """Values whose third, then second part falls under bfloat16's smallest ones: off by at most 2^-134 of a value and what the sums round."""
+    monkeypatch.setattr(K, "F32_TC_WORK", 0)
+    M, N, K_ = 96, 160, 512
+    x, w = rnd(M, K_, seed=1) * 2.0 ** e, rnd(N, K_, seed=2)
+    out = torch.empty(M, N, device=DEV)
+    K.linear(x.to(DEV), w.to(DEV), out)
+    ref, scale = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((out.cpu().double() - ref).abs() <= 8 * 2.0 ** -23 * scale + 2.0 ** -134 * w.double().abs().sum(1)).all())
+
+
 @pytest.mark.parametrize("which", ["x", "w", "w2"])
 def test_linear_float32_of_unaligned_rows_where_the_work_is_enough_for_the_tensor_cores(which):
     M, N, K_ = 300, 512, 512
